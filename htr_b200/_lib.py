@@ -81,7 +81,20 @@ def _load():
     return lib
 
 
+def _load_host():
+    """The native front (csrc/host_binding.cpp), bound to the entry points of the library loaded above."""
+    try:
+        import torch  # noqa: F401  (its libraries carry the symbols that the extension needs)
+
+        from . import _host
+    except ImportError as e:
+        raise ImportError(f"htr_b200/_host.so is missing or does not load ({e}): build it with `python -m htr_b200.build`") from e
+    _host.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in EXPORTS})
+    return _host
+
+
 lib = _load()
+host = _load_host()
 
 
 def check(status, what):

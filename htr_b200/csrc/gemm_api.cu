@@ -148,7 +148,12 @@ double codebook_scale() {
 int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return HTR_ERR_CUDA;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return HTR_ERR_CUDA;
+  static int seen_sms[64] = {0};                          // a device fact: asked once (every caller would store the same number)
+  if (dev >= 0 && dev < 64) sms = seen_sms[dev];
+  if (sms <= 0) {
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return HTR_ERR_CUDA;
+    if (dev >= 0 && dev < 64) seen_sms[dev] = sms;
+  }
   GemmPlan g;
   g.np = (M + 15) / 16 * 16;
   g.rbs = m / 128;

@@ -1,0 +1,287 @@
+// Native front of the operators: the part of a call that is the same every time (argument checks, output allocation, stream and
+// workspace lookup, the C call) without the interpreter.
+//
+// What bounds it: a small packed linear runs 5-15 us on the GPU, while the same steps in Python and ctypes took 26 us per call on
+// the host (attribute reads of six tensors, a device context manager, 16 converted arguments), so calls queued behind the host.
+// Here a call costs about the launch itself.
+//
+// Each function either enqueues the whole call and returns its result, or returns None having enqueued nothing that matters: a
+// wrong type, device or shape, a tensor subclass, a tensor that is not contiguous, a workspace that is missing or too small, or a
+// status of the library other than HTR_OK.  The caller then takes the general path (htr_b200/ops.py), which raises the error,
+// copies the operand or makes the workspace.  Entry points of the library arrive as addresses (bind), so that this module and the
+// ctypes binding use one loaded library.  Every function runs with the interpreter lock held: the launches of one call are never
+// interleaved with those of another thread on the same workspace.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <optional>
+#include <vector>
+
+#include "../../include/htr_b200.h"
+
+namespace {
+
+struct Entry {
+  decltype(&htr_linear_ex) linear_ex;
+  decltype(&htr_linear_gemm) linear_gemm;
+  decltype(&htr_linear_padded) linear_padded;
+  decltype(&htr_linear_fused) linear_fused;
+} g_lib = {};
+
+// ---- workspaces: buffers that ops.py owns (one per device, stream and kind); this table only remembers where they are
+enum Kind { kGemv = 0, kGemm = 1 };
+struct Workspace {
+  int kind, device;
+  void* stream;
+  at::Tensor buf;
+};
+std::vector<Workspace>& workspaces() {
+  static auto* table = new std::vector<Workspace>();     // never destroyed: the CUDA context may be gone by then
+  return *table;
+}
+const at::Tensor* find_workspace(int kind, int device, void* stream) {
+  for (const Workspace& w : workspaces())
+    if (w.stream == stream && w.device == device && w.kind == kind) return &w.buf;
+  return nullptr;
+}
+
+const at::Tensor* tensor(PyObject* o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kBFloat16: return HTR_DTYPE_BF16;
+    case at::kHalf: return HTR_DTYPE_F16;
+    case at::kFloat: return HTR_DTYPE_F32;
+    default: return -1;
+  }
+}
+
+bool plain(const at::Tensor& t, const at::Device& dev, at::ScalarType type) {
+  return t.scalar_type() == type && t.device() == dev && t.is_contiguous();
+}
+
+// the four wire tensors of one linear
+struct Weight {
+  const void *qw, *sc;
+  const uint8_t *su, *sv;
+  int mt, nt, K;
+};
+bool weight(PyObject* const* a, const at::Device& dev, Weight* w) {
+  const at::Tensor *qw = tensor(a[0]), *sc = tensor(a[1]), *su = tensor(a[2]), *sv = tensor(a[3]);
+  if (!qw || !sc || !su || !sv) return false;
+  if (!plain(*qw, dev, at::kInt) || !plain(*sc, dev, at::kHalf) || !plain(*su, dev, at::kByte) || !plain(*sv, dev, at::kByte)) return false;
+  if (qw->dim() != 3 || qw->size(2) % 8 || qw->size(0) > (1 << 24) || qw->size(1) > (1 << 24)) return false;
+  w->mt = (int)qw->size(0);
+  w->nt = (int)qw->size(1);
+  w->K = (int)(qw->size(2) / 8);
+  if (sc->numel() != (int64_t)w->mt * 16 || su->numel() != (int64_t)w->nt * 2 || sv->numel() != (int64_t)w->mt * 2) return false;
+  w->qw = qw->const_data_ptr();
+  w->sc = sc->const_data_ptr();
+  w->su = static_cast<const uint8_t*>(su->const_data_ptr());
+  w->sv = static_cast<const uint8_t*>(sv->const_data_ptr());
+  return true;
+}
+
+// None, or a bias of `count` elements of the activation type
+bool bias_of(PyObject* o, const at::Tensor& x, int64_t count, const void** out) {
+  *out = nullptr;
+  if (o == Py_None) return true;
+  const at::Tensor* b = tensor(o);
+  if (!b || !plain(*b, x.device(), x.scalar_type()) || b->numel() != count) return false;
+  *out = b->const_data_ptr();
+  return true;
+}
+
+at::Tensor output(const at::Tensor& x, int64_t columns) {
+  c10::DimVector shape(x.sizes().begin(), x.sizes().end());
+  shape.back() = columns;
+  return at::detail::empty_cuda(shape, x.scalar_type(), x.device(), std::nullopt);
+}
+
+// the device of the activations becomes the current one for the call (a CUDAGuard costs two runtime calls: only when it has to)
+struct OnDevice {
+  std::optional<c10::cuda::CUDAGuard> guard;
+  explicit OnDevice(int device) {
+    if (c10::cuda::current_device() != device) guard.emplace((c10::DeviceIndex)device);
+  }
+};
+
+PyObject* none() { Py_RETURN_NONE; }
+
+// linear(x, qweight, scales, su, sv, bias, flags, gemv_rows, gemm_rows): up to gemv_rows activation rows as one GEMV, up to
+// gemm_rows on the tensor-core GEMM
+PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 9) return none();
+  const at::Tensor* x = tensor(a[0]);
+  Weight w;
+  const void* bias;
+  if (!x || !x->is_cuda() || x->dim() < 1 || !x->is_contiguous() || !weight(a + 1, x->device(), &w)) return none();
+  const int dt = dtype_code(x->scalar_type());
+  const int64_t cols = (int64_t)w.nt * 16, rows64 = cols ? x->numel() / cols : 0;
+  const long flags = PyLong_AsLong(a[6]), gemv_rows = PyLong_AsLong(a[7]), gemm_rows = PyLong_AsLong(a[8]);
+  if (dt < 0 || x->size(-1) != cols || rows64 < 1 || !bias_of(a[5], *x, (int64_t)w.mt * 16, &bias)) return none();
+  const bool gemv = rows64 <= gemv_rows && rows64 <= HTR_GEMV_MAX_ROWS;
+  if (!gemv && (rows64 <= gemv_rows || rows64 > gemm_rows)) return none();
+  const int rows = (int)rows64, dev = x->get_device();
+  OnDevice on(dev);
+  void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const at::Tensor* ws = find_workspace(gemv ? kGemv : kGemm, dev, st);
+  if (!ws) return none();
+  at::Tensor y = output(*x, (int64_t)w.mt * 16);
+  const char* xp = static_cast<const char*>(x->const_data_ptr());
+  char* yp = static_cast<char*>(y.data_ptr());
+  if (gemv) {
+    if (g_lib.linear_ex(xp, dt, rows, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, bias, yp, ws->data_ptr(), ws->numel(), st, (unsigned)flags) != HTR_OK)
+      return none();
+  } else {
+    const int step = dt == HTR_DTYPE_F32 ? HTR_GEMM_MAX_ROWS_F32 : HTR_GEMM_MAX_ROWS;
+    const int64_t esize = x->element_size();
+    for (int r = 0; r < rows; r += step) {
+      const int here = rows - r < step ? rows - r : step;
+      if (g_lib.linear_gemm(xp + r * cols * esize, dt, here, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, bias, yp + (int64_t)r * w.mt * 16 * esize,
+                            ws->data_ptr(), ws->numel(), st) != HTR_OK)
+        return none();
+    }
+  }
+  return THPVariable_Wrap(std::move(y));
+}
+
+// linear_padded(x, qweight, scales, su, sv, bias, m_out)
+PyObject* py_linear_padded(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 7) return none();
+  const at::Tensor* x = tensor(a[0]);
+  Weight w;
+  const void* bias;
+  if (!x || !x->is_cuda() || x->dim() < 1 || !x->is_contiguous() || !weight(a + 1, x->device(), &w)) return none();
+  const int dt = dtype_code(x->scalar_type());
+  const int64_t n_in = x->size(-1), m_out = PyLong_AsLong(a[6]);
+  if (dt < 0 || n_in < 1 || n_in > (int64_t)w.nt * 16 || m_out < 1 || m_out > (int64_t)w.mt * 16 || !bias_of(a[5], *x, m_out, &bias)) return none();
+  const int64_t rows = x->numel() / n_in, esize = x->element_size();
+  if (rows < 1) return none();
+  const int dev = x->get_device();
+  OnDevice on(dev);
+  void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const at::Tensor* ws = find_workspace(kGemv, dev, st);
+  if (!ws) return none();
+  at::Tensor y = output(*x, m_out);
+  const char* xp = static_cast<const char*>(x->const_data_ptr());
+  char* yp = static_cast<char*>(y.data_ptr());
+  for (int64_t r = 0; r < rows; r += HTR_GEMV_MAX_ROWS) {
+    const int here = (int)(rows - r < HTR_GEMV_MAX_ROWS ? rows - r : HTR_GEMV_MAX_ROWS);
+    if (g_lib.linear_padded(xp + r * n_in * esize, dt, here, (int)n_in, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, bias, yp + r * m_out * esize,
+                            (int)m_out, ws->data_ptr(), ws->numel(), st) != HTR_OK)
+      return none();
+  }
+  return THPVariable_Wrap(std::move(y));
+}
+
+// linear_fused(x2, qweight, scales, su, sv, out, prologue, norm_weight, eps, residual)
+PyObject* py_linear_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 10) return none();
+  const at::Tensor* x = tensor(a[0]);
+  Weight w;
+  if (!x || !x->is_cuda() || x->dim() != 2 || x->scalar_type() != at::kBFloat16 || !x->is_contiguous() || !weight(a + 1, x->device(), &w)) return none();
+  const long prologue = PyLong_AsLong(a[6]);
+  const double eps = PyFloat_AsDouble(a[8]);
+  if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
+  const bool residual = PyObject_IsTrue(a[9]) == 1;
+  const int64_t rows = x->size(0), cols = (int64_t)w.nt * 16 * (prologue == HTR_PROLOGUE_SWIGLU ? 2 : 1), m = (int64_t)w.mt * 16;
+  if (rows < 1 || rows > HTR_GEMV_MAX_ROWS || x->size(1) != cols) return none();
+  const void* norm = nullptr;
+  if (a[7] != Py_None) {
+    const at::Tensor* g = tensor(a[7]);
+    if (!g || !plain(*g, x->device(), at::kBFloat16) || g->numel() != (int64_t)w.nt * 16) return none();
+    norm = g->const_data_ptr();
+  }
+  const int dev = x->get_device();
+  OnDevice on(dev);
+  void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const at::Tensor* ws = find_workspace(kGemv, dev, st);
+  if (!ws) return none();
+  at::Tensor y;
+  if (a[5] == Py_None) {
+    if (residual) return none();
+    y = output(*x, m);
+  } else {
+    const at::Tensor* o = tensor(a[5]);
+    if (!o || !plain(*o, x->device(), at::kBFloat16) || o->dim() != 2 || o->size(0) != rows || o->size(1) != m) return none();
+    y = *o;
+  }
+  if (g_lib.linear_fused(x->const_data_ptr(), (int)rows, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, y.data_ptr(), ws->data_ptr(), ws->numel(), st,
+                         (int)prologue, norm, (float)eps, residual ? 1 : 0) != HTR_OK)
+    return none();
+  if (a[5] != Py_None) return Py_NewRef(a[5]);
+  return THPVariable_Wrap(std::move(y));
+}
+
+// set_workspace(kind, device index, stream, buffer): the buffer that calls on this device and stream use from now on
+PyObject* py_set_workspace(PyObject*, PyObject* args) {
+  int kind, device;
+  unsigned long long stream;
+  PyObject* buf;
+  if (!PyArg_ParseTuple(args, "iiKO", &kind, &device, &stream, &buf)) return nullptr;
+  if (!THPVariable_Check(buf)) {
+    PyErr_SetString(PyExc_TypeError, "set_workspace wants a tensor");
+    return nullptr;
+  }
+  void* st = reinterpret_cast<void*>(stream);
+  for (Workspace& w : workspaces())
+    if (w.stream == st && w.device == device && w.kind == kind) {
+      w.buf = THPVariable_Unpack(buf);
+      Py_RETURN_NONE;
+    }
+  workspaces().push_back({kind, device, st, THPVariable_Unpack(buf)});
+  Py_RETURN_NONE;
+}
+
+// bind(dict name -> address of the loaded library's entry point)
+PyObject* py_bind(PyObject*, PyObject* table) {
+  const auto at_name = [&](const char* name) -> void* {
+    PyObject* v = PyDict_Check(table) ? PyDict_GetItemString(table, name) : nullptr;
+    return v ? PyLong_AsVoidPtr(v) : nullptr;
+  };
+  g_lib.linear_ex = reinterpret_cast<decltype(g_lib.linear_ex)>(at_name("htr_linear_ex"));
+  g_lib.linear_gemm = reinterpret_cast<decltype(g_lib.linear_gemm)>(at_name("htr_linear_gemm"));
+  g_lib.linear_padded = reinterpret_cast<decltype(g_lib.linear_padded)>(at_name("htr_linear_padded"));
+  g_lib.linear_fused = reinterpret_cast<decltype(g_lib.linear_fused)>(at_name("htr_linear_fused"));
+  if (!g_lib.linear_ex || !g_lib.linear_gemm || !g_lib.linear_padded || !g_lib.linear_fused) {
+    PyErr_SetString(PyExc_ImportError, "bind: an entry point of libhtr_b200 is missing");
+    return nullptr;
+  }
+  Py_RETURN_NONE;
+}
+
+// C++ exceptions (out of memory in the allocator, a sticky CUDA error) become the Python exceptions torch uses
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  return F(self, a, n);
+  END_HANDLE_TH_ERRORS
+}
+
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyMethodDef fast(const char* name) {
+  return {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&guarded<F>)), METH_FASTCALL, nullptr};
+}
+
+PyMethodDef g_methods[] = {
+    fast<py_linear>("linear"),
+    fast<py_linear_padded>("linear_padded"),
+    fast<py_linear_fused>("linear_fused"),
+    {"set_workspace", py_set_workspace, METH_VARARGS, nullptr},
+    {"bind", py_bind, METH_O, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_host", "native front of the packed-linear operators", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&g_module); }

@@ -6,8 +6,14 @@ namespace htr {
 template <>
 int launch_packed_gemm_tc<HTR_INST_K>(const GemmParams& p, int grid, cudaStream_t st) {
   const int smem = gemm_smem_bytes(p.np, p.planes, HTR_INST_K, p.stages);
-  cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);   // the 227 KB limit includes the static part
-  if (e != cudaSuccess) return (int)e;
+  static bool allowed[64] = {false};                      // shared memory beyond 48 KB: opted in once per device
+  int dev = 0;
+  if (const cudaError_t e = cudaGetDevice(&dev)) return (int)e;
+  if (dev < 0 || dev >= 64 || !allowed[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);   // the 227 KB limit includes the static part
+    if (e != cudaSuccess) return (int)e;
+    if (dev >= 0 && dev < 64) allowed[dev] = true;
+  }
   // programmatic stream serialisation: the kernel may start while the activation transform before it still runs; it
   // fetches packed words at once and waits (griddepcontrol.wait) before it touches anything that kernel writes
   cudaLaunchConfig_t cfg = {};
@@ -34,8 +40,7 @@ int launch_packed_gemm_tc<HTR_INST_K>(const GemmParams& p, int grid, cudaStream_
     struct Seen { int dev, split, smem, clusters; };
     static thread_local Seen seen[8] = {};
     static thread_local int next_slot = 0;
-    int dev = 0, clusters = -1;
-    cudaGetDevice(&dev);
+    int clusters = -1;
     for (const Seen& c : seen)
       if (c.split == p.split && c.smem == smem && c.dev == dev) clusters = c.clusters;
     if (clusters < 0) {

@@ -25,6 +25,7 @@ import torch
 
 from . import _lib, wire
 
+_host = _lib.host
 CB = wire.cbscale()
 GEMV_MAX_M = _lib.GEMV_MAX_ROWS
 GEMV_LOOP_MAX = int(os.environ.get("HTR_GEMV_LOOP_MAX", "64"))
@@ -61,6 +62,7 @@ def workspace(device, nbytes, stream=None):
         size = max(_MIN_WORKSPACE, 1 << (int(nbytes) - 1).bit_length())
         buf = torch.zeros(size, dtype=torch.uint8, device=device)
         _WORKSPACES[key] = buf
+        _host.set_workspace(0, *key, buf)
     return buf
 
 
@@ -111,6 +113,9 @@ def linear_padded(x, qweight, scales, su, sv, bias=None, m_out=None):
     written).  n_in and m_out must be multiples of 8.  Batches above 8 rows run as 8-row launches."""
     mt, nt, W = qweight.shape
     m_out = mt * 16 if m_out is None else int(m_out)
+    y = _host.linear_padded(x, qweight, scales, su, sv, bias, m_out)     # the usual case; None: whatever it does not take
+    if y is not None:
+        return y
     n_in = x.shape[-1]
     x2 = x.reshape(-1, n_in).contiguous()
     if not x2.is_cuda:
@@ -147,6 +152,9 @@ def linear_fused(x2, qweight, scales, su, sv, out=None, prologue=PROLOGUE_NONE, 
 
     Returns `out` (allocated when not given and residual is False).  The reference runs these steps as separate kernels of its
     serving stack; results equal the unfused bf16 operators up to the summation order of the norm."""
+    y = _host.linear_fused(x2, qweight, scales, su, sv, out, prologue, norm_weight, eps, residual)
+    if y is not None:
+        return y
     if x2.dtype != torch.bfloat16 or not x2.is_cuda or x2.dim() != 2:
         raise _lib.HTRError("htr_linear_fused: activations must be a 2-D bf16 CUDA tensor")
     M = x2.shape[0]
@@ -190,6 +198,7 @@ def _gemm(x2, qweight, scales, su, sv, bias, out, peer_ptrs=None, elem_offset=0)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 24), dtype=torch.uint8, device=x2.device)
         _GEMM_WS[key] = ws
+        _host.set_workspace(1, *key, ws)
     if peer_ptrs is None:
         rc = _lib.lib.htr_linear_gemm(x2.data_ptr(), _DTYPES[x2.dtype], M, qweight.data_ptr(), mt, nt, K, scales.data_ptr(), su.data_ptr(),
                                       sv.data_ptr(), None if bias is None else bias.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), st)
@@ -385,10 +394,16 @@ def _(x2, qweight, scales, su, sv, bias):
 
 def linear(x, qweight, scales, su, sv, bias=None):
     """y = x @ W^T (+ bias) for an HTR-W1 weight; x [..., n] -> [..., m] in x.dtype (htr/ops.py:118-122)."""
+    compiling = torch.compiler.is_compiling()
+    if not compiling:
+        # eager: one native call checks, allocates and launches; None: nothing it takes (other routes, copies, growth, errors)
+        y = _host.linear(x, qweight, scales, su, sv, bias, _STATE.flags, GEMV_ROUTE_MAX, GEMM_ROUTE_MAX if USE_GEMM else 0)
+        if y is not None:
+            return y
     lead = x.shape[:-1]
     x2 = x.reshape(-1, x.shape[-1])
-    if torch.compiler.is_compiling():
+    if compiling:
         y = htr_linear_op(x2, qweight, scales, su, sv, bias)      # traced programs see the registered op
     else:
-        y = _linear_impl(x2.contiguous(), qweight, scales, su, sv, bias)   # eager: skip the dispatcher round trip
+        y = _linear_impl(x2.contiguous(), qweight, scales, su, sv, bias)
     return y.reshape(*lead, qweight.shape[0] * 16)

@@ -1,0 +1,37 @@
+"""The native front of the operators (csrc/host_binding.cpp) against the general path in Python: the same kernels, so equal bits;
+what it does not take (strided rows, wrong types, CPU tensors) must still work or raise as the general path does."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,dtype", ((1, torch.bfloat16), (4, torch.float32), (5, torch.float16), (129, torch.float32), (300, torch.bfloat16), (600, torch.bfloat16)))
+def test_front_equals_general_path(M, dtype, monkeypatch):
+    from htr_b200 import _lib, ops, wire
+
+    dev = torch.device("cuda:0")
+    m, n, K = 384, 256, 3
+    w = wire.random_packed(m, n, K, seed=M, device=dev)
+    x = torch.randn(M, n, generator=torch.Generator().manual_seed(M)).to(dtype).to(dev)
+    bias = torch.randn(m, device=dev).to(dtype)
+    ops.linear(x, *w, bias)                                              # the workspaces exist from here on
+    got, padded = ops.linear(x.view(1, M, n), *w, bias), ops.linear_padded(x[:, :200].contiguous(), *w, bias[:136].contiguous(), m_out=136)
+    assert got.shape == (1, M, m)
+    strided = torch.zeros(M, 2 * n, dtype=dtype, device=dev)
+    strided[:, :n] = x
+    assert torch.equal(ops.linear(strided[:, :n], *w, bias), got[0])     # rows with a gap: copied by the general path
+    with pytest.raises(_lib.HTRError):
+        ops.linear(x, *w, bias.double())
+    with pytest.raises(_lib.HTRError):
+        ops.linear(x[:, :128].contiguous(), *w)
+    side = torch.cuda.Stream()                                            # a stream without workspaces yet
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        other = ops.linear(x, *w, bias)
+    side.synchronize()
+    assert torch.equal(other, got[0])
+    for name in ("linear", "linear_padded"):
+        monkeypatch.setattr(ops._host, name, lambda *a: None)
+    assert torch.equal(ops.linear(x, *w, bias), got[0])
+    assert torch.equal(ops.linear_padded(x[:, :200].contiguous(), *w, bias[:136].contiguous(), m_out=136), padded)
