@@ -1,4 +1,4 @@
-// C entry points of the tensor-core packed GEMM (batches of 9..128 activation rows per call).
+// C entry points of the tensor-core packed GEMM (batches of up to 256 activation rows per call).
 #include <cmath>
 
 #include "packed_gemm_tc.cuh"
@@ -7,14 +7,15 @@ namespace htr {
 
 // ------------------------------------------------------------------------------------------------
 // Activation transform for the GEMM: xt = H128(su * x) / sqrt(128) / tok as one or two fp16 planes, their sums, tok.
-// Output layout = the B operand tiles of the GEMM, ready for one bulk copy per 64-column chunk:
-//   xb[chunk][column group g][k-group kc][column r][8 k]   column = g*8 + r: activation row (hi plane), np + row (lo plane)
-// grid (np, slices): a CTA transforms one 1024-column slice of one activation row (one 128-column block per warp), after
-// finding the range of the whole row itself (every CTA of a row reads the row once; that is cheaper than a second launch
-// or a grid-wide exchange).  xsum[row][slice] holds the slice's sum, added up in slice order by the GEMM's epilogue.
-// Rows beyond `rows` are written as zeros so that the padded batch is harmless.
+// Output layout = the B operand tiles of the GEMM, one contiguous block per 128 columns of x:
+//   xb[64-column unit][column group g][k-group kc][column r][8 k]   column = g*8 + r: activation row (hi plane), np + row (lo plane)
+// with the k order of the A operand inside a unit (packed_gemm_tc.cuh): position 16 j + 4 c + e holds column 16 c + 4 j + e.
+// grid (np, slices): a CTA transforms one slice of one activation row (one 128-column block per warp and turn), after finding the
+// range of the whole row itself (every CTA of a row reads the row once, 16 bytes per load and all of them in flight; that is
+// cheaper than a second launch or a grid-wide exchange).  xsum[row][slice] holds the slice's sum, added up in slice order by the
+// GEMM's epilogue.  Rows beyond `rows` are written as zeros so that the padded batch is harmless; columns from n_in on read as zeros.
 template <int DT>
-__global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x, int rows, int np, int n, int planes, int per,
+__global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x, int rows, int np, int n, int n_in, int planes, int per,
                                                       const uint8_t* __restrict__ su, __half* __restrict__ xb, float* __restrict__ xsum,
                                                       float* __restrict__ tok) {
   __shared__ float red[8];
@@ -23,13 +24,14 @@ __global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x
   const int blocks = n >> 7;
   const int hb0 = slice * 8 * per + warp;                    // this warp's 128-column blocks: hb0, hb0 + 8, ... (`per` of them)
   const int ncols = np * planes;
-  const size_t chunk_halves = (size_t)ncols * 64;
-  // element offset of (column c, k) = chunk*chunk_halves + ((c/8)*8 + (k%64)/8)*64 + (c%8)*8 + k%8
+  const size_t unit_halves = (size_t)ncols * 64;
   const size_t col_hi = (size_t)(r >> 3) * 512 + (r & 7) * 8, col_lo = (size_t)((np + r) >> 3) * 512 + ((np + r) & 7) * 8;
-  auto tile_offset = [&](int hb) {
-    const int k0 = hb * 128 + 4 * lane;                      // four consecutive k, inside one 8-wide k group
-    return (size_t)(k0 >> 6) * chunk_halves + (size_t)((k0 & 63) >> 3) * 64 + (k0 & 7);
-  };
+  // four consecutive columns 4 lane .. + 3 of a block: tile c = (lane % 16) / 4, step j = lane % 4 of unit lane / 16
+  const int c = (lane & 15) >> 2, j = lane & 3;
+  const size_t in_unit = (size_t)(2 * j + (c >> 1)) * 64 + 4 * (c & 1);
+  auto tile_offset = [&](int hb) { return (size_t)(2 * hb + (lane >> 4)) * unit_halves + in_unit; };
+  const unsigned sg_first = hb0 < blocks ? sign_nibble(su, hb0 * 32 + lane) : 0u;   // the signs do not depend on earlier kernels
+  asm volatile("griddepcontrol.wait;" ::: "memory");         // x may come from the preceding kernel, the last GEMM may still read xb
   if (r >= rows) {
     for (int i = 0; i < per; ++i) {
       const int hb = hb0 + 8 * i;
@@ -44,19 +46,37 @@ __global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x
     }
     return;
   }
-  float amax = 0.f;
-#pragma unroll 4
-  for (int e = tid; e < n / 4; e += 256) {                   // range of the whole row
-    const float4 v = load_quad(x, (size_t)r * n + 4 * e, DT);
-    amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+  // this lane's values of its first block: the load is in flight beside those of the scan
+  auto values = [&](int hb) {
+    const int col = hb * 128 + 4 * lane;
+    return hb < blocks && col < n_in ? load_quad(x, (size_t)r * n_in + col, DT) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  const float4 first = values(hb0);
+  // range of the whole row: magnitudes of floats compare like their bit patterns, so 16-bit pairs take the packed integer maximum
+  uint32_t top = 0u;
+  constexpr int kPer16 = DT == HTR_DTYPE_F32 ? 4 : 8;        // elements in 16 bytes
+  const uint4* row16 = reinterpret_cast<const uint4*>(static_cast<const char*>(x) + (size_t)r * n_in * (16 / kPer16));
+#pragma unroll 8
+  for (int e = tid; e < n_in / kPer16; e += 256) {
+    const uint4 v = __ldg(row16 + e);
+    if constexpr (DT == HTR_DTYPE_F32) {
+      constexpr uint32_t m = 0x7FFFFFFFu;
+      top = max(max(top, v.x & m), max(v.y & m, max(v.z & m, v.w & m)));
+    } else {
+      constexpr uint32_t m = 0x7FFF7FFFu;
+      top = __vmaxu2(__vmaxu2(top, v.x & m), __vmaxu2(v.y & m, __vmaxu2(v.z & m, v.w & m)));
+    }
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(kFullWarp, amax, o));
-  if (lane == 0) red[warp] = amax;
+  if constexpr (DT != HTR_DTYPE_F32) top = max(top >> 16, top & 0xFFFFu);
+  top = __reduce_max_sync(kFullWarp, top);
+  if (lane == 0) red[warp] = __uint_as_float(top);
   __syncthreads();
-  float mx = 0.f;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) mx = fmaxf(mx, red[k]);
+  for (int k = 0; k < 8; ++k) top = max(top, __float_as_uint(red[k]));
+  float mx;
+  if constexpr (DT == HTR_DTYPE_F32) mx = __uint_as_float(top);
+  else if constexpr (DT == HTR_DTYPE_BF16) mx = __uint_as_float(top << 16);
+  else mx = __half2float(__ushort_as_half((unsigned short)top));
   const float bound = mx * 11.32f;                           // |H128 x| / sqrt(128) <= sqrt(128) * amax
   const float scale = bound > 16384.f ? exp2f(ceilf(log2f(bound / 16384.f))) : 1.f;
   if (tid == 0 && slice == 0) tok[r] = scale;
@@ -66,8 +86,8 @@ __global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x
   for (int i = 0; i < per; ++i) {
     const int hb = hb0 + 8 * i;
     if (hb >= blocks) break;                                 // warp-uniform: the shuffles inside stay converged
-    const float4 mine = load_quad(x, (size_t)r * n + hb * 128 + 4 * lane, DT);   // second touch: L1
-    const unsigned sg = sign_nibble(su, hb * 32 + lane);
+    const float4 mine = i == 0 ? first : values(hb);         // (second touch: L1)
+    const unsigned sg = i == 0 ? sg_first : sign_nibble(su, hb * 32 + lane);
     float v[4] = {flip(mine.x, sg & 1u), flip(mine.y, (sg >> 1) & 1u), flip(mine.z, (sg >> 2) & 1u), flip(mine.w, sg >> 3)};
     wht128(v, lane);
     __half hi[4], lo[4];
@@ -106,16 +126,23 @@ int gemm_rht_slices(int np, int n) {
   return (n / 128 + 8 * per - 1) / (8 * per);
 }
 
-int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
+int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
                 cudaStream_t st) {
-  const dim3 grid(np, gemm_rht_slices(np, n));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(np, gemm_rht_slices(np, n));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // resident early, waits before its first read
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   const int per = gemm_rht_per(np, n);
   switch (dtype) {
-    case HTR_DTYPE_BF16: rht_f16_kernel<HTR_DTYPE_BF16><<<grid, 256, 0, st>>>(x, rows, np, n, planes, per, su, xb, xsum, tok); break;
-    case HTR_DTYPE_F16: rht_f16_kernel<HTR_DTYPE_F16><<<grid, 256, 0, st>>>(x, rows, np, n, planes, per, su, xb, xsum, tok); break;
-    default: rht_f16_kernel<HTR_DTYPE_F32><<<grid, 256, 0, st>>>(x, rows, np, n, planes, per, su, xb, xsum, tok); break;
+    case HTR_DTYPE_BF16: return (int)cudaLaunchKernelEx(&cfg, rht_f16_kernel<HTR_DTYPE_BF16>, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
+    case HTR_DTYPE_F16: return (int)cudaLaunchKernelEx(&cfg, rht_f16_kernel<HTR_DTYPE_F16>, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
+    default: return (int)cudaLaunchKernelEx(&cfg, rht_f16_kernel<HTR_DTYPE_F32>, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
   }
-  return (int)cudaGetLastError();
 }
 
 namespace {
@@ -125,7 +152,7 @@ constexpr size_t kCounterRegion = 1 << 16;   // same fixed counter region as the
 constexpr size_t kErrorRegion = 256;
 
 struct GemmPlan {
-  int np, rbs, hb, split, grid, stages;
+  int np, rbs, hb, split, grid, stages, smem;
   size_t off_xb, off_xsum, off_tok, off_part, total;
 };
 
@@ -145,6 +172,21 @@ double codebook_scale() {
   return value;
 }
 
+int gemm_clusters(int K, int smem, int split) {
+  switch (K) {
+    case 2: return packed_gemm_tc_clusters<2>(smem, split);
+    case 3: return packed_gemm_tc_clusters<3>(smem, split);
+    case 4: return packed_gemm_tc_clusters<4>(smem, split);
+    case 5: return packed_gemm_tc_clusters<5>(smem, split);
+    case 6: return packed_gemm_tc_clusters<6>(smem, split);
+    case 8: return packed_gemm_tc_clusters<8>(smem, split);
+  }
+  return 0;
+}
+
+// activation rows per launch after padding: accumulator columns come in multiples of 16
+int padded_rows(int M, int planes) { return planes == 2 ? (M + 7) / 8 * 8 : (M + 15) / 16 * 16; }
+
 int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return HTR_ERR_CUDA;
@@ -155,42 +197,36 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
     if (dev >= 0 && dev < 64) seen_sms[dev] = sms;
   }
   GemmPlan g;
-  g.np = (M + 15) / 16 * 16;
+  g.np = padded_rows(M, planes);
   g.rbs = m / 128;
   g.hb = n / 128;
   const int ncols = g.np * planes;
-  int tmem_cols = 32;
-  while (tmem_cols < ncols) tmem_cols <<= 1;
-  // two CTAs per SM when shared memory and the 512 TMEM columns allow, else one; the deepest ring of chunk pairs that fits
-#ifndef HTR_GEMM_MAX_CTAS
-#define HTR_GEMM_MAX_CTAS 2
-#endif
-  const int budget = 227 * 1024;
-  int per_sm = 1;
-  g.stages = 2;
-  bool found = false;
-  for (int ctas = HTR_GEMM_MAX_CTAS; ctas >= 1 && !found; --ctas) {
-    if (ctas * tmem_cols > 512) continue;
-    for (int st = kMaxStages; st >= 2; --st) {
-      if (ctas * (gemm_smem_bytes(g.np, planes, K, st) + 1024) <= budget) {
-        per_sm = ctas;
-        g.stages = st;
-        found = true;
-        break;
-      }
-    }
-  }
-  if (!found) return HTR_ERR_TOO_LARGE;
-  long long s = (long long)sms * per_sm / g.rbs;
-  if (s < 1) s = 1;
+  if (ncols > kGemmMaxCols) return HTR_ERR_TOO_LARGE;
+  // one thread block per SM; as many stages as its tensor memory and shared memory hold
+  const int words = gemm_word_bytes(K), budget = 226 * 1024;
+  g.stages = (kGemmTmemCols - gemm_acc_cols(ncols)) / 64;
+  if (g.stages > kGemmMaxStages) g.stages = kGemmMaxStages;
+  while (g.stages > 1 && gemm_smem_bytes(g.np, planes, g.stages, words) > budget) --g.stages;
+  g.smem = gemm_smem_bytes(g.np, planes, g.stages, words);
+  if (g.stages < 2) return HTR_ERR_TOO_LARGE;
+  // Few row blocks: up to eight thread blocks share one as a cluster and reduce on chip.  Even runs over the whole GPU (flat) give
+  // every thread block the same work, but a row block's partial sums then meet in global memory at one last arriver: they have
+  // to be a fifth shorter to win.
+  const long long slots = (long long)sms, units = (long long)g.rbs * g.hb;
+  long long s = slots / g.rbs;
+  if (s > 8) s = 8;
   if (s > g.hb) s = g.hb;
-  g.split = (int)s;
-  g.grid = g.rbs * g.split;
+  const long long flat_grid = slots < units ? slots : units, flat_run = (units + flat_grid - 1) / flat_grid;
+  g.split = 0;
+  if (s >= 1 && (g.hb + s - 1) / s * 5 <= flat_run * 6 && (s == 1 || gemm_clusters(K, g.smem, (int)s) >= g.rbs)) g.split = (int)s;
+  else if (s == 8 && gemm_clusters(K, g.smem, 8) >= g.rbs) g.split = 8;   // too few row blocks to fill the GPU: short runs either way
+  g.grid = g.split > 0 ? g.rbs * g.split : (int)flat_grid;
   size_t off = kCounterRegion + kErrorRegion;
   g.off_xb = off; off += align256((size_t)ncols * n * 2);
   g.off_xsum = off; off += align256((size_t)g.np * gemm_rht_slices(g.np, n) * 4);
   g.off_tok = off; off += align256((size_t)g.np * 4);
-  g.off_part = off; off += align256((size_t)g.rbs * g.split * g.np * 128 * 4);
+  g.off_part = off;
+  if (g.split == 0) off += align256((size_t)g.grid * 2 * g.np * 128 * 4);
   g.total = off;
   *out = g;
   return HTR_OK;
@@ -203,15 +239,9 @@ using namespace htr;
 
 extern "C" {
 
-// rows of the first launch when a batch is too wide for the shared memory of one CTA (two fp16 planes of many rows, wide streams)
-static int first_half_rows(int M) { return ((M + 1) / 2 + 15) / 16 * 16; }
-
 static size_t plan_bytes(int M, int m, int n, int K, int planes) {
   GemmPlan g;
-  const int rc = make_gemm_plan(M, m, n, K, planes, &g);
-  if (rc == HTR_OK) return g.total;
-  if (rc == HTR_ERR_TOO_LARGE && M > 16) return plan_bytes(first_half_rows(M), m, n, K, planes);   // the halves run one after the other
-  return 0;
+  return make_gemm_plan(M, m, n, K, planes, &g) == HTR_OK ? g.total : 0;
 }
 
 size_t htr_linear_gemm_workspace_bytes(int M, int m, int n, int K) {
@@ -237,10 +267,6 @@ int htr_linear_gemm_peers(const void* x, int dtype, int M, const void* qweight, 
   if (npeer < 1 || npeer > 8 || !peer_y || peer_offset < 0 || (peer_offset & 7)) return HTR_ERR_BAD_SHAPE;
   for (int i = 0; i < npeer; ++i)
     if (!peer_y[i] || (reinterpret_cast<uintptr_t>(peer_y[i]) & 15u)) return peer_y[i] ? HTR_ERR_ALIGNMENT : HTR_ERR_NULL;
-  // a batch too wide for one launch would need the halves at different offsets: the row-shard form serves one launch
-  GemmPlan g;
-  if (M > 0 && width_ok(K) && mt > 0 && nt > 0 && make_gemm_plan(M, mt * 16, nt * 16, K, dtype == HTR_DTYPE_F32 ? 2 : 1, &g) != HTR_OK)
-    return HTR_ERR_TOO_LARGE;
   return gemm_launch(x, dtype, M, qweight, mt, nt, K, scales, su, sv, bias, nullptr, peer_y, npeer, peer_offset, workspace, workspace_bytes, stream);
 }
 
@@ -260,14 +286,6 @@ static int gemm_launch(const void* x, int dtype, int M, const void* qweight, int
   const int planes = dtype == HTR_DTYPE_F32 ? 2 : 1;      // 16-bit activations need no lo plane
   if (planes == 2 && M > HTR_GEMM_MAX_ROWS_F32) return HTR_ERR_BAD_SHAPE;
   const int rc = make_gemm_plan(M, m, n, K, planes, &g);
-  if (rc == HTR_ERR_TOO_LARGE && M > 16 && npeer == 0) {  // too wide for one CTA's shared memory: two launches over row halves
-    const int M1 = first_half_rows(M);
-    const size_t esz = dtype == HTR_DTYPE_F32 ? 4 : 2;
-    const int r1 = htr_linear_gemm(x, dtype, M1, qweight, mt, nt, K, scales, su, sv, bias, y, workspace, workspace_bytes, stream);
-    if (r1 != HTR_OK) return r1;
-    return htr_linear_gemm(static_cast<const char*>(x) + (size_t)M1 * n * esz, dtype, M - M1, qweight, mt, nt, K, scales, su, sv, bias,
-                           static_cast<char*>(y) + (size_t)M1 * m * esz, workspace, workspace_bytes, stream);
-  }
   if (rc != HTR_OK) return rc;
   if (!workspace || workspace_bytes < g.total) return HTR_ERR_WORKSPACE;
   char* ws = static_cast<char*>(workspace);
@@ -293,21 +311,22 @@ static int gemm_launch(const void* x, int dtype, int M, const void* qweight, int
   p.hb = g.hb;
   p.split = g.split;
   p.stages = g.stages;
+  p.m_out = m;
   p.xsum_slices = gemm_rht_slices(g.np, n);
   p.cb = (float)codebook_scale();
   p.npeer = npeer;
   p.peer_offset = peer_offset;
   for (int i = 0; i < 8; ++i) p.peer_y[i] = i < npeer ? peer_y[i] : nullptr;
-  int e = run_rht_f16(x, dtype, M, g.np, n, planes, su, reinterpret_cast<__half*>(ws + g.off_xb), reinterpret_cast<float*>(ws + g.off_xsum),
+  int e = run_rht_f16(x, dtype, M, g.np, n, n, planes, su, reinterpret_cast<__half*>(ws + g.off_xb), reinterpret_cast<float*>(ws + g.off_xsum),
                       reinterpret_cast<float*>(ws + g.off_tok), st);
   if (e) { t_gemm_cuda = e; return HTR_ERR_CUDA; }
   switch (K) {
-    case 2: e = launch_packed_gemm_tc<2>(p, g.grid, st); break;
-    case 3: e = launch_packed_gemm_tc<3>(p, g.grid, st); break;
-    case 4: e = launch_packed_gemm_tc<4>(p, g.grid, st); break;
-    case 5: e = launch_packed_gemm_tc<5>(p, g.grid, st); break;
-    case 6: e = launch_packed_gemm_tc<6>(p, g.grid, st); break;
-    case 8: e = launch_packed_gemm_tc<8>(p, g.grid, st); break;
+    case 2: e = launch_packed_gemm_tc<2>(p, g.grid, g.smem, st); break;
+    case 3: e = launch_packed_gemm_tc<3>(p, g.grid, g.smem, st); break;
+    case 4: e = launch_packed_gemm_tc<4>(p, g.grid, g.smem, st); break;
+    case 5: e = launch_packed_gemm_tc<5>(p, g.grid, g.smem, st); break;
+    case 6: e = launch_packed_gemm_tc<6>(p, g.grid, g.smem, st); break;
+    case 8: e = launch_packed_gemm_tc<8>(p, g.grid, g.smem, st); break;
   }
   if (e) t_gemm_cuda = e;
   return e ? HTR_ERR_CUDA : HTR_OK;

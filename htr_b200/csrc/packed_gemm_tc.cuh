@@ -1,72 +1,65 @@
-// Packed GEMM for prefill-sized batches on sm_100a: decoded tiles feed tcgen05.mma, accumulators live in TMEM.
+// Packed GEMM for batches on sm_100a: decoded tiles feed tcgen05.mma from tensor memory, accumulators live there too.
 //
-//   Y[j, i] = sum_k Xt[j, k] * V[i, k]   for one 128-row block i of the weight, batch rows j (up to 128 per launch)
+//   Y[j, i] = sum_k Xt[j, k] * V[i, k]   for one 128-row block i of the weight, activation rows j (up to 256 per launch)
 //
 // Replaces the reference's prefill route (dequant_w to bf16 in DRAM + library GEMM, htr/ops.py:89-93, kernels
-// htr_kernels.cu:658-903): the packed words are decoded once per launch straight into the shared-memory A operand
-// and never reach DRAM as 16-bit weights.  This is the only kernel of the library that uses tensor cores.
+// htr_kernels.cu:658-903): the packed words are decoded once per launch straight into the A operand and never reach memory as
+// 16-bit weights.
 //
-// Operands.  A (128 x 64 per k-chunk) holds the codebook integers as exact fp16 values 1024 + bytesum (the fp16 bit
-// pattern 0x6400 + bytesum needs no conversion instruction); the constant 1534 = 1024 + 510 is removed in the
-// epilogue with the row sums of the activations, as the reference does (htr_kernels.cu:312-313).  B holds the
-// transformed activations as two fp16 planes, hi and lo = fp16(xt - hi), concatenated along N, so that the
-// products carry ~22 bits of the activations; the two accumulator halves are added after the MMA.  A per-row
-// power-of-two scale keeps |xt| inside the fp16 range (htr_kernels.cu:205-206).
+// Operands.  A holds the codebook integers as exact fp16 values 1024 + bytesum (the fp16 bit pattern 0x6400 + bytesum needs no
+// conversion instruction); the constant 1534 = 1024 + 510 is removed in the epilogue with the row sums of the activations, as the
+// reference does (htr_kernels.cu:312-313).  B holds the transformed activations as one fp16 plane `hi`, or two, hi and
+// lo = fp16(xt - hi), concatenated along N, so that the products carry ~22 bits of the activations; the two accumulator halves are
+// added after the MMA.  A per-row power-of-two scale keeps |xt| inside the fp16 range (htr_kernels.cu:205-206).
 //
-// Both operands use the K-major, no-swizzle canonical layout of the UMMA shared-memory descriptor: 8 rows x 16 bytes
-// form a contiguous 128-byte core matrix; core matrices adjacent in K are LBO = 128 bytes apart, 8-row groups are
-// SBO bytes apart.  For A, SBO is padded by 16 bytes so that the decode threads' 16-byte stores spread over all
-// banks.  The activation transform writes B to global memory already in this layout, one contiguous block per
-// 64-column chunk, so a B tile arrives with a single bulk copy.
+// What bounds it: producing A.  A weight costs about four issue slots (window, hash multiply-add, byte sum, half a pack) whatever
+// the batch, so the goal is that the decode warps do nothing else.  Two properties of the layout serve that:
+//  * A lives in tensor memory, not in shared memory.  An fp16 weight that is stored to and fetched from shared memory takes 4 of
+//    its 128 bytes per cycle and SM, a bound of 32 weights per cycle by itself beside B and the packed words; the tensor-memory
+//    path carries A alone (the MMA fetches 4 KB in 32 cycles: 64 weights per cycle).
+//  * tcgen05.st.16x256b gives a thread a piece of two rows, which is the decode unit (a row pair of one tile, whose 32 windows
+//    share words): lane (g, c) decodes rows 2g, 2g+1 of tile c of a 16-row strip's four tiles and one store per unit places them.
+//    Tensor-memory lane l < 8 of a strip holds weight row 2l, lane 8 + l row 2l + 1, and MMA step j takes columns 4j..4j+3 of each
+//    of the four tiles; the activation transform writes B in that k order.
+// The packed words take a ring per warp (16-byte cp.async, all slots but one in flight): plain loads into registers one block ahead
+// keep 16 KB per SM in flight and measured 12 weights per cycle and SM, the ring 22 (at any depth from 3 slots on), which is the
+// decode alone: 4.8 instructions per weight at 82 % of the issue slots.
 //
-// Roles (576 threads).  Warps 0-15 decode: two groups of eight warps take alternate 64-column chunks; inside a group
-// warp w owns the 16-row strip w of the 128-row block, fetches that strip's packed words itself (cp.async ring, the
-// same scheme as the GEMV) and writes its rows of the A tile.  One lane of warp 16 brings the B tiles (one bulk copy
-// per pair of chunks, completion counted on an mbarrier); one lane of warp 17 issues the MMAs.  The ring holds pairs of
-// consecutive chunks (one chunk per decode group): {A tile, A tile, B tile, B tile} with a_full[s] (all sixteen decode
-// warps stored and fenced), b_full[s] (bytes landed) and freed[s] (tcgen05.commit: the MMAs that read the pair have
-// retired), so the MMA lane pays one round of barrier traffic per 128 columns.  No CTA-wide barrier inside the main loop.
+// Roles (22 warps, one thread block per SM).  Warps 0-15 decode, as two groups of eight that take alternate 128-column blocks;
+// inside a group warp w owns tensor-memory quadrant w % 4 and strip 2 (w % 4) + (w / 4) % 2.  One lane of warp 16 brings the B tile
+// of each block (one bulk copy, completion counted on an mbarrier); one lane of warp 17 issues the eight MMAs of a block.  Stage s of
+// the ring is {64 tensor-memory columns of A, one B tile} with full[s] and freed[s] (tcgen05.commit); with up to seven
+// stages the decode runs ahead while the activation transform before the launch still works and while an accumulator is read.
+// Warps 18-21 finish row blocks: they move the accumulator to a partial sum in memory and, where it is the last, add the partials,
+// apply scales, output transform and signs, and store.  (Done by the decode warps, that chain of dependent loads cost 12 000 cycles
+// per row block, a fifth of the LM head at 8 rows.)  The last row block of a thread block is finished by all its warps.
 //
-// Every wait on an mbarrier is bounded: when it expires the CTA records an error code, stops issuing work, waits
-// (bounded) for its copies in flight, frees its TMEM columns and returns; the host sees the code in the workspace
-// header.
+// Decomposition.  Work = (row block) x (128-column blocks).  Where the row blocks are few, `split` thread blocks share one as a
+// cluster and reduce through distributed shared memory; else every thread block takes an even contiguous run that may cross row
+// blocks (flat), publishes a partial [np][128] per row block it touches, and the last arriver adds them in thread-block order.
+// Both are deterministic and nobody waits for another thread block except inside a cluster.  One thread block per SM, not two: the
+// partial sums of a row block are half as many, and no SM waits for the slower of two.
+//
+// Every wait on an mbarrier is bounded: when it expires the thread block records an error code, stops issuing work, waits (bounded)
+// for its copies and MMAs in flight, writes NaN into the rows it owed, frees its tensor memory and returns; the host sees the code
+// in the workspace header.
 #pragma once
 #include "htr_codec.cuh"
 #include "htr_common.cuh"
 
 namespace htr {
 
-constexpr int kStripWarps = 8;                              // warps of one decode group = 16-row strips of a row block
-constexpr int kDecodeGroups = 2;                            // groups take alternate chunks
-constexpr int kGemmDecodeWarps = kStripWarps * kDecodeGroups;
-constexpr int kGemmWarps = kGemmDecodeWarps + 2;            // + B-tile warp + MMA warp
+constexpr int kGemmMaxStages = 7;
+constexpr int kGemmDecodeWarps = 16, kGemmGroupWarps = 8;
+constexpr int kGemmFinishWarps = 4;
+constexpr int kGemmWarps = kGemmDecodeWarps + 2 + kGemmFinishWarps;
 constexpr int kGemmThreads = kGemmWarps * 32;
-constexpr int kChunkK = 64;                                 // k extent of one stage
-constexpr int kLbo = 128;                                   // bytes between core matrices adjacent in K
-#ifndef HTR_GEMM_SBOA_PAD
-#define HTR_GEMM_SBOA_PAD 16
-#endif
-#ifndef HTR_GEMM_MMAS
-#define HTR_GEMM_MMAS (kChunkK / 16)
-#endif
-constexpr int kSboA = (kChunkK / 8) * 128 + HTR_GEMM_SBOA_PAD;   // bytes between 8-row groups of A (padded: 1040)
-constexpr int kSboB = (kChunkK / 8) * 128;                  // ... of B (as written by the activation transform)
-constexpr int kATileBytes = (128 / 8) * kSboA;              // 16640
-constexpr int kMaxStages = 3;                               // stage pairs in flight (2..3, chosen by the host); a pair = two consecutive
-                                                            // chunks, one per decode group: {A tile, A tile, B tile, B tile}
-constexpr unsigned kSpinLimit = 4000000u;                   // iterations of a try_wait loop before giving up
+constexpr int kGemmTmemCols = 512;                          // the accumulator first, then 64 columns of A per stage
 constexpr int kGemmMaxCols = 256;                           // accumulator columns (activation rows x planes) per launch
-#ifndef HTR_GEMM_WAIT_HINT
-#define HTR_GEMM_WAIT_HINT 200
-#endif
-#ifndef HTR_GEMM_PACK_MODE
-#define HTR_GEMM_PACK_MODE 1
-#endif
-// packed-word ring of a decode warp: chunks in flight + the one being read
-#ifndef HTR_GEMM_RAW_SLOTS
-#define HTR_GEMM_RAW_SLOTS(K) ((K) <= 2 ? 6 : (K) <= 3 ? 5 : 4)
-#endif
-__host__ __device__ constexpr int gemm_raw_slots(int K) { return HTR_GEMM_RAW_SLOTS(K); }
+constexpr int kLbo = 128;                                   // bytes between core matrices of B adjacent in K
+constexpr int kSboB = 1024;                                 // bytes between its 8-column groups (64 k x 8 columns x 2 bytes)
+constexpr unsigned kSleepNs = 100u;                         // between polls of a role that is ahead of the decode warps
+constexpr unsigned kSpinLimit = 2000000u;                   // iterations of a try_wait loop before giving up
 
 struct GemmParams {
   const uint32_t* qw;
@@ -74,22 +67,21 @@ struct GemmParams {
   const uint8_t* sv;
   const void* bias;
   void* y;
-  const __half* xb;       // transformed activations, [chunk][column group of 8][8 k-groups][8 columns][8 k] fp16:
-                          // columns 0..np-1 = hi plane of the activation rows, np..2np-1 = lo plane (planes == 2)
-  const float* xsum;      // [np][xsum_slices] sums over k (per 1024-column slice) of the planes in use (hi, or hi + lo)
+  const __half* xb;       // transformed activations in B tile layout (see rht_f16_kernel): columns 0..np-1 = hi plane of the
+                          // activation rows, np..2np-1 = lo plane (planes == 2)
+  const float* xsum;      // [np][xsum_slices] sums over k (per slice of the transform) of the planes in use
   const float* tok;       // [np] power-of-two range scale per activation row
-  float* part;            // [row blocks][slots][np][128]
+  float* part;            // [thread blocks][2][np][128]: flat form, the partial of a thread block's first row block and of a later one
   int* counters;          // [row blocks]
-  int* error;             // one word: first failure code seen by any CTA (0 = none)
-  int rows, np;           // activation rows present / padded to a multiple of 16
-  int planes;             // 1: hi plane only (16-bit activations), 2: hi + lo (float32 activations)
+  int* error;             // one word: first failure code seen by any thread block (0 = none)
+  int rows, np;           // activation rows present / padded (to 16, or 8 with two planes)
+  int planes;
   int mt, nt;
+  int m_out;              // rows of the weight that are written (row stride of y, length of bias)
   int dtype;
-  int hb;                 // 128-column blocks per row (n / 128) = units per row block
-  int split;              // CTAs per row block
-  int cluster;            // 1: the CTAs of a row block were launched as one thread-block cluster (split <= 8): the split reduction
-                          // goes through distributed shared memory instead of global partial sums
-  int stages;             // stage pairs in the ring (2..kMaxStages)
+  int hb;                 // 128-column blocks per row block (n / 128)
+  int split;              // > 0: thread blocks per row block (cluster form); 0: flat ranges
+  int stages;
   int xsum_slices;
   float cb;
   // row-shard form: the output rows go, with plain peer stores, to element offset peer_offset + j * m + row of every buffer in
@@ -99,70 +91,63 @@ struct GemmParams {
   long long peer_offset;
 };
 
-__device__ __forceinline__ void gemm_store_rows(const GemmParams& p, int j, int m, int row0, float4 o) {
+__device__ __forceinline__ void gemm_store_rows(const GemmParams& p, int j, int row0, float4 o) {
   if (p.npeer == 0) {
-    store_quad(p.y, (size_t)j * m + row0, p.dtype, o);
+    if (row0 < p.m_out) store_quad(p.y, (size_t)j * p.m_out + row0, p.dtype, o);
   } else {
 #pragma unroll 1
-    for (int pe = 0; pe < p.npeer; ++pe) store_quad(p.peer_y[pe], (size_t)p.peer_offset + (size_t)j * m + row0, p.dtype, o);
+    for (int pe = 0; pe < p.npeer; ++pe) store_quad(p.peer_y[pe], (size_t)p.peer_offset + (size_t)j * p.m_out + row0, p.dtype, o);
   }
+}
+
+// One lane of the (converged) warp.  The branch on elect.sync tells the compiler that one thread runs it, so the operands of
+// tcgen05 and bulk-copy instructions go to uniform registers once; behind `lane == 0` every MMA took 125 cycles to issue, behind
+// the election 50 (measured back to back at N = 16..64, A in tensor memory).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(is));
+  return is != 0;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr, int sbo_bytes) {
+__device__ __forceinline__ uint64_t umma_desc_b(uint32_t smem_addr) {
   // start address, LBO, SBO in 16-byte units; descriptor version 1 (sm_100); layout type 0 = no swizzle
-  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)((kLbo >> 4) & 0x3FFF) << 16) | ((uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32) |
+  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)((kLbo >> 4) & 0x3FFF) << 16) | ((uint64_t)((kSboB >> 4) & 0x3FFF) << 32) |
          (1ull << 46);
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-
-// bounded wait for the phase with the given parity; false when the limit ran out or another role has already failed
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* fail) {
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity, unsigned hint_ns) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity), "r"(hint_ns)
+      : "memory");
+  return done != 0;
+}
+// (a role that waits most of the time sleeps between polls: the issue slots are the decode warps')
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, const volatile int* fail, unsigned sleep_ns) {
   for (unsigned it = 0; it < kSpinLimit; ++it) {
-    uint32_t done;
-#if HTR_GEMM_WAIT_HINT > 0
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity), "r"((unsigned)HTR_GEMM_WAIT_HINT)
-        : "memory");
-#else
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-#endif
-    if (done) return true;
-    if ((it & 255u) == 255u && *fail) return false;
+    if (mbar_try(bar, parity, 1000u)) return true;
+    if ((it & 255u) == 255u && fail && *fail) return false;
+    if (sleep_ns) __nanosleep(sleep_ns);
   }
   return false;
 }
-
-// the same without the early exit: used on the failure path to let copies and MMAs in flight drain
-__device__ __forceinline__ bool mbar_wait_plain(uint32_t bar, uint32_t parity) {
-  for (unsigned it = 0; it < kSpinLimit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
+// bounded wait for the phase with the given parity; false when the limit ran out or another role has already failed
+// (`fail` null: no early exit -- used on the failure path to let copies and MMAs in flight drain)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* fail, unsigned sleep_ns = 0) {
+  return mbar_try(bar, parity, 1000u) || mbar_wait_slow(bar, parity, fail, sleep_ns);
 }
 
 // global -> shared bulk copy (16-byte aligned, size a multiple of 16), completion counted in bytes on an mbarrier
@@ -172,282 +157,458 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// D[128 x N] (+)= A[128 x 16 f16, tensor memory] * B[N x 16 f16, shared memory]
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// 16 consecutive accumulator columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_load16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// 16 lanes x 32 columns of tensor memory from one warp: registers 4j, 4j+1 of lane (g, c) = columns 8j + 2c, +1 of row g,
+// registers 4j+2, 4j+3 the same of row g + 8
+__device__ __forceinline__ void tmem_store_strip(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+               "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+               "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+               : "memory");
+}
+
+// 8 consecutive accumulator columns of this thread's tensor-memory lane (complete after tcgen05.wait::ld)
+__device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+
+// dynamic shared memory: the B ring (the cluster form reuses it for the [np][128] float partial of the thread block), then the
+// packed-word rings of the decode warps (`words` bytes)
+__host__ __device__ inline int gemm_stage_bytes(int ncols) { return ncols * 256; }
+__host__ __device__ inline int gemm_ring_bytes(int np, int planes, int stages) {
+  const int ring = stages * gemm_stage_bytes(np * planes), result = np * 128 * 4;
+  return ring > result ? ring : result;
+}
+__host__ __device__ inline int gemm_smem_bytes(int np, int planes, int stages, int words) { return gemm_ring_bytes(np, planes, stages) + words + 128; }
+__host__ __device__ inline int gemm_acc_cols(int ncols) { return ncols < 32 ? 32 : ncols; }
+
+// ---- packed-word ring of a decode warp: one slot = the tiles of its strip in one 128-column block (two units of four tiles).
+// A lane reads the words of row pair g of tile c; for K a multiple of 4 the 16-byte chunks of a tile are stored in an order that
+// spreads the eight lanes of a read phase (two g, four c) over all banks.
+template <int K>
+struct GemmRing {
+  static constexpr int slot_bytes = 256 * K;
+  static constexpr int slots = K <= 3 ? 6 : K <= 5 ? 4 : 3;  // 40 to 64 KB in flight per SM
+  static constexpr int bytes = kGemmDecodeWarps * slots * slot_bytes;
+  static constexpr int chunks = slot_bytes / 16, copies = (chunks + 31) / 32;
+};
+// position (in 16-byte chunks, inside the four tiles of a unit) of chunk ch of tile c
+template <int K>
+__device__ __forceinline__ int ring_chunk(int c, int ch) {
+  if constexpr (K == 4) return c * 8 + (ch ^ (2 * c));
+  else if constexpr (K == 8) return c * 16 + (ch ^ ((c & 1) | ((c & 2) << 1)));
+  else return c * 2 * K + ch;
+}
+template <int K>
+__device__ __forceinline__ void read_own_words(const unsigned char* unit, int c, int g, uint32_t (&V)[K]) {
+  if constexpr (K % 4 == 0) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < K / 4; ++i) {
+      const uint4 t = *reinterpret_cast<const uint4*>(unit + 16 * ring_chunk<K>(c, (K / 4) * g + i));
+      V[4 * i] = t.x; V[4 * i + 1] = t.y; V[4 * i + 2] = t.z; V[4 * i + 3] = t.w;
+    }
+  } else if constexpr (K % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < K / 2; ++i) {
+      const uint2 t = *reinterpret_cast<const uint2*>(unit + c * (32 * K) + g * (4 * K) + 8 * i);
+      V[2 * i] = t.x; V[2 * i + 1] = t.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < K; ++i) V[i] = *reinterpret_cast<const uint32_t*>(unit + c * (32 * K) + g * (4 * K) + 4 * i);
+  }
 }
 
-// dynamic shared memory: stages {A tile, B tile}, then the packed-word rings of the decode warps -- later reused for
-// the [np][128] float result
-__host__ __device__ inline int gemm_stage_bytes(int ncols) { return kDecodeGroups * (kATileBytes + ncols * 128); }   // one pair
-__host__ __device__ inline int gemm_smem_bytes(int np, int planes, int K, int stages) {
-  const int pipe = stages * gemm_stage_bytes(np * planes) + kGemmDecodeWarps * gemm_raw_slots(K) * (4 * 32 * K);
-  const int result = np * 128 * 4;
-  return (pipe > result ? pipe : result) + 128;
+// 32 codebook integers of a lane unit as fp16 pairs (1024 + bytesum), in the register order of tmem_store_strip
+template <int K>
+__device__ __forceinline__ void decode_unit(const uint32_t (&own)[K], int lane, uint32_t (&out)[16]) {
+  uint32_t V[K + 1], s[32];
+#pragma unroll
+  for (int i = 0; i < K; ++i) V[i + 1] = own[i];
+  V[0] = __shfl_sync(kFullWarp, own[K - 1], (lane - 4) & 31);          // last word of the row pair before, circularly inside the tile
+  unit_states<K>(V, s);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = rr * 16 + 4 * j + 2 * h;
+        const uint32_t lo = bytesum_add(s[t] * kGenMul + kGenAdd, 0x6400u), hi = bytesum_add(s[t + 1] * kGenMul + kGenAdd, 0x6400u);
+        // the pack goes to whichever pipe the width leaves free: shift/logic (PRMT) or multiply (IMAD)
+        const bool alu = PairStride<K>::value > 1 || h == 0;
+        out[4 * j + 2 * rr + h] = alu ? __byte_perm(lo, hi, 0x5410) : hi * 65536u + lo;
+      }
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// barrier of the finisher warps; true where every thread brought true
+__device__ __forceinline__ bool finishers_all(bool mine) {
+  int all;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %1, 0;\n\tbar.red.and.pred p, 1, %2, q;\n\tselp.s32 %0, 1, 0, p;\n\t}"
+               : "=r"(all)
+               : "r"((int)mine), "n"(kGemmFinishWarps * 32)
+               : "memory");
+  return all != 0;
+}
+
+// ---- finishing of a row block: one warp per activation row, lane holds rows 4 lane .. + 3 of the block
+struct GemmTail {
+  float s[4];                                               // row scales
+  unsigned sv_bits;
+  float4 bias;
+  int row0;
+  __device__ __forceinline__ GemmTail(const GemmParams& p, int rb, int lane) {
+    row0 = rb * 128 + 4 * lane;
+    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(p.scales + row0));
+    const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+    s[0] = s01.x; s[1] = s01.y; s[2] = s23.x; s[3] = s23.y;
+    sv_bits = sign_nibble(p.sv, rb * 32 + lane);
+    bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.bias && row0 < p.m_out) bias = load_quad(p.bias, row0, p.dtype);
+  }
+};
+// this lane's share of the row sum of the activations; the warp adds the shares (a fixed tree: results do not depend on scheduling)
+__device__ __forceinline__ float gemm_xsum_share(const GemmParams& p, int j, int lane) {
+  float xs = 0.f;
+  for (int y = lane; y < p.xsum_slices; y += 32) xs += __ldcg(p.xsum + (size_t)j * p.xsum_slices + y);
+  return xs;
+}
+__device__ __forceinline__ void gemm_finish_row(const GemmParams& p, const GemmTail& t, int j, int lane, float4 r4, float xs, float tok) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) xs += __shfl_xor_sync(kFullWarp, xs, o);
+  const float off = 1534.0f * xs, rs = p.cb * tok;
+  float v[4] = {(r4.x - off) * (t.s[0] * rs), (r4.y - off) * (t.s[1] * rs), (r4.z - off) * (t.s[2] * rs), (r4.w - off) * (t.s[3] * rs)};
+  wht128(v, lane);
+  gemm_store_rows(p, j, t.row0, make_float4(flip(v[0] * kInvSqrt128, t.sv_bits & 1u) + t.bias.x, flip(v[1] * kInvSqrt128, (t.sv_bits >> 1) & 1u) + t.bias.y,
+                                            flip(v[2] * kInvSqrt128, (t.sv_bits >> 2) & 1u) + t.bias.z, flip(v[3] * kInvSqrt128, t.sv_bits >> 3) + t.bias.w));
+}
+
+// flat form: even runs of 128-column blocks, the first `rem` thread blocks hold one more
+struct GemmRuns {
+  int q, rem;
+  __device__ __forceinline__ GemmRuns(int units, int grid) : q(units / grid), rem(units - (units / grid) * grid) {}
+  __device__ __forceinline__ int begin(int b) const { return b * q + min(b, rem); }
+  __device__ __forceinline__ int owner(int u) const { return u < rem * (q + 1) ? u / (q + 1) : rem + (u - rem * (q + 1)) / q; }
+};
+
+// rows j0, j0 + step, ... of row block rb from the partial sums of thread blocks first .. first + contributors - 1, added in that
+// order.  Two rows at a time: the loads of both are in flight together.  head: which partial of thread block `first`.
+__device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, int first, int contributors, int head, int j0, int step, int lane) {
+  const GemmTail tail(p, rb, lane);
+  const float4* slot0 = reinterpret_cast<const float4*>(p.part + (size_t)(2 * first) * ((size_t)p.np * 128)) + lane;
+  const size_t stride = (size_t)p.np * 32;
+  for (int j = j0; j < p.rows; j += 2 * step) {
+    const int jb = j + step < p.rows ? j + step : j;
+    const float xa = gemm_xsum_share(p, j, lane), xb = gemm_xsum_share(p, jb, lane), ta = __ldcg(p.tok + j), tb = __ldcg(p.tok + jb);
+    float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb4 = ra;
+    for (int base = 0; base < contributors; base += 4) {
+      float4 va[4], vb[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = base + q;
+        const float4* src = slot0 + (size_t)(i == 0 ? head : 2 * i) * stride;
+        va[q] = i < contributors ? __ldcg(src + j * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+        vb[q] = i < contributors ? __ldcg(src + jb * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        ra.x += va[q].x; ra.y += va[q].y; ra.z += va[q].z; ra.w += va[q].w;
+        rb4.x += vb[q].x; rb4.y += vb[q].y; rb4.z += vb[q].z; rb4.w += vb[q].w;
+      }
+    }
+    gemm_finish_row(p, tail, j, lane, ra, xa, ta);
+    if (jb != j) gemm_finish_row(p, tail, jb, lane, rb4, xb, tb);
+  }
 }
 
 template <int K>
-__global__ void __launch_bounds__(kGemmThreads) packed_gemm_tc_kernel(const GemmParams p) {
+__global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const GemmParams p) {
   extern __shared__ __align__(128) unsigned char gsm[];
-  __shared__ __align__(8) unsigned long long s_afull[kMaxStages], s_bfull[kMaxStages], s_freed[kMaxStages], s_done;
+  __shared__ __align__(8) unsigned long long s_full[kGemmMaxStages], s_freed[kGemmMaxStages], s_done, s_drained;
   __shared__ uint32_t s_tmem;
   __shared__ int s_arrival;
+  __shared__ int s_owed[kGemmFinishWarps];                  // row blocks below it have been delivered by the finisher warp
   __shared__ volatile int s_fail;
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  constexpr int DW = kGemmDecodeWarps;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int np = p.np, ncols = p.planes * np;               // accumulator columns: hi plane, then lo plane if present
-  const int nt = p.nt, m = p.mt * 16, HB = p.hb, NS = p.stages;
-  const int rb = blockIdx.x / p.split, part_id = blockIdx.x - rb * p.split;
-  const int hb_begin = part_id * HB / p.split, hb_end = (part_id + 1) * HB / p.split;
-  const int chunks = (hb_end - hb_begin) * 2;                // two 64-column chunks per 128-column block
-  constexpr int kStripBytes = 4 * 32 * K, R = gemm_raw_slots(K);
-  const int b_tile_bytes = ncols * 128, stage_bytes = kDecodeGroups * (kATileBytes + b_tile_bytes);   // pair: A0 | A1 | B0 | B1
-  unsigned char* stage0 = gsm + (128 - (smem_u32(gsm) & 127)) % 128;   // 128-byte aligned start: stage s = {A tile, B tile}
-  unsigned char* raw0 = stage0 + NS * stage_bytes;                     // packed-word rings [decode warp][slot][4 tiles][8K words]
-  const uint32_t stage0_addr = smem_u32(stage0), raw0_addr = smem_u32(raw0);
+  const int nt = p.nt, HB = p.hb, NS = p.stages;
+  const int U = (p.mt >> 3) * HB;
+  const GemmRuns runs(U, gridDim.x);
+  int u_begin, u_end, part_id = 0;
+  if (p.split > 0) {
+    const int rb = blockIdx.x / p.split;
+    part_id = blockIdx.x - rb * p.split;
+    u_begin = rb * HB + part_id * HB / p.split;
+    u_end = rb * HB + (part_id + 1) * HB / p.split;
+  } else {
+    u_begin = runs.begin(blockIdx.x);
+    u_end = runs.begin(blockIdx.x + 1);
+  }
+  const int b_tile_bytes = ncols * 256;
+  unsigned char* ring = gsm + (128 - (smem_u32(gsm) & 127)) % 128;
+  const uint32_t ring_addr = smem_u32(ring);
+  const int a_col = gemm_acc_cols(ncols);
 
-  uint32_t tmem_cols = 32;
-  while ((int)tmem_cols < ncols) tmem_cols <<= 1;
   if (tid == 0) {
-    for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(smem_u32(&s_afull[s]), kGemmDecodeWarps);              // one arrival per decode warp (both groups)
-      mbar_init(smem_u32(&s_bfull[s]), 1);                             // the B lane's arrive.expect_tx
-      mbar_init(smem_u32(&s_freed[s]), 1);                             // tcgen05.commit
+    for (int s = 0; s < kGemmMaxStages; ++s) {
+      mbar_init(smem_u32(&s_full[s]), kGemmGroupWarps + 1);             // the warps of the group that decodes the block, and the B
+                                                                        // lane's arrive.expect_tx (with the bytes of the tile)
+      mbar_init(smem_u32(&s_freed[s]), 1);                              // tcgen05.commit
     }
-    mbar_init(smem_u32(&s_done), 1);
+    mbar_init(smem_u32(&s_done), 1);                                    // tcgen05.commit: the MMAs of a row block have retired
+    mbar_init(smem_u32(&s_drained), kGemmFinishWarps);                  // one arrival per finisher warp: its accumulator has been read
     s_fail = 0;
+    for (int i = 0; i < kGemmFinishWarps; ++i) s_owed[i] = u_begin / HB;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(tmem_cols) : "memory");
+  if (warp == DW + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"((uint32_t)kGemmTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  if (warp == kGemmWarps - 1 && lane < 6) {
+    // the row scales and signs of the first and the last row block are needed at the very end, in a chain of dependent loads:
+    // bring them to L2 now (256 bytes of scales and 16 of signs per row block)
+    const size_t rb = lane & 1 ? (u_end - 1) / HB : u_begin / HB;
+    const char* at = lane < 4 ? reinterpret_cast<const char*>(p.scales + rb * 128) + (lane >> 1) * 128 : reinterpret_cast<const char*>(p.sv + rb * 16);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+  }
 
-  if (warp < kGemmDecodeWarps) {
-    // ================= decode warps: group = warp / 8 takes chunks group, group + 2, ...; strip = warp % 8;
-    // inside the strip: tile column tc = lane >> 3, row pair q = lane & 7
-    const int group = warp / kStripWarps, strip = warp % kStripWarps;
-    const int tc = lane >> 3, q = lane & 7;
-    const uint32_t ring_addr = raw0_addr + warp * (R * kStripBytes);
-    const unsigned char* ring = raw0 + warp * (R * kStripBytes);
-    const char* wsrc = reinterpret_cast<const char*>(p.qw) + ((size_t)(rb * 8 + strip) * nt + (size_t)hb_begin * 8) * (32 * K);
-    // asynchronous fetch of chunk c (contiguous: four tiles of this strip) into ring slot `slot`; always commits a group
-    auto prefetch = [&](int c, int slot) {
-      if (c < chunks) {
-        const char* src = wsrc + (size_t)c * kStripBytes;
-        const uint32_t dst = ring_addr + slot * kStripBytes;
+  if (warp < DW) {
+    // ================= decode warps
+    const int quad = warp & 3, half = (warp >> 2) & 1, strip = 2 * quad + half, group = warp >> 3;
+    const int g = lane >> 2, c = lane & 3;
+    using Ring = GemmRing<K>;
+    constexpr int R = Ring::slots;
+    const unsigned char* words = ring + gemm_ring_bytes(np, p.planes, NS) + warp * (R * Ring::slot_bytes);
+    // copy cursor: every second block of the run, across row blocks; past the end of the run the copies are predicated off
+    uint32_t cp_dst[Ring::copies];
 #pragma unroll
-        for (int j = 0; j < (kStripBytes / 16 + 31) / 32; ++j)
-          if (32 * j + 32 <= kStripBytes / 16 || lane + 32 * j < kStripBytes / 16) cp_async16(dst + (lane + 32 * j) * 16, src + (lane + 32 * j) * 16);
+    for (int i = 0; i < Ring::copies; ++i) {
+      const int ch = lane + 32 * i, unit = ch / (8 * K), within = ch % (8 * K);
+      cp_dst[i] = smem_u32(words) + unit * (128 * K) + 16 * ring_chunk<K>(within / (2 * K), within % (2 * K));
+    }
+    // from the end of a strip's row to the same strip of the next row block (a row of one block is left twice per step of two)
+    const size_t next_strip = (size_t)7 * nt * (32 * K) * (HB == 1 ? 2 : 1);
+    int pf_left = u_end - u_begin - group, pf_in_rb;
+    const char* pf;
+    {
+      const int u = u_begin + group, rb = u / HB, hb = u - rb * HB;
+      pf = reinterpret_cast<const char*>(p.qw) + ((size_t)(rb * 8 + strip) * nt + (size_t)hb * 8) * (32 * K) + lane * 16;
+      pf_in_rb = HB - hb;
+    }
+    auto fetch = [&](uint32_t at) {
+#pragma unroll
+      for (int i = 0; i < Ring::copies; ++i) {
+        const int on = (32 * i + 32 <= Ring::chunks || lane + 32 * i < Ring::chunks) ? pf_left : 0;
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(cp_dst[i] + at),
+                     "l"(pf + 512 * i), "r"(on)
+                     : "memory");
       }
+      pf_left -= 2;
+      const bool wrap = pf_in_rb <= 2;
+      pf_in_rb += wrap ? HB - 2 : -2;
+      pf += wrap ? next_strip + 512 * K : (size_t)(512 * K);
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
-    for (int i = 0; i < R - 1; ++i) prefetch(group + kDecodeGroups * i, i);   // the weights do not depend on the preceding kernel
-    // the barriers and the TMEM address become visible here (first CTA-wide barrier)
+    for (int i = 0; i < R - 1; ++i) fetch(i * Ring::slot_bytes);   // the weights do not depend on the preceding kernel
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    const int hist = history_word<K>(q);
-    const int row_a = strip * 16 + 2 * q;
-    const uint32_t a_off = (uint32_t)((row_a >> 3) * kSboA + (row_a & 7) * 16 + (2 * tc) * kLbo);
-    int slot = 0;
-    int st_idx = 0;                                         // ring slot of the pair (c / 2) % NS
-    uint32_t use = 0u;                                      // how many times that slot was used before this pair
+    __syncthreads();                                        // the barriers and the tensor-memory address are visible from here on
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t a_addr = s_tmem + ((uint32_t)(32 * quad + 16 * half) << 16) + (uint32_t)a_col;
+    // (this loop is what bounds the kernel: no branches but the two below, no divisions, no counters beside the ring positions)
+    uint32_t at = 0u, refill = (R - 1) * Ring::slot_bytes;  // ring slots of this block and of the one before it
+    int stage = group;
+    uint32_t parity = 1u;                                   // of freed[stage]: passes at once on the first round
     bool ok = true;
-    for (int c = group; c < chunks; c += kDecodeGroups) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(R - 2) : "memory");   // this chunk's words have landed (own copies) ...
-      __syncwarp();                                                       // ... and those of the other lanes; slot of the previous chunk is free
-      prefetch(c + kDecodeGroups * (R - 1), slot == 0 ? R - 1 : slot - 1);
-      uint32_t V[K + 1];
-      {
-        const uint32_t* tile = reinterpret_cast<const uint32_t*>(ring + slot * kStripBytes) + tc * (8 * K);
-        const uint32_t* own = tile + q * K;
-        if constexpr (K % 4 == 0) {
-#pragma unroll
-          for (int i = 0; i < K / 4; ++i) {
-            const uint4 t = *reinterpret_cast<const uint4*>(own + 4 * i);
-            V[4 * i + 1] = t.x; V[4 * i + 2] = t.y; V[4 * i + 3] = t.z; V[4 * i + 4] = t.w;
-          }
-        } else if constexpr (K % 2 == 0) {
-#pragma unroll
-          for (int i = 0; i < K / 2; ++i) {
-            const uint2 t = *reinterpret_cast<const uint2*>(own + 2 * i);
-            V[2 * i + 1] = t.x; V[2 * i + 2] = t.y;
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < K; ++k) V[k + 1] = own[k];
-        }
-        V[0] = tile[hist];
-      }
-      // the MMAs that read this ring slot (NS pairs ago) must have retired
-      if (use > 0 && !__all_sync(kFullWarp, mbar_wait(smem_u32(&s_freed[st_idx]), (use - 1u) & 1u, &s_fail))) { ok = false; break; }
-      unsigned char* dst0 = stage0 + st_idx * stage_bytes + group * kATileBytes + a_off;
-      // 32 codebook integers of this lane unit as fp16 (1024 + bytesum): rows 2q and 2q+1 of the strip, 16 k each
-      uint32_t st[32];
-      unit_states<K>(V, st);
-#pragma unroll
-      for (int rr = 0; rr < 2; ++rr) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-#if HTR_GEMM_PACK_MODE == 0
-            const uint32_t lo = bytesum_add_alu(st[rr * 16 + half * 8 + 2 * e] * kGenMul + kGenAdd, 0x6400u);
-            const uint32_t hi = bytesum_add(st[rr * 16 + half * 8 + 2 * e + 1] * kGenMul + kGenAdd, 0x6400u);
-            w[e] = __byte_perm(lo, hi, 0x5410);
-#elif HTR_GEMM_PACK_MODE == 1
-            const uint32_t lo = bytesum_add(st[rr * 16 + half * 8 + 2 * e] * kGenMul + kGenAdd, 0x6400u);
-            const uint32_t hi = bytesum_add(st[rr * 16 + half * 8 + 2 * e + 1] * kGenMul + kGenAdd, 0x6400u);
-            w[e] = hi * 65536u + lo;                         // multiply-add: keeps the pack off the shift/logic pipe
-#else
-            const uint32_t lo = bytesum_add_alu(st[rr * 16 + half * 8 + 2 * e] * kGenMul + kGenAdd, 0x6400u);
-            const uint32_t hi = bytesum_add(st[rr * 16 + half * 8 + 2 * e + 1] * kGenMul + kGenAdd, 0x6400u);
-            w[e] = hi * 65536u + lo;
-#endif
-          }
-          *reinterpret_cast<uint4*>(dst0 + rr * 16 + half * kLbo) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core
+#pragma unroll 1
+    for (int left = u_end - u_begin - group; left > 0; left -= 2) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(R - 2) : "memory");   // this block's words have landed (own copies) ...
+      __syncwarp();                                                       // ... and those of the other lanes; the slot before it is free
+      fetch(refill);
+      const unsigned char* blk = words + at;
+      refill = at;
+      at = at == (R - 1) * Ring::slot_bytes ? 0u : at + Ring::slot_bytes;
+      uint32_t V[K], w[16];
+      read_own_words<K>(blk, c, g, V);
+      decode_unit<K>(V, lane, w);
+      // the MMAs that read this stage NS blocks ago must have retired
+      const uint32_t bar = smem_u32(&s_freed[0]) + 8u * stage;
+      if (!__all_sync(kFullWarp, mbar_try(bar, parity, 1000u)) && !__all_sync(kFullWarp, mbar_wait_slow(bar, parity, &s_fail, 0u))) { ok = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tmem_store_strip(a_addr + 64 * stage, w);
+      read_own_words<K>(blk + 128 * K, c, g, V);
+      decode_unit<K>(V, lane, w);
+      tmem_store_strip(a_addr + 64 * stage + 32, w);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_afull[st_idx]));
-      if (++slot == R) slot = 0;
-      if (++st_idx == NS) { st_idx = 0; ++use; }
+      if (lane == 0) mbar_arrive(smem_u32(&s_full[0]) + 8u * stage);
+      const bool around = stage + 2 >= NS;
+      stage += around ? 2 - NS : 2;
+      parity ^= around ? 1u : 0u;
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (!ok) s_fail = 1;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == kGemmDecodeWarps) {
-      // ================= B lane: one bulk copy per chunk (the activation transform wrote the tiles contiguously)
-      if (lane == 0) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");   // the transformed activations come from the preceding kernel
-        const char* bsrc = reinterpret_cast<const char*>(p.xb) + (size_t)(hb_begin * 2) * b_tile_bytes;
-        int s = 0, issued = 0;
+    if (warp == DW) {
+      // ================= B lane: one bulk copy per 128-column block (the activation transform wrote the tiles contiguously)
+      if (elect_one()) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // the transformed activations come from the preceding kernel
+        int s = 0, issued = 0, hb = u_begin % HB;
         uint32_t use = 0u;
-        const uint32_t pair_b_bytes = (uint32_t)(kDecodeGroups * b_tile_bytes);
-        for (int pr = 0; pr < chunks / kDecodeGroups; ++pr) {      // the B tiles of a pair are contiguous in global memory: one copy
-          if (use > 0 && !mbar_wait(smem_u32(&s_freed[s]), (use - 1u) & 1u, &s_fail)) { s_fail = 1; break; }
-          const uint32_t bar = smem_u32(&s_bfull[s]);
-          mbar_expect_tx(bar, pair_b_bytes);
-          bulk_load(stage0_addr + s * stage_bytes + kDecodeGroups * kATileBytes, bsrc + (size_t)pr * pair_b_bytes, pair_b_bytes, bar);
+        for (int u = u_begin; u < u_end; ++u) {
+          if (use > 0 && !mbar_wait(smem_u32(&s_freed[s]), (use - 1u) & 1u, &s_fail, kSleepNs)) { s_fail = 1; break; }
+          const uint32_t bar = smem_u32(&s_full[s]);
+          mbar_expect_tx(bar, (uint32_t)b_tile_bytes);
+          bulk_load(ring_addr + s * b_tile_bytes, reinterpret_cast<const char*>(p.xb) + (size_t)hb * b_tile_bytes, (uint32_t)b_tile_bytes, bar);
           ++issued;
+          if (++hb == HB) hb = 0;
           if (++s == NS) { s = 0; ++use; }
         }
         if (s_fail) {
-          // copies still in flight write into this CTA's shared memory: wait (bounded) for every slot last filled
-          for (int pr = issued > NS ? issued - NS : 0; pr < issued; ++pr) mbar_wait_plain(smem_u32(&s_bfull[pr % NS]), (uint32_t)(pr / NS) & 1u);
+          // copies still in flight write into this thread block's shared memory, and the decode warps' arrivals may never come to
+          // complete their barriers: give the copies far longer than a copy takes
+          if (issued) __nanosleep(1000000u);
         }
       }
-    } else if (lane == 0) {
+    } else if (warp == DW + 1) {
       // ================= MMA lane
-      const uint32_t tmem_acc = s_tmem;
-      // instruction descriptor: D = f32, A = B = f16, both K-major, M = 128, N = ncols
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(ncols >> 3) << 17) | ((128u >> 4) << 24);
-      int s = 0;
-      uint32_t ph = 0u;
-      bool ok = true;
-      for (int pr = 0; pr < chunks / kDecodeGroups; ++pr) {
-        if (!mbar_wait(smem_u32(&s_afull[s]), ph, &s_fail)) { ok = false; break; }
-        if (!mbar_wait(smem_u32(&s_bfull[s]), ph, &s_fail)) { ok = false; break; }
+      if (elect_one()) {
+        const uint32_t tmem = s_tmem;
+        // instruction descriptor: D = f32, A = B = f16, both K-major, M = 128, N = ncols
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(ncols >> 3) << 17) | ((128u >> 4) << 24);
+        const uint64_t desc0 = umma_desc_b(ring_addr);
+        int s = 0, seg = 0;
+        uint32_t ph = 0u;
+        bool ok = true;
+        for (int u = u_begin; u < u_end && ok; ++seg) {
+          const int stop = min(u_end, (u / HB + 1) * HB);
+          if (seg > 0 && !mbar_wait(smem_u32(&s_drained), (uint32_t)(seg - 1) & 1u, &s_fail)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          uint32_t fresh = 0u;                               // 0: the first MMA of a row block overwrites the accumulator
+          for (; u < stop; ++u) {
+            if (!mbar_wait(smem_u32(&s_full[s]), ph, &s_fail)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t desc = desc0 + (uint64_t)(s * (b_tile_bytes >> 4));   // (shared memory addresses fit the field: no carry)
+            const uint32_t a_addr = tmem + (uint32_t)(a_col + 64 * s);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                umma_f16_ts(tmem, a_addr + 32 * q + 8 * j, desc + (uint64_t)(q * (b_tile_bytes >> 5) + j * ((2 * kLbo) >> 4)), idesc, (q | j) ? 1u : fresh);
+            fresh = 1u;
+            umma_commit(smem_u32(&s_freed[s]));
+            if (++s == NS) { s = 0; ph ^= 1u; }
+          }
+          if (!ok) break;
+          umma_commit(smem_u32(&s_done));                    // covers every MMA issued so far
+        }
+        if (!ok) {
+          s_fail = 1;                                        // the other threads stop waiting at once ...
+          __threadfence_block();
+          umma_commit(smem_u32(&s_done));
+          mbar_wait(smem_u32(&s_done), (uint32_t)seg & 1u, nullptr);   // ... this one lets the MMAs in flight retire first
+        }
+      }
+    } else {
+      // ================= finishers
+      const int fw = warp - (DW + 2), quad = warp & 3;
+      const uint32_t acc_addr = s_tmem + ((uint32_t)(32 * quad) << 16);
+      const int li = lane & 15, row = 32 * quad + (lane & 16) + (li < 8 ? 2 * li : 2 * li - 15);   // weight row of this tensor-memory lane
+      bool ok = true, predecessor_done = false;
+      int seg = 0;
+      for (int u = u_begin; u < u_end; ++seg) {
+        const int rb = u / HB, stop = (rb + 1) * HB;
+        ok = __all_sync(kFullWarp, mbar_wait(smem_u32(&s_done), (uint32_t)seg & 1u, &s_fail, kSleepNs));
+        if (s_fail) ok = false;
+        if (!ok) s_fail = 1;
+        // all finishers go on together or none does (they meet in barriers below)
+        if (!finishers_all(ok)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_addr = stage0_addr + s * stage_bytes, b_addr = a_addr + kDecodeGroups * kATileBytes;
+        if (!predecessor_done) {
+          asm volatile("griddepcontrol.wait;" ::: "memory");   // scratch and outputs of earlier launches
+          predecessor_done = true;
+        }
+        // accumulator -> partial [np][128], hi + lo added here.  A thread block has two partials: its first row block's, which other
+        // thread blocks may read, and one for all later ones (of which only the last is read by others)
+        float* mine = p.split > 0 ? reinterpret_cast<float*>(ring) : p.part + (size_t)(2 * blockIdx.x + (seg > 0 ? 1 : 0)) * ((size_t)np * 128);
+        for (int j0 = 0; j0 < np; j0 += 8) {
+          uint32_t hi[8], lo[8];
+          tmem_load8(acc_addr + j0, hi);
+          if (p.planes == 2) tmem_load8(acc_addr + np + j0, lo);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int g = 0; g < kDecodeGroups; ++g)
-#pragma unroll
-          for (int kk = 0; kk < HTR_GEMM_MMAS; ++kk)
-            umma_f16(tmem_acc, umma_desc(a_addr + g * kATileBytes + kk * 2 * kLbo, kSboA), umma_desc(b_addr + g * b_tile_bytes + kk * 2 * kLbo, kSboB),
-                     idesc, (pr | g | kk) ? 1u : 0u);
-        umma_commit(smem_u32(&s_freed[s]));
-        if (++s == NS) { s = 0; ph ^= 1u; }
+          for (int j = 0; j < 8; ++j) {
+            const float v = p.planes == 2 ? __uint_as_float(hi[j]) + __uint_as_float(lo[j]) : __uint_as_float(hi[j]);
+            if (p.split > 0) mine[(j0 + j) * 128 + row] = v;
+            else __stcg(mine + (j0 + j) * 128 + row, v);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&s_drained));    // the MMAs of the next row block may start
+        if (p.split > 0 || stop >= u_end) break;             // the last row block: all warps finish it, below
+        // only the run's first row block can have other contributors here, thread blocks before this one
+        const int first = runs.owner(rb * HB), contributors = blockIdx.x - first + 1;
+        bool finish = true;
+        finishers_all(true);
+        if (contributors > 1) {
+          if (fw == 0 && lane == 0) {
+            __threadfence();                                 // the partials of the whole thread block (ordered by the barrier) before the arrival
+            s_arrival = atomicAdd(p.counters + rb, 1);       // (they are read with loads served by L2, after this atomic)
+          }
+          finishers_all(true);
+          finish = s_arrival == contributors - 1;
+          if (finish && fw == 0 && lane == 0) p.counters[rb] = 0;
+        }
+        if (finish) gemm_finish_flat(p, rb, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, fw, kGemmFinishWarps, lane);
+        __syncwarp();
+        if (lane == 0) s_owed[fw] = rb + 1;
+        finishers_all(true);                                 // the partial has been read by all of them: it may be written again
+        u = stop;
       }
-      umma_commit(smem_u32(&s_done));                        // covers every MMA issued above
-      if (!ok) {
-        s_fail = 1;                                          // the other threads stop waiting at once ...
-        mbar_wait_plain(smem_u32(&s_done), 0u);              // ... this one lets the MMAs in flight retire first
-      }
+      if (!ok) s_fail = 1;
     }
     __syncwarp();
   }
-  const uint32_t tmem_base = s_tmem;
-
-  // ---- all MMAs of this CTA done?
-  if (!mbar_wait(smem_u32(&s_done), 0u, &s_fail)) s_fail = 1;
-  asm volatile("griddepcontrol.wait;" ::: "memory");         // row sums / scales of the activations, scratch of earlier launches
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
   const bool bad = s_fail != 0;
   if (bad && tid == 0) atomicCAS(p.error, 0, 1);
 
-  // ---- accumulator -> registers -> shared [np][128]: thread = row of the block, hi + lo added here
-  float* result = reinterpret_cast<float*>(stage0);          // the stages are idle now
-  if (!bad) {
-    if (warp < 16) {
-      const int row = 32 * (warp & 3) + lane;                // a warp reads the TMEM lanes of its quadrant (warp % 4)
-      const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
-      for (int j0 = (warp >> 2) * 16; j0 < np; j0 += 64) {   // the four warps of a quadrant take alternate groups of 16 batch rows
-        float hi[16], lo[16];
-        tmem_load16(lane_addr + j0, hi);
-        if (p.planes == 2) {
-          tmem_load16(lane_addr + np + j0, lo);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) hi[j] += lo[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) result[(j0 + j) * 128 + row] = hi[j];
-      }
-    }
-  } else {
-    // a bounded wait gave up: the rows of this block come out as NaN (visible to any consumer), beside the error word
-    for (int e = tid; e < np * 128; e += kGemmThreads) result[e] = __uint_as_float(0x7FC00000u);
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
-
-  if (p.cluster) {
-    // ---- split reduction inside the cluster: every CTA keeps its partial [np][128] where it is; CTA r of the cluster sums rows
-    // r, r + split, ... over all CTAs (in rank order: the same additions as the global path) and finishes those rows itself
+  if (p.split > 0) {
+    // ---- split reduction inside the cluster: every thread block keeps its partial [np][128] where it is; thread block r of the
+    // cluster sums rows r, r + split, ... over all of them (in rank order) and finishes those rows itself
+    float* result = reinterpret_cast<float*>(ring);
+    if (bad)                                                 // a bounded wait gave up: the rows come out as NaN, beside the error word
+      for (int e = tid; e < np * 128; e += kGemmThreads) result[e] = __uint_as_float(0x7FC00000u);
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    const int row0 = rb * 128 + 4 * lane;
-    const uint2 sc_raw = __ldg(reinterpret_cast<const uint2*>(p.scales + row0));
-    const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.y));
-    const unsigned sv_bits = sign_nibble(p.sv, rb * 32 + lane);
-    float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.bias) bias4 = load_quad(p.bias, row0, p.dtype);
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // (done before by the roles that needed it)
+    const GemmTail tail(p, blockIdx.x / p.split, lane);
     const uint32_t result_addr = smem_u32(result);
     for (int j = part_id + p.split * warp; j < p.rows; j += p.split * kGemmWarps) {
+      const float xs = gemm_xsum_share(p, j, lane), tok = __ldcg(p.tok + j);
       float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int r = 0; r < p.split; ++r) {
         uint32_t remote;
@@ -456,75 +617,55 @@ __global__ void __launch_bounds__(kGemmThreads) packed_gemm_tc_kernel(const Gemm
         asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
         r4.x += v.x; r4.y += v.y; r4.z += v.z; r4.w += v.w;
       }
-      float xs = 0.f;
-      for (int y = 0; y < p.xsum_slices; ++y) xs += p.xsum[j * p.xsum_slices + y];
-      const float off = 1534.0f * xs, rs = p.cb * p.tok[j];
-      float v[4] = {(r4.x - off) * (s01.x * rs), (r4.y - off) * (s01.y * rs), (r4.z - off) * (s23.x * rs), (r4.w - off) * (s23.y * rs)};
-      wht128(v, lane);
-      float4 o = make_float4(flip(v[0] * kInvSqrt128, sv_bits & 1u), flip(v[1] * kInvSqrt128, (sv_bits >> 1) & 1u),
-                             flip(v[2] * kInvSqrt128, (sv_bits >> 2) & 1u), flip(v[3] * kInvSqrt128, sv_bits >> 3));
-      o.x += bias4.x; o.y += bias4.y; o.z += bias4.z; o.w += bias4.w;
-      gemm_store_rows(p, j, m, row0, o);
+      gemm_finish_row(p, tail, j, lane, r4, xs, tok);
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // nobody leaves while its shared memory may still be read
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    return;
-  }
-
-  // ---- split reduction across the CTAs of this row block (same scheme as the GEMV), then the epilogue
-  bool finish = true;
-  const int contributors = p.split;
-  if (contributors > 1) {
-    float4* mine = reinterpret_cast<float4*>(p.part + ((size_t)rb * contributors + part_id) * ((size_t)np * 128));
-    for (int e = tid; e < np * 32; e += kGemmThreads) __stcg(mine + e, reinterpret_cast<const float4*>(result)[e]);
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      s_arrival = atomicAdd(p.counters + rb, 1);
-      __threadfence();
-    }
-    __syncthreads();
-    finish = (s_arrival == contributors - 1);
-    if (finish) {
-      const float4* slot0 = reinterpret_cast<const float4*>(p.part + (size_t)rb * contributors * ((size_t)np * 128));
-      for (int e = tid; e < np * 32; e += kGemmThreads) {
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int sl = 0; sl < contributors; ++sl) {
-          const float4 v = __ldcg(slot0 + (size_t)sl * np * 32 + e);
-          sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-        }
-        reinterpret_cast<float4*>(result)[e] = sum;
+  } else {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int rb = (u_end - 1) / HB;
+    bool finish = !bad;
+    const int first = runs.owner(rb * HB), contributors = runs.owner((rb + 1) * HB - 1) - first + 1;
+    if (!bad && contributors > 1) {
+      if (tid == 0) {
+        __threadfence();                                    // the partials of the whole thread block (ordered by the barrier above) before the arrival
+        s_arrival = atomicAdd(p.counters + rb, 1);
       }
-      if (tid == 0) p.counters[rb] = 0;
+      __syncthreads();
+      finish = s_arrival == contributors - 1;
+      if (finish && tid == 0) p.counters[rb] = 0;
     }
-    __syncthreads();
+    if (finish) gemm_finish_flat(p, rb, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, warp, kGemmWarps, lane);
+    if (bad) {
+      // the row blocks this thread block still owed never complete (nobody arrives for them): their rows come out as NaN
+      const float nan = __uint_as_float(0x7FC00000u);
+      for (int b = min(min(s_owed[0], s_owed[1]), min(s_owed[2], s_owed[3])); b <= rb; ++b)
+        for (int j = warp; j < p.rows; j += kGemmWarps) gemm_store_rows(p, j, b * 128 + 4 * lane, make_float4(nan, nan, nan, nan));
+    }
   }
-  if (!finish) return;
-  // epilogue: one warp per activation row j; lane holds rows 4*lane .. 4*lane+3 of the block
-  const int row0 = rb * 128 + 4 * lane;
-  const uint2 sc_raw = __ldg(reinterpret_cast<const uint2*>(p.scales + row0));
-  const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.y));
-  const unsigned sv_bits = sign_nibble(p.sv, rb * 32 + lane);
-  float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (p.bias) bias4 = load_quad(p.bias, row0, p.dtype);
-  for (int j = warp; j < p.rows; j += kGemmWarps) {
-    float xs = 0.f;
-    for (int y = 0; y < p.xsum_slices; ++y) xs += p.xsum[j * p.xsum_slices + y];   // fixed order: results do not depend on scheduling
-    const float off = 1534.0f * xs, rs = p.cb * p.tok[j];
-    const float4 r4 = *reinterpret_cast<const float4*>(result + j * 128 + 4 * lane);
-    float v[4] = {(r4.x - off) * (s01.x * rs), (r4.y - off) * (s01.y * rs), (r4.z - off) * (s23.x * rs), (r4.w - off) * (s23.y * rs)};
-    wht128(v, lane);
-    float4 o = make_float4(flip(v[0] * kInvSqrt128, sv_bits & 1u), flip(v[1] * kInvSqrt128, (sv_bits >> 1) & 1u),
-                           flip(v[2] * kInvSqrt128, (sv_bits >> 2) & 1u), flip(v[3] * kInvSqrt128, sv_bits >> 3));
-    o.x += bias4.x; o.y += bias4.y; o.z += bias4.z; o.w += bias4.w;
-    gemm_store_rows(p, j, m, row0, o);
-  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == DW + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem), "r"((uint32_t)kGemmTmemCols) : "memory");
 }
 
 int gemm_rht_slices(int np, int n);
-int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
+int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
                 cudaStream_t st);
 template <int K>
-int launch_packed_gemm_tc(const GemmParams& p, int grid, cudaStream_t st);
+int launch_packed_gemm_tc(const GemmParams& p, int grid, int smem, cudaStream_t st);
+// clusters of `split` thread blocks that the GPU holds at once (0: none), for the cluster form of the plan
+template <int K>
+int packed_gemm_tc_clusters(int smem, int split);
+// bytes of the packed-word rings of a thread block
+inline int gemm_word_bytes(int K) {
+  switch (K) {
+    case 2: return GemmRing<2>::bytes;
+    case 3: return GemmRing<3>::bytes;
+    case 4: return GemmRing<4>::bytes;
+    case 5: return GemmRing<5>::bytes;
+    case 6: return GemmRing<6>::bytes;
+    default: return GemmRing<8>::bytes;
+  }
+}
 
 }  // namespace htr

@@ -1,62 +1,85 @@
 // Instantiates the tensor-core packed GEMM for one stream width; included by packed_gemm_tc_k<K>.cu with HTR_INST_K set.
+#include <map>
+#include <mutex>
+#include <tuple>
+
 #include "packed_gemm_tc.cuh"
 
 namespace htr {
+namespace {
+
+// shared memory beyond 48 KB: opted in once per device (the 227 KB limit includes the static part)
+int allow_smem(int dev) {
+  static bool allowed[64] = {false};
+  if (dev >= 0 && dev < 64 && allowed[dev]) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+  if (e != cudaSuccess) return (int)e;
+  if (dev >= 0 && dev < 64) allowed[dev] = true;
+  return 0;
+}
+
+}  // namespace
 
 template <>
-int launch_packed_gemm_tc<HTR_INST_K>(const GemmParams& p, int grid, cudaStream_t st) {
-  const int smem = gemm_smem_bytes(p.np, p.planes, HTR_INST_K, p.stages);
-  static bool allowed[64] = {false};                      // shared memory beyond 48 KB: opted in once per device
+int packed_gemm_tc_clusters<HTR_INST_K>(int smem, int split) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  // the query costs tens of microseconds on the host: remember the answer
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, int>, int> seen;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(dev, smem, split);
+  const auto it = seen.find(key);
+  if (it != seen.end()) return it->second;
+  int clusters = 0;
+  if (allow_smem(dev) == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)split);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)split;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&clusters, packed_gemm_tc_kernel<HTR_INST_K>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      clusters = 0;
+    }
+  }
+  seen[key] = clusters;
+  return clusters;
+}
+
+template <>
+int launch_packed_gemm_tc<HTR_INST_K>(const GemmParams& p, int grid, int smem, cudaStream_t st) {
   int dev = 0;
   if (const cudaError_t e = cudaGetDevice(&dev)) return (int)e;
-  if (dev < 0 || dev >= 64 || !allowed[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);   // the 227 KB limit includes the static part
-    if (e != cudaSuccess) return (int)e;
-    if (dev >= 0 && dev < 64) allowed[dev] = true;
-  }
+  if (const int e = allow_smem(dev)) return e;
   // programmatic stream serialisation: the kernel may start while the activation transform before it still runs; it
   // fetches packed words at once and waits (griddepcontrol.wait) before it touches anything that kernel writes
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kGemmThreads);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  GemmParams q = p;
-  q.cluster = 0;
-#ifndef HTR_GEMM_NO_CLUSTER
-  if (p.split >= 2 && p.split <= 8) {
-    // the CTAs of a row block as one cluster, when every cluster of the grid can be resident at once
+  if (p.split > 1) {
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = (unsigned)p.split;
     attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = 1;
     cfg.numAttrs = 2;
-    // the occupancy query costs tens of microseconds on the host: remember the answer per (device, cluster size, shared memory)
-    struct Seen { int dev, split, smem, clusters; };
-    static thread_local Seen seen[8] = {};
-    static thread_local int next_slot = 0;
-    int clusters = -1;
-    for (const Seen& c : seen)
-      if (c.split == p.split && c.smem == smem && c.dev == dev) clusters = c.clusters;
-    if (clusters < 0) {
-      if (cudaOccupancyMaxActiveClusters(&clusters, packed_gemm_tc_kernel<HTR_INST_K>, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();
-        clusters = 0;
-      }
-      seen[next_slot] = Seen{dev, p.split, smem, clusters};
-      next_slot = (next_slot + 1) % 8;
-    }
-    if (clusters * p.split >= grid) q.cluster = 1;
-    else cfg.numAttrs = 1;
   }
-#endif
-  return (int)cudaLaunchKernelEx(&cfg, packed_gemm_tc_kernel<HTR_INST_K>, q);
+  GemmParams q = p;
+  void* args[1] = {&q};
+  return (int)cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(packed_gemm_tc_kernel<HTR_INST_K>), args);
 }
 
 }  // namespace htr
-
