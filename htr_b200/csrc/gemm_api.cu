@@ -114,6 +114,176 @@ __global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Plan of a mixture-of-experts step for the grouped GEMM: the (token, slot) pairs sorted by expert and cut into tiles of up to
+// kGroupRows pairs, so that an expert's weights are decoded once per tile instead of once per pair.  One thread block; a warp
+// takes every 32nd expert and finds its pairs, in order, with one ballot per 32 route entries (a few hundred to a few thousand
+// entries: the launch is what it costs).  Entries outside the tables and absent experts (null weight) get no tile.
+// slot_of[pair] (behind the plan) = tile * kGroupRows + row, or -1.
+constexpr int kPlanThreads = 1024;
+__global__ void __launch_bounds__(kPlanThreads) route_plan_kernel(const long long* __restrict__ route, int count, int experts, const uint32_t* const* qw,
+                                                                  int* __restrict__ plan, int cap) {
+  extern __shared__ int plan_smem[];                         // [experts] pairs, then first tile of every expert; [count] routes
+  int* first_tile = plan_smem;
+  int* ids = plan_smem + experts;
+  __shared__ int warp_sum[kPlanThreads / 32];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");         // the route comes from the router's kernel, the last step may still read the plan
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int* slot_of = plan + group_plan_ints(cap);
+  for (int i = tid; i < count; i += kPlanThreads) {
+    const long long e = route[i];
+    const bool ok = e >= 0 && e < experts && qw[e] != nullptr;
+    ids[i] = ok ? (int)e : -1;
+    if (!ok) slot_of[i] = -1;
+  }
+  __syncthreads();
+  for (int e = warp; e < experts; e += kPlanThreads / 32) {
+    int n = 0;
+    for (int base = 0; base < count; base += 32) n += __popc(__ballot_sync(kFullWarp, base + lane < count && ids[base + lane] == e));
+    if (lane == 0) first_tile[e] = (n + kGroupRows - 1) / kGroupRows;
+  }
+  __syncthreads();
+  // exclusive sum of the tile counts over the experts
+  int running = 0;
+  for (int base = 0; base < experts; base += kPlanThreads) {
+    const int e = base + tid, own = e < experts ? first_tile[e] : 0;
+    int incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(kFullWarp, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < kPlanThreads / 32; ++w) {
+      if (w < warp) before += warp_sum[w];
+      all += warp_sum[w];
+    }
+    __syncthreads();
+    if (e < experts) first_tile[e] = running + before + incl - own;
+    running += all;
+  }
+  __syncthreads();
+  if (tid == 0) plan[0] = running;
+  for (int e = warp; e < experts; e += kPlanThreads / 32) {
+    const int t0 = first_tile[e];
+    int n = 0;
+    for (int base = 0; base < count; base += 32) {
+      const bool hit = base + lane < count && ids[base + lane] == e;
+      const unsigned mask = __ballot_sync(kFullWarp, hit);
+      if (hit) {
+        const int at = n + __popc(mask & ((1u << lane) - 1u)), t = t0 + at / kGroupRows, j = at % kGroupRows;
+        plan[4 + 2 * cap + t * kGroupRows + j] = base + lane;
+        slot_of[base + lane] = t * kGroupRows + j;
+      }
+      n += __popc(mask);
+    }
+    for (int t = lane; t < (n + kGroupRows - 1) / kGroupRows; t += 32) {
+      plan[4 + t0 + t] = e;
+      plan[4 + cap + t0 + t] = min(kGroupRows, n - t * kGroupRows);
+    }
+  }
+}
+
+// Activation transform of the grouped GEMM: one thread block per (token, slot) pair, two fp16 planes (the float32 activations of the
+// routed GEMV must not lose precision here), B operand tiles per plan tile as in rht_f16_kernel.  The row stays in registers
+// between the range scan and the transform.  SWIGLU: the row is [gate | up] of 2n bf16 values and the linear sees silu(gate) * up
+// with the roundings of the unfused operators.  Columns of B without a pair are left as they are: they reach only accumulator
+// columns that nobody reads.
+constexpr int kGroupRhtWarps = 16, kGroupRhtBlocks = 8;      // n <= 16 * 8 * 128
+template <bool SWIGLU>
+__global__ void __launch_bounds__(kGroupRhtWarps * 32) rht_group_kernel(const void* __restrict__ x, int dtype, int x_div, long long x_stride, int n,
+                                                                        const int* __restrict__ plan, int cap, const uint8_t* const* su_table,
+                                                                        __half* __restrict__ xb, float* __restrict__ xsum, float* __restrict__ tok) {
+  __shared__ float red[kGroupRhtWarps];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int pair = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blocks = n >> 7;
+  const int slot = __ldcg(plan + group_plan_ints(cap) + pair);
+  if (slot < 0) return;
+  const int t = slot / kGroupRows, r = slot % kGroupRows;
+  const uint8_t* su = su_table[group_expert(plan, cap, t)];
+  const size_t row = (size_t)(pair / x_div) * x_stride;
+  float v[kGroupRhtBlocks][4];
+  float mx = 0.f;
+#pragma unroll
+  for (int i = 0; i < kGroupRhtBlocks; ++i) {
+    const int hb = warp + kGroupRhtWarps * i, col = hb * 128 + 4 * lane;
+    if (hb >= blocks) break;
+    float4 q = load_quad(x, row + col, dtype);
+    if constexpr (SWIGLU) {
+      const float4 u = load_quad(x, row + n + col, dtype);
+      const auto rnd = [](float f) { return __bfloat162float(__float2bfloat16_rn(f)); };
+      q = make_float4(rnd(rnd(q.x / (1.f + __expf(-q.x))) * u.x), rnd(rnd(q.y / (1.f + __expf(-q.y))) * u.y), rnd(rnd(q.z / (1.f + __expf(-q.z))) * u.z),
+                      rnd(rnd(q.w / (1.f + __expf(-q.w))) * u.w));
+    }
+    v[i][0] = q.x; v[i][1] = q.y; v[i][2] = q.z; v[i][3] = q.w;
+    mx = fmaxf(mx, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFullWarp, mx, o));
+  if (lane == 0) red[warp] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kGroupRhtWarps; ++k) mx = fmaxf(mx, red[k]);
+  const float bound = mx * 11.32f;                           // |H128 x| / sqrt(128) <= sqrt(128) * amax
+  const float scale = bound > 16384.f ? exp2f(ceilf(log2f(bound / 16384.f))) : 1.f;
+  if (tid == 0) tok[slot] = scale;
+  const float inv = kInvSqrt128 / scale;
+  const int c = (lane & 15) >> 2, j = lane & 3;
+  constexpr size_t unit_halves = 2 * kGroupRows * 64;
+  __half* out = xb + (size_t)t * (2 * blocks) * unit_halves + (size_t)(2 * j + (c >> 1)) * 64 + 4 * (c & 1);
+  const size_t col_hi = (size_t)(r >> 3) * 512 + (r & 7) * 8, col_lo = col_hi + (kGroupRows >> 3) * 512;
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < kGroupRhtBlocks; ++i) {
+    const int hb = warp + kGroupRhtWarps * i;
+    if (hb >= blocks) break;                                 // warp-uniform
+    const unsigned sg = sign_nibble(su, hb * 32 + lane);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[i][k] = flip(v[i][k], (sg >> k) & 1u);
+    wht128(v[i], lane);
+    __half hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float f = v[i][k] * inv;
+      hi[k] = __float2half_rn(f);
+      lo[k] = __float2half_rn(f - __half2float(hi[k]));
+      sum += __half2float(hi[k]) + __half2float(lo[k]);      // exactly what the MMA will see
+    }
+    __half* at = out + (size_t)(2 * hb + (lane >> 4)) * unit_halves;
+    *reinterpret_cast<uint2*>(at + col_hi) = *reinterpret_cast<const uint2*>(hi);
+    *reinterpret_cast<uint2*>(at + col_lo) = *reinterpret_cast<const uint2*>(lo);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullWarp, sum, o);
+  __syncthreads();
+  if (lane == 0) red[warp] = sum;
+  __syncthreads();
+  if (tid == 0) {
+    float s = 0.f;
+    for (int k = 0; k < kGroupRhtWarps; ++k) s += red[k];
+    xsum[slot] = s;
+  }
+}
+
+template <typename... P, typename... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // resident early, waits before its first read
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // 128-column blocks per warp of the transform: one for small batches (most CTAs), more when the rows alone fill the GPU
 int gemm_rht_per(int np, int n) {
   const int max_per = (n / 128 + 7) / 8;
@@ -128,20 +298,12 @@ int gemm_rht_slices(int np, int n) {
 
 int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
                 cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(np, gemm_rht_slices(np, n));
-  cfg.blockDim = dim3(256);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // resident early, waits before its first read
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const int per = gemm_rht_per(np, n);
+  const dim3 grid(np, gemm_rht_slices(np, n));
   switch (dtype) {
-    case HTR_DTYPE_BF16: return (int)cudaLaunchKernelEx(&cfg, rht_f16_kernel<HTR_DTYPE_BF16>, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
-    case HTR_DTYPE_F16: return (int)cudaLaunchKernelEx(&cfg, rht_f16_kernel<HTR_DTYPE_F16>, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
-    default: return (int)cudaLaunchKernelEx(&cfg, rht_f16_kernel<HTR_DTYPE_F32>, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
+    case HTR_DTYPE_BF16: return launch_chained(rht_f16_kernel<HTR_DTYPE_BF16>, grid, 256, 0, st, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
+    case HTR_DTYPE_F16: return launch_chained(rht_f16_kernel<HTR_DTYPE_F16>, grid, 256, 0, st, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
+    default: return launch_chained(rht_f16_kernel<HTR_DTYPE_F32>, grid, 256, 0, st, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
   }
 }
 
@@ -152,7 +314,7 @@ constexpr size_t kCounterRegion = 1 << 16;   // same fixed counter region as the
 constexpr size_t kErrorRegion = 256;
 
 struct GemmPlan {
-  int np, rbs, hb, split, grid, stages, smem;
+  int np, rbs, hb, split, grid, stages, smem, sms;
   size_t off_xb, off_xsum, off_tok, off_part, total;
 };
 
@@ -184,6 +346,18 @@ int gemm_clusters(int K, int smem, int split) {
   return 0;
 }
 
+int launch_gemm(int K, const GemmParams& p, int grid, int smem, cudaStream_t st) {
+  switch (K) {
+    case 2: return launch_packed_gemm_tc<2>(p, grid, smem, st);
+    case 3: return launch_packed_gemm_tc<3>(p, grid, smem, st);
+    case 4: return launch_packed_gemm_tc<4>(p, grid, smem, st);
+    case 5: return launch_packed_gemm_tc<5>(p, grid, smem, st);
+    case 6: return launch_packed_gemm_tc<6>(p, grid, smem, st);
+    case 8: return launch_packed_gemm_tc<8>(p, grid, smem, st);
+  }
+  return (int)cudaErrorInvalidValue;
+}
+
 // activation rows per launch after padding: accumulator columns come in multiples of 16
 int padded_rows(int M, int planes) { return planes == 2 ? (M + 7) / 8 * 8 : (M + 15) / 16 * 16; }
 
@@ -197,6 +371,7 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
     if (dev >= 0 && dev < 64) seen_sms[dev] = sms;
   }
   GemmPlan g;
+  g.sms = sms;
   g.np = padded_rows(M, planes);
   g.rbs = m / 128;
   g.hb = n / 128;
@@ -314,20 +489,124 @@ static int gemm_launch(const void* x, int dtype, int M, const void* qweight, int
   p.m_out = m;
   p.xsum_slices = gemm_rht_slices(g.np, n);
   p.cb = (float)codebook_scale();
+  p.plan = nullptr;
   p.npeer = npeer;
   p.peer_offset = peer_offset;
   for (int i = 0; i < 8; ++i) p.peer_y[i] = i < npeer ? peer_y[i] : nullptr;
   int e = run_rht_f16(x, dtype, M, g.np, n, n, planes, su, reinterpret_cast<__half*>(ws + g.off_xb), reinterpret_cast<float*>(ws + g.off_xsum),
                       reinterpret_cast<float*>(ws + g.off_tok), st);
   if (e) { t_gemm_cuda = e; return HTR_ERR_CUDA; }
-  switch (K) {
-    case 2: e = launch_packed_gemm_tc<2>(p, g.grid, g.smem, st); break;
-    case 3: e = launch_packed_gemm_tc<3>(p, g.grid, g.smem, st); break;
-    case 4: e = launch_packed_gemm_tc<4>(p, g.grid, g.smem, st); break;
-    case 5: e = launch_packed_gemm_tc<5>(p, g.grid, g.smem, st); break;
-    case 6: e = launch_packed_gemm_tc<6>(p, g.grid, g.smem, st); break;
-    case 8: e = launch_packed_gemm_tc<8>(p, g.grid, g.smem, st); break;
-  }
+  e = launch_gemm(K, p, g.grid, g.smem, st);
+  if (e) t_gemm_cuda = e;
+  return e ? HTR_ERR_CUDA : HTR_OK;
+}
+
+// ---- grouped form: the experts of a mixture-of-experts step
+static int group_cap(int count, int table_rows) {
+  const int most = table_rows + count / kGroupRows;          // every expert may end in a part tile
+  return count < most ? count : most;
+}
+
+struct GroupLayout {
+  int cap, stages, smem, grid;
+  size_t off_xb, off_xsum, off_tok, off_part, total;
+};
+
+static int group_layout(int count, int table_rows, int m, int n, int K, GroupLayout* g) {
+  if (count < 1 || count > 4096 || table_rows < 1 || table_rows + count > 12288 || n > kGroupRhtWarps * kGroupRhtBlocks * 128) return HTR_ERR_TOO_LARGE;
+  g->cap = group_cap(count, table_rows);
+  if (g->cap > kGroupMaxTiles || (long long)g->cap * (m / 128) > (int)(kCounterRegion / 4) || (long long)g->cap * (m / 128) * (n / 128) > 0x3FFFFFFF)
+    return HTR_ERR_TOO_LARGE;
+  GemmPlan plan;                                             // stages, shared memory and thread blocks of a launch with these columns
+  const int rc = make_gemm_plan(kGroupRows, m, n, K, 2, &plan);
+  if (rc != HTR_OK) return rc;
+  g->stages = plan.stages;
+  g->smem = plan.smem;
+  g->grid = plan.sms;
+  size_t off = kCounterRegion + kErrorRegion;
+  g->off_xb = off; off += align256((size_t)g->cap * n * (2 * kGroupRows) * 2);
+  g->off_xsum = off; off += align256((size_t)g->cap * kGroupRows * 4);
+  g->off_tok = off; off += align256((size_t)g->cap * kGroupRows * 4);
+  g->off_part = off; off += align256((size_t)g->grid * 2 * kGroupRows * 128 * 4);
+  g->total = off;
+  return HTR_OK;
+}
+
+size_t htr_route_plan_bytes(int count, int table_rows) {
+  if (count < 1 || count > 4096 || table_rows < 1 || table_rows + count > 12288) return 0;
+  return align256(((size_t)group_plan_ints(group_cap(count, table_rows)) + count) * sizeof(int));
+}
+
+int htr_route_plan(const int64_t* route, int count, int table_rows, const void* const* qweight_table, void* plan, size_t plan_bytes,
+                   htr_stream_t stream) {
+  const size_t need = htr_route_plan_bytes(count, table_rows);
+  if (need == 0) return HTR_ERR_TOO_LARGE;
+  if (!route || !qweight_table || !plan) return HTR_ERR_NULL;
+  if (plan_bytes < need) return HTR_ERR_WORKSPACE;
+  const int e = launch_chained(route_plan_kernel, dim3(1), kPlanThreads, (size_t)(table_rows + count) * sizeof(int), static_cast<cudaStream_t>(stream),
+                               reinterpret_cast<const long long*>(route), count, table_rows, reinterpret_cast<const uint32_t* const*>(qweight_table),
+                               static_cast<int*>(plan), group_cap(count, table_rows));
+  if (e) { t_gemm_cuda = e; return HTR_ERR_CUDA; }
+  return HTR_OK;
+}
+
+size_t htr_linear_routed_gemm_workspace_bytes(int count, int table_rows, int m, int n, int K) {
+  if (!width_ok(K) || m <= 0 || n <= 0 || m % 128 || n % 128) return 0;
+  GroupLayout g;
+  return group_layout(count, table_rows, m, n, K, &g) == HTR_OK ? g.total : 0;
+}
+
+int htr_linear_routed_gemm(const void* x, int dtype, int x_div, int64_t x_row_stride, const void* plan, int count, int table_rows,
+                           const void* const* qweight_table, const void* const* scales_table, const uint8_t* const* su_table,
+                           const uint8_t* const* sv_table, int mt, int nt, int K, void* y, int prologue, void* workspace, size_t workspace_bytes,
+                           htr_stream_t stream) {
+  if (!width_ok(K)) return HTR_ERR_BAD_K;
+  if (dtype < HTR_DTYPE_BF16 || dtype > HTR_DTYPE_F32) return HTR_ERR_BAD_DTYPE;
+  if (prologue == HTR_PROLOGUE_SWIGLU && dtype != HTR_DTYPE_BF16) return HTR_ERR_BAD_DTYPE;
+  if (x_div < 1 || x_row_stride < 0 || x_row_stride % 4 || mt <= 0 || nt <= 0 || mt % 8 || nt % 8 || (prologue != HTR_PROLOGUE_NONE && prologue != HTR_PROLOGUE_SWIGLU))
+    return HTR_ERR_BAD_SHAPE;
+  if (!x || !y || !plan || !qweight_table || !scales_table || !su_table || !sv_table) return HTR_ERR_NULL;
+  const auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  if (!a16(x) || !a16(y) || !a16(workspace) || !a16(plan)) return HTR_ERR_ALIGNMENT;
+  const int m = mt * 16, n = nt * 16;
+  GroupLayout g;
+  const int rc = group_layout(count, table_rows, m, n, K, &g);
+  if (rc != HTR_OK) return rc;
+  if (!workspace || workspace_bytes < g.total) return HTR_ERR_WORKSPACE;
+  char* ws = static_cast<char*>(workspace);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  __half* xb = reinterpret_cast<__half*>(ws + g.off_xb);
+  float *xsum = reinterpret_cast<float*>(ws + g.off_xsum), *tok = reinterpret_cast<float*>(ws + g.off_tok);
+  const int* pl = static_cast<const int*>(plan);
+  int e = prologue == HTR_PROLOGUE_SWIGLU
+              ? launch_chained(rht_group_kernel<true>, dim3(count), kGroupRhtWarps * 32, 0, st, x, dtype, x_div, (long long)x_row_stride, n, pl, g.cap, su_table, xb, xsum, tok)
+              : launch_chained(rht_group_kernel<false>, dim3(count), kGroupRhtWarps * 32, 0, st, x, dtype, x_div, (long long)x_row_stride, n, pl, g.cap, su_table, xb, xsum, tok);
+  if (e) { t_gemm_cuda = e; return HTR_ERR_CUDA; }
+  GemmParams p = {};
+  p.y = y;
+  p.xb = xb;
+  p.xsum = xsum;
+  p.tok = tok;
+  p.part = reinterpret_cast<float*>(ws + g.off_part);
+  p.counters = reinterpret_cast<int*>(ws);
+  p.error = reinterpret_cast<int*>(ws + kCounterRegion);
+  p.rows = p.np = kGroupRows;
+  p.planes = 2;
+  p.mt = mt;
+  p.nt = nt;
+  p.m_out = m;
+  p.dtype = dtype;
+  p.hb = n / 128;
+  p.stages = g.stages;
+  p.xsum_slices = 1;
+  p.cb = (float)codebook_scale();
+  p.plan = pl;
+  p.tile_cap = g.cap;
+  p.rb_per_tile = m / 128;
+  p.g_qw = reinterpret_cast<const uint32_t* const*>(qweight_table);
+  p.g_scales = reinterpret_cast<const __half* const*>(scales_table);
+  p.g_sv = sv_table;
+  e = launch_gemm(K, p, g.grid, g.smem, st);
   if (e) t_gemm_cuda = e;
   return e ? HTR_ERR_CUDA : HTR_OK;
 }

@@ -84,12 +84,29 @@ struct GemmParams {
   int stages;
   int xsum_slices;
   float cb;
+  // Grouped form (GROUP instantiations: the experts of a mixture-of-experts step): the problems are the tiles of a device-side plan
+  // (route_plan_kernel in gemm_api.cu), each an expert and up to kGroupRows (token, slot) pairs; row blocks are numbered tile-major,
+  // xb holds one B operand per tile, xsum / tok kGroupRows entries per tile, and activation row j of tile t is output row pair(t, j).
+  const int* plan;
+  int tile_cap;           // tiles the plan has room for
+  int rb_per_tile;
+  const uint32_t* const* g_qw;
+  const __half* const* g_scales;
+  const uint8_t* const* g_sv;
   // row-shard form: the output rows go, with plain peer stores, to element offset peer_offset + j * m + row of every buffer in
   // peer_y (the gather buffers of all ranks of an NVLink box as mapped into this process) instead of y
   void* peer_y[8];
   int npeer;
   long long peer_offset;
 };
+
+// layout of the plan (ints): tile count, three spare, then per tile the expert, the number of pairs, and kGroupRows pair numbers
+constexpr int kGroupRows = 16, kGroupMaxTiles = 512;
+__host__ __device__ inline int group_plan_ints(int cap) { return 4 + cap * (2 + kGroupRows); }
+__device__ __forceinline__ int group_tiles(const int* plan) { return __ldcg(plan); }
+__device__ __forceinline__ int group_expert(const int* plan, int, int t) { return __ldcg(plan + 4 + t); }
+__device__ __forceinline__ int group_count(const int* plan, int cap, int t) { return __ldcg(plan + 4 + cap + t); }
+__device__ __forceinline__ const int* group_pairs(const int* plan, int cap, int t) { return plan + 4 + 2 * cap + t * kGroupRows; }
 
 __device__ __forceinline__ void gemm_store_rows(const GemmParams& p, int j, int row0, float4 o) {
   if (p.npeer == 0) {
@@ -270,13 +287,31 @@ struct GemmTail {
   float s[4];                                               // row scales
   unsigned sv_bits;
   float4 bias;
-  int row0;
-  __device__ __forceinline__ GemmTail(const GemmParams& p, int rb, int lane) {
+  int row0;                                                 // row of this problem's weight
+  int rows;                                                 // activation rows
+  int base;                                                 // of its entries of xsum and tok
+  const int* pairs;                                         // grouped form: output row of every activation row
+  template <bool GROUP>
+  __device__ __forceinline__ void load(const GemmParams& p, int rb, int lane) {
+    const __half* scales = p.scales;
+    const uint8_t* sv = p.sv;
+    rows = p.rows;
+    base = 0;
+    pairs = nullptr;
+    if constexpr (GROUP) {
+      const int t = rb / p.rb_per_tile, e = group_expert(p.plan, p.tile_cap, t);
+      rb -= t * p.rb_per_tile;
+      scales = p.g_scales[e];
+      sv = p.g_sv[e];
+      rows = group_count(p.plan, p.tile_cap, t);
+      base = t * kGroupRows;
+      pairs = group_pairs(p.plan, p.tile_cap, t);
+    }
     row0 = rb * 128 + 4 * lane;
-    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(p.scales + row0));
+    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(scales + row0));
     const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
     s[0] = s01.x; s[1] = s01.y; s[2] = s23.x; s[3] = s23.y;
-    sv_bits = sign_nibble(p.sv, rb * 32 + lane);
+    sv_bits = sign_nibble(sv, rb * 32 + lane);
     bias = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p.bias && row0 < p.m_out) bias = load_quad(p.bias, row0, p.dtype);
   }
@@ -293,8 +328,9 @@ __device__ __forceinline__ void gemm_finish_row(const GemmParams& p, const GemmT
   const float off = 1534.0f * xs, rs = p.cb * tok;
   float v[4] = {(r4.x - off) * (t.s[0] * rs), (r4.y - off) * (t.s[1] * rs), (r4.z - off) * (t.s[2] * rs), (r4.w - off) * (t.s[3] * rs)};
   wht128(v, lane);
-  gemm_store_rows(p, j, t.row0, make_float4(flip(v[0] * kInvSqrt128, t.sv_bits & 1u) + t.bias.x, flip(v[1] * kInvSqrt128, (t.sv_bits >> 1) & 1u) + t.bias.y,
-                                            flip(v[2] * kInvSqrt128, (t.sv_bits >> 2) & 1u) + t.bias.z, flip(v[3] * kInvSqrt128, t.sv_bits >> 3) + t.bias.w));
+  gemm_store_rows(p, t.pairs ? __ldcg(t.pairs + j) : j, t.row0,
+                  make_float4(flip(v[0] * kInvSqrt128, t.sv_bits & 1u) + t.bias.x, flip(v[1] * kInvSqrt128, (t.sv_bits >> 1) & 1u) + t.bias.y,
+                              flip(v[2] * kInvSqrt128, (t.sv_bits >> 2) & 1u) + t.bias.z, flip(v[3] * kInvSqrt128, t.sv_bits >> 3) + t.bias.w));
 }
 
 // flat form: even runs of 128-column blocks, the first `rem` thread blocks hold one more
@@ -307,13 +343,16 @@ struct GemmRuns {
 
 // rows j0, j0 + step, ... of row block rb from the partial sums of thread blocks first .. first + contributors - 1, added in that
 // order.  Two rows at a time: the loads of both are in flight together.  head: which partial of thread block `first`.
+template <bool GROUP>
 __device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, int first, int contributors, int head, int j0, int step, int lane) {
-  const GemmTail tail(p, rb, lane);
+  GemmTail tail;
+  tail.load<GROUP>(p, rb, lane);
   const float4* slot0 = reinterpret_cast<const float4*>(p.part + (size_t)(2 * first) * ((size_t)p.np * 128)) + lane;
   const size_t stride = (size_t)p.np * 32;
-  for (int j = j0; j < p.rows; j += 2 * step) {
-    const int jb = j + step < p.rows ? j + step : j;
-    const float xa = gemm_xsum_share(p, j, lane), xb = gemm_xsum_share(p, jb, lane), ta = __ldcg(p.tok + j), tb = __ldcg(p.tok + jb);
+  for (int j = j0; j < tail.rows; j += 2 * step) {
+    const int jb = j + step < tail.rows ? j + step : j;
+    const float xa = gemm_xsum_share(p, tail.base + j, lane), xb = gemm_xsum_share(p, tail.base + jb, lane);
+    const float ta = __ldcg(p.tok + tail.base + j), tb = __ldcg(p.tok + tail.base + jb);
     float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb4 = ra;
     for (int base = 0; base < contributors; base += 4) {
       float4 va[4], vb[4];
@@ -335,7 +374,7 @@ __device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, in
   }
 }
 
-template <int K>
+template <int K, bool GROUP>
 __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const GemmParams p) {
   extern __shared__ __align__(128) unsigned char gsm[];
   __shared__ __align__(8) unsigned long long s_full[kGemmMaxStages], s_freed[kGemmMaxStages], s_done, s_drained;
@@ -349,10 +388,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int np = p.np, ncols = p.planes * np;               // accumulator columns: hi plane, then lo plane if present
   const int nt = p.nt, HB = p.hb, NS = p.stages;
-  const int U = (p.mt >> 3) * HB;
+  int tiles = 1;
+  if constexpr (GROUP) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // the plan comes from an earlier kernel
+    tiles = group_tiles(p.plan);
+  }
+  const int U = (GROUP ? tiles * p.rb_per_tile : p.mt >> 3) * HB;
   const GemmRuns runs(U, gridDim.x);
   int u_begin, u_end, part_id = 0;
-  if (p.split > 0) {
+  if (!GROUP && p.split > 0) {
     const int rb = blockIdx.x / p.split;
     part_id = blockIdx.x - rb * p.split;
     u_begin = rb * HB + part_id * HB / p.split;
@@ -361,6 +405,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     u_begin = runs.begin(blockIdx.x);
     u_end = runs.begin(blockIdx.x + 1);
   }
+  if (GROUP && u_begin == u_end) return;                    // fewer blocks than thread blocks (an empty plan among others)
   const int b_tile_bytes = ncols * 256;
   unsigned char* ring = gsm + (128 - (smem_u32(gsm) & 127)) % 128;
   const uint32_t ring_addr = smem_u32(ring);
@@ -382,7 +427,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"((uint32_t)kGemmTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (warp == kGemmWarps - 1 && lane < 6) {
+  __shared__ const uint32_t* s_qw[GROUP ? kGroupMaxTiles : 1];   // packed words of every tile's expert
+  if constexpr (GROUP) {
+    for (int t = tid; t < tiles; t += kGemmThreads) s_qw[t] = p.g_qw[group_expert(p.plan, p.tile_cap, t)];
+    __syncthreads();
+  }
+  if (!GROUP && warp == kGemmWarps - 1 && lane < 6) {
     // the row scales and signs of the first and the last row block are needed at the very end, in a chain of dependent loads:
     // bring them to L2 now (256 bytes of scales and 16 of signs per row block)
     const size_t rb = lane & 1 ? (u_end - 1) / HB : u_begin / HB;
@@ -406,11 +456,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     }
     // from the end of a strip's row to the same strip of the next row block (a row of one block is left twice per step of two)
     const size_t next_strip = (size_t)7 * nt * (32 * K) * (HB == 1 ? 2 : 1);
-    int pf_left = u_end - u_begin - group, pf_in_rb;
+    int pf_left = u_end - u_begin - group, pf_in_rb, pf_rb;
     const char* pf;
+    auto strip_row = [&](int rb) {                          // this lane's first chunk of this warp's strip of row block rb
+      const uint32_t* base = p.qw;
+      if constexpr (GROUP) {
+        const int t = min(rb / p.rb_per_tile, tiles - 1);    // (past the last tile nothing is copied any more)
+        rb -= t * p.rb_per_tile;
+        base = s_qw[t];
+      }
+      return reinterpret_cast<const char*>(base) + (size_t)(rb * 8 + strip) * nt * (32 * K) + lane * 16;
+    };
     {
-      const int u = u_begin + group, rb = u / HB, hb = u - rb * HB;
-      pf = reinterpret_cast<const char*>(p.qw) + ((size_t)(rb * 8 + strip) * nt + (size_t)hb * 8) * (32 * K) + lane * 16;
+      const int u = u_begin + group, hb = u % HB;
+      pf_rb = u / HB;
+      pf = strip_row(pf_rb) + (size_t)hb * (256 * K);
       pf_in_rb = HB - hb;
     }
     auto fetch = [&](uint32_t at) {
@@ -422,9 +482,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
                      : "memory");
       }
       pf_left -= 2;
-      const bool wrap = pf_in_rb <= 2;
-      pf_in_rb += wrap ? HB - 2 : -2;
-      pf += wrap ? next_strip + 512 * K : (size_t)(512 * K);
+      if constexpr (GROUP) {
+        pf += 512 * K;
+        pf_in_rb -= 2;
+        if (pf_in_rb <= 0) {
+          while (pf_in_rb <= 0) { pf_in_rb += HB; ++pf_rb; }
+          pf = strip_row(pf_rb) + (size_t)(HB - pf_in_rb) * (256 * K);
+        }
+      } else {
+        const bool wrap = pf_in_rb <= 2;
+        pf_in_rb += wrap ? HB - 2 : -2;
+        pf += wrap ? next_strip + 512 * K : (size_t)(512 * K);
+      }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
@@ -476,14 +545,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       if (elect_one()) {
         asm volatile("griddepcontrol.wait;" ::: "memory");  // the transformed activations come from the preceding kernel
         int s = 0, issued = 0, hb = u_begin % HB;
+        int rb_left = GROUP ? p.rb_per_tile - (u_begin / HB) % p.rb_per_tile : 0;   // row blocks of this tile still to come, this one included
+        const char* xb = reinterpret_cast<const char*>(p.xb);
+        if constexpr (GROUP) xb += (size_t)(u_begin / HB / p.rb_per_tile) * HB * b_tile_bytes;
         uint32_t use = 0u;
         for (int u = u_begin; u < u_end; ++u) {
           if (use > 0 && !mbar_wait(smem_u32(&s_freed[s]), (use - 1u) & 1u, &s_fail, kSleepNs)) { s_fail = 1; break; }
           const uint32_t bar = smem_u32(&s_full[s]);
           mbar_expect_tx(bar, (uint32_t)b_tile_bytes);
-          bulk_load(ring_addr + s * b_tile_bytes, reinterpret_cast<const char*>(p.xb) + (size_t)hb * b_tile_bytes, (uint32_t)b_tile_bytes, bar);
+          bulk_load(ring_addr + s * b_tile_bytes, xb + (size_t)hb * b_tile_bytes, (uint32_t)b_tile_bytes, bar);
           ++issued;
-          if (++hb == HB) hb = 0;
+          if (++hb == HB) {
+            hb = 0;
+            if (GROUP && --rb_left == 0) {
+              rb_left = p.rb_per_tile;
+              xb += (size_t)HB * b_tile_bytes;
+            }
+          }
           if (++s == NS) { s = 0; ++use; }
         }
         if (s_fail) {
@@ -552,7 +630,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         }
         // accumulator -> partial [np][128], hi + lo added here.  A thread block has two partials: its first row block's, which other
         // thread blocks may read, and one for all later ones (of which only the last is read by others)
-        float* mine = p.split > 0 ? reinterpret_cast<float*>(ring) : p.part + (size_t)(2 * blockIdx.x + (seg > 0 ? 1 : 0)) * ((size_t)np * 128);
+        float* mine = !GROUP && p.split > 0 ? reinterpret_cast<float*>(ring) : p.part + (size_t)(2 * blockIdx.x + (seg > 0 ? 1 : 0)) * ((size_t)np * 128);
         for (int j0 = 0; j0 < np; j0 += 8) {
           uint32_t hi[8], lo[8];
           tmem_load8(acc_addr + j0, hi);
@@ -561,14 +639,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float v = p.planes == 2 ? __uint_as_float(hi[j]) + __uint_as_float(lo[j]) : __uint_as_float(hi[j]);
-            if (p.split > 0) mine[(j0 + j) * 128 + row] = v;
+            if (!GROUP && p.split > 0) mine[(j0 + j) * 128 + row] = v;
             else __stcg(mine + (j0 + j) * 128 + row, v);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&s_drained));    // the MMAs of the next row block may start
-        if (p.split > 0 || stop >= u_end) break;             // the last row block: all warps finish it, below
+        if ((!GROUP && p.split > 0) || stop >= u_end) break;             // the last row block: all warps finish it, below
         // only the run's first row block can have other contributors here, thread blocks before this one
         const int first = runs.owner(rb * HB), contributors = blockIdx.x - first + 1;
         bool finish = true;
@@ -582,7 +660,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
           finish = s_arrival == contributors - 1;
           if (finish && fw == 0 && lane == 0) p.counters[rb] = 0;
         }
-        if (finish) gemm_finish_flat(p, rb, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, fw, kGemmFinishWarps, lane);
+        if (finish) gemm_finish_flat<GROUP>(p, rb, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, fw, kGemmFinishWarps, lane);
         __syncwarp();
         if (lane == 0) s_owed[fw] = rb + 1;
         finishers_all(true);                                 // the partial has been read by all of them: it may be written again
@@ -596,7 +674,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   const bool bad = s_fail != 0;
   if (bad && tid == 0) atomicCAS(p.error, 0, 1);
 
-  if (p.split > 0) {
+  if (!GROUP && p.split > 0) {
     // ---- split reduction inside the cluster: every thread block keeps its partial [np][128] where it is; thread block r of the
     // cluster sums rows r, r + split, ... over all of them (in rank order) and finishes those rows itself
     float* result = reinterpret_cast<float*>(ring);
@@ -605,7 +683,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");      // (done before by the roles that needed it)
-    const GemmTail tail(p, blockIdx.x / p.split, lane);
+    GemmTail tail;
+    tail.load<false>(p, blockIdx.x / p.split, lane);
     const uint32_t result_addr = smem_u32(result);
     for (int j = part_id + p.split * warp; j < p.rows; j += p.split * kGemmWarps) {
       const float xs = gemm_xsum_share(p, j, lane), tok = __ldcg(p.tok + j);
@@ -635,12 +714,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       finish = s_arrival == contributors - 1;
       if (finish && tid == 0) p.counters[rb] = 0;
     }
-    if (finish) gemm_finish_flat(p, rb, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, warp, kGemmWarps, lane);
+    if (finish) gemm_finish_flat<GROUP>(p, rb, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, warp, kGemmWarps, lane);
     if (bad) {
       // the row blocks this thread block still owed never complete (nobody arrives for them): their rows come out as NaN
       const float nan = __uint_as_float(0x7FC00000u);
-      for (int b = min(min(s_owed[0], s_owed[1]), min(s_owed[2], s_owed[3])); b <= rb; ++b)
-        for (int j = warp; j < p.rows; j += kGemmWarps) gemm_store_rows(p, j, b * 128 + 4 * lane, make_float4(nan, nan, nan, nan));
+      for (int b = min(min(s_owed[0], s_owed[1]), min(s_owed[2], s_owed[3])); b <= rb; ++b) {
+        GemmTail tail;
+        tail.load<GROUP>(p, b, lane);
+        for (int j = warp; j < tail.rows; j += kGemmWarps) gemm_store_rows(p, tail.pairs ? tail.pairs[j] : j, tail.row0, make_float4(nan, nan, nan, nan));
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -652,7 +734,7 @@ int gemm_rht_slices(int np, int n);
 int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
                 cudaStream_t st);
 template <int K>
-int launch_packed_gemm_tc(const GemmParams& p, int grid, int smem, cudaStream_t st);
+int launch_packed_gemm_tc(const GemmParams& p, int grid, int smem, cudaStream_t st);   // p.plan set: the grouped form
 // clusters of `split` thread blocks that the GPU holds at once (0: none), for the cluster form of the plan
 template <int K>
 int packed_gemm_tc_clusters(int smem, int split);

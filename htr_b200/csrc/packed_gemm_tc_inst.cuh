@@ -12,8 +12,10 @@ namespace {
 int allow_smem(int dev) {
   static bool allowed[64] = {false};
   if (dev >= 0 && dev < 64 && allowed[dev]) return 0;
-  const cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+  const cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
   if (e != cudaSuccess) return (int)e;
+  const cudaError_t e2 = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  if (e2 != cudaSuccess) return (int)e2;
   if (dev >= 0 && dev < 64) allowed[dev] = true;
   return 0;
 }
@@ -44,7 +46,7 @@ int packed_gemm_tc_clusters<HTR_INST_K>(int smem, int split) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&clusters, packed_gemm_tc_kernel<HTR_INST_K>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, packed_gemm_tc_kernel<HTR_INST_K, false>, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
       clusters = 0;
     }
@@ -79,7 +81,7 @@ int launch_packed_gemm_tc<HTR_INST_K>(const GemmParams& p, int grid, int smem, c
   }
   GemmParams q = p;
   void* args[1] = {&q};
-  return (int)cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(packed_gemm_tc_kernel<HTR_INST_K>), args);
+  return (int)cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(p.plan ? packed_gemm_tc_kernel<HTR_INST_K, true> : packed_gemm_tc_kernel<HTR_INST_K, false>), args);
 }
 
 }  // namespace htr

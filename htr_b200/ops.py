@@ -183,6 +183,17 @@ def linear_fused(x2, qweight, scales, su, sv, out=None, prologue=PROLOGUE_NONE, 
 _GEMM_WS = {}
 
 
+def _gemm_workspace(device, st, need):
+    """Scratch of the tensor-core GEMM, one per (device, stream), as `workspace` is for the GEMV."""
+    key = (device.index, st)
+    ws = _GEMM_WS.get(key)
+    if ws is None or ws.numel() < need:
+        ws = torch.zeros(max(need, 1 << 24), dtype=torch.uint8, device=device)
+        _GEMM_WS[key] = ws
+        _host.set_workspace(1, *key, ws)
+    return ws
+
+
 def _gemm(x2, qweight, scales, su, sv, bias, out, peer_ptrs=None, elem_offset=0):
     """One C call of the tensor-core GEMM: up to 256 rows of x2 (128 for float32) against the packed weight.  With peer_ptrs the
     rows go to element offset `elem_offset` of every buffer in the list instead of `out` (htr_linear_gemm_peers)."""
@@ -193,12 +204,7 @@ def _gemm(x2, qweight, scales, su, sv, bias, out, peer_ptrs=None, elem_offset=0)
     if need == 0:
         raise _lib.HTRError("htr_linear_gemm: unsupported sizes")
     st = torch.cuda.current_stream(x2.device).cuda_stream
-    key = (x2.device.index, st)
-    ws = _GEMM_WS.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(max(need, 1 << 24), dtype=torch.uint8, device=x2.device)
-        _GEMM_WS[key] = ws
-        _host.set_workspace(1, *key, ws)
+    ws = _gemm_workspace(x2.device, st, need)
     if peer_ptrs is None:
         rc = _lib.lib.htr_linear_gemm(x2.data_ptr(), _DTYPES[x2.dtype], M, qweight.data_ptr(), mt, nt, K, scales.data_ptr(), su.data_ptr(),
                                       sv.data_ptr(), None if bias is None else bias.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), st)
@@ -322,6 +328,39 @@ def linear_routed(x, route, tables, mt, nt, K, x_div=1, prologue=PROLOGUE_NONE, 
                                                   tables[3].data_ptr(), mt, nt, K, out.data_ptr(), host if peers else None, len(peers),
                                                   int(share), int(prologue), ws.data_ptr(), ws.numel(), st)
         _lib.check(rc, "htr_linear_routed")
+    return out
+
+
+def route_plan(route, tables):
+    """The pairs of a mixture-of-experts step sorted by expert (htr_route_plan), for `linear_routed_gemm`; None where the sizes are
+    beyond the grouped GEMM."""
+    count, rows, dev = route.numel(), int(tables[0].numel()), route.device
+    need = _lib.lib.htr_route_plan_bytes(count, rows)
+    if need == 0:
+        return None
+    plan = torch.empty(need, dtype=torch.uint8, device=dev)
+    with torch.cuda.device(dev):
+        rc = _lib.lib.htr_route_plan(route.data_ptr(), count, rows, tables[0].data_ptr(), plan.data_ptr(), need, torch.cuda.current_stream(dev).cuda_stream)
+    _lib.check(rc, "htr_route_plan")
+    return plan
+
+
+def linear_routed_gemm(x, plan, count, tables, mt, nt, K, x_div=1, prologue=PROLOGUE_NONE, out=None):
+    """`linear_routed` for steps in which pairs share experts: `plan` (from `route_plan`) in place of the route, each expert's weights
+    decoded once per 16 of its pairs on the tensor cores.  Returns None where the sizes are beyond the grouped GEMM."""
+    dev, rows = x.device, int(tables[0].numel())
+    need = _lib.lib.htr_linear_routed_gemm_workspace_bytes(count, rows, mt * 16, nt * 16, K)
+    if need == 0:
+        return None
+    if out is None:
+        out = torch.empty((count, mt * 16), dtype=x.dtype, device=dev)
+    with torch.cuda.device(dev):
+        st = torch.cuda.current_stream(dev).cuda_stream
+        ws = _gemm_workspace(dev, st, need)
+        rc = _lib.lib.htr_linear_routed_gemm(x.data_ptr(), _DTYPES[x.dtype], int(x_div), x.shape[1], plan.data_ptr(), count, rows, tables[0].data_ptr(),
+                                             tables[1].data_ptr(), tables[2].data_ptr(), tables[3].data_ptr(), mt, nt, K, out.data_ptr(), int(prologue),
+                                             ws.data_ptr(), ws.numel(), st)
+    _lib.check(rc, "htr_linear_routed_gemm")
     return out
 
 

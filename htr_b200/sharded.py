@@ -29,6 +29,18 @@ import torch.distributed as dist
 PEER_ORDER = "kernel"
 
 
+# On one GPU the grouped GEMM decodes an expert's weights once for the pairs that share it, the routed GEMV once per pair.  Both
+# decode 4.2 to 4.5e12 weights a second (float32 activations stay on the GEMV, whose sums carry 24 bits), the GEMM's three extra launches and its reductions cost about 20 us: it wins from this many
+# weights saved on (64 experts of 4096 x 1536, top 8: from 4 tokens; 16 experts of 2048 x 1024, top 4: from 8 tokens).
+GROUPED_GEMM_MIN_SAVED = 90_000_000
+
+
+def grouped_gemm_pays(pairs, experts, weights_per_expert):
+    """Whether `pairs` (token, slot) pairs over `experts` experts are expected to share them enough for the grouped GEMM."""
+    met = experts * (1.0 - (1.0 - 1.0 / experts) ** pairs)
+    return (pairs - met) * weights_per_expert >= GROUPED_GEMM_MIN_SAVED
+
+
 def row_block_partition(m, world):
     """Split m/128 row blocks into `world` contiguous runs of equal padded length.
     Returns (blocks_per_rank, [(first_block, real_blocks), ...]).  151936 rows = 1187 blocks over 8 ranks -> 149 per rank,
@@ -354,6 +366,17 @@ class ExpertParallelMoE:
         mt_dn, nt_dn, _ = any_e["down"][0].shape
         K = W // 8
         x = x.contiguous()
+        if self.world == 1 and x.is_cuda and x.dtype != torch.float32 and grouped_gemm_pays(T * k, self.num_experts, 256 * (mt_gu * nt_gu + mt_dn * nt_dn)):
+            plan = ops.route_plan(route, tabs["gate_up"])
+            gu = None if plan is None else ops.linear_routed_gemm(x, plan, T * k, tabs["gate_up"], mt_gu, nt_gu, K, x_div=k)
+            if gu is not None:
+                if x.dtype == torch.bfloat16:
+                    act, prologue = gu, ops.PROLOGUE_SWIGLU
+                else:
+                    act, prologue = (torch.nn.functional.silu(gu[:, :mt_gu * 8]) * gu[:, mt_gu * 8:]).contiguous(), ops.PROLOGUE_NONE
+                dn = ops.linear_routed_gemm(act, plan, T * k, tabs["down"], mt_dn, nt_dn, K, prologue=prologue)
+                if dn is not None:
+                    return dn
         skip = self.world > 1 and not exchange                          # rows of skipped pairs must read as zero
         alloc = torch.zeros if skip else torch.empty
         # (with `exchange`, the gate_up rows of pairs owned elsewhere are never read: the down launch skips the same pairs)

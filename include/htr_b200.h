@@ -188,6 +188,21 @@ int htr_linear_routed_peers(const void* x, int dtype, int x_div, int64_t x_row_s
                             const uint8_t* const* sv_table, int mt, int nt, int K, void* y, void* const* peer_y, int npeer, int share,
                             int prologue, void* workspace, size_t workspace_bytes, htr_stream_t stream);
 
+/* Routed launches for steps in which several pairs share an expert: htr_route_plan sorts the pairs by expert on the device (one small
+ * kernel; tiles of up to 16 pairs of one expert), and htr_linear_routed_gemm decodes an expert's weights once per tile, on the
+ * tensor cores (activations as two fp16 planes, float32 sums), where htr_linear_routed decodes them once per pair.  Arguments and result
+ * as for htr_linear_routed, with the plan in place of the route; the plan serves every launch of the step whose tables have the
+ * same rows.  Limits: 4096 pairs, table_rows + pairs/16 <= 512 tiles (or fewer pairs than that), n <= 16384, tiles * m/128 <= 16384;
+ * beyond them the workspace function returns 0 and the launches HTR_ERR_TOO_LARGE.  The workspace is one of htr_linear_gemm's. */
+size_t htr_route_plan_bytes(int count, int table_rows);
+int htr_route_plan(const int64_t* route, int count, int table_rows, const void* const* qweight_table, void* plan, size_t plan_bytes,
+                   htr_stream_t stream);
+size_t htr_linear_routed_gemm_workspace_bytes(int count, int table_rows, int m, int n, int K);
+int htr_linear_routed_gemm(const void* x, int dtype, int x_div, int64_t x_row_stride, const void* plan, int count, int table_rows,
+                           const void* const* qweight_table, const void* const* scales_table, const uint8_t* const* su_table,
+                           const uint8_t* const* sv_table, int mt, int nt, int K, void* y, int prologue, void* workspace,
+                           size_t workspace_bytes, htr_stream_t stream);
+
 /* Padded form (the reference's HTRHCLinearMethod.apply, htr/vllm_plugin.py:313-326: F.pad of the input to n_pad, slice of
  * the output to m_out, both as separate copies there): the stored tensors cover a padded [m = 16*mt, n = 16*nt] matrix, x has
  * only n_in <= n columns per row (row stride n_in; the missing columns count as zeros) and y receives only the first
