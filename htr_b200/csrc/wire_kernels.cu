@@ -52,61 +52,150 @@ __global__ void __launch_bounds__(256) rht_kernel(const void* __restrict__ x, in
 }
 
 // ------------------------------------------------------------------------------------------------
-// W block (128 x 128) = sv * Ho Q Hi * su.  One CTA per block: decode into shared memory, transform down
-// the columns, then along the rows, apply the signs and write.
-constexpr int kDqLd = 129;  // padded leading dimension: conflict-free for both transform directions
+// W block (128 x 128) = sv * Ho Q Hi * su, one thread block of 128 threads per block: 14 butterfly stages and the decode per weight.
+// What bounds it: the 14 additions (the FMA pipes take 124 of them per cycle and SM: 20 us at 4096 x 12288), then the decode
+// (6 us); 100 MB of bf16 output take 15 us.  So every stage runs in registers, two elements per instruction where they are
+// independent, and the block crosses shared memory once:
+//   phase 1  thread = a row pair (q) of one strip x 64 columns (four tiles): 128 values, seven index bits in registers -- four
+//            column bits and two tile bits as packed pairs (row 2q, row 2q+1), then the row bit;
+//   phase 2  thread = columns c, c + 64 of the 64 rows of one parity: the six row bits as packed pairs (c, c + 64), then the last
+//            column bit, signs, cast, store.
+// The exchange buffer swaps 16-byte groups by row pair so that both sides are free of bank conflicts.  16-bit results change
+// hands with the neighbour lane so that a store carries two adjacent columns.
+// Measured at 4096 x 12288 K4, bf16: 54 us, where one value per shuffle and shared-memory access with scalar stores took 108; issue
+// slots 52 % busy, a quarter of the stalls are instruction fetches of the unrolled body.
+constexpr int kDqThreads = 128;
+constexpr int kDqSmem = 128 * 128 * 4;
 
-template <int K>
-__global__ void __launch_bounds__(256) dequant_w_kernel(const uint32_t* __restrict__ qw, const __half* __restrict__ scales,
-                                                        const uint8_t* __restrict__ su, const uint8_t* __restrict__ sv, float cb,
-                                                        void* __restrict__ W, int out_dtype, int nt) {
-  extern __shared__ float blk[];  // [128][kDqLd]
+__device__ __forceinline__ int dq_at(int row, int col) { return row * 128 + ((((col >> 2) ^ ((row >> 1) & 7)) << 2) | (col & 3)); }
+
+// butterflies over index bit BIT of N packed pairs
+template <int N, int BIT>
+__device__ __forceinline__ void dq_stage(float2 (&v)[N]) {
+  const float2 minus = make_float2(-1.f, -1.f);
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (!(i & (1 << BIT))) {
+      const float2 a = v[i], b = v[i | (1 << BIT)];
+      v[i] = __fadd2_rn(a, b);
+      v[i | (1 << BIT)] = __ffma2_rn(b, minus, a);           // a - b, exactly as rounded
+    }
+}
+
+template <int K, int OUT>
+__global__ void __launch_bounds__(kDqThreads, 3) dequant_w_kernel(const uint32_t* __restrict__ qw, const __half* __restrict__ scales,
+                                                                  const uint8_t* __restrict__ su, const uint8_t* __restrict__ sv, float cb,
+                                                                  void* __restrict__ W, int nt) {
+  extern __shared__ __align__(16) float blk[];               // [128][128], groups of four columns swapped by row pair
+  __shared__ __align__(16) uint32_t s_sign[128];             // sign mask of a row, rows of one parity together
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cbk = blockIdx.x, rb = blockIdx.y, n = nt * 16;
-
-  // decode: 64 tiles x 8 row pairs = 512 lane units, two per thread
-  for (int unit = tid; unit < 512; unit += 256) {
-    const int q = unit & 7, tl = unit >> 3, tr = tl >> 3, tc = tl & 7;  // tile (tr, tc) of the block
-    const uint32_t* words = qw + ((size_t)(rb * 8 + tr) * nt + (cbk * 8 + tc)) * (8 * K);
-    uint32_t V[K + 1];
-    V[0] = words[history_word<K>(q)];
+  s_sign[(tid & 1) * 64 + (tid >> 1)] = ((sv[rb * 16 + (tid >> 3)] >> (tid & 7)) & 1) ? 0x80008000u : 0u;
+  {
+    const int q = lane & 7, half = (lane >> 3) & 1, strip = 2 * warp + (lane >> 4);
+    const uint32_t* words = qw + ((size_t)(rb * 8 + strip) * nt + (size_t)(cbk * 8 + half * 4)) * (8 * K) + q * K;
+    uint32_t own[4][K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) V[k + 1] = words[q * K + k];
-    uint32_t s[32];
-    unit_states<K>(V, s);
+    for (int t = 0; t < 4; ++t) {
+      const uint32_t* w = words + t * (8 * K);
+      if constexpr (K % 4 == 0) {
 #pragma unroll
-    for (int u = 0; u < 32; ++u) {
-      const int row = tr * 16 + 2 * q + (u >> 4), col = tc * 16 + (u & 15);
-      blk[row * kDqLd + col] = (float)code_value(s[u]) * (__half2float(scales[rb * 128 + row]) * cb);
+        for (int i = 0; i < K / 4; ++i) {
+          const uint4 r = __ldg(reinterpret_cast<const uint4*>(w) + i);
+          own[t][4 * i] = r.x; own[t][4 * i + 1] = r.y; own[t][4 * i + 2] = r.z; own[t][4 * i + 3] = r.w;
+        }
+      } else if constexpr (K % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < K / 2; ++i) {
+          const uint2 r = __ldg(reinterpret_cast<const uint2*>(w) + i);
+          own[t][2 * i] = r.x; own[t][2 * i + 1] = r.y;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < K; ++i) own[t][i] = __ldg(w + i);
+      }
+    }
+    const int row = strip * 16 + 2 * q;
+    const float2 sc = make_float2(__half2float(scales[rb * 128 + row]), __half2float(scales[rb * 128 + row + 1]));
+    const float2 s2 = make_float2(sc.x * cb * (1.0f / 128.0f), sc.y * cb * (1.0f / 128.0f));
+    const float2 unbias = make_float2(-kMagic, -kMagic);
+    float2 v[64];                                            // [tile][column] of (row, row + 1)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      uint32_t V[K + 1], s[32];
+#pragma unroll
+      for (int i = 0; i < K; ++i) V[i + 1] = own[t][i];
+      V[0] = __shfl_sync(kFullWarp, own[t][K - 1], (lane & 24) | ((q - 1) & 7));   // last word of the row pair before
+      unit_states<K>(V, s);
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        v[t * 16 + u] = __fmul2_rn(__fadd2_rn(make_float2(__uint_as_float(code_magic_bits_alu(s[u])), __uint_as_float(code_magic_bits(s[16 + u]))), unbias), s2);
+    }
+    dq_stage<64, 0>(v);
+    dq_stage<64, 1>(v);
+    dq_stage<64, 2>(v);
+    dq_stage<64, 3>(v);
+    dq_stage<64, 4>(v);
+    dq_stage<64, 5>(v);
+#pragma unroll
+    for (int g = 0; g < 16; ++g) {
+      const float2 *p = v + 4 * g;
+      const int col = half * 64 + 4 * g;
+      *reinterpret_cast<float4*>(blk + dq_at(row, col)) = make_float4(p[0].x + p[0].y, p[1].x + p[1].y, p[2].x + p[2].y, p[3].x + p[3].y);
+      *reinterpret_cast<float4*>(blk + dq_at(row + 1, col)) = make_float4(p[0].x - p[0].y, p[1].x - p[1].y, p[2].x - p[2].y, p[3].x - p[3].y);
     }
   }
   __syncthreads();
-  // Hadamard over the 128 rows, column by column (htr/wire.py:111): lane holds rows lane + 32k
-  for (int col = warp; col < 128; col += 8) {
-    float v[4];
+  const int parity = warp >> 1, c = (warp & 1) * 32 + lane;
+  float2 v[64];                                              // row 2i + parity, columns (c, c + 64)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = blk[(lane + 32 * k) * kDqLd + col];
-    wht128(v, lane);
+  for (int i = 0; i < 64; ++i) v[i] = make_float2(blk[dq_at(2 * i + parity, c)], blk[dq_at(2 * i + parity, c + 64)]);
+  dq_stage<64, 0>(v);
+  dq_stage<64, 1>(v);
+  dq_stage<64, 2>(v);
+  dq_stage<64, 3>(v);
+  dq_stage<64, 4>(v);
+  dq_stage<64, 5>(v);
+  const int gc = cbk * 128 + c;
+  const uint32_t su0 = (su[gc >> 3] >> (gc & 7)) & 1u, su1 = (su[(gc + 64) >> 3] >> (gc & 7)) & 1u;
+  const uint32_t* masks = s_sign + parity * 64;
+  const size_t row0 = (size_t)rb * 128 + parity;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) blk[(lane + 32 * k) * kDqLd + col] = v[k];
-  }
-  __syncthreads();
-  // Hadamard over the 128 columns of each row (htr/wire.py:112), signs (htr/wire.py:113), store
-  for (int row = warp; row < 128; row += 8) {
-    float v[4];
+  for (int i = 0; i < 64; i += 4) {
+    const uint4 m4 = *reinterpret_cast<const uint4*>(masks + i);
+    const uint32_t m[4] = {m4.x, m4.y, m4.z, m4.w};
+    if constexpr (OUT == HTR_DTYPE_F32) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = blk[row * kDqLd + lane + 32 * k];
-    wht128(v, lane);
-    const int gi = rb * 128 + row;
-    const float rs = sign_of(sv, gi) * (1.0f / 128.0f);
+      for (int k = 0; k < 4; ++k) {
+        const float2 a = v[i + k];
+        float* dst = static_cast<float*>(W) + (row0 + 2 * (i + k)) * n + gc;
+        dst[0] = __uint_as_float(__float_as_uint(a.x + a.y) ^ ((m[k] & 0x80000000u) ^ (su0 << 31)));
+        dst[64] = __uint_as_float(__float_as_uint(a.x - a.y) ^ ((m[k] & 0x80000000u) ^ (su1 << 31)));
+      }
+    } else {
+      const uint32_t flips = (su0 << 15) | (su1 << 31);
+      uint32_t w[4];                                         // columns c (low half) and c + 64 (high half)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int gj = cbk * 128 + lane + 32 * k;
-      const float w = v[k] * rs * sign_of(su, gj);
-      const size_t at = (size_t)gi * n + gj;
-      if (out_dtype == HTR_DTYPE_F32) static_cast<float*>(W)[at] = w;
-      else if (out_dtype == HTR_DTYPE_BF16) static_cast<__nv_bfloat16*>(W)[at] = __float2bfloat16_rn(w);
-      else static_cast<__half*>(W)[at] = __float2half_rn(w);
+      for (int k = 0; k < 4; ++k) {
+        const float2 a = v[i + k];
+        if constexpr (OUT == HTR_DTYPE_BF16) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(a.x + a.y, a.x - a.y);
+          w[k] = *reinterpret_cast<const uint32_t*>(&h) ^ m[k] ^ flips;
+        } else {
+          const __half2 h = __floats2half2_rn(a.x + a.y, a.x - a.y);
+          w[k] = *reinterpret_cast<const uint32_t*>(&h) ^ m[k] ^ flips;
+        }
+      }
+      const bool odd = lane & 1;
+#pragma unroll
+      for (int k = 0; k < 4; k += 2) {
+        // the even lane keeps row k and takes its neighbour's, the odd lane row k + 1
+        const uint32_t other = __shfl_xor_sync(kFullWarp, odd ? w[k] : w[k + 1], 1), mine = odd ? w[k + 1] : w[k];
+        const uint32_t left = odd ? other : mine, right = odd ? mine : other;
+        uint32_t* dst = reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(W) + (row0 + 2 * (i + k + (odd ? 1 : 0))) * n + (gc & ~1));
+        dst[0] = __byte_perm(left, right, 0x5410);
+        dst[32] = __byte_perm(left, right, 0x7632);
+      }
     }
   }
 }
@@ -118,14 +207,29 @@ static int launch_decode_raw(const uint32_t* qw, int16_t* out, long long ntiles,
   return (int)cudaGetLastError();
 }
 
+template <int K, int OUT>
+static int launch_dequant_w_as(const uint32_t* qw, const __half* scales, const uint8_t* su, const uint8_t* sv, float cb, void* W, int mt, int nt,
+                               cudaStream_t st) {
+  static bool allowed[64] = {false};                         // shared memory beyond 48 KB: opted in once per device
+  int dev = 0;
+  if (const cudaError_t e = cudaGetDevice(&dev)) return (int)e;
+  if (dev < 0 || dev >= 64 || !allowed[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(dequant_w_kernel<K, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmem);
+    if (e != cudaSuccess) return (int)e;
+    if (dev >= 0 && dev < 64) allowed[dev] = true;
+  }
+  dequant_w_kernel<K, OUT><<<dim3(nt / 8, mt / 8), kDqThreads, kDqSmem, st>>>(qw, scales, su, sv, cb, W, nt);
+  return (int)cudaGetLastError();
+}
+
 template <int K>
 static int launch_dequant_w(const uint32_t* qw, const __half* scales, const uint8_t* su, const uint8_t* sv, float cb, void* W,
                             int out_dtype, int mt, int nt, cudaStream_t st) {
-  const size_t smem = sizeof(float) * 128 * kDqLd;
-  cudaError_t e = cudaFuncSetAttribute(dequant_w_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  dequant_w_kernel<K><<<dim3(nt / 8, mt / 8), 256, smem, st>>>(qw, scales, su, sv, cb, W, out_dtype, nt);
-  return (int)cudaGetLastError();
+  switch (out_dtype) {
+    case HTR_DTYPE_BF16: return launch_dequant_w_as<K, HTR_DTYPE_BF16>(qw, scales, su, sv, cb, W, mt, nt, st);
+    case HTR_DTYPE_F16: return launch_dequant_w_as<K, HTR_DTYPE_F16>(qw, scales, su, sv, cb, W, mt, nt, st);
+    default: return launch_dequant_w_as<K, HTR_DTYPE_F32>(qw, scales, su, sv, cb, W, mt, nt, st);
+  }
 }
 
 int run_decode_raw(int K, const uint32_t* qw, int16_t* out, long long ntiles, cudaStream_t st) {
