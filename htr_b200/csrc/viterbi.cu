@@ -9,11 +9,23 @@
 // Formulation.  The reference keeps all 65536 path costs; here only their minima over the top K bits survive a step:
 //   m_{t+1}[j] = min_top ( m_t[(top << (16-2K)) | (j >> K)] + w_t * (x_t - cb[(top << (16-K)) | j])^2 ),   bp_t[j] = argmin,
 // with m_0 = 0 (or, in the second pass, +inf except at the required start).  That is 2 * 2^(16-K) floats of state, which fits
-// shared memory for every K (128 KB at K = 2), so one CTA owns a tile from the first step to the traceback and touches global
-// memory only for the back-pointers (one byte per (step, j), second pass only; each resident CTA has its own region).
-// The codebook value is recomputed per candidate from the hash: v(s) lands in a float through the 1.5 * 2^23 mantissa trick
-// and float32(v / rms) = fma(v, inv_hi, v * inv_lo) with 1/rms split in two floats -- exact for all 1021 possible v (checked
-// by the tests against the oracle's table, bit for bit), so no table lookups with their bank conflicts.
+// shared memory for every K (128 KB at K = 2), so one thread block owns a tile from the first step to the traceback and touches
+// global memory only for the back-pointers (one byte per (step, j), second pass only; each resident block has its own region).
+//
+// What bounds it: per candidate the reference's operations x - c, d * d, w * (d * d), prev + ... occupy the FMA pipes for four
+// cycles of a warp (packed or not), the minimum the shift/logic pipe for two.  So everything else has to go:
+//  * A thread owns the same 128 states in every step, hence the same 128 codebook values: 64 of them stay in registers, 64 in shared
+//    memory (one 16-byte read per four; K = 2 has no room there and recomputes them from the state hash).  Recomputing all of them
+//    cost 3.5 instructions per candidate.
+//  * The first pass needs no argument of the minimum except in its last step.
+//  * The traceback is a chain of dependent loads; the K unknown bits per step are few enough to load two to five steps' candidates
+//    at once, so a warp resolves that many steps per memory latency.
+// Measured, 256 tiles (K = 2, 3, 4, 5, 6, 8): 3.91, 3.69, 3.48, 3.60, 3.82, 3.89 ms with the values recomputed and one state per
+// latency in the traceback; 2.65, 2.05, 2.01, 2.08, 2.25, 2.63 ms in this form.
+//
+// The codebook value in float: v(s) lands in a float through the 1.5 * 2^23 mantissa trick and float32(v / rms) =
+// fma(v, inv_hi, v * inv_lo) with 1/rms split in two floats -- exact for all 1021 possible v (checked by the tests against the
+// oracle's table, bit for bit).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -39,12 +51,18 @@ struct VitParams {
 
 template <int K>
 struct VitCfg {
-  static constexpr int kSj = 1 << (16 - K);
-  // a thread owns groups of kJb consecutive j (they share the predecessor minima: kJb divides 2^K) and works on them in pairs
-  static constexpr int kJb = K == 2 ? 4 : K <= 4 ? 8 : K == 5 ? 4 : 2;
-  static constexpr int kThreads = K == 2 ? 1024 : (kSj / kJb < 512 ? kSj / kJb : 512);
-  static constexpr int kGroups = kSj / (kThreads * kJb);
-  static constexpr int kSmem = 2 * kSj * 4 + 2 * kVitMaxT * 4 + kSj;   // two cost arrays, targets, weights, last back-pointers
+  static constexpr int kNB = 1 << K, kSj = 1 << (16 - K);
+  static constexpr int kThreads = 512;                                    // x 128 states = all of them
+  static constexpr int kTT = kNB < 16 ? kNB : 16;                         // tops of one thread; kSub neighbouring lanes share the others
+  static constexpr int kSub = kNB / kTT;
+  static constexpr int kJb = K == 2 ? 4 : 8;                              // consecutive j of a group: they share their predecessor minima
+  static constexpr int kGroups = 128 / (kTT * kJb);                       // groups of a thread: K = 2: 8, K = 3: 2, else 1
+  static constexpr int kBlocks = 128 / kJb;                               // (group, top) blocks of kJb states, in that order
+  static constexpr int kRegBlocks = kBlocks / 2;                          // ... whose codebook values stay in registers
+  static constexpr bool kTable = K != 2;                                  // the others': in shared memory, else from the hash
+  static constexpr int kTableBytes = kTable ? 64 * kThreads * 4 : 0;
+  static constexpr int kSmem = kTableBytes + 2 * kSj * 4 + 2 * kVitMaxT * 4 + kSj;   // table, two cost arrays, targets, weights, last back-pointers
+  static constexpr int kLevels = K == 2 ? 5 : K <= 4 ? 3 : 2;             // steps of the traceback per memory latency: kNB^(levels-1) <= 256
 };
 
 __device__ __forceinline__ float codebook_value(uint32_t hash, float inv_hi, float inv_lo) {
@@ -55,7 +73,6 @@ __device__ __forceinline__ float codebook_value(uint32_t hash, float inv_hi, flo
 // packed float32 pairs: one instruction, two candidates
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
 struct Best {
   float v;
@@ -63,13 +80,111 @@ struct Best {
 };
 __device__ __forceinline__ bool better(const Best& a, const Best& b) { return a.v < b.v || (a.v == b.v && a.key < b.key); }
 
+// one candidate: the first minimum wins, as torch.min does
+template <bool ARG>
+__device__ __forceinline__ void take(float val, int top, float& best, int& arg) {
+  if constexpr (ARG) {
+    if (val < best) { best = val; arg = top; }
+  } else {
+    best = fminf(best, val);
+  }
+}
+
+// One step of all states: costs mc -> mn and, with ARG, the arguments to bp and lastarg (either may be null).
+template <int K, bool ARG>
+__device__ __forceinline__ void vit_step(const float* __restrict__ mc, float* __restrict__ mn, float xt, float wt, const float2 (&negc)[32],
+                                         const float4* __restrict__ table, float inv_hi, float inv_lo, uint8_t* __restrict__ bp,
+                                         uint8_t* __restrict__ lastarg) {
+  using C = VitCfg<K>;
+  constexpr int JB = C::kJb, SH = 16 - 2 * K, TT = C::kTT, SUB = C::kSub;
+  const int tid = threadIdx.x, sub = tid % SUB;
+  const float2 xt2 = make_float2(xt, xt), wt2 = make_float2(wt, wt);
+#pragma unroll
+  for (int g = 0; g < C::kGroups; ++g) {
+    const int jbase = (g * (C::kThreads / SUB) + tid / SUB) * JB;
+    const float* prev_col = mc + (jbase >> K) + ((sub * TT) << SH);        // predecessor minima of this group: stride 2^(16-2K) per top
+    float best[JB];
+    int arg[JB];                                                          // relative to this lane's first top
+#pragma unroll
+    for (int b = 0; b < JB; ++b) { best[b] = INFINITY; arg[b] = 0; }
+#pragma unroll
+    for (int tt = 0; tt < TT; ++tt) {
+      const float prev = prev_col[tt << SH];
+      constexpr int kQuads = JB / 4;
+      const int blk = g * TT + tt;
+#pragma unroll
+      for (int q = 0; q < kQuads; ++q) {
+        float2 nc[2];
+        if (blk < C::kRegBlocks) {
+          nc[0] = negc[(blk * kQuads + q) * 2];
+          nc[1] = negc[(blk * kQuads + q) * 2 + 1];
+        } else if constexpr (C::kTable) {
+          const float4 f = table[((blk - C::kRegBlocks) * kQuads + q) * C::kThreads];
+          nc[0] = make_float2(f.x, f.y);
+          nc[1] = make_float2(f.z, f.w);
+        } else {
+          const uint32_t h0 = ((uint32_t)((sub * TT + tt) << (16 - K)) + (uint32_t)(jbase + 4 * q)) * kGenMul + kGenAdd;
+          const float2 unmagic = make_float2(-12582912.0f, -12582912.0f), hi = make_float2(-inv_hi, -inv_hi), lo = make_float2(-inv_lo, -inv_lo);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float2 v = add2(make_float2(__uint_as_float(bytesum_add_alu(h0 + (2 * e) * kGenMul, kMagicBits - 510u)),
+                                              __uint_as_float(bytesum_add(h0 + (2 * e + 1) * kGenMul, kMagicBits - 510u))), unmagic);
+            nc[e] = __ffma2_rn(v, hi, mul2(v, lo));                         // -c: negation commutes with rounding
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float2 d = add2(xt2, nc[e]);
+          const float2 wd = mul2(wt2, mul2(d, d));
+          // the last addition stays scalar: a packed multiply followed by a packed add was observed to come out fused (one
+          // rounding instead of two, costs 1 ulp off the reference's), which separate scalar adds rule out
+          take<ARG>(__fadd_rn(prev, wd.x), tt, best[4 * q + 2 * e], arg[4 * q + 2 * e]);
+          take<ARG>(__fadd_rn(prev, wd.y), tt, best[4 * q + 2 * e + 1], arg[4 * q + 2 * e + 1]);
+        }
+      }
+    }
+    if constexpr (ARG && SUB > 1) {
+#pragma unroll
+      for (int b = 0; b < JB; ++b) arg[b] += sub * TT;
+    }
+    // neighbouring lanes hold the other tops: the smaller cost, then the smaller top
+#pragma unroll
+    for (int o = 1; o < SUB; o <<= 1)
+#pragma unroll
+      for (int b = 0; b < JB; ++b) {
+        const float ov = __shfl_xor_sync(0xFFFFFFFFu, best[b], o);
+        if constexpr (ARG) {
+          const int oa = __shfl_xor_sync(0xFFFFFFFFu, arg[b], o);
+          const bool other = ov < best[b] || (ov == best[b] && oa < arg[b]);
+          best[b] = other ? ov : best[b];
+          arg[b] = other ? oa : arg[b];
+        } else {
+          best[b] = fminf(best[b], ov);
+        }
+      }
+    if (sub == 0) {
+#pragma unroll
+      for (int q = 0; q < JB / 4; ++q)
+        *reinterpret_cast<float4*>(mn + jbase + 4 * q) = make_float4(best[4 * q], best[4 * q + 1], best[4 * q + 2], best[4 * q + 3]);
+      if constexpr (ARG) {
+#pragma unroll
+        for (int q = 0; q < JB / 4; ++q) {
+          const uint32_t packed = (uint32_t)arg[4 * q] | ((uint32_t)arg[4 * q + 1] << 8) | ((uint32_t)arg[4 * q + 2] << 16) | ((uint32_t)arg[4 * q + 3] << 24);
+          if (bp) *reinterpret_cast<uint32_t*>(bp + jbase + 4 * q) = packed;
+          if (lastarg) *reinterpret_cast<uint32_t*>(lastarg + jbase + 4 * q) = packed;
+        }
+      }
+    }
+  }
+}
+
 template <int K>
-__global__ void __launch_bounds__(VitCfg<K>::kThreads) viterbi_kernel(const VitParams p) {
-  constexpr int NB = 1 << K, SJ = VitCfg<K>::kSj, SH = 16 - 2 * K, THREADS = VitCfg<K>::kThreads, JB = VitCfg<K>::kJb, GROUPS = VitCfg<K>::kGroups;
-  static_assert(JB >= 2 && JB % 2 == 0 && NB % JB == 0 && GROUPS * THREADS * JB == SJ, "thread-to-state mapping");
-  constexpr uint32_t kTopStep = kGenMul << (16 - K);                      // hash difference between consecutive top values
+__global__ void __launch_bounds__(VitCfg<K>::kThreads, 1) viterbi_kernel(const VitParams p) {
+  using C = VitCfg<K>;
+  constexpr int NB = C::kNB, SJ = C::kSj, THREADS = C::kThreads, JB = C::kJb;
   extern __shared__ __align__(16) unsigned char vsm[];
-  float* m_a = reinterpret_cast<float*>(vsm);
+  float4* table = reinterpret_cast<float4*>(vsm) + threadIdx.x;
+  float* m_a = reinterpret_cast<float*>(vsm + C::kTableBytes);
   float* m_b = m_a + SJ;
   float* xs = m_b + SJ;
   float* ws = xs + kVitMaxT;
@@ -79,8 +194,26 @@ __global__ void __launch_bounds__(VitCfg<K>::kThreads) viterbi_kernel(const VitP
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int T = p.T;
   uint8_t* bp = p.bps + (size_t)blockIdx.x * T * SJ;
-  const float2 unmagic = make_float2(-12582912.0f, -12582912.0f);
-  const float2 ninv_hi = make_float2(-p.inv_hi, -p.inv_hi), ninv_lo = make_float2(-p.inv_lo, -p.inv_lo);
+
+  // the negated codebook values of this thread's states, in block order (group, top): half here, half in shared memory
+  float2 negc[32];
+#pragma unroll
+  for (int blk = 0; blk < (C::kTable ? C::kBlocks : C::kRegBlocks); ++blk) {
+    const int g = blk / C::kTT, top = (tid % C::kSub) * C::kTT + blk % C::kTT;
+    const int jbase = (g * (THREADS / C::kSub) + tid / C::kSub) * JB;
+#pragma unroll
+    for (int q = 0; q < JB / 4; ++q) {
+      float f[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f[e] = -codebook_value((((uint32_t)top << (16 - K)) | (uint32_t)(jbase + 4 * q + e)) * kGenMul + kGenAdd, p.inv_hi, p.inv_lo);
+      if (blk < C::kRegBlocks) {
+        negc[(blk * (JB / 4) + q) * 2] = make_float2(f[0], f[1]);
+        negc[(blk * (JB / 4) + q) * 2 + 1] = make_float2(f[2], f[3]);
+      } else {
+        table[((blk - C::kRegBlocks) * (JB / 4) + q) * THREADS] = make_float4(f[0], f[1], f[2], f[3]);
+      }
+    }
+  }
 
   for (int tile = blockIdx.x; tile < p.B; tile += gridDim.x) {
     __syncthreads();                                                     // the previous tile's traceback is over
@@ -97,65 +230,10 @@ __global__ void __launch_bounds__(VitCfg<K>::kThreads) viterbi_kernel(const VitP
       for (int j = tid; j < SJ; j += THREADS) mc[j] = (j0 < 0 || j == j0) ? 0.f : INFINITY;
       __syncthreads();
       for (int t = 0; t < T; ++t) {
-        const float2 xt2 = make_float2(xs[t], xs[t]), wt2 = make_float2(ws[t], ws[t]);
+        const float xt = xs[t], wt = ws[t];
         const bool last = t == T - 1;
-#pragma unroll 1
-        for (int g = 0; g < GROUPS; ++g) {
-          const int jbase = (g * THREADS + tid) * JB;
-          const float* prev_col = mc + (jbase >> K);                     // predecessor minima of this group: stride 2^(16-2K) per top
-          uint32_t hash[JB];
-          float best[JB];
-          int arg[JB];
-#pragma unroll
-          for (int b = 0; b < JB; ++b) {
-            hash[b] = (uint32_t)(jbase + b) * kGenMul + kGenAdd;
-            best[b] = INFINITY;
-            arg[b] = 0;
-          }
-#pragma unroll 4
-          for (int top = 0; top < NB; ++top) {
-            const float prev = prev_col[top << SH];
-#pragma unroll
-            for (int b = 0; b < JB; b += 2) {
-              // two candidates per packed float instruction; per lane the reference's operation order:
-              // c = float32(v / rms); d = x - c; cost = prev + w * (d * d)
-              const float2 vm = make_float2(__uint_as_float(bytesum_add_alu(hash[b], kMagicBits - 510u)),
-                                            __uint_as_float(bytesum_add(hash[b + 1], kMagicBits - 510u)));
-              const float2 v = add2(vm, unmagic);
-              const float2 negc = fma2(v, ninv_hi, mul2(v, ninv_lo));              // -c: negation commutes with rounding
-              const float2 d = add2(xt2, negc);
-              const float2 wd = mul2(wt2, mul2(d, d));
-              // the last addition stays scalar: a packed multiply followed by a packed add was observed to come out fused (one
-              // rounding instead of two, costs 1 ulp off the reference's), which separate scalar adds rule out
-              const float2 val = make_float2(__fadd_rn(prev, wd.x), __fadd_rn(prev, wd.y));
-              if (val.x < best[b]) { best[b] = val.x; arg[b] = top; }              // strict: the first minimum wins, as torch.min does
-              if (val.y < best[b + 1]) { best[b + 1] = val.y; arg[b + 1] = top; }
-              hash[b] += kTopStep;
-              hash[b + 1] += kTopStep;
-            }
-          }
-          uint32_t packed_arg[(JB + 3) / 4];
-#pragma unroll
-          for (int q = 0; q < (JB + 3) / 4; ++q) packed_arg[q] = 0u;
-#pragma unroll
-          for (int b = 0; b < JB; ++b) {
-            mn[jbase + b] = best[b];
-            packed_arg[b >> 2] |= (uint32_t)arg[b] << (8 * (b & 3));
-          }
-          if constexpr (JB >= 4) {
-            if (keep) {
-#pragma unroll
-              for (int q = 0; q < JB / 4; ++q) *reinterpret_cast<uint32_t*>(bp + (size_t)t * SJ + jbase + 4 * q) = packed_arg[q];
-            }
-            if (last) {
-#pragma unroll
-              for (int q = 0; q < JB / 4; ++q) *reinterpret_cast<uint32_t*>(lastarg + jbase + 4 * q) = packed_arg[q];
-            }
-          } else {
-            if (keep) *reinterpret_cast<uint16_t*>(bp + (size_t)t * SJ + jbase) = (uint16_t)packed_arg[0];
-            if (last) *reinterpret_cast<uint16_t*>(lastarg + jbase) = (uint16_t)packed_arg[0];
-          }
-        }
+        if (keep || last) vit_step<K, true>(mc, mn, xt, wt, negc, table, p.inv_hi, p.inv_lo, keep ? bp + (size_t)t * SJ : nullptr, last ? lastarg : nullptr);
+        else vit_step<K, false>(mc, mn, xt, wt, negc, table, p.inv_hi, p.inv_lo, nullptr, nullptr);
         __syncthreads();
         float* sw = mc; mc = mn; mn = sw;
       }
@@ -183,16 +261,48 @@ __global__ void __launch_bounds__(VitCfg<K>::kThreads) viterbi_kernel(const VitP
         __syncthreads();
         j0 = (int)(s_win.key & 0xFFFFu);                                 // low 16-K bits of the winner (j < 2^(16-K))
       }
-      if (keep && tid == 0) {
+      if (keep && warp == 0) {
         // last state: with tail-biting the cheapest state whose low bits equal j0, else the overall winner
         uint32_t s = p.tailbite ? ((uint32_t)lastarg[j0] * SJ + (uint32_t)j0) : ((s_win.key >> 16) * SJ + (s_win.key & 0xFFFFu));
-        if (p.total) p.total[tile] = p.tailbite ? mc[j0] : s_win.v;
         int32_t* out = p.states + (size_t)tile * T;
-        out[T - 1] = (int32_t)s;
-        for (int t = T - 1; t >= 1; --t) {                                // htr/reference.py:45-49
-          const uint32_t low = s >> K;
-          s = (uint32_t)bp[(size_t)(t - 1) * SJ + low] * SJ + low;
-          out[t - 1] = (int32_t)s;
+        if (lane == 0) {
+          if (p.total) p.total[tile] = p.tailbite ? mc[j0] : s_win.v;
+          out[T - 1] = (int32_t)s;
+        }
+        // back along the path (htr/reference.py:45-49): s_{t-1} = bp_{t-1}[s_t >> K] * SJ + (s_t >> K).  The back-pointers of kLevels
+        // steps are loaded together: for every value of the tops still unknown, candidate id = those tops as a number in base NB
+        constexpr int LV = C::kLevels;
+        for (int t = T - 1; t >= 1; t -= LV) {
+          constexpr int kMost = 8;                                       // loads of a lane per level: NB^(LV-1) <= 256
+          uint32_t got[LV][kMost];
+          int ids = 1;
+#pragma unroll
+          for (int l = 0; l < LV; ++l, ids *= NB) {
+#pragma unroll
+            for (int r = 0; r < kMost; ++r) {
+              got[l][r] = 0u;
+              const int id = 32 * r + lane;
+              if (32 * r < ids && id < ids && t - 1 - l >= 0) {
+                uint32_t low = s >> K;
+#pragma unroll
+                for (int k = l - 1; k >= 0; --k) low = ((((uint32_t)(id >> (k * K)) & (NB - 1)) * SJ) + low) >> K;   // the earliest step's top is the leading digit
+                got[l][r] = __ldcg(bp + (size_t)(t - 1 - l) * SJ + low);
+              }
+            }
+          }
+          int id = 0;
+#pragma unroll
+          for (int l = 0; l < LV; ++l) {
+            if (t - 1 - l < 0) break;
+            uint32_t mine = got[l][0];
+#pragma unroll
+            for (int r = 1; r < kMost; ++r)
+              if (r == id >> 5) mine = got[l][r];
+            const uint32_t top = __shfl_sync(0xFFFFFFFFu, mine, id & 31);
+            s = top * SJ + (s >> K);
+            if (lane == 0) out[t - 1 - l] = (int32_t)s;
+            id = id * NB + (int)top;
+          }
         }
       }
       __syncthreads();
