@@ -172,6 +172,11 @@ static int gemv_kind(int M, int dtype = HTR_DTYPE_BF16, int n = 0, int prologue 
   return kind == 0 || kind == 1 ? kind : (M >= 2 ? 1 : 0);
 }
 
+// From two 16-bit rows on, linears of at least this many weights run on the tensor-core GEMM (htr_linear_route_rows).  Measured at
+// K4, two / four bf16 rows, GEMV -> GEMM: 1024x4096 10.3 / 14.4 -> 7.8 us, 4096x12288 18.4 / 22.8 -> 17.1, 151936x4096 169 / 219 -> 126;
+// at 2 million weights and below the second launch costs what the decode saves (1024x1024, four fp16 rows: 5.9 against 7.0).
+constexpr long long kRouteSmall = 1 << 22;
+
 static int make_plan(int M, int m, int n, int K, Plan* out, int kind = 0) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -282,6 +287,14 @@ int htr_last_cuda_error(void) { return t_last_cuda; }
 int htr_version(void) { return 100; }
 
 void htr_set_gemv_kernel(int kind) { g_kind_override = kind < 0 || kind > 2 ? -1 : kind; }   // -1: back to the default
+
+int htr_linear_route_rows(int dtype, int mt, int nt, unsigned flags) {
+  // float32 rows and the forms that promise exact sums or a kernel stay on the GEMV kernels; so do small linears, where the GEMM's
+  // second launch costs more than its decode saves
+  const bool chosen = g_kind_override >= 0 || gemv_kind_default() >= 0;
+  if (dtype == HTR_DTYPE_F32 || (flags & HTR_LINEAR_EXACT_SUMS) || chosen || (long long)mt * nt * 256 < kRouteSmall) return 4;
+  return 1;
+}
 
 size_t htr_linear_fault_offset(void) { return (size_t)kTmFaultWord * 4; }
 

@@ -384,17 +384,23 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   while (g.stages > 1 && gemm_smem_bytes(g.np, planes, g.stages, words) > budget) --g.stages;
   g.smem = gemm_smem_bytes(g.np, planes, g.stages, words);
   if (g.stages < 2) return HTR_ERR_TOO_LARGE;
-  // Few row blocks: up to eight thread blocks share one as a cluster and reduce on chip.  Even runs over the whole GPU (flat) give
-  // every thread block the same work, but a row block's partial sums then meet in global memory at one last arriver: they have
-  // to be a fifth shorter to win.
-  const long long slots = (long long)sms, units = (long long)g.rbs * g.hb;
-  long long s = slots / g.rbs;
-  if (s > 8) s = 8;
-  if (s > g.hb) s = g.hb;
+  // Up to eight thread blocks share a row block as a cluster and reduce on chip, or every thread block of the GPU takes an even run
+  // (flat) and a row block's partial sums meet in global memory at one last arriver.  Costs in units of one decoded 128 x 128 block
+  // (0.43 us): the longest run, and for the flat form nine for the hand-over (measured 2 to 3 us) plus the partials that the last
+  // arriver reads at about 100 bytes a nanosecond.  At 2048x2048, 8 / 200 rows, this chose clusters of four over flat runs: 11.5 / 33.2
+  // -> 7.6 / 16.9 us; 6144x4096, 8 rows: 14.6 -> 12.7.
+  const long long slots = sms, units = (long long)g.rbs * g.hb;
   const long long flat_grid = slots < units ? slots : units, flat_run = (units + flat_grid - 1) / flat_grid;
+  long long best = flat_run + 9 + (g.hb / flat_run + 1) * g.np / 84;
   g.split = 0;
-  if (s >= 1 && (g.hb + s - 1) / s * 5 <= flat_run * 6 && (s == 1 || gemm_clusters(K, g.smem, (int)s) >= g.rbs)) g.split = (int)s;
-  else if (s == 8 && gemm_clusters(K, g.smem, 8) >= g.rbs) g.split = 8;   // too few row blocks to fill the GPU: short runs either way
+  for (int s = (int)(slots / g.rbs < 8 ? slots / g.rbs : 8); s >= 1; --s) {
+    const long long run = (g.hb + s - 1) / s;
+    if (s > g.hb || run >= best) continue;
+    if (s == 1 || gemm_clusters(K, g.smem, s) >= g.rbs) {
+      g.split = s;
+      best = run;
+    }
+  }
   g.grid = g.split > 0 ? g.rbs * g.split : (int)flat_grid;
   size_t off = kCounterRegion + kErrorRegion;
   g.off_xb = off; off += align256((size_t)ncols * n * 2);
@@ -427,13 +433,24 @@ size_t htr_linear_gemm_workspace_bytes(int M, int m, int n, int K) {
   return b1 > b2 ? b1 : b2;
 }
 
-static int gemm_launch(const void* x, int dtype, int M, const void* qweight, int mt, int nt, int K, const void* scales, const uint8_t* su,
-                       const uint8_t* sv, const void* bias, void* y, void* const* peer_y, int npeer, int64_t peer_offset, void* workspace,
-                       size_t workspace_bytes, htr_stream_t stream);
+// fp16 planes of the activations: two (hi + lo, 22 bits) for float32 inputs, for callers that ask, and for up to 8 rows, which fill the
+// 16 accumulator columns of the smallest MMA either way; else one
+static int gemm_planes(int dtype, int M, bool fine) { return dtype == HTR_DTYPE_F32 || fine || M <= 8 ? 2 : 1; }
+
+static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qweight, int mt, int nt, int K, const void* scales, const uint8_t* su,
+                       const uint8_t* sv, const void* bias, void* y, int m_out, bool fine, void* const* peer_y, int npeer, int64_t peer_offset,
+                       void* workspace, size_t workspace_bytes, htr_stream_t stream);
 
 int htr_linear_gemm(const void* x, int dtype, int M, const void* qweight, int mt, int nt, int K, const void* scales, const uint8_t* su,
                     const uint8_t* sv, const void* bias, void* y, void* workspace, size_t workspace_bytes, htr_stream_t stream) {
-  return gemm_launch(x, dtype, M, qweight, mt, nt, K, scales, su, sv, bias, y, nullptr, 0, 0, workspace, workspace_bytes, stream);
+  return gemm_launch(x, dtype, M, nt * 16, qweight, mt, nt, K, scales, su, sv, bias, y, mt * 16, false, nullptr, 0, 0, workspace, workspace_bytes, stream);
+}
+
+int htr_linear_gemm_padded(const void* x, int dtype, int M, int n_in, const void* qweight, int mt, int nt, int K, const void* scales, const uint8_t* su,
+                           const uint8_t* sv, const void* bias, void* y, int m_out, void* workspace, size_t workspace_bytes, htr_stream_t stream) {
+  if (mt <= 0 || nt <= 0 || M > HTR_GEMM_MAX_ROWS_F32) return HTR_ERR_BAD_SHAPE;
+  if (n_in < 8 || n_in > nt * 16 || n_in % 8 || m_out < 8 || m_out > mt * 16 || m_out % 8) return HTR_ERR_BAD_SHAPE;
+  return gemm_launch(x, dtype, M, n_in, qweight, mt, nt, K, scales, su, sv, bias, y, m_out, true, nullptr, 0, 0, workspace, workspace_bytes, stream);
 }
 
 int htr_linear_gemm_peers(const void* x, int dtype, int M, const void* qweight, int mt, int nt, int K, const void* scales, const uint8_t* su,
@@ -442,12 +459,13 @@ int htr_linear_gemm_peers(const void* x, int dtype, int M, const void* qweight, 
   if (npeer < 1 || npeer > 8 || !peer_y || peer_offset < 0 || (peer_offset & 7)) return HTR_ERR_BAD_SHAPE;
   for (int i = 0; i < npeer; ++i)
     if (!peer_y[i] || (reinterpret_cast<uintptr_t>(peer_y[i]) & 15u)) return peer_y[i] ? HTR_ERR_ALIGNMENT : HTR_ERR_NULL;
-  return gemm_launch(x, dtype, M, qweight, mt, nt, K, scales, su, sv, bias, nullptr, peer_y, npeer, peer_offset, workspace, workspace_bytes, stream);
+  return gemm_launch(x, dtype, M, nt * 16, qweight, mt, nt, K, scales, su, sv, bias, nullptr, mt * 16, false, peer_y, npeer, peer_offset, workspace,
+                     workspace_bytes, stream);
 }
 
-static int gemm_launch(const void* x, int dtype, int M, const void* qweight, int mt, int nt, int K, const void* scales, const uint8_t* su,
-                       const uint8_t* sv, const void* bias, void* y, void* const* peer_y, int npeer, int64_t peer_offset, void* workspace,
-                       size_t workspace_bytes, htr_stream_t stream) {
+static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qweight, int mt, int nt, int K, const void* scales, const uint8_t* su,
+                       const uint8_t* sv, const void* bias, void* y, int m_out, bool fine, void* const* peer_y, int npeer, int64_t peer_offset,
+                       void* workspace, size_t workspace_bytes, htr_stream_t stream) {
   if (!width_ok(K)) return HTR_ERR_BAD_K;
   if (dtype < HTR_DTYPE_BF16 || dtype > HTR_DTYPE_F32) return HTR_ERR_BAD_DTYPE;
   if (M < 0 || M > HTR_GEMM_MAX_ROWS || mt <= 0 || nt <= 0 || mt % 8 || nt % 8) return HTR_ERR_BAD_SHAPE;
@@ -458,7 +476,7 @@ static int gemm_launch(const void* x, int dtype, int M, const void* qweight, int
   if (!a16(x) || !a16(qweight) || !a16(y) || (bias && !a16(bias)) || !a16(workspace) || !a16(scales)) return HTR_ERR_ALIGNMENT;
   const int m = mt * 16, n = nt * 16;
   GemmPlan g;
-  const int planes = dtype == HTR_DTYPE_F32 ? 2 : 1;      // 16-bit activations need no lo plane
+  const int planes = gemm_planes(dtype, M, fine);
   if (planes == 2 && M > HTR_GEMM_MAX_ROWS_F32) return HTR_ERR_BAD_SHAPE;
   const int rc = make_gemm_plan(M, m, n, K, planes, &g);
   if (rc != HTR_OK) return rc;
@@ -486,14 +504,14 @@ static int gemm_launch(const void* x, int dtype, int M, const void* qweight, int
   p.hb = g.hb;
   p.split = g.split;
   p.stages = g.stages;
-  p.m_out = m;
+  p.m_out = m_out;
   p.xsum_slices = gemm_rht_slices(g.np, n);
   p.cb = (float)codebook_scale();
   p.plan = nullptr;
   p.npeer = npeer;
   p.peer_offset = peer_offset;
   for (int i = 0; i < 8; ++i) p.peer_y[i] = i < npeer ? peer_y[i] : nullptr;
-  int e = run_rht_f16(x, dtype, M, g.np, n, n, planes, su, reinterpret_cast<__half*>(ws + g.off_xb), reinterpret_cast<float*>(ws + g.off_xsum),
+  int e = run_rht_f16(x, dtype, M, g.np, n, n_in, planes, su, reinterpret_cast<__half*>(ws + g.off_xb), reinterpret_cast<float*>(ws + g.off_xsum),
                       reinterpret_cast<float*>(ws + g.off_tok), st);
   if (e) { t_gemm_cuda = e; return HTR_ERR_CUDA; }
   e = launch_gemm(K, p, g.grid, g.smem, st);

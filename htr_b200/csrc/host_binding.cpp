@@ -21,6 +21,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <optional>
 #include <vector>
 
@@ -33,6 +34,8 @@ struct Entry {
   decltype(&htr_linear_gemm) linear_gemm;
   decltype(&htr_linear_padded) linear_padded;
   decltype(&htr_linear_fused) linear_fused;
+  decltype(&htr_linear_gemm_padded) linear_gemm_padded;
+  decltype(&htr_linear_route_rows) route_rows;
 } g_lib = {};
 
 // ---- workspaces: buffers that ops.py owns (one per device, stream and kind); this table only remembers where they are
@@ -127,8 +130,11 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t cols = (int64_t)w.nt * 16, rows64 = cols ? x->numel() / cols : 0;
   const long flags = PyLong_AsLong(a[6]), gemv_rows = PyLong_AsLong(a[7]), gemm_rows = PyLong_AsLong(a[8]);
   if (dt < 0 || x->size(-1) != cols || rows64 < 1 || !bias_of(a[5], *x, (int64_t)w.mt * 16, &bias)) return none();
-  const bool gemv = rows64 <= gemv_rows && rows64 <= HTR_GEMV_MAX_ROWS;
-  if (!gemv && (rows64 <= gemv_rows || rows64 > gemm_rows)) return none();
+  // (the rule of ops._gemv_rows)
+  int64_t most = gemv_rows;
+  if (gemv_rows <= 4 && rows64 <= gemv_rows && gemm_rows > 0) most = std::min<int64_t>(most, g_lib.route_rows(dt, w.mt, w.nt, (unsigned)flags));
+  const bool gemv = rows64 <= most && rows64 <= HTR_GEMV_MAX_ROWS;
+  if (!gemv && (rows64 <= most || rows64 > gemm_rows)) return none();
   const int rows = (int)rows64, dev = x->get_device();
   OnDevice on(dev);
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
@@ -153,9 +159,9 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(y));
 }
 
-// linear_padded(x, qweight, scales, su, sv, bias, m_out)
+// linear_padded(x, qweight, scales, su, sv, bias, m_out, gemv_rows): up to gemv_rows rows in GEMV launches, more on the tensor-core GEMM
 PyObject* py_linear_padded(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 7) return none();
+  if (n != 8) return none();
   const at::Tensor* x = tensor(a[0]);
   Weight w;
   const void* bias;
@@ -168,14 +174,17 @@ PyObject* py_linear_padded(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int dev = x->get_device();
   OnDevice on(dev);
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
-  const at::Tensor* ws = find_workspace(kGemv, dev, st);
+  const bool gemm = rows > PyLong_AsLong(a[7]);
+  const at::Tensor* ws = find_workspace(gemm ? kGemm : kGemv, dev, st);
   if (!ws) return none();
   at::Tensor y = output(*x, m_out);
   const char* xp = static_cast<const char*>(x->const_data_ptr());
   char* yp = static_cast<char*>(y.data_ptr());
-  for (int64_t r = 0; r < rows; r += HTR_GEMV_MAX_ROWS) {
-    const int here = (int)(rows - r < HTR_GEMV_MAX_ROWS ? rows - r : HTR_GEMV_MAX_ROWS);
-    if (g_lib.linear_padded(xp + r * n_in * esize, dt, here, (int)n_in, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, bias, yp + r * m_out * esize,
+  const int64_t step = gemm ? HTR_GEMM_MAX_ROWS_F32 : HTR_GEMV_MAX_ROWS;
+  const auto launch = gemm ? g_lib.linear_gemm_padded : g_lib.linear_padded;
+  for (int64_t r = 0; r < rows; r += step) {
+    const int here = (int)(rows - r < step ? rows - r : step);
+    if (launch(xp + r * n_in * esize, dt, here, (int)n_in, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, bias, yp + r * m_out * esize,
                             (int)m_out, ws->data_ptr(), ws->numel(), st) != HTR_OK)
       return none();
   }
@@ -251,7 +260,9 @@ PyObject* py_bind(PyObject*, PyObject* table) {
   g_lib.linear_gemm = reinterpret_cast<decltype(g_lib.linear_gemm)>(at_name("htr_linear_gemm"));
   g_lib.linear_padded = reinterpret_cast<decltype(g_lib.linear_padded)>(at_name("htr_linear_padded"));
   g_lib.linear_fused = reinterpret_cast<decltype(g_lib.linear_fused)>(at_name("htr_linear_fused"));
-  if (!g_lib.linear_ex || !g_lib.linear_gemm || !g_lib.linear_padded || !g_lib.linear_fused) {
+  g_lib.linear_gemm_padded = reinterpret_cast<decltype(g_lib.linear_gemm_padded)>(at_name("htr_linear_gemm_padded"));
+  g_lib.route_rows = reinterpret_cast<decltype(g_lib.route_rows)>(at_name("htr_linear_route_rows"));
+  if (!g_lib.linear_gemm_padded || !g_lib.route_rows || !g_lib.linear_ex || !g_lib.linear_gemm || !g_lib.linear_padded || !g_lib.linear_fused) {
     PyErr_SetString(PyExc_ImportError, "bind: an entry point of libhtr_b200 is missing");
     return nullptr;
   }

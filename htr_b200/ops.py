@@ -37,6 +37,22 @@ GEMM_ROUTE_MAX = int(os.environ.get("HTR_GEMM_ROUTE_MAX", "512"))
 # on the GEMM is faster: 25 us against 41-44 us at 4096x12288, 190 us against 384-408 us on the 151936x4096 head)
 GEMV_ROUTE_MAX = min(GEMV_MAX_M, int(os.environ.get("HTR_GEMV_ROUTE_MAX", "4")))
 
+
+def _gemv_rows(dtype, mt, nt):
+    """Rows up to which a linear stays on the GEMV: GEMV_ROUTE_MAX, unless the library knows fewer to be faster (16-bit rows of large
+    linears, htr_linear_route_rows); 5 and more keep every batch of that size there."""
+    return min(GEMV_ROUTE_MAX, _lib.lib.htr_linear_route_rows(_DTYPES[dtype], mt, nt, _STATE.flags)) if GEMV_ROUTE_MAX <= 4 else GEMV_ROUTE_MAX
+
+
+def _padded_gemv_rows(dtype):
+    """The same for padded linears, whose larger batches run as GEMV launches of 8 rows: two of those where GEMV_ROUTE_MAX keeps 8
+    rows on the GEMV, and float32 rows always (their sums carry 24 bits there)."""
+    if dtype == torch.float32 or not USE_GEMM:
+        return 1 << 30
+    return GEMV_ROUTE_MAX if GEMV_ROUTE_MAX < GEMV_MAX_M else 2 * GEMV_MAX_M
+
+
+
 class _ThreadState(threading.local):
     flags = 0       # flags of htr_linear_ex applied to every GEMV launch of this thread (see independent_inputs)
 
@@ -110,10 +126,10 @@ def linear_padded(x, qweight, scales, su, sv, bias=None, m_out=None):
 
     The reference's `HTRHCLinearMethod.apply` (htr/vllm_plugin.py:313-326) pads the input with `F.pad` and slices the output
     with `.contiguous()`; here both happen inside the kernel (missing columns are read as zeros, rows beyond m_out are not
-    written).  n_in and m_out must be multiples of 8.  Batches above 8 rows run as 8-row launches."""
+    written).  n_in and m_out must be multiples of 8.  16-bit batches run on the tensor-core GEMM, float32 ones as 8-row GEMV launches."""
     mt, nt, W = qweight.shape
     m_out = mt * 16 if m_out is None else int(m_out)
-    y = _host.linear_padded(x, qweight, scales, su, sv, bias, m_out)     # the usual case; None: whatever it does not take
+    y = _host.linear_padded(x, qweight, scales, su, sv, bias, m_out, _padded_gemv_rows(x.dtype))     # the usual case; None: whatever it does not take
     if y is not None:
         return y
     n_in = x.shape[-1]
@@ -130,6 +146,15 @@ def linear_padded(x, qweight, scales, su, sv, bias=None, m_out=None):
         qweight, scales, su, sv = qweight.contiguous(), scales.contiguous(), su.contiguous(), sv.contiguous()
         with torch.cuda.device(x2.device):
             st = torch.cuda.current_stream(x2.device).cuda_stream
+            if M > _padded_gemv_rows(x2.dtype):
+                for r0 in range(0, M, _lib.GEMM_MAX_ROWS_F32):
+                    rows = min(_lib.GEMM_MAX_ROWS_F32, M - r0)
+                    ws = _gemm_workspace(x2.device, st, _lib.lib.htr_linear_gemm_workspace_bytes(rows, mt * 16, nt * 16, K))
+                    rc = _lib.lib.htr_linear_gemm_padded(x2[r0:].data_ptr(), _DTYPES[x2.dtype], rows, n_in, qweight.data_ptr(), mt, nt, K,
+                                                         scales.data_ptr(), su.data_ptr(), sv.data_ptr(), None if bias is None else bias.data_ptr(),
+                                                         y[r0:].data_ptr(), m_out, ws.data_ptr(), ws.numel(), st)
+                    _lib.check(rc, "htr_linear_gemm_padded")
+                return y.reshape(*x.shape[:-1], m_out)
             for r0 in range(0, M, GEMV_MAX_M):
                 rows = min(GEMV_MAX_M, M - r0)
                 ws = workspace(x2.device, _lib.lib.htr_linear_workspace_bytes(rows, mt * 16, nt * 16, K))
@@ -403,7 +428,7 @@ def _linear_impl(x2, qweight, scales, su, sv, bias):
     qweight, scales, su, sv = qweight.contiguous(), scales.contiguous(), su.contiguous(), sv.contiguous()
     bias = None if bias is None else bias.contiguous()
     with torch.cuda.device(x2.device):
-        if GEMV_ROUTE_MAX < M <= GEMM_ROUTE_MAX and USE_GEMM:
+        if USE_GEMM and _gemv_rows(x2.dtype, mt, qweight.shape[1]) < M <= GEMM_ROUTE_MAX:
             y = torch.empty((M, mt * 16), dtype=x2.dtype, device=x2.device)
             step = _lib.GEMM_MAX_ROWS_F32 if x2.dtype == torch.float32 else GEMM_MAX_M
             for r0 in range(0, M, step):

@@ -237,6 +237,15 @@ int htr_linear_gemm(const void* x, int dtype, int M, const void* qweight, int mt
                     const uint8_t* su, const uint8_t* sv, const void* bias /* may be NULL */, void* y, void* workspace,
                     size_t workspace_bytes, htr_stream_t stream);
 
+/* htr_linear_gemm in the padded form of htr_linear_padded (n_in columns of x, m_out rows of y), always with two fp16 planes of the
+ * activations, up to HTR_GEMM_MAX_ROWS_F32 rows per call. */
+int htr_linear_gemm_padded(const void* x, int dtype, int M, int n_in, const void* qweight, int mt, int nt, int K, const void* scales,
+                           const uint8_t* su, const uint8_t* sv, const void* bias, void* y, int m_out, void* workspace,
+                           size_t workspace_bytes, htr_stream_t stream);
+/* Up to how many activation rows htr_linear (the GEMV) is the faster or the more exact choice for a linear of this type and size; beyond
+ * them htr_linear_gemm.  Honours HTR_LINEAR_EXACT_SUMS in `flags` and htr_set_gemv_kernel. */
+int htr_linear_route_rows(int dtype, int mt, int nt, unsigned flags);
+
 /* Row-shard form of htr_linear_gemm (one launch: batches that htr_linear_gemm would split into two are refused with
  * HTR_ERR_TOO_LARGE): the epilogue stores row j, rows [0, m) of this shard, at element offset peer_offset + j * m of every buffer in
  * peer_y (the gather buffers of all ranks of an NVLink box as mapped into this process, plain peer stores) instead of y; the caller
