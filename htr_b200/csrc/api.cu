@@ -3,6 +3,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "packed_gemv1.cuh"
 #include "packed_gemv_mma.cuh"
 #include "packed_gemv_tm.cuh"
 
@@ -248,6 +249,26 @@ static int make_plan(int M, int m, int n, int K, Plan* out, int kind = 0) {
   return HTR_OK;
 }
 
+// One row in a chain of dependent launches (packed_gemv1.cuh): one thread block per SM.  Small linears stay on the three small
+// blocks per SM of packed_gemv.cuh.
+constexpr long long kChainSmall = 1 << 21;
+static bool chain_serves(int m, int n) { return n <= kG1MaxCols && (long long)m * n >= kChainSmall; }
+static size_t chain_partial_bytes(int grid) { return (size_t)grid * 2 * 128 * sizeof(float); }
+static int make_chain_plan(int m, int n, Plan* out) {
+  int dev = 0;
+  if (const cudaError_t e = cudaGetDevice(&dev)) return cuda_fail((int)e);
+  const int sms = device_sms(dev);
+  if (sms <= 0) return cuda_fail((int)cudaErrorInvalidDevice);
+  const int units = (m / 128) * (n / 128);
+  *out = Plan{};
+  out->rbs = m / 128;
+  out->rows_t = 1;
+  out->units = units;
+  out->cg = n / 64;
+  out->grid = sms < units ? sms : units;
+  return HTR_OK;
+}
+
 // the counter region has one fixed size, so that calls of any shape share a workspace without moving it
 static size_t counter_bytes(int) { return (size_t)kCounterBytes; }
 
@@ -335,8 +356,10 @@ size_t htr_linear_workspace_bytes(int M, int m, int n, int K) {
       if ((size_t)tm.slots > slots) slots = (size_t)tm.slots;
     }
   }
+  const size_t chain = M == 1 && chain_serves(m, n) && make_chain_plan(m, n, &pl) == HTR_OK ? chain_partial_bytes(pl.grid) : 0;
   // up to four rows may run in an integer-exact form, whose partial sums are 64-bit
-  return counter_bytes(m) + (size_t)pl.rbs * slots * pl.rows_t * 128 * (M <= kMmaRows ? sizeof(long long) : sizeof(float));
+  const size_t part = (size_t)(m / 128) * slots * template_rows(M) * 128 * (M <= kMmaRows ? sizeof(long long) : sizeof(float));
+  return counter_bytes(m) + (part > chain ? part : chain);
 }
 
 int htr_linear_plan(int M, int m, int n, int K, int* grid, int* slots_per_block) {
@@ -425,9 +448,10 @@ static int launch_linear(const void* x, int dtype, int M, int n_in, const void* 
   int kind = gemv_kind(M, dtype, n, prologue);
   const bool exact = (flags & HTR_LINEAR_EXACT_SUMS) && prologue == 0 && (M <= 2 || kind == 2);
   if (exact && kind != 2) kind = 1;
-  const int rc = make_plan(M, m, n, K, &pl, kind);
+  const bool chain = kind == 0 && M == 1 && npeer == 0 && !(flags & HTR_LINEAR_INPUT_INDEPENDENT) && chain_serves(m, n);
+  const int rc = chain ? make_chain_plan(m, n, &pl) : make_plan(M, m, n, K, &pl, kind);
   if (rc != HTR_OK) return rc;
-  const size_t need = counter_bytes(m) + (size_t)pl.rbs * pl.slots * pl.rows_t * 128 * ((exact || kind == 2) ? sizeof(long long) : sizeof(float));
+  const size_t need = chain ? counter_bytes(m) + chain_partial_bytes(pl.grid) : counter_bytes(m) + (size_t)pl.rbs * pl.slots * pl.rows_t * 128 * ((exact || kind == 2) ? sizeof(long long) : sizeof(float));
   if (!workspace || workspace_bytes < need) return HTR_ERR_WORKSPACE;
 
   GemvParams p;
@@ -475,6 +499,17 @@ static int launch_linear(const void* x, int dtype, int M, int n_in, const void* 
   p.cb = (float)codebook_scale();
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int e = 0;
+  if (chain) {
+    switch (K) {
+      case 2: e = launch_packed_gemv1<2>(p, pl.grid, st); break;
+      case 3: e = launch_packed_gemv1<3>(p, pl.grid, st); break;
+      case 4: e = launch_packed_gemv1<4>(p, pl.grid, st); break;
+      case 5: e = launch_packed_gemv1<5>(p, pl.grid, st); break;
+      case 6: e = launch_packed_gemv1<6>(p, pl.grid, st); break;
+      case 8: e = launch_packed_gemv1<8>(p, pl.grid, st); break;
+    }
+    return e ? cuda_fail(e) : HTR_OK;
+  }
   if (kind == 2) {
     switch (K) {
       case 2: e = launch_packed_gemv_tm<2>(p, pl.grid, st); break;

@@ -333,14 +333,6 @@ __device__ __forceinline__ void gemm_finish_row(const GemmParams& p, const GemmT
                               flip(v[2] * kInvSqrt128, (t.sv_bits >> 2) & 1u) + t.bias.z, flip(v[3] * kInvSqrt128, t.sv_bits >> 3) + t.bias.w));
 }
 
-// flat form: even runs of 128-column blocks, the first `rem` thread blocks hold one more
-struct GemmRuns {
-  int q, rem;
-  __device__ __forceinline__ GemmRuns(int units, int grid) : q(units / grid), rem(units - (units / grid) * grid) {}
-  __device__ __forceinline__ int begin(int b) const { return b * q + min(b, rem); }
-  __device__ __forceinline__ int owner(int u) const { return u < rem * (q + 1) ? u / (q + 1) : rem + (u - rem * (q + 1)) / q; }
-};
-
 // rows j0, j0 + step, ... of row block rb from the partial sums of thread blocks first .. first + contributors - 1, added in that
 // order.  Two rows at a time: the loads of both are in flight together.  head: which partial of thread block `first`.
 template <bool GROUP>
@@ -394,7 +386,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     tiles = group_tiles(p.plan);
   }
   const int U = (GROUP ? tiles * p.rb_per_tile : p.mt >> 3) * HB;
-  const GemmRuns runs(U, gridDim.x);
+  const EvenRuns runs(U, gridDim.x);
   int u_begin, u_end, part_id = 0;
   if (!GROUP && p.split > 0) {
     const int rb = blockIdx.x / p.split;

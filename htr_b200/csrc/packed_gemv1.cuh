@@ -1,0 +1,270 @@
+// Packed GEMV for one activation row in a chain of dependent launches: one thread block per SM, decode and finishing overlapped.
+//
+//   y = sv * Ho( diag(scale * CB) * V * Hi(su * x) ),  V[i,j] = bytesum(h_ij) - 510      (the linear of packed_gemv.cuh)
+//
+// What bounds a dependent launch (a token of the decoder: four of them per layer): the decode at an SM's issue rate, and what no
+// weight is decoded in -- the release behind the predecessor, the staging of the activations, the hand-over of partial sums, the
+// tail.  packed_gemv.cuh with three small thread blocks per SM hides those parts of overlapping launches from one another, but in a
+// chain they add up, its blocks get 7 or 8 units each where 6.9 would do, and a scheduler serves its oldest warps first, so that
+// the three blocks of an SM end one after the other and the last one decodes alone (12288x4096: 10 to 23 us).  Here
+//  * every SM gets an even run of 128 x 128 blocks (flat over the row blocks), 16 decode warps take alternate blocks in two groups,
+//    each group kept together by a barrier per trip;
+//  * activations are staged once per SM, from one load per value also where a norm is folded in (the row stays in registers between
+//    its sum of squares and the transform);
+//  * at the end of a row block the decode warps leave their sums in shared memory and go on; four finisher warps add them, publish
+//    and finish;
+//  * a weight costs half an instruction less: its byte sum, as the bits of a float, is a subnormal number (n * 2^-149 exactly), and
+//    multiplied with activations staged times 2^80 it needs neither a magic constant nor its subtraction.  The constant 510 goes in
+//    per 16 columns, as -510 times their sum added to the accumulator first, so that the sums stay centred (no cancellation at the end).
+// MEASURED.
+#pragma once
+#include "packed_gemv.cuh"
+
+namespace htr {
+
+constexpr int kG1DecodeWarps = 16, kG1FinishWarps = 4, kG1Warps = kG1DecodeWarps + kG1FinishWarps, kG1Threads = kG1Warps * 32;
+#ifndef G1A
+#define G1A 2
+#endif
+constexpr int kG1Alu = G1A;
+constexpr int kG1MaxCols = 16384;                            // staged activations of a row: 64 KB
+constexpr float kG1Up = 1.2089258196146292e24f;              // 2^80: staged activations
+constexpr float kG1Down = 1.6940658945086007e-21f;           // 2^-69 = 2^80 * 2^-149: unit of the accumulators
+constexpr float kG1Out = 5.902958103587057e20f;              // 2^69
+
+template <int K>
+struct G1Ring {
+  static constexpr int tile_bytes = 32 * K, slot_bytes = 8 * tile_bytes;      // one warp, one trip: four strips x two units
+  static constexpr int slots = K <= 3 ? 5 : K <= 5 ? 4 : 3;
+  static constexpr int bytes = kG1DecodeWarps * slots * slot_bytes;
+};
+template <int K>
+constexpr int gemv1_smem_bytes(int n) { return G1Ring<K>::bytes + n * 4 + (n / 16) * 4; }
+
+template <int ID, int COUNT>
+__device__ __forceinline__ void named_sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory"); }
+__device__ __forceinline__ void named_sync_at(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+__device__ __forceinline__ void named_arrive_at(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+
+// 32 weights (two tile rows x 16 columns) of a lane against the tile's staged activations
+template <int K, int ALU4>
+__device__ __forceinline__ void unit_fma_subnormal(const uint32_t (&V)[K + 1], const float* __restrict__ xs, float offset, float2 (&acc)[2]) {
+  uint32_t s[32];
+  unit_states<K>(V, s);
+  acc[0].x += offset;
+  acc[1].x += offset;
+#pragma unroll
+  for (int quad = 0; quad < 4; ++quad) {
+    const float4 xv = *reinterpret_cast<const float4*>(xs + quad * 4);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int c0 = staged_col_inv<K>(quad * 4 + half * 2), c1 = staged_col_inv<K>(quad * 4 + half * 2 + 1);
+      const float2 xp = half ? make_float2(xv.z, xv.w) : make_float2(xv.x, xv.y);
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const uint32_t h0 = s[rr * 16 + c0] * kGenMul + kGenAdd, h1 = s[rr * 16 + c1] * kGenMul + kGenAdd;
+        const uint32_t b0 = (2 * half + 2 * rr) % 4 < ALU4 ? bytesum_add_alu(h0, 0u) : bytesum_add(h0, 0u);
+        const uint32_t b1 = (2 * half + 2 * rr + 1) % 4 < ALU4 ? bytesum_add_alu(h1, 0u) : bytesum_add(h1, 0u);
+        acc[rr] = __ffma2_rn(make_float2(__uint_as_float(b0), __uint_as_float(b1)), xp, acc[rr]);
+      }
+    }
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvParams p) {
+  using Ring = G1Ring<K>;
+  constexpr int kTileBytes = Ring::tile_bytes, kSlotBytes = Ring::slot_bytes, R = Ring::slots;
+  extern __shared__ __align__(128) unsigned char dyn_smem[];
+  __shared__ __align__(16) float s_red[2][kG1DecodeWarps][64];   // sums of a row block: [buffer][decode warp][its 64 rows]
+  __shared__ __align__(16) float ytil[128];
+  __shared__ float s_ss[kG1Warps];
+  __shared__ int s_arrival;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nt = p.nt, n = nt * 16, HB = nt >> 3;
+  const EvenRuns runs((p.mt >> 3) * HB, gridDim.x);
+  const int u_begin = runs.begin(blockIdx.x), u_end = runs.begin(blockIdx.x + 1);
+  float* xs = reinterpret_cast<float*>(dyn_smem + Ring::bytes);  // [n] staged activations, by column
+  float* xoff = xs + n;                                          // [n / 16] offset of every tile
+
+  // ---- decode warps: copy cursor over every second block of the run (warp = 64 rows h x tile column c of either unit)
+  const int h = warp & 1, c = (warp >> 1) & 3, group = warp >> 3, g = lane >> 3, q = lane & 7;
+  const unsigned char* my_ring = dyn_smem + ((warp < kG1DecodeWarps ? warp : 0) * R * 8 + g) * kTileBytes;
+  const uint32_t ring_dst = (uint32_t)__cvta_generic_to_shared(my_ring) + q * 16;
+  const int on_tail = (q + 8 * ((2 * K - 1) / 8) < 2 * K) ? -1 : 0;
+  const size_t next_strip = (size_t)7 * nt * kTileBytes * (HB == 1 ? 2 : 1);
+  int pf_left = 0, pf_in_rb = 1;
+  const char* pf = nullptr;
+  auto fetch = [&](uint32_t at) {
+    GemvTripCopies<K, 0, 0>::run(ring_dst + at, pf, pf_left, pf_left & on_tail);
+    pf_left -= 2;
+    const bool wrap = pf_in_rb <= 2;
+    pf_in_rb += wrap ? HB - 2 : -2;
+    pf += wrap ? next_strip + 16 * kTileBytes : (size_t)(16 * kTileBytes);
+    async_commit();
+  };
+  if (warp < kG1DecodeWarps) {
+    const int u = u_begin + group, rb = u / HB, hb = u - rb * HB;
+    pf_left = max(u_end - u, 0);
+    pf_in_rb = HB - hb;
+    pf = reinterpret_cast<const char*>(p.qw) + ((size_t)(rb * 8 + 4 * h + g) * nt + (size_t)hb * 8 + c) * kTileBytes + q * 16;
+#pragma unroll
+    for (int i = 0; i < R - 1; ++i) fetch(i * kSlotBytes);   // the weights do not depend on the preceding kernel
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // ---- activations of every column this thread block meets
+  const bool one_rb = u_begin / HB == (u_end - 1) / HB;
+  const int hb_first = one_rb ? u_begin % HB : 0, hb_last = one_rb ? hb_first + (u_end - u_begin) : HB;
+  auto stage = [&](int hb, float4 x4) {
+    const unsigned sg = sign_nibble(p.su, hb * 32 + lane);
+    float v[4] = {flip(x4.x, sg & 1u), flip(x4.y, (sg >> 1) & 1u), flip(x4.z, (sg >> 2) & 1u), flip(x4.w, sg >> 3)};
+    wht128(v, lane);
+    float* dst = xs + hb * 128 + (lane >> 2) * 16;
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float f = v[k] * kInvSqrt128;
+      dst[staged_col<K>(4 * (lane & 3) + k)] = f * kG1Up;
+      sum += f;
+    }
+    sum += __shfl_xor_sync(kFullWarp, sum, 1);
+    sum += __shfl_xor_sync(kFullWarp, sum, 2);
+    if ((lane & 3) == 0) xoff[hb * 8 + (lane >> 2)] = -510.0f * sum * kG1Down;
+  };
+  if (p.prologue == 1) {
+    constexpr int kHeld = (kG1MaxCols / 128 + kG1Warps - 1) / kG1Warps;
+    float4 held[kHeld];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int hb = warp + kG1Warps * i;
+      held[i] = hb < HB ? load_quad(p.x, hb * 128 + 4 * lane, p.dtype) : make_float4(0.f, 0.f, 0.f, 0.f);
+      ss += held[i].x * held[i].x + held[i].y * held[i].y + held[i].z * held[i].z + held[i].w * held[i].w;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(kFullWarp, ss, o);
+    if (lane == 0) s_ss[warp] = ss;
+    __syncthreads();
+    float tot = 0.f;
+#pragma unroll
+    for (int k = 0; k < kG1Warps; ++k) tot += s_ss[k];
+    const float inv = rsqrtf(tot / (float)n + p.eps);
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int hb = warp + kG1Warps * i;
+      if (hb >= hb_first && hb < hb_last) {
+        const float4 v = held[i], w = load_quad(p.norm_w, hb * 128 + 4 * lane, p.dtype);   // (the roundings of the unfused operators)
+        stage(hb, make_float4(bf16_round(bf16_round(v.x * inv) * w.x), bf16_round(bf16_round(v.y * inv) * w.y),
+                              bf16_round(bf16_round(v.z * inv) * w.z), bf16_round(bf16_round(v.w * inv) * w.w)));
+      }
+    }
+  } else {
+    for (int hb = hb_first + warp; hb < hb_last; hb += kG1Warps) stage(hb, fused_x(p, p.x, 0, hb * 128 + 4 * lane, 1.f));
+  }
+  __syncthreads();
+
+  if (warp < kG1DecodeWarps) {
+    float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    uint32_t at = 0u, refill = (R - 1) * kSlotBytes;         // ring slots of this trip and of the one before it
+    int seg = 0, u = u_begin + group;
+    for (int start = u_begin; start < u_end; ++seg) {
+      const int rb = start / HB, stop = min(u_end, (rb + 1) * HB);
+      const float* xt = xs + (u - rb * HB) * 128 + c * 16;
+      const float* ot = xoff + (u - rb * HB) * 8 + c;
+#pragma unroll 1
+      for (; u < stop; u += 2) {
+        async_wait<R - 2>();                                 // this trip's words have landed (own copies) ...
+        named_sync_at(6 + group, 256);                       // ... and those of the other lanes; the group's warps stay together
+        fetch(refill);
+        const uint32_t* tiles = reinterpret_cast<const uint32_t*>(my_ring + at);
+        refill = at;
+        at = at == (R - 1) * kSlotBytes ? 0u : at + kSlotBytes;
+        uint32_t V[K + 1];
+        read_unit_words<K>(tiles, q, V);
+        unit_fma_subnormal<K, kG1Alu>(V, xt, ot[0], acc);
+        read_unit_words<K>(tiles + 8 * K * 4, q, V);
+        unit_fma_subnormal<K, kG1Alu>(V, xt + 64, ot[4], acc);
+        xt += 256;
+        ot += 16;
+      }
+      // ---- this warp's part of row block rb: leave it for the finishers (two buffers)
+      const int buf = seg & 1;
+      if (seg >= 2) named_sync_at(3 + buf, kG1Threads);
+      *reinterpret_cast<float2*>(&s_red[buf][warp][g * 16 + 2 * q]) = make_float2(acc[0].x + acc[0].y, acc[1].x + acc[1].y);
+      acc[0] = acc[1] = make_float2(0.f, 0.f);
+      named_arrive_at(1 + buf, kG1Threads);
+      start = stop;
+    }
+    async_wait<0>();
+    return;
+  }
+
+  // ---- finishers: thread r owns row r of the row block
+  const int r = tid - kG1DecodeWarps * 32, segs = (u_end - 1) / HB - u_begin / HB + 1;
+  for (int seg = 0, start = u_begin; seg < segs; ++seg) {
+    const int rb = start / HB, buf = seg & 1;
+    const int first = runs.owner(rb * HB), contributors = runs.owner((rb + 1) * HB - 1) - first + 1;
+    start = (rb + 1) * HB;
+    // operands of the epilogue are fetched now so that their latency hides behind the hand-over
+    const int row0 = rb * 128 + 4 * lane;
+    const uint2 sc_raw = __ldg(reinterpret_cast<const uint2*>(p.scales + row0));
+    const unsigned sv_bits = sign_nibble(p.sv, rb * 32 + lane);
+    float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), old = bias4;
+    if (r < 32 && row0 < p.m_out) {
+      if (p.bias) bias4 = load_quad(p.bias, row0, p.dtype);
+      if (p.residual) old = load_quad(p.y, row0, p.dtype);
+    }
+    named_sync_at(1 + buf, kG1Threads);
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kG1DecodeWarps / 2; ++w) sum += s_red[buf][2 * w + (r >> 6)][r & 63];
+    if (seg + 2 < segs) named_arrive_at(3 + buf, kG1Threads);
+    bool finish = true;
+    if (contributors > 1) {
+      // a thread block has two partials: its first row block's and that of a later one (only its last is read by others)
+      __stcg(p.part + (size_t)(2 * blockIdx.x + (seg > 0 ? 1 : 0)) * 128 + r, sum);
+      named_sync<5, kG1FinishWarps * 32>();
+      if (r == 0) {
+        __threadfence();                                     // the partials of the thread block (ordered by the barrier) before the arrival
+        s_arrival = atomicAdd(p.counters + rb, 1);           // (they are read with loads served by L2, after this atomic)
+      }
+      named_sync<5, kG1FinishWarps * 32>();
+      finish = s_arrival == contributors - 1;
+      if (finish) {
+        if (r == 0) p.counters[rb] = 0;
+        const int head = runs.begin(first) < rb * HB ? 1 : 0;
+        const float* slot0 = p.part + (size_t)(2 * first) * 128 + r;
+        sum = 0.f;
+        for (int base = 0; base < contributors; base += 8) { // loads in flight together, added in thread-block order
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = base + j < contributors ? __ldcg(slot0 + (size_t)(base + j == 0 ? head : 2 * (base + j)) * 128) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) sum += v[j];
+        }
+      }
+    }
+    if (!finish) continue;
+    ytil[r] = sum * kG1Out;
+    named_sync<5, kG1FinishWarps * 32>();
+    if (r < 32) {
+      const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.y));
+      const float4 y4 = *reinterpret_cast<const float4*>(ytil + 4 * lane);
+      float v[4] = {y4.x * (s01.x * p.cb), y4.y * (s01.y * p.cb), y4.z * (s23.x * p.cb), y4.w * (s23.y * p.cb)};
+      wht128(v, lane);
+      float4 o = make_float4(flip(v[0] * kInvSqrt128, sv_bits & 1u) + bias4.x, flip(v[1] * kInvSqrt128, (sv_bits >> 1) & 1u) + bias4.y,
+                             flip(v[2] * kInvSqrt128, (sv_bits >> 2) & 1u) + bias4.z, flip(v[3] * kInvSqrt128, sv_bits >> 3) + bias4.w);
+      if (p.residual) o = make_float4(old.x + bf16_round(o.x), old.y + bf16_round(o.y), old.z + bf16_round(o.z), old.w + bf16_round(o.w));
+      if (row0 < p.m_out) store_quad(p.y, row0, p.dtype, o);
+    }
+    // (ytil is written again only behind the next barrier with the decode warps, which warp 0 reaches after this)
+  }
+}
+
+// host side, defined once per K in packed_gemv_k*.cu
+template <int K>
+int launch_packed_gemv1(const GemvParams& p, int grid, cudaStream_t stream);
+
+}  // namespace htr

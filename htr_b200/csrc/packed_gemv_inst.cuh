@@ -1,5 +1,6 @@
 // Instantiates the packed GEMV for one stream width; included by packed_gemv_k<K>.cu with HTR_INST_K set.
 #include "packed_gemv.cuh"
+#include "packed_gemv1.cuh"
 
 namespace htr {
 
@@ -51,6 +52,29 @@ int launch_packed_gemv<HTR_INST_K>(const GemvParams& p, int mt_rows, int grid, c
     case 8: return launch_one<HTR_INST_K, 8>(p, grid, stream);
   }
   return (int)cudaErrorInvalidValue;
+}
+
+template <>
+int launch_packed_gemv1<HTR_INST_K>(const GemvParams& p, int grid, cudaStream_t stream) {
+  static bool allowed[64] = {false};                      // shared memory beyond 48 KB: opted in once per device
+  int dev = 0;
+  if (const cudaError_t e = cudaGetDevice(&dev)) return (int)e;
+  if (dev < 0 || dev >= 64 || !allowed[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(packed_gemv1_kernel<HTR_INST_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemv1_smem_bytes<HTR_INST_K>(kG1MaxCols));
+    if (e != cudaSuccess) return (int)e;
+    if (dev >= 0 && dev < 64) allowed[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kG1Threads);
+  cfg.dynamicSmemBytes = (size_t)gemv1_smem_bytes<HTR_INST_K>(p.nt * 16);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = gemv_overlap_enabled() ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, packed_gemv1_kernel<HTR_INST_K>, p);
 }
 
 template <>
