@@ -7,8 +7,8 @@
 // tail.  packed_gemv.cuh with three small thread blocks per SM hides those parts of overlapping launches from one another, but in a
 // chain they add up, its blocks get 7 or 8 units each where 6.9 would do, and a scheduler serves its oldest warps first, so that
 // the three blocks of an SM end one after the other and the last one decodes alone (12288x4096: 10 to 23 us).  Here
-//  * every SM gets an even run of 128 x 128 blocks (flat over the row blocks), 16 decode warps take alternate blocks in two groups,
-//    each group kept together by a barrier per trip;
+//  * every SM gets an even run of 128 x 128 blocks (flat over the row blocks), 16 decode warps take alternate blocks in two groups
+//    (a barrier per trip to keep the warps of a group together cost 4 to 8 %);
 //  * activations are staged once per SM, from one load per value also where a norm is folded in (the row stays in registers between
 //    its sum of squares and the transform);
 //  * at the end of a row block the decode warps leave their sums in shared memory and go on; four finisher warps add them, publish
@@ -16,17 +16,15 @@
 //  * a weight costs half an instruction less: its byte sum, as the bits of a float, is a subnormal number (n * 2^-149 exactly), and
 //    multiplied with activations staged times 2^80 it needs neither a magic constant nor its subtraction.  The constant 510 goes in
 //    per 16 columns, as -510 times their sum added to the accumulator first, so that the sums stay centred (no cancellation at the end).
-// MEASURED.
+// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.5 -> 4.6, 12288x4096 K4 14.5 -> 13.1, 151936x4096 K4
+// 131 -> 102 (6.1e12 weights a second, 21 per cycle and SM).
 #pragma once
 #include "packed_gemv.cuh"
 
 namespace htr {
 
 constexpr int kG1DecodeWarps = 16, kG1FinishWarps = 4, kG1Warps = kG1DecodeWarps + kG1FinishWarps, kG1Threads = kG1Warps * 32;
-#ifndef G1A
-#define G1A 2
-#endif
-constexpr int kG1Alu = G1A;
+constexpr int kG1Alu = 2;                                    // byte sums of four that go to the shift/logic pipe (1, 3, 4: 2 to 3 % slower)
 constexpr int kG1MaxCols = 16384;                            // staged activations of a row: 64 KB
 constexpr float kG1Up = 1.2089258196146292e24f;              // 2^80: staged activations
 constexpr float kG1Down = 1.6940658945086007e-21f;           // 2^-69 = 2^80 * 2^-149: unit of the accumulators
@@ -176,7 +174,7 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
 #pragma unroll 1
       for (; u < stop; u += 2) {
         async_wait<R - 2>();                                 // this trip's words have landed (own copies) ...
-        named_sync_at(6 + group, 256);                       // ... and those of the other lanes; the group's warps stay together
+        __syncwarp();                                        // ... and those of the other lanes; the slot before it is free
         fetch(refill);
         const uint32_t* tiles = reinterpret_cast<const uint32_t*>(my_ring + at);
         refill = at;
