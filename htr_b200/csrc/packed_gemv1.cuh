@@ -110,13 +110,26 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     for (int i = 0; i < R - 1; ++i) fetch(i * kSlotBytes);   // the weights do not depend on the preceding kernel
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // ---- activations of every column this thread block meets: `count` blocks from its first one on, around the end of the row.
+  // A warp takes every 20th; signs and norm weights do not depend on the preceding kernel and are fetched before the wait
+  constexpr int kHeld = (kG1MaxCols / 128 + kG1Warps - 1) / kG1Warps;
+  const int hb0 = u_begin % HB, count = min(u_end - u_begin, HB);
+  auto block_at = [&](int i) { const int hb = hb0 + warp + kG1Warps * i; return hb >= HB ? hb - HB : hb; };
+  unsigned signs[kHeld];
+  uint2 gain[kHeld];
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    signs[i] = 0u;
+    gain[i] = make_uint2(0u, 0u);
+    if (warp + kG1Warps * i < count) {
+      // (in assembly so that nothing waits for the byte here)
+      asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(signs[i]) : "l"(p.su + block_at(i) * 16 + (lane >> 1)));
+      if (p.prologue == 1) gain[i] = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(p.norm_w) + block_at(i) * 128 + 4 * lane));
+    }
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // ---- activations of every column this thread block meets
-  const bool one_rb = u_begin / HB == (u_end - 1) / HB;
-  const int hb_first = one_rb ? u_begin % HB : 0, hb_last = one_rb ? hb_first + (u_end - u_begin) : HB;
-  auto stage = [&](int hb, float4 x4) {
-    const unsigned sg = sign_nibble(p.su, hb * 32 + lane);
+  auto stage = [&](int hb, unsigned sg, float4 x4) {
     float v[4] = {flip(x4.x, sg & 1u), flip(x4.y, (sg >> 1) & 1u), flip(x4.z, (sg >> 2) & 1u), flip(x4.w, sg >> 3)};
     wht128(v, lane);
     float* dst = xs + hb * 128 + (lane >> 2) * 16;
@@ -131,16 +144,14 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     sum += __shfl_xor_sync(kFullWarp, sum, 2);
     if ((lane & 3) == 0) xoff[hb * 8 + (lane >> 2)] = -510.0f * sum * kG1Down;
   };
+  float4 held[kHeld];                                        // every load of a warp is in flight before the first is used
   if (p.prologue == 1) {
-    constexpr int kHeld = (kG1MaxCols / 128 + kG1Warps - 1) / kG1Warps;
-    float4 held[kHeld];
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < kHeld; ++i) {
-      const int hb = warp + kG1Warps * i;
-      held[i] = hb < HB ? load_quad(p.x, hb * 128 + 4 * lane, p.dtype) : make_float4(0.f, 0.f, 0.f, 0.f);
-      ss += held[i].x * held[i].x + held[i].y * held[i].y + held[i].z * held[i].z + held[i].w * held[i].w;
-    }
+    for (int i = 0; i < kHeld; ++i)                          // the whole row, for its sum of squares
+      held[i] = warp + kG1Warps * i < HB ? load_quad(p.x, block_at(i) * 128 + 4 * lane, p.dtype) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) ss += held[i].x * held[i].x + held[i].y * held[i].y + held[i].z * held[i].z + held[i].w * held[i].w;
 #pragma unroll
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(kFullWarp, ss, o);
     if (lane == 0) s_ss[warp] = ss;
@@ -150,17 +161,20 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     for (int k = 0; k < kG1Warps; ++k) tot += s_ss[k];
     const float inv = rsqrtf(tot / (float)n + p.eps);
 #pragma unroll
-    for (int i = 0; i < kHeld; ++i) {
-      const int hb = warp + kG1Warps * i;
-      if (hb >= hb_first && hb < hb_last) {
-        const float4 v = held[i], w = load_quad(p.norm_w, hb * 128 + 4 * lane, p.dtype);   // (the roundings of the unfused operators)
-        stage(hb, make_float4(bf16_round(bf16_round(v.x * inv) * w.x), bf16_round(bf16_round(v.y * inv) * w.y),
-                              bf16_round(bf16_round(v.z * inv) * w.z), bf16_round(bf16_round(v.w * inv) * w.w)));
-      }
+    for (int i = 0; i < kHeld; ++i) {                        // (the roundings of the unfused operators)
+      const float4 v = held[i], w = make_float4(__uint_as_float(gain[i].x << 16), __uint_as_float(gain[i].x & 0xFFFF0000u),
+                                                __uint_as_float(gain[i].y << 16), __uint_as_float(gain[i].y & 0xFFFF0000u));
+      held[i] = make_float4(bf16_round(bf16_round(v.x * inv) * w.x), bf16_round(bf16_round(v.y * inv) * w.y),
+                            bf16_round(bf16_round(v.z * inv) * w.z), bf16_round(bf16_round(v.w * inv) * w.w));
     }
   } else {
-    for (int hb = hb_first + warp; hb < hb_last; hb += kG1Warps) stage(hb, fused_x(p, p.x, 0, hb * 128 + 4 * lane, 1.f));
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i)
+      if (warp + kG1Warps * i < count) held[i] = fused_x(p, p.x, 0, block_at(i) * 128 + 4 * lane, 1.f);
   }
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i)
+    if (warp + kG1Warps * i < count) stage(block_at(i), (signs[i] >> (4 * (lane & 1))) & 15u, held[i]);
   __syncthreads();
 
   if (warp < kG1DecodeWarps) {

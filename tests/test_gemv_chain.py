@@ -24,10 +24,11 @@ def test_one_row(coracle, K, m, n):
     x[0, :: 131] *= 500.0
     ref = coracle.linear(x.numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy(), bias=bias.numpy())
     y = ops.linear(x.to(dev), *d, bias.to(dev))
-    assert rel(y.cpu().numpy(), ref) <= 2e-6 and torch.equal(ops.linear(x.to(dev), *d, bias.to(dev)), y)
+    assert rel(y.cpu().numpy(), ref) <= 5e-6 and torch.equal(ops.linear(x.to(dev), *d, bias.to(dev)), y)
+    plain = coracle.linear(x.numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy())
     for scale in (1e-12, 1e9):                                        # the subnormal products keep their bits at either end
         z = ops.linear((x * scale).to(dev), *d)
-        assert rel(z.cpu().numpy() / scale, ref - bias.numpy()) <= 2e-6
+        assert rel(z.cpu().numpy() / scale, plain) <= 5e-6
     ones = torch.ones(1, n) * (1 - 2 * torch.from_numpy(np.unpackbits(su.numpy(), bitorder="little").astype(np.float32)))   # one spike per block
     assert rel(ops.linear(ones.to(dev), *d).cpu().numpy(), coracle.linear(ones.numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy())) <= 5e-6
     for dt in (torch.bfloat16, torch.float16):
