@@ -249,10 +249,11 @@ static int make_plan(int M, int m, int n, int K, Plan* out, int kind = 0) {
   return HTR_OK;
 }
 
-// One row in a chain of dependent launches (packed_gemv1.cuh): one thread block per SM.  Small linears stay on the three small
-// blocks per SM of packed_gemv.cuh.
-constexpr long long kChainSmall = 1 << 21;
-static bool chain_serves(int m, int n) { return n <= kG1MaxCols && (long long)m * n >= kChainSmall; }
+// One row in a chain of dependent launches (packed_gemv1.cuh): one thread block per SM.  At least as fast as the three small blocks per
+// SM of packed_gemv.cuh from 256 thousand weights on (512x512 4.1 us either way, 1024x1024 4.5 -> 4.1, 256x16384 10.5 -> 6.6), except
+// where most blocks of a run end a row block (32768x256: 5.2 against 5.6).
+constexpr long long kChainSmall = 1 << 18;
+static bool chain_serves(int m, int n) { return n <= kG1MaxCols && (long long)m * n >= kChainSmall && (n >= 512 || m < 16384); }
 static size_t chain_partial_bytes(int grid) { return (size_t)grid * 2 * 128 * sizeof(float); }
 static int make_chain_plan(int m, int n, Plan* out) {
   int dev = 0;

@@ -16,7 +16,7 @@
 //  * a weight costs half an instruction less: its byte sum, as the bits of a float, is a subnormal number (n * 2^-149 exactly), and
 //    multiplied with activations staged times 2^80 it needs neither a magic constant nor its subtraction.  The constant 510 goes in
 //    per 16 columns, as -510 times their sum added to the accumulator first, so that the sums stay centred (no cancellation at the end).
-// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.5 -> 4.6, 12288x4096 K4 14.5 -> 13.1, 151936x4096 K4
+// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.4 -> 4.9, 4096x12288 K4 13.8 -> 12.7, 151936x4096 K4
 // 131 -> 102 (6.1e12 weights a second, 21 per cycle and SM).
 #pragma once
 #include "packed_gemv.cuh"
