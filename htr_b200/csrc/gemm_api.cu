@@ -384,7 +384,7 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   while (g.stages > 1 && gemm_smem_bytes(g.np, planes, g.stages, words) > budget) --g.stages;
   g.smem = gemm_smem_bytes(g.np, planes, g.stages, words);
   if (g.stages < 2) return HTR_ERR_TOO_LARGE;
-  // Up to eight thread blocks share a row block as a cluster and reduce on chip, or every thread block of the GPU takes an even run
+  // Up to sixteen thread blocks share a row block as a cluster and reduce on chip, or every thread block of the GPU takes an even run
   // (flat) and a row block's partial sums meet in global memory at one last arriver.  Costs in units of one decoded 128 x 128 block
   // (0.43 us): the longest run, and for the flat form nine for the hand-over (measured 2 to 3 us) plus the partials that the last
   // arriver reads at about 100 bytes a nanosecond.  At 2048x2048, 8 / 200 rows, this chose clusters of four over flat runs: 11.5 / 33.2
@@ -393,7 +393,7 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   const long long flat_grid = slots < units ? slots : units, flat_run = (units + flat_grid - 1) / flat_grid;
   long long best = flat_run + 9 + (g.hb / flat_run + 1) * g.np / 84;
   g.split = 0;
-  for (int s = (int)(slots / g.rbs < 8 ? slots / g.rbs : 8); s >= 1; --s) {
+  for (int s = (int)(slots / g.rbs < 16 ? slots / g.rbs : 16); s >= 1; --s) {
     const long long run = (g.hb + s - 1) / s;
     if (s > g.hb || run >= best) continue;
     if (s == 1 || gemm_clusters(K, g.smem, s) >= g.rbs) {

@@ -16,6 +16,8 @@ int allow_smem(int dev) {
   if (e != cudaSuccess) return (int)e;
   const cudaError_t e2 = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
   if (e2 != cudaSuccess) return (int)e2;
+  const cudaError_t e3 = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // up to 16
+  if (e3 != cudaSuccess) return (int)e3;
   if (dev >= 0 && dev < 64) allowed[dev] = true;
   return 0;
 }

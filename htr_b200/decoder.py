@@ -9,9 +9,9 @@ projections (q|k|v, gate|up) are single packed linears, as the format prescribes
 Every packed linear goes through `htr_b200.ops.linear`.  The glue between them (residual add + RMSNorm, rotary embedding
 + KV-cache write, single-query grouped attention, SwiGLU) runs as four small fused kernels of the library
 (`htr_dec_*`, launched with programmatic stream serialisation so the following packed GEMV prefetches its weights while
-they run); `fused=False` evaluates the same glue with plain torch ops, which is how the kernels are checked.  Steps of at
-most 8 rows (decoding) fold the norms, the SwiGLU and the residual adds into the packed GEMVs themselves
-(`ops.linear_fused`) and, for a single token, the rotary embedding and cache write into the attention kernel: five launches
+they run); `fused=False` evaluates the same glue with plain torch ops, which is how the kernels are checked.  A single token
+(and two of small layers) folds the norms, the SwiGLU and the residual adds into the packed GEMVs themselves
+(`ops.linear_fused`) and the rotary embedding and cache write into the attention kernel: five launches
 per layer.  A decode step reads its position from a device tensor, so one CUDA graph captured once serves every step.
 """
 import dataclasses
@@ -191,11 +191,21 @@ class PackedDecoder:
         out = torch.stack((t1 * cos - t2 * sin, t1 * sin + t2 * cos), dim=-1)
         return out.flatten(-2).to(t.dtype)
 
+    def _folds(self, T):
+        """Whether a step of T rows runs with the glue folded into the GEMVs: one row; two rows of small layers, where launches count.
+        From there on the linears are faster on the tensor-core GEMM between separate glue kernels (8 layers of the 9B class,
+        2 / 3 / 8 rows: 810 / 946 / 1750 -> 774 / 788 / 815 us)."""
+        return T == 1 or (T == 2 and 2 * self.cfg.intermediate * self.cfg.hidden < 1 << 25)
+
+    def _cache_rows(self):
+        """Addresses of the first layer's cache rows and the bytes between layers."""
+        return self.k_cache.data_ptr(), self.v_cache.data_ptr(), self.k_cache.stride(0) * self.k_cache.element_size()
+
     def forward_fused(self, ids, pos):
         """The same step with the library's glue kernels (bf16 only)."""
         c, L_ = self.cfg, _lib.lib
         T = ids.shape[0]
-        if T <= ops.GEMV_MAX_M and self.fold:
+        if self.fold and self._folds(T):
             return self.forward_folded(ids, pos)
         dev = self.device
         st = torch.cuda.current_stream(dev).cuda_stream
@@ -205,15 +215,18 @@ class PackedDecoder:
         att = torch.empty_like(q)
         act = torch.empty(T, c.intermediate, dtype=self.dtype, device=dev)
         delta = None
+        kp, vp, layer_bytes = self._cache_rows()
+        cosp, sinp, posp, statp = self.cos.data_ptr(), self.sin.data_ptr(), pos.data_ptr(), self.status.data_ptr()
         for li, L in enumerate(self.layers):
+            kl, vl = kp + li * layer_bytes, vp + li * layer_bytes
             _lib.check(L_.htr_dec_add_rmsnorm(x.data_ptr(), None if delta is None else delta.data_ptr(), L["ln1"].data_ptr(), h.data_ptr(),
                                               T, c.hidden, c.eps, st), "htr_dec_add_rmsnorm")
             qkv = ops.linear(h, *L["qkv"])
-            _lib.check(L_.htr_dec_rope_cache(qkv.data_ptr(), pos.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), q.data_ptr(),
-                                             self.k_cache[li].data_ptr(), self.v_cache[li].data_ptr(), T, c.q_heads, c.kv_heads, c.head_dim,
-                                             c.max_len, self.status.data_ptr(), st), "htr_dec_rope_cache")
-            _lib.check(L_.htr_dec_attention(q.data_ptr(), self.k_cache[li].data_ptr(), self.v_cache[li].data_ptr(), pos.data_ptr(),
-                                            att.data_ptr(), T, c.q_heads, c.kv_heads, c.head_dim, c.max_len, self.status.data_ptr(), st),
+            _lib.check(L_.htr_dec_rope_cache(qkv.data_ptr(), posp, cosp, sinp, q.data_ptr(),
+                                             kl, vl, T, c.q_heads, c.kv_heads, c.head_dim,
+                                             c.max_len, statp, st), "htr_dec_rope_cache")
+            _lib.check(L_.htr_dec_attention(q.data_ptr(), kl, vl, posp,
+                                            att.data_ptr(), T, c.q_heads, c.kv_heads, c.head_dim, c.max_len, statp, st),
                        "htr_dec_attention")
             o = ops.linear(att.view(T, c.q_heads * c.head_dim), *L["o"])
             _lib.check(L_.htr_dec_add_rmsnorm(x.data_ptr(), o.data_ptr(), L["ln2"].data_ptr(), h.data_ptr(), T, c.hidden, c.eps, st),
@@ -226,7 +239,7 @@ class PackedDecoder:
         return ops.linear(h, *self.head)
 
     def forward_folded(self, ids, pos):
-        """Decode-sized step (at most 8 rows) with the norms, the SwiGLU and the residual adds folded into the packed GEMVs
+        """Decode-sized step (at most 8 rows; see `_folds`) with the norms, the SwiGLU and the residual adds folded into the packed GEMVs
         (`ops.linear_fused`): six launches per layer instead of nine, five for a single token."""
         c, L_ = self.cfg, _lib.lib
         T = ids.shape[0]
@@ -235,19 +248,22 @@ class PackedDecoder:
         x = self.embed.index_select(0, ids)                     # residual stream, updated in place by the o and down projections
         q = torch.empty(T, c.q_heads, c.head_dim, dtype=self.dtype, device=dev)
         att = torch.empty_like(q)
+        kp, vp, layer_bytes = self._cache_rows()
+        cosp, sinp, posp, statp = self.cos.data_ptr(), self.sin.data_ptr(), pos.data_ptr(), self.status.data_ptr()
         for li, L in enumerate(self.layers):
+            kl, vl = kp + li * layer_bytes, vp + li * layer_bytes
             qkv = ops.linear_fused(x, *L["qkv"], prologue=ops.PROLOGUE_RMSNORM, norm_weight=L["ln1"], eps=c.eps)
             if T == 1:                                          # one token: rotary embedding, cache write and attention in one launch
-                _lib.check(L_.htr_dec_rope_attention(qkv.data_ptr(), pos.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(),
-                                                     self.k_cache[li].data_ptr(), self.v_cache[li].data_ptr(), att.data_ptr(),
-                                                     c.q_heads, c.kv_heads, c.head_dim, c.max_len, self.status.data_ptr(), st),
+                _lib.check(L_.htr_dec_rope_attention(qkv.data_ptr(), posp, cosp, sinp,
+                                                     kl, vl, att.data_ptr(),
+                                                     c.q_heads, c.kv_heads, c.head_dim, c.max_len, statp, st),
                            "htr_dec_rope_attention")
             else:
-                _lib.check(L_.htr_dec_rope_cache(qkv.data_ptr(), pos.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), q.data_ptr(),
-                                                 self.k_cache[li].data_ptr(), self.v_cache[li].data_ptr(), T, c.q_heads, c.kv_heads, c.head_dim,
-                                                 c.max_len, self.status.data_ptr(), st), "htr_dec_rope_cache")
-                _lib.check(L_.htr_dec_attention(q.data_ptr(), self.k_cache[li].data_ptr(), self.v_cache[li].data_ptr(), pos.data_ptr(),
-                                                att.data_ptr(), T, c.q_heads, c.kv_heads, c.head_dim, c.max_len, self.status.data_ptr(), st),
+                _lib.check(L_.htr_dec_rope_cache(qkv.data_ptr(), posp, cosp, sinp, q.data_ptr(),
+                                                 kl, vl, T, c.q_heads, c.kv_heads, c.head_dim,
+                                                 c.max_len, statp, st), "htr_dec_rope_cache")
+                _lib.check(L_.htr_dec_attention(q.data_ptr(), kl, vl, posp,
+                                                att.data_ptr(), T, c.q_heads, c.kv_heads, c.head_dim, c.max_len, statp, st),
                        "htr_dec_attention")
             ops.linear_fused(att.view(T, c.q_heads * c.head_dim), *L["o"], out=x, residual=True)
             gu = ops.linear_fused(x, *L["gate_up"], prologue=ops.PROLOGUE_RMSNORM, norm_weight=L["ln2"], eps=c.eps)
