@@ -314,8 +314,7 @@ constexpr size_t kCounterRegion = 1 << 16;   // same fixed counter region as the
 constexpr size_t kErrorRegion = 256;
 
 struct GemmPlan {
-  int np, rbs, hb, split, grid, stages, smem, sms, rbp, direct;
-  double cost;
+  int np, rbs, hb, split, grid, stages, smem, sms;
   size_t off_xb, off_xsum, off_tok, off_part, total;
 };
 
@@ -335,26 +334,26 @@ double codebook_scale() {
   return value;
 }
 
-int gemm_clusters(int K, int rbp, int smem, int split) {
+int gemm_clusters(int K, int smem, int split) {
   switch (K) {
-    case 2: return packed_gemm_tc_clusters<2>(rbp, smem, split);
-    case 3: return packed_gemm_tc_clusters<3>(rbp, smem, split);
-    case 4: return packed_gemm_tc_clusters<4>(rbp, smem, split);
-    case 5: return packed_gemm_tc_clusters<5>(rbp, smem, split);
-    case 6: return packed_gemm_tc_clusters<6>(rbp, smem, split);
-    case 8: return packed_gemm_tc_clusters<8>(rbp, smem, split);
+    case 2: return packed_gemm_tc_clusters<2>(smem, split);
+    case 3: return packed_gemm_tc_clusters<3>(smem, split);
+    case 4: return packed_gemm_tc_clusters<4>(smem, split);
+    case 5: return packed_gemm_tc_clusters<5>(smem, split);
+    case 6: return packed_gemm_tc_clusters<6>(smem, split);
+    case 8: return packed_gemm_tc_clusters<8>(smem, split);
   }
   return 0;
 }
 
-int launch_gemm(int K, const GemmParams& p, int rbp, int grid, int smem, cudaStream_t st) {
+int launch_gemm(int K, const GemmParams& p, int grid, int smem, cudaStream_t st) {
   switch (K) {
-    case 2: return launch_packed_gemm_tc<2>(p, rbp, grid, smem, st);
-    case 3: return launch_packed_gemm_tc<3>(p, rbp, grid, smem, st);
-    case 4: return launch_packed_gemm_tc<4>(p, rbp, grid, smem, st);
-    case 5: return launch_packed_gemm_tc<5>(p, rbp, grid, smem, st);
-    case 6: return launch_packed_gemm_tc<6>(p, rbp, grid, smem, st);
-    case 8: return launch_packed_gemm_tc<8>(p, rbp, grid, smem, st);
+    case 2: return launch_packed_gemm_tc<2>(p, grid, smem, st);
+    case 3: return launch_packed_gemm_tc<3>(p, grid, smem, st);
+    case 4: return launch_packed_gemm_tc<4>(p, grid, smem, st);
+    case 5: return launch_packed_gemm_tc<5>(p, grid, smem, st);
+    case 6: return launch_packed_gemm_tc<6>(p, grid, smem, st);
+    case 8: return launch_packed_gemm_tc<8>(p, grid, smem, st);
   }
   return (int)cudaErrorInvalidValue;
 }
@@ -362,79 +361,7 @@ int launch_gemm(int K, const GemmParams& p, int rbp, int grid, int smem, cudaStr
 // activation rows per launch after padding: accumulator columns come in multiples of 16
 int padded_rows(int M, int planes) { return planes == 2 ? (M + 7) / 8 * 8 : (M + 15) / 16 * 16; }
 
-// One launch of `rbp` row blocks per unit; false where it does not fit.  Costs are in units of one decoded 128 x 128 block (0.43 us).
-// A unit takes the longest of its decode, its MMAs (50 cycles each up to 92 columns, then by their width) and the way of its B tile from
-// L2: 60 bytes a cycle into one SM, 2600 into all of them together.  Up to sixteen thread blocks share a row block (pair) as a cluster
-// and reduce on chip, or every thread block of the GPU takes an even run (flat) and a row block's partial sums meet in global memory at
-// one last arriver: nine more for the hand-over (measured 2 to 3 us) and the partials, which that one reads at 100 bytes a nanosecond.
-// Measured, flat -> as chosen: 2048x2048, 8 / 200 rows 11.5 / 33.2 -> 7.6 / 16.9 us; 6144x4096, 8 rows 14.6 -> 12.7.
-bool plan_launch(int sms, int m, int n, int K, int planes, int np, int rbp, GemmPlan* out) {
-  GemmPlan g;
-  g.sms = sms;
-  g.np = np;
-  g.rbp = rbp;
-  g.rbs = m / 128;
-  g.hb = n / 128;
-  const int ncols = np * planes, words = gemm_word_bytes(K), rows = (g.rbs + rbp - 1) / rbp;   // rows of units
-  // one thread block per SM; as many stages as its tensor memory and shared memory hold, the finishers' exchange buffer where it fits
-  const int most = (kGemmTmemCols - rbp * gemm_acc_cols(ncols)) / (64 * rbp);
-  for (g.direct = 1; g.direct >= 0; --g.direct) {
-    g.stages = most > kGemmMaxStages ? kGemmMaxStages : most;
-    const int extra = words + (g.direct ? kExchangeBytes : 0);
-    while (g.stages > 1 && gemm_smem_bytes(np, planes, g.stages, rbp, extra) > kGemmMaxSmem) --g.stages;
-    g.smem = gemm_smem_bytes(np, planes, g.stages, rbp, extra);
-    if (g.stages >= 2 && g.smem <= kGemmMaxSmem) break;
-  }
-  if (g.direct < 0) return false;
-  const double mma = 8.0 * (ncols > 92 ? 0.54 * ncols : 50.0) / 845.0;
-  const auto unit = [&](int active) {
-    const double b = ncols * (active > 43 ? active / 8680.0 : 0.005), work = rbp * (mma > 1.0 ? mma : 1.0);
-    return b > work ? b : work;
-  };
-  const long long units = (long long)rows * g.hb, flat_grid = sms < units ? sms : units, flat_run = (units + flat_grid - 1) / flat_grid;
-  g.cost = flat_run * unit((int)flat_grid) + 9.0 + (g.hb / flat_run + 1) * rbp * np / 84.0;
-  g.split = 0;
-  g.grid = (int)flat_grid;
-  for (int s = sms / rows < 16 ? sms / rows : 16; s >= 1; --s) {
-    if (s > g.hb) continue;
-    const double cost = (double)((g.hb + s - 1) / s) * unit(rows * s);
-    if (cost >= g.cost) continue;
-    if (s == 1 || gemm_clusters(K, rbp, g.smem, s) >= rows) {
-      g.split = s;
-      g.grid = rows * s;
-      g.cost = cost;
-    }
-  }
-  size_t off = kCounterRegion + kErrorRegion;
-  g.off_xb = off; off += align256((size_t)ncols * n * 2);
-  g.off_xsum = off; off += align256((size_t)np * gemm_rht_slices(np, n) * 4);
-  g.off_tok = off; off += align256((size_t)np * 4);
-  g.off_part = off;
-  if (g.split == 0) off += align256((size_t)g.grid * 2 * rbp * np * 128 * 4);
-  g.total = off;
-  *out = g;
-  return true;
-}
-
-// How M rows are run: `rows` of them per launch, each as plan_launch finds cheapest with one or two row blocks per unit.  (Several
-// launches decode the weight several times, but a launch of 256 columns waits four times as long for its B tiles as for its decode.)
-// `bytes`: workspace that any of the launches needs.  Remembered per thread: the answer costs a few microseconds.
-struct GemmSchedule {
-  int rows;
-  GemmPlan plan;      // of a launch with `rows` rows
-  GemmPlan last;      // of the last launch, which may have fewer
-  size_t bytes;
-};
-int schedule_rows(int sms, int M, int m, int n, int K, int planes, GemmPlan* out) {
-  const int np = padded_rows(M, planes);
-  if (np * planes > kGemmMaxCols) return HTR_ERR_TOO_LARGE;
-  GemmPlan two;
-  const bool one_fits = plan_launch(sms, m, n, K, planes, np, 1, out);
-  const bool two_fits = np * planes > 32 && m > 128 && plan_launch(sms, m, n, K, planes, np, 2, &two);
-  if (two_fits && (!one_fits || two.cost < out->cost)) *out = two;
-  return one_fits || two_fits ? HTR_OK : HTR_ERR_TOO_LARGE;
-}
-int make_schedule(int M, int m, int n, int K, int planes, GemmSchedule* out) {
+int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return HTR_ERR_CUDA;
   static int seen_sms[64] = {0};                          // a device fact: asked once (every caller would store the same number)
@@ -443,35 +370,46 @@ int make_schedule(int M, int m, int n, int K, int planes, GemmSchedule* out) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return HTR_ERR_CUDA;
     if (dev >= 0 && dev < 64) seen_sms[dev] = sms;
   }
-  struct Seen { int dev, M, m, n, K, planes; GemmSchedule schedule; };
-  static thread_local Seen seen[64] = {};
-  Seen& slot = seen[((unsigned)M * 2654435761u + (unsigned)m * 40503u + (unsigned)n * 9973u + (unsigned)(K * 2 + planes)) >> 7 & 63u];
-  if (slot.M == M && slot.m == m && slot.n == n && slot.K == K && slot.planes == planes && slot.dev == dev) {
-    *out = slot.schedule;
-    return HTR_OK;
-  }
-  GemmSchedule best;
-  best.rows = 0;
-  double best_cost = 0;
-  const int unit = planes == 2 ? 8 : 16;
-  for (int parts = 1; parts <= 4; ++parts) {
-    GemmSchedule c;
-    c.rows = ((M + parts - 1) / parts + unit - 1) / unit * unit;
-    if (c.rows > M) c.rows = M;
-    if (parts > 1 && c.rows * planes < 64) break;
-    if (schedule_rows(sms, c.rows, m, n, K, planes, &c.plan) != HTR_OK) continue;
-    const int launches = (M + c.rows - 1) / c.rows, rest = M - (launches - 1) * c.rows;
-    if (schedule_rows(sms, rest, m, n, K, planes, &c.last) != HTR_OK) continue;
-    c.bytes = c.plan.total > c.last.total ? c.plan.total : c.last.total;
-    const double cost = (launches - 1) * (c.plan.cost + 6.0) + c.last.cost + 6.0;
-    if (best.rows == 0 || cost < best_cost) {
-      best = c;
-      best_cost = cost;
+  GemmPlan g;
+  g.sms = sms;
+  g.np = padded_rows(M, planes);
+  g.rbs = m / 128;
+  g.hb = n / 128;
+  const int ncols = g.np * planes;
+  if (ncols > kGemmMaxCols) return HTR_ERR_TOO_LARGE;
+  // one thread block per SM; as many stages as its tensor memory and shared memory hold
+  const int words = gemm_word_bytes(K), budget = 226 * 1024;
+  g.stages = (kGemmTmemCols - gemm_acc_cols(ncols)) / 64;
+  if (g.stages > kGemmMaxStages) g.stages = kGemmMaxStages;
+  while (g.stages > 1 && gemm_smem_bytes(g.np, planes, g.stages, words) > budget) --g.stages;
+  g.smem = gemm_smem_bytes(g.np, planes, g.stages, words);
+  if (g.stages < 2) return HTR_ERR_TOO_LARGE;
+  // Up to sixteen thread blocks share a row block as a cluster and reduce on chip, or every thread block of the GPU takes an even run
+  // (flat) and a row block's partial sums meet in global memory at one last arriver.  Costs in units of one decoded 128 x 128 block
+  // (0.43 us): the longest run, and for the flat form nine for the hand-over (measured 2 to 3 us) plus the partials that the last
+  // arriver reads at about 100 bytes a nanosecond.  At 2048x2048, 8 / 200 rows, this chose clusters of four over flat runs: 11.5 / 33.2
+  // -> 7.6 / 16.9 us; 6144x4096, 8 rows: 14.6 -> 12.7.
+  const long long slots = sms, units = (long long)g.rbs * g.hb;
+  const long long flat_grid = slots < units ? slots : units, flat_run = (units + flat_grid - 1) / flat_grid;
+  long long best = flat_run + 9 + (g.hb / flat_run + 1) * g.np / 84;
+  g.split = 0;
+  for (int s = (int)(slots / g.rbs < 16 ? slots / g.rbs : 16); s >= 1; --s) {
+    const long long run = (g.hb + s - 1) / s;
+    if (s > g.hb || run >= best) continue;
+    if (s == 1 || gemm_clusters(K, g.smem, s) >= g.rbs) {
+      g.split = s;
+      best = run;
     }
   }
-  if (best.rows == 0) return HTR_ERR_TOO_LARGE;
-  slot = Seen{dev, M, m, n, K, planes, best};
-  *out = best;
+  g.grid = g.split > 0 ? g.rbs * g.split : (int)flat_grid;
+  size_t off = kCounterRegion + kErrorRegion;
+  g.off_xb = off; off += align256((size_t)ncols * n * 2);
+  g.off_xsum = off; off += align256((size_t)g.np * gemm_rht_slices(g.np, n) * 4);
+  g.off_tok = off; off += align256((size_t)g.np * 4);
+  g.off_part = off;
+  if (g.split == 0) off += align256((size_t)g.grid * 2 * g.np * 128 * 4);
+  g.total = off;
+  *out = g;
   return HTR_OK;
 }
 
@@ -483,8 +421,8 @@ using namespace htr;
 extern "C" {
 
 static size_t plan_bytes(int M, int m, int n, int K, int planes) {
-  GemmSchedule g;
-  return make_schedule(M, m, n, K, planes, &g) == HTR_OK ? g.bytes : 0;
+  GemmPlan g;
+  return make_gemm_plan(M, m, n, K, planes, &g) == HTR_OK ? g.total : 0;
 }
 
 size_t htr_linear_gemm_workspace_bytes(int M, int m, int n, int K) {
@@ -537,54 +475,48 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   const auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
   if (!a16(x) || !a16(qweight) || !a16(y) || (bias && !a16(bias)) || !a16(workspace) || !a16(scales)) return HTR_ERR_ALIGNMENT;
   const int m = mt * 16, n = nt * 16;
+  GemmPlan g;
   const int planes = gemm_planes(dtype, M, fine);
   if (planes == 2 && M > HTR_GEMM_MAX_ROWS_F32) return HTR_ERR_BAD_SHAPE;
-  GemmSchedule schedule;
-  const int rc = make_schedule(M, m, n, K, planes, &schedule);
+  const int rc = make_gemm_plan(M, m, n, K, planes, &g);
   if (rc != HTR_OK) return rc;
-  if (!workspace || workspace_bytes < schedule.bytes) return HTR_ERR_WORKSPACE;
+  if (!workspace || workspace_bytes < g.total) return HTR_ERR_WORKSPACE;
   char* ws = static_cast<char*>(workspace);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t esize = dtype == HTR_DTYPE_F32 ? 4 : 2;
-  GemmParams p = {};
+  GemmParams p;
   p.qw = static_cast<const uint32_t*>(qweight);
   p.scales = static_cast<const __half*>(scales);
   p.sv = sv;
   p.bias = bias;
+  p.y = y;
+  p.xb = reinterpret_cast<const __half*>(ws + g.off_xb);
+  p.xsum = reinterpret_cast<const float*>(ws + g.off_xsum);
+  p.tok = reinterpret_cast<const float*>(ws + g.off_tok);
+  p.part = reinterpret_cast<float*>(ws + g.off_part);
   p.counters = reinterpret_cast<int*>(ws);
   p.error = reinterpret_cast<int*>(ws + kCounterRegion);
+  p.rows = M;
+  p.np = g.np;
   p.planes = planes;
   p.mt = mt;
   p.nt = nt;
-  p.rbs = m / 128;
   p.dtype = dtype;
-  p.hb = n / 128;
+  p.hb = g.hb;
+  p.split = g.split;
+  p.stages = g.stages;
   p.m_out = m_out;
+  p.xsum_slices = gemm_rht_slices(g.np, n);
   p.cb = (float)codebook_scale();
+  p.plan = nullptr;
   p.npeer = npeer;
+  p.peer_offset = peer_offset;
   for (int i = 0; i < 8; ++i) p.peer_y[i] = i < npeer ? peer_y[i] : nullptr;
-  for (int r0 = 0; r0 < M; r0 += schedule.rows) {
-    const int rows = M - r0 < schedule.rows ? M - r0 : schedule.rows;
-    const GemmPlan& g = r0 + rows == M ? schedule.last : schedule.plan;
-    float *xsum = reinterpret_cast<float*>(ws + g.off_xsum), *tok = reinterpret_cast<float*>(ws + g.off_tok);
-    __half* xb = reinterpret_cast<__half*>(ws + g.off_xb);
-    p.y = y ? static_cast<char*>(y) + (size_t)r0 * m_out * esize : nullptr;
-    p.peer_offset = peer_offset + (int64_t)r0 * m_out;
-    p.xb = xb;
-    p.xsum = xsum;
-    p.tok = tok;
-    p.part = reinterpret_cast<float*>(ws + g.off_part);
-    p.rows = rows;
-    p.np = g.np;
-    p.split = g.split;
-    p.stages = g.stages;
-    p.direct = g.direct && g.split == 0 && npeer == 0 ? 1 : 0;
-    p.xsum_slices = gemm_rht_slices(g.np, n);
-    int e = run_rht_f16(static_cast<const char*>(x) + (size_t)r0 * n_in * esize, dtype, rows, g.np, n, n_in, planes, su, xb, xsum, tok, st);
-    if (!e) e = launch_gemm(K, p, g.rbp, g.grid, g.smem, st);
-    if (e) { t_gemm_cuda = e; return HTR_ERR_CUDA; }
-  }
-  return HTR_OK;
+  int e = run_rht_f16(x, dtype, M, g.np, n, n_in, planes, su, reinterpret_cast<__half*>(ws + g.off_xb), reinterpret_cast<float*>(ws + g.off_xsum),
+                      reinterpret_cast<float*>(ws + g.off_tok), st);
+  if (e) { t_gemm_cuda = e; return HTR_ERR_CUDA; }
+  e = launch_gemm(K, p, g.grid, g.smem, st);
+  if (e) t_gemm_cuda = e;
+  return e ? HTR_ERR_CUDA : HTR_OK;
 }
 
 // ---- grouped form: the experts of a mixture-of-experts step
@@ -603,10 +535,9 @@ static int group_layout(int count, int table_rows, int m, int n, int K, GroupLay
   g->cap = group_cap(count, table_rows);
   if (g->cap > kGroupMaxTiles || (long long)g->cap * (m / 128) > (int)(kCounterRegion / 4) || (long long)g->cap * (m / 128) * (n / 128) > 0x3FFFFFFF)
     return HTR_ERR_TOO_LARGE;
-  GemmSchedule schedule;                                     // stages and shared memory of a launch with these columns
-  const int rc = make_schedule(kGroupRows, m, n, K, 2, &schedule);
+  GemmPlan plan;                                             // stages, shared memory and thread blocks of a launch with these columns
+  const int rc = make_gemm_plan(kGroupRows, m, n, K, 2, &plan);
   if (rc != HTR_OK) return rc;
-  const GemmPlan& plan = schedule.last;
   g->stages = plan.stages;
   g->smem = plan.smem;
   g->grid = plan.sms;
@@ -693,7 +624,7 @@ int htr_linear_routed_gemm(const void* x, int dtype, int x_div, int64_t x_row_st
   p.g_qw = reinterpret_cast<const uint32_t* const*>(qweight_table);
   p.g_scales = reinterpret_cast<const __half* const*>(scales_table);
   p.g_sv = sv_table;
-  e = launch_gemm(K, p, 1, g.grid, g.smem, st);
+  e = launch_gemm(K, p, g.grid, g.smem, st);
   if (e) t_gemm_cuda = e;
   return e ? HTR_ERR_CUDA : HTR_OK;
 }

@@ -34,11 +34,7 @@
 // apply scales, output transform and signs, and store.  (Done by the decode warps, that chain of dependent loads cost 12 000 cycles
 // per row block, a fifth of the LM head at 8 rows.)  The last row block of a thread block is finished by all its warps.
 //
-// RBP row blocks per unit: 1, or 2 for batches above some 60 rows, whose B tile then takes longer to come from L2 (all SMs read the same
-// tiles: about 5 TB/s together) than a block takes to decode.  With 2 each decode group owns one row block of every unit, a stage holds
-// both A tiles beside one B tile, and B crosses from L2 half as often (RBPFIG).
-//
-// Decomposition.  Work = (row block or pair) x (128-column blocks).  Where the row blocks are few, `split` thread blocks share one as a
+// Decomposition.  Work = (row block) x (128-column blocks).  Where the row blocks are few, `split` thread blocks share one as a
 // cluster and reduce through distributed shared memory; else every thread block takes an even contiguous run that may cross row
 // blocks (flat), publishes a partial [np][128] per row block it touches, and the last arriver adds them in thread-block order.
 // Both are deterministic and nobody waits for another thread block except inside a cluster.  One thread block per SM, not two: the
@@ -59,7 +55,6 @@ constexpr int kGemmFinishWarps = 4;
 constexpr int kGemmWarps = kGemmDecodeWarps + 2 + kGemmFinishWarps;
 constexpr int kGemmThreads = kGemmWarps * 32;
 constexpr int kGemmTmemCols = 512;                          // the accumulator first, then 64 columns of A per stage
-constexpr int kGemmMaxSmem = 222 * 1024;                    // dynamic shared memory of a thread block (the static part holds the rest)
 constexpr int kGemmMaxCols = 256;                           // accumulator columns (activation rows x planes) per launch
 constexpr int kLbo = 128;                                   // bytes between core matrices of B adjacent in K
 constexpr int kSboB = 1024;                                 // bytes between its 8-column groups (64 k x 8 columns x 2 bytes)
@@ -82,8 +77,6 @@ struct GemmParams {
   int rows, np;           // activation rows present / padded (to 16, or 8 with two planes)
   int planes;
   int mt, nt;
-  int rbs;                // row blocks of the weight
-  int direct;             // 1: the finishers keep a column exchange buffer behind the packed-word rings (flat form)
   int m_out;              // rows of the weight that are written (row stride of y, length of bias)
   int dtype;
   int hb;                 // 128-column blocks per row block (n / 128)
@@ -213,12 +206,11 @@ __device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&r)[8]) {
 // dynamic shared memory: the B ring (the cluster form reuses it for the [np][128] float partial of the thread block), then the
 // packed-word rings of the decode warps (`words` bytes)
 __host__ __device__ inline int gemm_stage_bytes(int ncols) { return ncols * 256; }
-__host__ __device__ inline int gemm_ring_bytes(int np, int planes, int stages, int rbp) {
-  const int ring = stages * gemm_stage_bytes(np * planes), result = rbp * np * 128 * 4;
+__host__ __device__ inline int gemm_ring_bytes(int np, int planes, int stages) {
+  const int ring = stages * gemm_stage_bytes(np * planes), result = np * 128 * 4;
   return ring > result ? ring : result;
 }
-__host__ __device__ inline int gemm_smem_bytes(int np, int planes, int stages, int rbp, int words) { return gemm_ring_bytes(np, planes, stages, rbp) + words + 128; }
-constexpr int kExchangeCols = 16, kExchangeBytes = 2 * 4 * kExchangeCols * 32 * 4;   // of the finishers: two buffers of [quadrant][column][lane]
+__host__ __device__ inline int gemm_smem_bytes(int np, int planes, int stages, int words) { return gemm_ring_bytes(np, planes, stages) + words + 128; }
 __host__ __device__ inline int gemm_acc_cols(int ncols) { return ncols < 32 ? 32 : ncols; }
 
 // ---- packed-word ring of a decode warp: one slot = the tiles of its strip in one 128-column block (two units of four tiles).
@@ -342,14 +334,13 @@ __device__ __forceinline__ void gemm_finish_row(const GemmParams& p, const GemmT
 }
 
 // rows j0, j0 + step, ... of row block rb from the partial sums of thread blocks first .. first + contributors - 1, added in that
-// order.  Two rows at a time: the loads of both are in flight together (four spill).  head: which partial of thread block `first`; rbp: which
-// of the row blocks that a partial covers.
+// order.  Two rows at a time: the loads of both are in flight together.  head: which partial of thread block `first`.
 template <bool GROUP>
-__device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, int rbp, int per, int first, int contributors, int head, int j0, int step, int lane) {
+__device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, int first, int contributors, int head, int j0, int step, int lane) {
   GemmTail tail;
   tail.load<GROUP>(p, rb, lane);
-  const size_t stride = (size_t)per * p.np * 32;               // float4s between the partials of a thread block (`per` row blocks each)
-  const float4* slot0 = reinterpret_cast<const float4*>(p.part) + (size_t)(2 * first) * stride + (size_t)rbp * p.np * 32 + lane;
+  const float4* slot0 = reinterpret_cast<const float4*>(p.part + (size_t)(2 * first) * ((size_t)p.np * 128)) + lane;
+  const size_t stride = (size_t)p.np * 32;
   for (int j = j0; j < tail.rows; j += 2 * step) {
     const int jb = j + step < tail.rows ? j + step : j;
     const float xa = gemm_xsum_share(p, tail.base + j, lane), xb = gemm_xsum_share(p, tail.base + jb, lane);
@@ -375,93 +366,7 @@ __device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, in
   }
 }
 
-// Finishing of a row block that this thread block decoded alone, by the four finisher warps: thread = weight row of its quadrant (the
-// accumulator's own layout), 16 activation rows at a time.  Five of the seven butterfly stages run across the lanes, with 16 values in
-// flight, the two over the quadrants through shared memory; the partial is read back by the thread that wrote it.  (One warp per
-// activation row, as in gemm_finish_row, is a chain of dependent loads that four warps cannot hide: at 200 rows it took longer than
-// the decode of the row block.)  colinfo: offset and scale of every activation row.
-__device__ __forceinline__ void gemm_finish_direct(const GemmParams& p, int rb, const float* mine, const float2* colinfo, float* exchange, int quad, int lane) {
-  const int li = lane & 15, own = (lane & 16) + (li < 8 ? 2 * li : 2 * li - 15);      // weight row inside the quadrant
-  const float scale = __half2float(p.scales[rb * 128 + 32 * quad + own]);
-  float bias[4];
-  unsigned flips = 0u;                                       // bit q: sign of row own of quadrant q
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int row = rb * 128 + 32 * q + own;
-    flips |= ((p.sv[row >> 3] >> (row & 7)) & 1u) << q;
-    bias[q] = 0.f;
-    if (p.bias && row < p.m_out)
-      bias[q] = p.dtype == HTR_DTYPE_F32 ? static_cast<const float*>(p.bias)[row]
-                : p.dtype == HTR_DTYPE_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[row])
-                                            : __half2float(static_cast<const __half*>(p.bias)[row]);
-  }
-  const float* src = mine + 32 * quad + own;
-  const bool high = (lane & 8) != 0;
-  int buf = 0;
-  for (int j0 = 0; j0 < p.rows; j0 += kExchangeCols, buf ^= 1) {
-    float v[kExchangeCols];
-#pragma unroll
-    for (int j = 0; j < kExchangeCols; ++j) v[j] = j0 + j < p.rows ? __ldcg(src + (size_t)(j0 + j) * 128) : 0.f;
-#pragma unroll
-    for (int j = 0; j < kExchangeCols; ++j) {
-      const float2 info = colinfo[min(j0 + j, p.rows - 1)];
-      v[j] = (v[j] - info.x) * (scale * info.y);
-    }
-#pragma unroll
-    for (int bit = 1; bit < 32; bit <<= 1) {
-      const float sgn = (lane & bit) ? -1.0f : 1.0f;
-      const float2 sgn2 = make_float2(sgn, sgn);
-#pragma unroll
-      for (int j = 0; j < kExchangeCols; j += 2) {
-        const float2 other = make_float2(__shfl_xor_sync(kFullWarp, v[j], bit), __shfl_xor_sync(kFullWarp, v[j + 1], bit));
-        const float2 r = __ffma2_rn(sgn2, make_float2(v[j], v[j + 1]), other);
-        v[j] = r.x;
-        v[j + 1] = r.y;
-      }
-    }
-    float* ex = exchange + buf * (4 * kExchangeCols * 32);
-#pragma unroll
-    for (int j = 0; j < kExchangeCols; ++j) ex[(quad * kExchangeCols + j) * 32 + lane] = v[j];
-    finishers_all(true);                                     // (the other buffer is written before the next of these, read before the one after)
-#pragma unroll
-    for (int k = 0; k < kExchangeCols / 4; ++k) {            // this warp closes the columns 4 quad .. + 3
-      const int j = j0 + 4 * quad + k;
-      if (j >= p.rows) break;                                // warp-uniform
-      const float* col = ex + (4 * quad + k) * 32 + lane;
-      const float a = col[0], b = col[kExchangeCols * 32], c = col[2 * kExchangeCols * 32], d = col[3 * kExchangeCols * 32];
-      const float s0 = a + b, s1 = a - b, s2 = c + d, s3 = c - d;
-      const float o[4] = {s0 + s2, s1 + s3, s0 - s2, s1 - s3};
-      float f[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) f[q] = flip(o[q] * kInvSqrt128, (flips >> q) & 1u) + bias[q];
-      const size_t at = (size_t)j * p.m_out + rb * 128;
-      if (p.dtype == HTR_DTYPE_F32) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (rb * 128 + 32 * q + own < p.m_out) static_cast<float*>(p.y)[at + 32 * q + own] = f[q];
-      } else {
-        // rows 2l and 2l + 1 sit eight lanes apart: the low lanes store the pairs of quadrants 0 and 2, the high lanes of 1 and 3
-#pragma unroll
-        for (int h = 0; h < 4; h += 2) {
-          const float got = __shfl_xor_sync(kFullWarp, high ? f[h] : f[h + 1], 8);
-          const float lo = high ? got : f[h], hi = high ? f[h + 1] : got;
-          const int row = 32 * (h + (high ? 1 : 0)) + (lane & 16) + 2 * (lane & 7);
-          uint32_t packed;
-          if (p.dtype == HTR_DTYPE_BF16) {
-            const __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
-            packed = *reinterpret_cast<const uint32_t*>(&t);
-          } else {
-            const __half2 t = __floats2half2_rn(lo, hi);
-            packed = *reinterpret_cast<const uint32_t*>(&t);
-          }
-          if (rb * 128 + row < p.m_out) *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.y) + at + row) = packed;
-        }
-      }
-    }
-  }
-}
-
-template <int K, int RBP, bool GROUP>
+template <int K, bool GROUP>
 __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const GemmParams p) {
   extern __shared__ __align__(128) unsigned char gsm[];
   __shared__ __align__(8) unsigned long long s_full[kGemmMaxStages], s_freed[kGemmMaxStages], s_done, s_drained;
@@ -469,7 +374,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   __shared__ int s_arrival;
   __shared__ int s_owed[kGemmFinishWarps];                  // row blocks below it have been delivered by the finisher warp
   __shared__ volatile int s_fail;
-  __shared__ float2 s_colinfo[GROUP ? 1 : kGemmMaxCols];    // finishers: offset and scale of every activation row
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   constexpr int DW = kGemmDecodeWarps;
@@ -481,8 +385,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     asm volatile("griddepcontrol.wait;" ::: "memory");      // the plan comes from an earlier kernel
     tiles = group_tiles(p.plan);
   }
-  static_assert(RBP == 1 || (RBP == 2 && !GROUP), "row blocks per unit");
-  const int U = (GROUP ? tiles * p.rb_per_tile : (p.rbs + RBP - 1) / RBP) * HB;
+  const int U = (GROUP ? tiles * p.rb_per_tile : p.mt >> 3) * HB;
   const EvenRuns runs(U, gridDim.x);
   int u_begin, u_end, part_id = 0;
   if (!GROUP && p.split > 0) {
@@ -498,12 +401,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   const int b_tile_bytes = ncols * 256;
   unsigned char* ring = gsm + (128 - (smem_u32(gsm) & 127)) % 128;
   const uint32_t ring_addr = smem_u32(ring);
-  const int acc_cols = gemm_acc_cols(ncols), a_col = RBP * acc_cols;
-  constexpr int kStageCols = 64 * RBP;                       // tensor-memory columns of A per stage
+  const int a_col = gemm_acc_cols(ncols);
 
   if (tid == 0) {
     for (int s = 0; s < kGemmMaxStages; ++s) {
-      mbar_init(smem_u32(&s_full[s]), kGemmGroupWarps * RBP + 1);       // the warps that decode the unit, and the B
+      mbar_init(smem_u32(&s_full[s]), kGemmGroupWarps + 1);             // the warps of the group that decodes the block, and the B
                                                                         // lane's arrive.expect_tx (with the bytes of the tile)
       mbar_init(smem_u32(&s_freed[s]), 1);                              // tcgen05.commit
     }
@@ -525,7 +427,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   if (!GROUP && warp == kGemmWarps - 1 && lane < 6) {
     // the row scales and signs of the first and the last row block are needed at the very end, in a chain of dependent loads:
     // bring them to L2 now (256 bytes of scales and 16 of signs per row block)
-    const size_t rb = RBP * (lane & 1 ? (u_end - 1) / HB : u_begin / HB);
+    const size_t rb = lane & 1 ? (u_end - 1) / HB : u_begin / HB;
     const char* at = lane < 4 ? reinterpret_cast<const char*>(p.scales + rb * 128) + (lane >> 1) * 128 : reinterpret_cast<const char*>(p.sv + rb * 16);
     asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
   }
@@ -536,10 +438,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     const int g = lane >> 2, c = lane & 3;
     using Ring = GemmRing<K>;
     constexpr int R = Ring::slots;
-    const unsigned char* words = ring + gemm_ring_bytes(np, p.planes, NS, RBP) + warp * (R * Ring::slot_bytes);
-    // copy cursor: every second block of the run (RBP = 1) or this group's row block of every unit (RBP = 2), across row blocks;
-    // past the end of the run the copies are predicated off
-    constexpr int kStep = RBP == 1 ? 2 : 1;                 // blocks of its row that the cursor moves on per turn
+    const unsigned char* words = ring + gemm_ring_bytes(np, p.planes, NS) + warp * (R * Ring::slot_bytes);
+    // copy cursor: every second block of the run, across row blocks; past the end of the run the copies are predicated off
     uint32_t cp_dst[Ring::copies];
 #pragma unroll
     for (int i = 0; i < Ring::copies; ++i) {
@@ -547,9 +447,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       cp_dst[i] = smem_u32(words) + unit * (128 * K) + 16 * ring_chunk<K>(within / (2 * K), within % (2 * K));
     }
     // from the end of a strip's row to the same strip of the next row block (a row of one block is left twice per step of two)
-    const size_t next_strip = RBP == 1 ? (size_t)7 * nt * (32 * K) * (HB == 1 ? 2 : 1) : (size_t)15 * nt * (32 * K);
-    // (the last unit row of an odd number of row blocks has nothing for the second group: it decodes what its ring holds, for nobody)
-    int pf_left = RBP == 1 ? u_end - u_begin - group : min(u_end, (p.rbs - group + 1) / 2 * HB) - u_begin, pf_in_rb, pf_rb;
+    const size_t next_strip = (size_t)7 * nt * (32 * K) * (HB == 1 ? 2 : 1);
+    int pf_left = u_end - u_begin - group, pf_in_rb, pf_rb;
     const char* pf;
     auto strip_row = [&](int rb) {                          // this lane's first chunk of this warp's strip of row block rb
       const uint32_t* base = p.qw;
@@ -561,8 +460,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       return reinterpret_cast<const char*>(base) + (size_t)(rb * 8 + strip) * nt * (32 * K) + lane * 16;
     };
     {
-      const int u = RBP == 1 ? u_begin + group : u_begin, hb = u % HB;
-      pf_rb = RBP == 1 ? u / HB : 2 * (u / HB) + group;
+      const int u = u_begin + group, hb = u % HB;
+      pf_rb = u / HB;
       pf = strip_row(pf_rb) + (size_t)hb * (256 * K);
       pf_in_rb = HB - hb;
     }
@@ -574,7 +473,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
                      "l"(pf + 512 * i), "r"(on)
                      : "memory");
       }
-      pf_left -= kStep;
+      pf_left -= 2;
       if constexpr (GROUP) {
         pf += 512 * K;
         pf_in_rb -= 2;
@@ -583,9 +482,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
           pf = strip_row(pf_rb) + (size_t)(HB - pf_in_rb) * (256 * K);
         }
       } else {
-        const bool wrap = pf_in_rb <= kStep;
-        pf_in_rb += wrap ? HB - kStep : -kStep;
-        pf += wrap ? next_strip + kStep * 256 * K : (size_t)(kStep * 256 * K);
+        const bool wrap = pf_in_rb <= 2;
+        pf_in_rb += wrap ? HB - 2 : -2;
+        pf += wrap ? next_strip + 512 * K : (size_t)(512 * K);
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -594,14 +493,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();                                        // the barriers and the tensor-memory address are visible from here on
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t a_addr = s_tmem + ((uint32_t)(32 * quad + 16 * half) << 16) + (uint32_t)(a_col + (RBP == 2 ? 64 * group : 0));
+    const uint32_t a_addr = s_tmem + ((uint32_t)(32 * quad + 16 * half) << 16) + (uint32_t)a_col;
     // (this loop is what bounds the kernel: no branches but the two below, no divisions, no counters beside the ring positions)
     uint32_t at = 0u, refill = (R - 1) * Ring::slot_bytes;  // ring slots of this block and of the one before it
-    int stage = RBP == 1 ? group : 0;
+    int stage = group;
     uint32_t parity = 1u;                                   // of freed[stage]: passes at once on the first round
     bool ok = true;
 #pragma unroll 1
-    for (int left = u_end - u_begin - (RBP == 1 ? group : 0); left > 0; left -= kStep) {
+    for (int left = u_end - u_begin - group; left > 0; left -= 2) {
       asm volatile("cp.async.wait_group %0;" ::"n"(R - 2) : "memory");   // this block's words have landed (own copies) ...
       __syncwarp();                                                       // ... and those of the other lanes; the slot before it is free
       fetch(refill);
@@ -615,16 +514,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       const uint32_t bar = smem_u32(&s_freed[0]) + 8u * stage;
       if (!__all_sync(kFullWarp, mbar_try(bar, parity, 1000u)) && !__all_sync(kFullWarp, mbar_wait_slow(bar, parity, &s_fail, 0u))) { ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      tmem_store_strip(a_addr + kStageCols * stage, w);
+      tmem_store_strip(a_addr + 64 * stage, w);
       read_own_words<K>(blk + 128 * K, c, g, V);
       decode_unit<K>(V, lane, w);
-      tmem_store_strip(a_addr + kStageCols * stage + 32, w);
+      tmem_store_strip(a_addr + 64 * stage + 32, w);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&s_full[0]) + 8u * stage);
-      const bool around = stage + kStep >= NS;
-      stage += around ? kStep - NS : kStep;
+      const bool around = stage + 2 >= NS;
+      stage += around ? 2 - NS : 2;
       parity ^= around ? 1u : 0u;
     }
     if (!ok) s_fail = 1;
@@ -682,15 +581,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
             if (!mbar_wait(smem_u32(&s_full[s]), ph, &s_fail)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t desc = desc0 + (uint64_t)(s * (b_tile_bytes >> 4));   // (shared memory addresses fit the field: no carry)
-            const uint32_t a_addr = tmem + (uint32_t)(a_col + kStageCols * s);
+            const uint32_t a_addr = tmem + (uint32_t)(a_col + 64 * s);
 #pragma unroll
-            for (int rbp = 0; rbp < RBP; ++rbp)
+            for (int q = 0; q < 2; ++q)
 #pragma unroll
-              for (int q = 0; q < 2; ++q)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                  umma_f16_ts(tmem + (uint32_t)(rbp * acc_cols), a_addr + 64 * rbp + 32 * q + 8 * j, desc + (uint64_t)(q * (b_tile_bytes >> 5) + j * ((2 * kLbo) >> 4)),
-                              idesc, (q | j) ? 1u : fresh);
+              for (int j = 0; j < 4; ++j)
+                umma_f16_ts(tmem, a_addr + 32 * q + 8 * j, desc + (uint64_t)(q * (b_tile_bytes >> 5) + j * ((2 * kLbo) >> 4)), idesc, (q | j) ? 1u : fresh);
             fresh = 1u;
             umma_commit(smem_u32(&s_freed[s]));
             if (++s == NS) { s = 0; ph ^= 1u; }
@@ -710,7 +606,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       const int fw = warp - (DW + 2), quad = warp & 3;
       const uint32_t acc_addr = s_tmem + ((uint32_t)(32 * quad) << 16);
       const int li = lane & 15, row = 32 * quad + (lane & 16) + (li < 8 ? 2 * li : 2 * li - 15);   // weight row of this tensor-memory lane
-      float* exchange = reinterpret_cast<float*>(ring + gemm_ring_bytes(np, p.planes, NS, RBP) + GemmRing<K>::bytes);
       bool ok = true, predecessor_done = false;
       int seg = 0;
       for (int u = u_begin; u < u_end; ++seg) {
@@ -724,33 +619,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         if (!predecessor_done) {
           asm volatile("griddepcontrol.wait;" ::: "memory");   // scratch and outputs of earlier launches
           predecessor_done = true;
-          if (!GROUP && p.direct) {                            // offset and scale of every activation row, for all row blocks
-            for (int j = fw * 32 + lane; j < p.rows; j += kGemmFinishWarps * 32) {
-              float xs = 0.f;
-              for (int y = 0; y < p.xsum_slices; ++y) xs += __ldcg(p.xsum + (size_t)j * p.xsum_slices + y);
-              s_colinfo[j] = make_float2(1534.0f * xs, p.cb * __ldcg(p.tok + j));
-            }
-            finishers_all(true);
-          }
         }
         // accumulator -> partial [np][128], hi + lo added here.  A thread block has two partials: its first row block's, which other
         // thread blocks may read, and one for all later ones (of which only the last is read by others)
-        float* mine = !GROUP && p.split > 0 ? reinterpret_cast<float*>(ring)
-                                            : p.part + (size_t)(2 * blockIdx.x + (seg > 0 ? 1 : 0)) * ((size_t)RBP * np * 128);
-#pragma unroll 1
-        for (int rbp = 0; rbp < RBP; ++rbp)
-          for (int j0 = 0; j0 < np; j0 += 8) {
-            uint32_t hi[8], lo[8];
-            tmem_load8(acc_addr + rbp * acc_cols + j0, hi);
-            if (p.planes == 2) tmem_load8(acc_addr + rbp * acc_cols + np + j0, lo);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float* mine = !GROUP && p.split > 0 ? reinterpret_cast<float*>(ring) : p.part + (size_t)(2 * blockIdx.x + (seg > 0 ? 1 : 0)) * ((size_t)np * 128);
+        for (int j0 = 0; j0 < np; j0 += 8) {
+          uint32_t hi[8], lo[8];
+          tmem_load8(acc_addr + j0, hi);
+          if (p.planes == 2) tmem_load8(acc_addr + np + j0, lo);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float v = p.planes == 2 ? __uint_as_float(hi[j]) + __uint_as_float(lo[j]) : __uint_as_float(hi[j]);
-              if (!GROUP && p.split > 0) mine[(rbp * np + j0 + j) * 128 + row] = v;
-              else __stcg(mine + (rbp * np + j0 + j) * 128 + row, v);
-            }
+          for (int j = 0; j < 8; ++j) {
+            const float v = p.planes == 2 ? __uint_as_float(hi[j]) + __uint_as_float(lo[j]) : __uint_as_float(hi[j]);
+            if (!GROUP && p.split > 0) mine[(j0 + j) * 128 + row] = v;
+            else __stcg(mine + (j0 + j) * 128 + row, v);
           }
+        }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&s_drained));    // the MMAs of the next row block may start
@@ -768,15 +652,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
           finish = s_arrival == contributors - 1;
           if (finish && fw == 0 && lane == 0) p.counters[rb] = 0;
         }
-        if (finish) {
-#pragma unroll 1
-          for (int rbp = 0; rbp < RBP; ++rbp) {
-            const int block = RBP * rb + rbp;
-            if (RBP > 1 && block >= p.rbs) break;
-            if (!GROUP && p.direct && contributors == 1) gemm_finish_direct(p, block, mine + (size_t)rbp * np * 128, s_colinfo, exchange, quad, lane);
-            else gemm_finish_flat<GROUP>(p, block, rbp, RBP, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, fw, kGemmFinishWarps, lane);
-          }
-        }
+        if (finish) gemm_finish_flat<GROUP>(p, rb, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, fw, kGemmFinishWarps, lane);
         __syncwarp();
         if (lane == 0) s_owed[fw] = rb + 1;
         finishers_all(true);                                 // the partial has been read by all of them: it may be written again
@@ -795,29 +671,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     // cluster sums rows r, r + split, ... over all of them (in rank order) and finishes those rows itself
     float* result = reinterpret_cast<float*>(ring);
     if (bad)                                                 // a bounded wait gave up: the rows come out as NaN, beside the error word
-      for (int e = tid; e < RBP * np * 128; e += kGemmThreads) result[e] = __uint_as_float(0x7FC00000u);
+      for (int e = tid; e < np * 128; e += kGemmThreads) result[e] = __uint_as_float(0x7FC00000u);
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");      // (done before by the roles that needed it)
-#pragma unroll 1
-    for (int rbp = 0; rbp < RBP; ++rbp) {
-      const int block = RBP * (blockIdx.x / p.split) + rbp;
-      if (RBP > 1 && block >= p.rbs) break;
-      GemmTail tail;
-      tail.load<false>(p, block, lane);
-      const uint32_t result_addr = smem_u32(result + (size_t)rbp * np * 128);
-      for (int j = part_id + p.split * warp; j < p.rows; j += p.split * kGemmWarps) {
-        const float xs = gemm_xsum_share(p, j, lane), tok = __ldcg(p.tok + j);
-        float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int r = 0; r < p.split; ++r) {
-          uint32_t remote;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(result_addr + (uint32_t)(j * 128 + 4 * lane) * 4u), "r"(r));
-          float4 v;
-          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
-          r4.x += v.x; r4.y += v.y; r4.z += v.z; r4.w += v.w;
-        }
-        gemm_finish_row(p, tail, j, lane, r4, xs, tok);
+    GemmTail tail;
+    tail.load<false>(p, blockIdx.x / p.split, lane);
+    const uint32_t result_addr = smem_u32(result);
+    for (int j = part_id + p.split * warp; j < p.rows; j += p.split * kGemmWarps) {
+      const float xs = gemm_xsum_share(p, j, lane), tok = __ldcg(p.tok + j);
+      float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int r = 0; r < p.split; ++r) {
+        uint32_t remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(result_addr + (uint32_t)(j * 128 + 4 * lane) * 4u), "r"(r));
+        float4 v;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+        r4.x += v.x; r4.y += v.y; r4.z += v.z; r4.w += v.w;
       }
+      gemm_finish_row(p, tail, j, lane, r4, xs, tok);
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // nobody leaves while its shared memory may still be read
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -835,16 +706,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       finish = s_arrival == contributors - 1;
       if (finish && tid == 0) p.counters[rb] = 0;
     }
-    if (finish) {
-#pragma unroll 1
-      for (int rbp = 0; rbp < RBP; ++rbp)
-        if (RBP == 1 || RBP * rb + rbp < p.rbs)
-          gemm_finish_flat<GROUP>(p, RBP * rb + rbp, rbp, RBP, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, warp, kGemmWarps, lane);
-    }
+    if (finish) gemm_finish_flat<GROUP>(p, rb, first, contributors, runs.begin(first) < rb * HB ? 1 : 0, warp, kGemmWarps, lane);
     if (bad) {
       // the row blocks this thread block still owed never complete (nobody arrives for them): their rows come out as NaN
       const float nan = __uint_as_float(0x7FC00000u);
-      for (int b = RBP * min(min(s_owed[0], s_owed[1]), min(s_owed[2], s_owed[3])); b < (GROUP ? rb + 1 : min(RBP * (rb + 1), p.rbs)); ++b) {
+      for (int b = min(min(s_owed[0], s_owed[1]), min(s_owed[2], s_owed[3])); b <= rb; ++b) {
         GemmTail tail;
         tail.load<GROUP>(p, b, lane);
         for (int j = warp; j < tail.rows; j += kGemmWarps) gemm_store_rows(p, tail.pairs ? tail.pairs[j] : j, tail.row0, make_float4(nan, nan, nan, nan));
@@ -860,10 +726,10 @@ int gemm_rht_slices(int np, int n);
 int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
                 cudaStream_t st);
 template <int K>
-int launch_packed_gemm_tc(const GemmParams& p, int rbp, int grid, int smem, cudaStream_t st);   // p.plan set: the grouped form
+int launch_packed_gemm_tc(const GemmParams& p, int grid, int smem, cudaStream_t st);   // p.plan set: the grouped form
 // clusters of `split` thread blocks that the GPU holds at once (0: none), for the cluster form of the plan
 template <int K>
-int packed_gemm_tc_clusters(int rbp, int smem, int split);
+int packed_gemm_tc_clusters(int smem, int split);
 // bytes of the packed-word rings of a thread block
 inline int gemm_word_bytes(int K) {
   switch (K) {

@@ -12,11 +12,12 @@ namespace {
 int allow_smem(int dev) {
   static bool allowed[64] = {false};
   if (dev >= 0 && dev < 64 && allowed[dev]) return 0;
-  for (const void* f : {reinterpret_cast<const void*>(packed_gemm_tc_kernel<HTR_INST_K, 1, false>), reinterpret_cast<const void*>(packed_gemm_tc_kernel<HTR_INST_K, 2, false>),
-                        reinterpret_cast<const void*>(packed_gemm_tc_kernel<HTR_INST_K, 1, true>)}) {
-    if (const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmMaxSmem)) return (int)e;
-    if (const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) return (int)e;   // up to 16
-  }
+  const cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+  if (e != cudaSuccess) return (int)e;
+  const cudaError_t e2 = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  if (e2 != cudaSuccess) return (int)e2;
+  const cudaError_t e3 = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // up to 16
+  if (e3 != cudaSuccess) return (int)e3;
   if (dev >= 0 && dev < 64) allowed[dev] = true;
   return 0;
 }
@@ -24,14 +25,14 @@ int allow_smem(int dev) {
 }  // namespace
 
 template <>
-int packed_gemm_tc_clusters<HTR_INST_K>(int rbp, int smem, int split) {
+int packed_gemm_tc_clusters<HTR_INST_K>(int smem, int split) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   // the query costs tens of microseconds on the host: remember the answer
   static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int>, int> seen;
+  static std::map<std::tuple<int, int, int>, int> seen;
   std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_tuple(dev, rbp, smem, split);
+  const auto key = std::make_tuple(dev, smem, split);
   const auto it = seen.find(key);
   if (it != seen.end()) return it->second;
   int clusters = 0;
@@ -47,7 +48,7 @@ int packed_gemm_tc_clusters<HTR_INST_K>(int rbp, int smem, int split) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&clusters, reinterpret_cast<const void*>(rbp == 2 ? packed_gemm_tc_kernel<HTR_INST_K, 2, false> : packed_gemm_tc_kernel<HTR_INST_K, 1, false>), &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, packed_gemm_tc_kernel<HTR_INST_K, false>, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
       clusters = 0;
     }
@@ -57,7 +58,7 @@ int packed_gemm_tc_clusters<HTR_INST_K>(int rbp, int smem, int split) {
 }
 
 template <>
-int launch_packed_gemm_tc<HTR_INST_K>(const GemmParams& p, int rbp, int grid, int smem, cudaStream_t st) {
+int launch_packed_gemm_tc<HTR_INST_K>(const GemmParams& p, int grid, int smem, cudaStream_t st) {
   int dev = 0;
   if (const cudaError_t e = cudaGetDevice(&dev)) return (int)e;
   if (const int e = allow_smem(dev)) return e;
@@ -82,7 +83,7 @@ int launch_packed_gemm_tc<HTR_INST_K>(const GemmParams& p, int rbp, int grid, in
   }
   GemmParams q = p;
   void* args[1] = {&q};
-  return (int)cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(p.plan ? packed_gemm_tc_kernel<HTR_INST_K, 1, true> : rbp == 2 ? packed_gemm_tc_kernel<HTR_INST_K, 2, false> : packed_gemm_tc_kernel<HTR_INST_K, 1, false>), args);
+  return (int)cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(p.plan ? packed_gemm_tc_kernel<HTR_INST_K, true> : packed_gemm_tc_kernel<HTR_INST_K, false>), args);
 }
 
 }  // namespace htr
