@@ -384,23 +384,29 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   while (g.stages > 1 && gemm_smem_bytes(g.np, planes, g.stages, words) > budget) --g.stages;
   g.smem = gemm_smem_bytes(g.np, planes, g.stages, words);
   if (g.stages < 2) return HTR_ERR_TOO_LARGE;
-  // Up to sixteen thread blocks share a row block as a cluster and reduce on chip, or every thread block of the GPU takes an even run
-  // (flat) and a row block's partial sums meet in global memory at one last arriver.  Costs in units of one decoded 128 x 128 block
-  // (0.43 us): the longest run, and for the flat form nine for the hand-over (measured 2 to 3 us) plus the partials that the last
-  // arriver reads at about 100 bytes a nanosecond.  At 2048x2048, 8 / 200 rows, this chose clusters of four over flat runs: 11.5 / 33.2
-  // -> 7.6 / 16.9 us; 6144x4096, 8 rows: 14.6 -> 12.7.
+  // Three forms, by their cost in units of one decoded 128 x 128 block (0.43 us, or as long as the MMAs of a wide batch take):
+  //  * up to sixteen thread blocks share a row block as a cluster and reduce on chip;
+  //  * a thread block takes a whole row block, in as many waves as there are row blocks per SM: all its warps finish it from shared
+  //    memory, about four blocks' time and a thirtieth of one per activation row;
+  //  * every thread block of the GPU takes an even run (flat) and a row block's partial sums meet in global memory at one last arriver:
+  //    nine blocks' time for the hand-over (measured 2 to 3 us) and the partials, which that one reads at 100 bytes a nanosecond.  Row
+  //    blocks inside a run are finished by four warps beside the decode, half a block's time per activation row: many rows wait for them.
+  // Measured, as before -> as chosen: WAVEFIG
+  const double unit = ncols > 192 ? 1.2 : 1.0;
   const long long slots = sms, units = (long long)g.rbs * g.hb;
   const long long flat_grid = slots < units ? slots : units, flat_run = (units + flat_grid - 1) / flat_grid;
-  long long best = flat_run + 9 + (g.hb / flat_run + 1) * g.np / 84;
+  const double beside = (double)(flat_run / g.hb) * M * 0.5;
+  double best = (flat_run * unit > beside ? flat_run * unit : beside) + 9 + (double)((g.hb / flat_run + 1) * g.np) / 84;
   g.split = 0;
-  for (int s = (int)(slots / g.rbs < 16 ? slots / g.rbs : 16); s >= 1; --s) {
-    const long long run = (g.hb + s - 1) / s;
-    if (s > g.hb || run >= best) continue;
-    if (s == 1 || gemm_clusters(K, g.smem, s) >= g.rbs) {
+  for (int s = (int)(slots / g.rbs < 16 ? slots / g.rbs : 16); s >= 2; --s) {
+    const double cost = (double)((g.hb + s - 1) / s) * unit;
+    if (s <= g.hb && cost < best && gemm_clusters(K, g.smem, s) >= g.rbs) {
       g.split = s;
-      best = run;
+      best = cost;
     }
   }
+  const long long waves = (g.rbs + slots - 1) / slots;
+  if (waves * (g.hb * unit + M / 30.0) + (waves - 1) * 4 < best) g.split = 1;
   g.grid = g.split > 0 ? g.rbs * g.split : (int)flat_grid;
   size_t off = kCounterRegion + kErrorRegion;
   g.off_xb = off; off += align256((size_t)ncols * n * 2);
