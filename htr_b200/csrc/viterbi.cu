@@ -44,22 +44,25 @@ struct VitParams {
   const float* w;
   int32_t* states;
   float* total;
-  uint8_t* bps;      // [grid][T][2^(16-K)]
+  uint8_t* bps;      // [tiles at once][T][2^(16-K)]
   int B, T, tailbite;
   float inv_hi, inv_lo;
 };
 
-template <int K>
+// C: thread blocks of the cluster that share one tile (1, 2 or 4): each owns SJ / C consecutive j
+template <int K, int C>
 struct VitCfg {
   static constexpr int kNB = 1 << K, kSj = 1 << (16 - K);
-  static constexpr int kThreads = 512;                                    // x 128 states = all of them
+  static constexpr int kThreads = 512, kStates = 128 / C;                 // kThreads x kStates x C = all of them
   static constexpr int kTT = kNB < 16 ? kNB : 16;                         // tops of one thread; kSub neighbouring lanes share the others
   static constexpr int kSub = kNB / kTT;
-  static constexpr int kJb = K == 2 ? 4 : 8;                              // consecutive j of a group: they share their predecessor minima
-  static constexpr int kGroups = 128 / (kTT * kJb);                       // groups of a thread: K = 2: 8, K = 3: 2, else 1
-  static constexpr int kBlocks = 128 / kJb;                               // (group, top) blocks of kJb states, in that order
-  static constexpr int kRegBlocks = kBlocks / 2;                          // ... whose codebook values stay in registers
-  static constexpr bool kTable = K != 2;                                  // the others': in shared memory, else from the hash
+  static constexpr int kPer = kStates / kTT;                              // j of a thread
+  static constexpr int kJb = K == 2 ? 4 : kPer < 8 ? kPer : 8;            // consecutive j of a group: they share their predecessor minima
+  static constexpr int kGroups = kPer / kJb;                              // groups of a thread
+  static constexpr int kPairs = kJb / 2;                                  // candidates are handled two at a time
+  static constexpr int kBlocks = kStates / kJb;                           // (group, top) blocks of kJb states, in that order
+  static constexpr int kRegBlocks = C == 1 ? kBlocks / 2 : kBlocks;       // ... whose codebook values stay in registers
+  static constexpr bool kTable = C == 1 && K != 2;                        // the others': in shared memory, else from the hash
   static constexpr int kTableBytes = kTable ? 64 * kThreads * 4 : 0;
   static constexpr int kSmem = kTableBytes + 2 * kSj * 4 + 2 * kVitMaxT * 4 + kSj;   // table, two cost arrays, targets, weights, last back-pointers
   static constexpr int kLevels = K == 2 ? 5 : K <= 4 ? 3 : 2;             // steps of the traceback per memory latency: kNB^(levels-1) <= 256
@@ -90,18 +93,71 @@ __device__ __forceinline__ void take(float val, int top, float& best, int& arg) 
   }
 }
 
-// One step of all states: costs mc -> mn and, with ARG, the arguments to bp and lastarg (either may be null).
-template <int K, bool ARG>
-__device__ __forceinline__ void vit_step(const float* __restrict__ mc, float* __restrict__ mn, float xt, float wt, const float2 (&negc)[32],
-                                         const float4* __restrict__ table, float inv_hi, float inv_lo, uint8_t* __restrict__ bp,
-                                         uint8_t* __restrict__ lastarg) {
-  using C = VitCfg<K>;
-  constexpr int JB = C::kJb, SH = 16 - 2 * K, TT = C::kTT, SUB = C::kSub;
+// JB consecutive costs, or their arguments as bytes, to the same place in the shared memory of every block of the cluster
+template <int C, int JB>
+__device__ __forceinline__ void spread_costs(float* at, const float (&v)[JB]) {
+  if constexpr (C == 1) {
+    if constexpr (JB % 4 == 0) {
+#pragma unroll
+      for (int q = 0; q < JB / 4; ++q) *reinterpret_cast<float4*>(at + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else {
+      *reinterpret_cast<float2*>(at) = make_float2(v[0], v[1]);
+    }
+  } else {
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(at);
+#pragma unroll
+    for (int r = 0; r < C; ++r) {
+      uint32_t to;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine), "r"(r));
+      if constexpr (JB % 4 == 0) {
+#pragma unroll
+        for (int q = 0; q < JB / 4; ++q)
+          asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + 16 * q), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                       : "memory");
+      } else {
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(v[0]), "f"(v[1]) : "memory");
+      }
+    }
+  }
+}
+template <int C>
+__device__ __forceinline__ void spread_byte(uint8_t* at, uint32_t v) {
+  if constexpr (C == 1) {
+    *at = (uint8_t)v;
+  } else {
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(at);
+#pragma unroll
+    for (int r = 0; r < C; ++r) {
+      uint32_t to;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine), "r"(r));
+      asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(to), "r"(v) : "memory");
+    }
+  }
+}
+// barrier of all threads that work on the tile
+template <int C>
+__device__ __forceinline__ void tile_sync() {
+  if constexpr (C == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+// One step of this thread's states: costs mc -> mn (of every block of the cluster) and, with ARG, the arguments to bp and lastarg
+// (either may be null).
+template <int K, int C, bool ARG>
+__device__ __forceinline__ void vit_step(const float* __restrict__ mc, float* __restrict__ mn, float xt, float wt,
+                                         const float2 (&negc)[VitCfg<K, C>::kRegBlocks * VitCfg<K, C>::kPairs], const float4* __restrict__ table, int j_first,
+                                         float inv_hi, float inv_lo, uint8_t* __restrict__ bp, uint8_t* __restrict__ lastarg) {
+  using Cfg = VitCfg<K, C>;
+  constexpr int JB = Cfg::kJb, SH = 16 - 2 * K, TT = Cfg::kTT, SUB = Cfg::kSub, PAIRS = Cfg::kPairs;
   const int tid = threadIdx.x, sub = tid % SUB;
   const float2 xt2 = make_float2(xt, xt), wt2 = make_float2(wt, wt);
 #pragma unroll
-  for (int g = 0; g < C::kGroups; ++g) {
-    const int jbase = (g * (C::kThreads / SUB) + tid / SUB) * JB;
+  for (int g = 0; g < Cfg::kGroups; ++g) {
+    const int jbase = j_first + (g * (Cfg::kThreads / SUB) + tid / SUB) * JB;
     const float* prev_col = mc + (jbase >> K) + ((sub * TT) << SH);        // predecessor minima of this group: stride 2^(16-2K) per top
     float best[JB];
     int arg[JB];                                                          // relative to this lane's first top
@@ -110,16 +166,15 @@ __device__ __forceinline__ void vit_step(const float* __restrict__ mc, float* __
 #pragma unroll
     for (int tt = 0; tt < TT; ++tt) {
       const float prev = prev_col[tt << SH];
-      constexpr int kQuads = JB / 4;
       const int blk = g * TT + tt;
 #pragma unroll
-      for (int q = 0; q < kQuads; ++q) {
+      for (int q = 0; q < (PAIRS + 1) / 2; ++q) {
         float2 nc[2];
-        if (blk < C::kRegBlocks) {
-          nc[0] = negc[(blk * kQuads + q) * 2];
-          nc[1] = negc[(blk * kQuads + q) * 2 + 1];
-        } else if constexpr (C::kTable) {
-          const float4 f = table[((blk - C::kRegBlocks) * kQuads + q) * C::kThreads];
+        if (blk < Cfg::kRegBlocks) {
+          nc[0] = negc[blk * PAIRS + 2 * q];
+          nc[1] = negc[blk * PAIRS + (2 * q + 1 < PAIRS ? 2 * q + 1 : 2 * q)];
+        } else if constexpr (Cfg::kTable) {
+          const float4 f = table[((blk - Cfg::kRegBlocks) * (PAIRS / 2) + q) * Cfg::kThreads];
           nc[0] = make_float2(f.x, f.y);
           nc[1] = make_float2(f.z, f.w);
         } else {
@@ -134,6 +189,7 @@ __device__ __forceinline__ void vit_step(const float* __restrict__ mc, float* __
         }
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
+          if (2 * q + e >= PAIRS) break;
           const float2 d = add2(xt2, nc[e]);
           const float2 wd = mul2(wt2, mul2(d, d));
           // the last addition stays scalar: a packed multiply followed by a packed add was observed to come out fused (one
@@ -163,28 +219,33 @@ __device__ __forceinline__ void vit_step(const float* __restrict__ mc, float* __
         }
       }
     if (sub == 0) {
-#pragma unroll
-      for (int q = 0; q < JB / 4; ++q)
-        *reinterpret_cast<float4*>(mn + jbase + 4 * q) = make_float4(best[4 * q], best[4 * q + 1], best[4 * q + 2], best[4 * q + 3]);
+      spread_costs<C, JB>(mn + jbase, best);
       if constexpr (ARG) {
+        if (bp) {
+          if constexpr (JB % 4 == 0) {
 #pragma unroll
-        for (int q = 0; q < JB / 4; ++q) {
-          const uint32_t packed = (uint32_t)arg[4 * q] | ((uint32_t)arg[4 * q + 1] << 8) | ((uint32_t)arg[4 * q + 2] << 16) | ((uint32_t)arg[4 * q + 3] << 24);
-          if (bp) *reinterpret_cast<uint32_t*>(bp + jbase + 4 * q) = packed;
-          if (lastarg) *reinterpret_cast<uint32_t*>(lastarg + jbase + 4 * q) = packed;
+            for (int q = 0; q < JB / 4; ++q)
+              *reinterpret_cast<uint32_t*>(bp + jbase + 4 * q) = (uint32_t)arg[4 * q] | ((uint32_t)arg[4 * q + 1] << 8) | ((uint32_t)arg[4 * q + 2] << 16) | ((uint32_t)arg[4 * q + 3] << 24);
+          } else {
+            *reinterpret_cast<uint16_t*>(bp + jbase) = (uint16_t)((uint32_t)arg[0] | ((uint32_t)arg[1] << 8));
+          }
+        }
+        if (lastarg) {
+#pragma unroll
+          for (int b = 0; b < JB; ++b) spread_byte<C>(lastarg + jbase + b, (uint32_t)arg[b]);
         }
       }
     }
   }
 }
 
-template <int K>
-__global__ void __launch_bounds__(VitCfg<K>::kThreads, 1) viterbi_kernel(const VitParams p) {
-  using C = VitCfg<K>;
-  constexpr int NB = C::kNB, SJ = C::kSj, THREADS = C::kThreads, JB = C::kJb;
+template <int K, int C>
+__global__ void __launch_bounds__(VitCfg<K, C>::kThreads, 1) viterbi_kernel(const VitParams p) {
+  using Cfg = VitCfg<K, C>;
+  constexpr int NB = Cfg::kNB, SJ = Cfg::kSj, THREADS = Cfg::kThreads, JB = Cfg::kJb, PAIRS = Cfg::kPairs;
   extern __shared__ __align__(16) unsigned char vsm[];
   float4* table = reinterpret_cast<float4*>(vsm) + threadIdx.x;
-  float* m_a = reinterpret_cast<float*>(vsm + C::kTableBytes);
+  float* m_a = reinterpret_cast<float*>(vsm + Cfg::kTableBytes);
   float* m_b = m_a + SJ;
   float* xs = m_b + SJ;
   float* ws = xs + kVitMaxT;
@@ -193,30 +254,30 @@ __global__ void __launch_bounds__(VitCfg<K>::kThreads, 1) viterbi_kernel(const V
   __shared__ Best s_win;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int T = p.T;
-  uint8_t* bp = p.bps + (size_t)blockIdx.x * T * SJ;
+  const int cluster = blockIdx.x / C, rank = blockIdx.x % C, j_first = rank * (SJ / C);
+  uint8_t* bp = p.bps + (size_t)cluster * T * SJ;
 
-  // the negated codebook values of this thread's states, in block order (group, top): half here, half in shared memory
-  float2 negc[32];
+  // the negated codebook values of this thread's states, in block order (group, top): in registers, or half of them in shared memory
+  float2 negc[Cfg::kRegBlocks * PAIRS];
 #pragma unroll
-  for (int blk = 0; blk < (C::kTable ? C::kBlocks : C::kRegBlocks); ++blk) {
-    const int g = blk / C::kTT, top = (tid % C::kSub) * C::kTT + blk % C::kTT;
-    const int jbase = (g * (THREADS / C::kSub) + tid / C::kSub) * JB;
+  for (int blk = 0; blk < (Cfg::kTable ? Cfg::kBlocks : Cfg::kRegBlocks); ++blk) {
+    const int g = blk / Cfg::kTT, top = (tid % Cfg::kSub) * Cfg::kTT + blk % Cfg::kTT;
+    const int jbase = j_first + (g * (THREADS / Cfg::kSub) + tid / Cfg::kSub) * JB;
+    float f[JB];
 #pragma unroll
-    for (int q = 0; q < JB / 4; ++q) {
-      float f[4];
+    for (int e = 0; e < JB; ++e) f[e] = -codebook_value((((uint32_t)top << (16 - K)) | (uint32_t)(jbase + e)) * kGenMul + kGenAdd, p.inv_hi, p.inv_lo);
+    if (blk < Cfg::kRegBlocks) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) f[e] = -codebook_value((((uint32_t)top << (16 - K)) | (uint32_t)(jbase + 4 * q + e)) * kGenMul + kGenAdd, p.inv_hi, p.inv_lo);
-      if (blk < C::kRegBlocks) {
-        negc[(blk * (JB / 4) + q) * 2] = make_float2(f[0], f[1]);
-        negc[(blk * (JB / 4) + q) * 2 + 1] = make_float2(f[2], f[3]);
-      } else {
-        table[((blk - C::kRegBlocks) * (JB / 4) + q) * THREADS] = make_float4(f[0], f[1], f[2], f[3]);
-      }
+      for (int e = 0; e < PAIRS; ++e) negc[blk * PAIRS + e] = make_float2(f[2 * e], f[2 * e + 1]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < JB / 4; ++q)
+        table[((blk - Cfg::kRegBlocks) * (JB / 4) + q) * THREADS] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
     }
   }
 
-  for (int tile = blockIdx.x; tile < p.B; tile += gridDim.x) {
-    __syncthreads();                                                     // the previous tile's traceback is over
+  for (int tile = cluster; tile < p.B; tile += gridDim.x / C) {
+    tile_sync<C>();                                                      // the previous tile's traceback is over; every block of the cluster runs
     for (int t = tid; t < T; t += THREADS) {
       xs[t] = p.x[(size_t)tile * T + t];
       ws[t] = p.w[(size_t)tile * T + t];
@@ -228,13 +289,13 @@ __global__ void __launch_bounds__(VitCfg<K>::kThreads, 1) viterbi_kernel(const V
       float* mc = m_a;
       float* mn = m_b;
       for (int j = tid; j < SJ; j += THREADS) mc[j] = (j0 < 0 || j == j0) ? 0.f : INFINITY;
-      __syncthreads();
+      tile_sync<C>();                                                    // (the other cost array may be written by the cluster from here on)
       for (int t = 0; t < T; ++t) {
         const float xt = xs[t], wt = ws[t];
         const bool last = t == T - 1;
-        if (keep || last) vit_step<K, true>(mc, mn, xt, wt, negc, table, p.inv_hi, p.inv_lo, keep ? bp + (size_t)t * SJ : nullptr, last ? lastarg : nullptr);
-        else vit_step<K, false>(mc, mn, xt, wt, negc, table, p.inv_hi, p.inv_lo, nullptr, nullptr);
-        __syncthreads();
+        if (keep || last) vit_step<K, C, true>(mc, mn, xt, wt, negc, table, j_first, p.inv_hi, p.inv_lo, keep ? bp + (size_t)t * SJ : nullptr, last ? lastarg : nullptr);
+        else vit_step<K, C, false>(mc, mn, xt, wt, negc, table, j_first, p.inv_hi, p.inv_lo, nullptr, nullptr);
+        tile_sync<C>();
         float* sw = mc; mc = mn; mn = sw;
       }
       // mc[j] = min over top of the final costs, lastarg[j] = its first top.  First pass of a tail-biting search, or an open
@@ -261,7 +322,7 @@ __global__ void __launch_bounds__(VitCfg<K>::kThreads, 1) viterbi_kernel(const V
         __syncthreads();
         j0 = (int)(s_win.key & 0xFFFFu);                                 // low 16-K bits of the winner (j < 2^(16-K))
       }
-      if (keep && warp == 0) {
+      if (keep && warp == 0 && rank == 0) {
         // last state: with tail-biting the cheapest state whose low bits equal j0, else the overall winner
         uint32_t s = p.tailbite ? ((uint32_t)lastarg[j0] * SJ + (uint32_t)j0) : ((s_win.key >> 16) * SJ + (s_win.key & 0xFFFFu));
         int32_t* out = p.states + (size_t)tile * T;
@@ -271,7 +332,7 @@ __global__ void __launch_bounds__(VitCfg<K>::kThreads, 1) viterbi_kernel(const V
         }
         // back along the path (htr/reference.py:45-49): s_{t-1} = bp_{t-1}[s_t >> K] * SJ + (s_t >> K).  The back-pointers of kLevels
         // steps are loaded together: for every value of the tops still unknown, candidate id = those tops as a number in base NB
-        constexpr int LV = C::kLevels;
+        constexpr int LV = Cfg::kLevels;
         for (int t = T - 1; t >= 1; t -= LV) {
           constexpr int kMost = 8;                                       // loads of a lane per level: NB^(LV-1) <= 256
           uint32_t got[LV][kMost];
@@ -308,6 +369,7 @@ __global__ void __launch_bounds__(VitCfg<K>::kThreads, 1) viterbi_kernel(const V
       __syncthreads();
     }
   }
+  if (C > 1) tile_sync<C>();                                              // nobody leaves while its shared memory may still be written
 }
 
 // every codebook value through the device function above (test hook)
@@ -332,38 +394,84 @@ bool width_ok(int K) { return K == 2 || K == 3 || K == 4 || K == 5 || K == 6 || 
 
 thread_local int t_vit_cuda = 0;
 
-template <int K>
-int resident_ctas(int* out) {
+// thread blocks (C = 1) or clusters that the GPU holds at once
+template <int K, int C>
+int resident(int* out) {
   static int cached[64] = {0};
   int dev = 0, sms = 0, per = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return (int)cudaErrorInvalidDevice;
   if (dev >= 0 && dev < 64 && cached[dev]) { *out = cached[dev]; return 0; }
-  cudaError_t e = cudaFuncSetAttribute(viterbi_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, VitCfg<K>::kSmem);
+  using Cfg = VitCfg<K, C>;
+  cudaError_t e = cudaFuncSetAttribute(viterbi_kernel<K, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
   if (e != cudaSuccess) return (int)e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, viterbi_kernel<K>, VitCfg<K>::kThreads, VitCfg<K>::kSmem)) != cudaSuccess) return (int)e;
+  if constexpr (C == 1) {
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, viterbi_kernel<K, C>, Cfg::kThreads, Cfg::kSmem)) != cudaSuccess) return (int)e;
+    per *= sms;
+  } else {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(Cfg::kThreads);
+    cfg.dynamicSmemBytes = Cfg::kSmem;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if ((e = cudaOccupancyMaxActiveClusters(&per, viterbi_kernel<K, C>, &cfg)) != cudaSuccess) return (int)e;
+  }
   if (per < 1) return (int)cudaErrorLaunchOutOfResources;
-  *out = sms * per;
-  if (dev >= 0 && dev < 64) cached[dev] = *out;
+  *out = per;
+  if (dev >= 0 && dev < 64) cached[dev] = per;
   return 0;
 }
 
-int resident_for(int K, int* out) {
+// Thread blocks per tile: as many as leave every tile a cluster of its own at once (few tiles leave SMs idle otherwise; a step of a
+// shared tile pays a cluster barrier).  VITFIG
+template <int K>
+int tile_split(int B, int* split, int* at_once) {
+  int one = 0, two = 0, four = 0;
+  if (const int e = resident<K, 1>(&one)) return e;
+  if (resident<K, 2>(&two)) { (void)cudaGetLastError(); two = 0; }
+  if (resident<K, 4>(&four)) { (void)cudaGetLastError(); four = 0; }
+  *split = B <= four ? 4 : B <= two ? 2 : 1;
+  *at_once = *split == 4 ? four : *split == 2 ? two : one;
+  return 0;
+}
+
+int split_for(int K, int B, int* split, int* at_once) {
   switch (K) {
-    case 2: return resident_ctas<2>(out);
-    case 3: return resident_ctas<3>(out);
-    case 4: return resident_ctas<4>(out);
-    case 5: return resident_ctas<5>(out);
-    case 6: return resident_ctas<6>(out);
-    case 8: return resident_ctas<8>(out);
+    case 2: return tile_split<2>(B, split, at_once);
+    case 3: return tile_split<3>(B, split, at_once);
+    case 4: return tile_split<4>(B, split, at_once);
+    case 5: return tile_split<5>(B, split, at_once);
+    case 6: return tile_split<6>(B, split, at_once);
+    case 8: return tile_split<8>(B, split, at_once);
   }
   return (int)cudaErrorInvalidValue;
 }
 
+template <int K, int C>
+int launch_split(const VitParams& p, int tiles_at_once, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)(tiles_at_once * C));
+  cfg.blockDim = dim3(VitCfg<K, C>::kThreads);
+  cfg.dynamicSmemBytes = VitCfg<K, C>::kSmem;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, viterbi_kernel<K, C>, p);
+}
 template <int K>
-int launch(const VitParams& p, int grid, cudaStream_t st) {
-  viterbi_kernel<K><<<grid, VitCfg<K>::kThreads, VitCfg<K>::kSmem, st>>>(p);
-  return (int)cudaGetLastError();
+int launch(const VitParams& p, int split, int tiles_at_once, cudaStream_t st) {
+  return split == 4 ? launch_split<K, 4>(p, tiles_at_once, st) : split == 2 ? launch_split<K, 2>(p, tiles_at_once, st) : launch_split<K, 1>(p, tiles_at_once, st);
 }
 
 }  // namespace
@@ -375,9 +483,9 @@ extern "C" {
 
 size_t htr_viterbi_workspace_bytes(int B, int T, int K) {
   if (!width_ok(K) || B < 1 || T < 1 || T > kVitMaxT) return 0;
-  int resident = 0;
-  if (resident_for(K, &resident) != 0) return 0;
-  const int grid = B < resident ? B : resident;
+  int split = 0, at_once = 0;
+  if (split_for(K, B, &split, &at_once) != 0) return 0;
+  const int grid = B < at_once ? B : at_once;
   return (size_t)grid * T * ((size_t)65536 >> K);
 }
 
@@ -387,10 +495,10 @@ int htr_viterbi(const float* x, const float* w, int B, int T, int K, int tailbit
   if (B < 0 || T < 1 || T > kVitMaxT) return HTR_ERR_BAD_SHAPE;
   if (B == 0) return HTR_OK;
   if (!x || !w || !states) return HTR_ERR_NULL;
-  int resident = 0;
-  int e = resident_for(K, &resident);
+  int split = 0, at_once = 0;
+  int e = split_for(K, B, &split, &at_once);
   if (e) { t_vit_cuda = e; return HTR_ERR_CUDA; }
-  const int grid = B < resident ? B : resident;
+  const int grid = B < at_once ? B : at_once;
   if (!workspace || workspace_bytes < (size_t)grid * T * ((size_t)65536 >> K)) return HTR_ERR_WORKSPACE;
   const double inv = inverse_rms();
   VitParams p;
@@ -406,12 +514,12 @@ int htr_viterbi(const float* x, const float* w, int B, int T, int K, int tailbit
   p.inv_lo = (float)(inv - (double)p.inv_hi);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (K) {
-    case 2: e = launch<2>(p, grid, st); break;
-    case 3: e = launch<3>(p, grid, st); break;
-    case 4: e = launch<4>(p, grid, st); break;
-    case 5: e = launch<5>(p, grid, st); break;
-    case 6: e = launch<6>(p, grid, st); break;
-    case 8: e = launch<8>(p, grid, st); break;
+    case 2: e = launch<2>(p, split, grid, st); break;
+    case 3: e = launch<3>(p, split, grid, st); break;
+    case 4: e = launch<4>(p, split, grid, st); break;
+    case 5: e = launch<5>(p, split, grid, st); break;
+    case 6: e = launch<6>(p, split, grid, st); break;
+    case 8: e = launch<8>(p, split, grid, st); break;
   }
   if (e) { t_vit_cuda = e; return HTR_ERR_CUDA; }
   return HTR_OK;

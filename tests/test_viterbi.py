@@ -112,3 +112,18 @@ def test_arguments_are_checked():
     with pytest.raises(_lib.HTRError):
         encoder.viterbi(x.to(dev), w.to(dev), torch.zeros(65536, device=dev), 4)   # not the codebook
     assert encoder.viterbi(x[:0].to(dev), w[:0].to(dev), None, 4).shape == (0, 256)
+
+
+@pytest.mark.parametrize("K", (2, 3, 4, 5, 6, 8))
+@pytest.mark.parametrize("B", (1, 37, 74, 75))
+def test_tiles_shared_by_a_cluster_equal_tiles_of_one_block(K, B):
+    """Few tiles are searched by clusters of four or two thread blocks, more by one each: the same bits."""
+    from htr_b200 import encoder
+
+    dev = torch.device("cuda:0")
+    x, w = tiles(300, 256, 70 + K)
+    want, cost = encoder.viterbi(x.to(dev), w.to(dev), None, K, return_cost=True)
+    got, c = encoder.viterbi(x[:B].to(dev), w[:B].to(dev), None, K, return_cost=True)
+    assert torch.equal(got, want[:B]) and torch.equal(c, cost[:B])
+    opened, _ = encoder.viterbi(x.to(dev), w.to(dev), None, K, tailbite=False, return_cost=True)
+    assert torch.equal(encoder.viterbi(x[:B].to(dev), w[:B].to(dev), None, K, tailbite=False), opened[:B])
