@@ -21,7 +21,7 @@
 //  * The traceback is a chain of dependent loads; the K unknown bits per step are few enough to load two to five steps' candidates
 //    at once, so a warp resolves that many steps per memory latency.
 // Measured, 256 tiles (K = 2, 3, 4, 5, 6, 8): 3.91, 3.69, 3.48, 3.60, 3.82, 3.89 ms with the values recomputed and one state per
-// latency in the traceback; 2.65, 2.05, 2.01, 2.08, 2.25, 2.63 ms in this form.
+// latency in the traceback; 2.70, 1.98, 2.01, 2.10, 2.18, 2.54 ms in this form.
 //
 // The codebook value in float: v(s) lands in a float through the 1.5 * 2^23 mantissa trick and float32(v / rms) =
 // fma(v, inv_hi, v * inv_lo) with 1/rms split in two floats -- exact for all 1021 possible v (checked by the tests against the
@@ -429,13 +429,16 @@ int resident(int* out) {
 }
 
 // Thread blocks per tile: as many as leave every tile a cluster of its own at once (few tiles leave SMs idle otherwise; a step of a
-// shared tile pays a cluster barrier).  VITFIG
+// shared tile pays a cluster barrier and stores its costs several times: 2^(16-K) of them).  One block / two / four, ms: K = 2 1.34 / 1.01 /
+// 1.14, K = 3 1.00 / 1.16 / 0.88, K = 4 1.00 / 0.81 / 0.67, K = 5 1.05 / 0.79 / 0.64, K = 8 1.28 / 1.03 / 1.00.
 template <int K>
 int tile_split(int B, int* split, int* at_once) {
   int one = 0, two = 0, four = 0;
   if (const int e = resident<K, 1>(&one)) return e;
   if (resident<K, 2>(&two)) { (void)cudaGetLastError(); two = 0; }
   if (resident<K, 4>(&four)) { (void)cudaGetLastError(); four = 0; }
+  if (K == 2) four = 0;
+  if (K == 3) two = 0;
   *split = B <= four ? 4 : B <= two ? 2 : 1;
   *at_once = *split == 4 ? four : *split == 2 ? two : one;
   return 0;
