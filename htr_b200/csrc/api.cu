@@ -253,6 +253,10 @@ static int make_plan(int M, int m, int n, int K, Plan* out, int kind = 0) {
 // SM of packed_gemv.cuh from 256 thousand weights on (512x512 4.1 us either way, 1024x1024 4.5 -> 4.1, 256x16384 10.5 -> 6.6), except
 // where most blocks of a run end a row block (32768x256: 5.2 against 5.6).
 constexpr long long kChainSmall = 1 << 18;
+// The linears inside a decoder's layers (a residual or an activation folded in, a norm before fewer rows than a vocabulary has) stay on
+// packed_gemv.cuh.  The chain form would save 5 % of a token there, but it adds in another order: each rounding to bf16 between the
+// layers that falls the other way is carried on, and over 36 layers the logits move by 4.7 % (2-norm).  After the last one nothing follows.
+constexpr int kChainLastRows = 1 << 15;
 static bool chain_serves(int m, int n) { return n <= kG1MaxCols && (long long)m * n >= kChainSmall && (n >= 512 || m < 16384); }
 static size_t chain_partial_bytes(int grid) { return (size_t)grid * 2 * 128 * sizeof(float); }
 static int make_chain_plan(int m, int n, Plan* out) {
@@ -449,7 +453,8 @@ static int launch_linear(const void* x, int dtype, int M, int n_in, const void* 
   int kind = gemv_kind(M, dtype, n, prologue);
   const bool exact = (flags & HTR_LINEAR_EXACT_SUMS) && prologue == 0 && (M <= 2 || kind == 2);
   if (exact && kind != 2) kind = 1;
-  const bool chain = kind == 0 && M == 1 && npeer == 0 && !(flags & HTR_LINEAR_INPUT_INDEPENDENT) && chain_serves(m, n);
+  const bool chain = kind == 0 && M == 1 && npeer == 0 && !(flags & HTR_LINEAR_INPUT_INDEPENDENT) && chain_serves(m, n) &&
+                     !residual && (prologue == 0 || (prologue == 1 && m >= kChainLastRows));
   const int rc = chain ? make_chain_plan(m, n, &pl) : make_plan(M, m, n, K, &pl, kind);
   if (rc != HTR_OK) return rc;
   const size_t need = chain ? counter_bytes(m) + chain_partial_bytes(pl.grid) : counter_bytes(m) + (size_t)pl.rbs * pl.slots * pl.rows_t * 128 * ((exact || kind == 2) ? sizeof(long long) : sizeof(float));

@@ -174,41 +174,43 @@ __global__ void __launch_bounds__(128) attention_kernel(const __nv_bfloat16* __r
 // per query head: position -> rotation -> scores -> values, eight rows at a time, 17 us at position 200.  So
 //  * a cluster shares the positions of a key/value head (block r takes positions r, r + 4, ...) and a block serves the whole group of
 //    query heads, so that each key and value row is read once;
-//  * the rows of a block do not depend on the length, so the first keys and values (256 positions of the cluster) are loaded right
-//    after the wait, together with the position and the new row;
+//  * the rows of a block do not depend on the length, so the first keys and values (256 positions of the cluster) are copied to shared
+//    memory right after the wait, while the position and the new row arrive; later ones follow two buffers ahead;
 //  * the rows are usually in DRAM by then: before the wait the position is read as a hint, to bring them to L2 and
 //    to load the rotation, which is loaded again if the position turns out to be another.
-// The cluster's partial softmax results meet in distributed shared memory; block h % 4 finishes query head h of the group.  Same
-// roundings as rope_cache_kernel + attention_kernel up to the order of the float32 sums.  A token of the 36-layer decoder at position
-// 200: 2.97 -> 2.52 ms; of a small one (12 layers, 16 / 4 heads) at position 900: 1.10 -> 0.46 ms.
+// The order of every float32 sum is fixed and does not depend on the split: a score is one thread's sum along the row, the value rows
+// are added in four streams (positions t = r mod 4, a block each), and the weights as 128 threads would, then over their lanes and
+// warps.  A decoder of dozens of bf16 layers turns one other rounding into another result of percents, so this order stays.  Block h
+// of the cluster adds up and finishes query head h of the group: scores and streams meet in its shared memory.
+// A token of a small decoder (12 layers, 16 / 4 heads) at position 200: 617 -> 457 us, at position 900: 1265 -> 538.
 constexpr int kAttSplit = 4, kAttHeads = 4, kAttThreads = 256, kAttWarps = kAttThreads / 32;
+constexpr int kAttRows = 64, kAttPitch = 272;                // positions of a buffer; bytes of a row in it (17 x 16: no bank conflicts)
 constexpr int kAttLocal = HTR_DEC_MAX_LEN / kAttSplit;       // positions of one thread block at most
+constexpr int kAttBuffer = kAttRows * kAttPitch, kAttSmem = 4 * kAttBuffer;
 
-__device__ __forceinline__ void unpack8(const uint4 raw, float (&f)[8]) {
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = __uint_as_float(w[i] << 16);
-    f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
-}
 __device__ __forceinline__ void cluster_write(float* mine, unsigned rank, float v) {
   uint32_t remote;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
 __global__ void __cluster_dims__(kAttSplit, 1, 1) __launch_bounds__(kAttThreads, 1)
     rope_attention_kernel(const __nv_bfloat16* __restrict__ qkv, const long long* __restrict__ pos, const float* __restrict__ cosv,
-                          const float* __restrict__ sinv, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
+                          const float* __restrict__ sinv, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
                           __nv_bfloat16* __restrict__ out, int hq, int hkv, int capacity, int* __restrict__ status) {
   constexpr int D = 128, S = kAttSplit, H = kAttHeads;
+  static_assert(S == H && kAttThreads == kAttRows * H, "a block finishes one head; a thread per position and head");
+  extern __shared__ __align__(16) unsigned char rows[];        // two buffers of keys, two of values
   __shared__ __align__(16) float sq[H][D];
   __shared__ __align__(16) float sk[D], sv[D];
-  __shared__ float sc[H][kAttLocal];
-  __shared__ __align__(16) float part[kAttWarps][H][D];
-  __shared__ float s_m[H], s_l[H];
-  __shared__ float in_out[H][S][D], in_m[H][S], in_l[H][S];    // what the blocks of the cluster found for this block's query heads
+  __shared__ float sc[H][kAttLocal];                            // scores of this block's positions
+  __shared__ float all[HTR_DEC_MAX_LEN];                        // from the cluster, for the head this block finishes: scores ...
+  __shared__ float part[S][D];                                  // ... and weighted sums
+  __shared__ float in_m[H][S * 2];                              // largest scores: two warps per head and block
+  __shared__ float red[4];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this block runs: its shared memory may be written (waited for below)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -237,41 +239,32 @@ __global__ void __cluster_dims__(kAttSplit, 1, 1) __launch_bounds__(kAttThreads,
     const int src_head = who < H ? head0 + min(who, nh - 1) : who == 4 ? hq + kvh : hq + hkv + kvh;
     if (who < 6) raw[k] = *reinterpret_cast<const __nv_bfloat162*>(qkv + (size_t)src_head * D + 2 * pair);
   }
-  const int sub = lane >> 3, e = lane & 7;                     // scores: eight lanes per position, 16 dimensions each
-  constexpr int kKeys = 2;                                      // key rows of a lane group in flight
-  uint4 kr[kKeys][2];
-  auto load_keys = [&](int base, int end) {
+  const uint32_t rows_at = (uint32_t)__cvta_generic_to_shared(rows);
+  // positions [64 chunk, 64 chunk + 64) of this block below `end` into a buffer (16 threads per row); commits a group, also an empty one
+  auto copy_rows = [&](const __nv_bfloat16* base, int buffer, int chunk, int end) {
 #pragma unroll
-    for (int k = 0; k < kKeys; ++k) {
-      const int i = base + (k * kAttWarps + warp) * 4 + sub;
-      kr[k][0] = kr[k][1] = make_uint4(0u, 0u, 0u, 0u);
-      if (i < end) {
-        const uint4* row = reinterpret_cast<const uint4*>(kbase + (size_t)(i * S + rank) * stride + e * 16);
-        kr[k][0] = row[0];
-        kr[k][1] = row[1];
-      }
+    for (int k = 0; k < kAttRows * 16 / kAttThreads; ++k) {
+      const int row = k * (kAttThreads / 16) + (tid >> 4), i = chunk * kAttRows + row;
+      if (i < end)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(rows_at + buffer * kAttBuffer + row * kAttPitch + (tid & 15) * 16),
+                     "l"(base + (size_t)(i * S + rank) * stride + (tid & 15) * 8) : "memory");
     }
-  };
-  constexpr int kAhead = 8;                                     // value rows of a warp in flight: warp, warp + 8, ... of the block
-  uint2 vr[kAhead];
-  auto load_values = [&](int base, int end) {
-#pragma unroll
-    for (int j = 0; j < kAhead; ++j) {
-      const int i = base + warp + kAttWarps * j;
-      vr[j] = i < end ? *reinterpret_cast<const uint2*>(vbase + (size_t)(i * S + rank) * stride + 4 * lane) : make_uint2(0u, 0u);
-    }
+    copy_commit();
   };
   const int local_limit = (limit - rank + S - 1) / S;           // positions of this block inside the caches
-  load_keys(0, local_limit);
-  load_values(0, local_limit);
+  copy_rows(kbase, 0, 0, local_limit);
+  copy_rows(vbase, 2, 0, local_limit);
   if (p0 < 0 || p0 >= limit) {                                  // outside the cache: no cache row is touched, zeros come out (the whole cluster)
     if (status && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) atomicOr(status, 4);
     for (int x = tid; x < nh * D && rank == 0; x += kAttThreads) out[(size_t)head0 * D + x] = __float2bfloat16_rn(0.f);
+    copy_wait<0>();
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     return;
   }
-  const int p = (int)p0, mine = p >= rank ? (p - rank) / S + 1 : 0;   // positions of this block
-  const bool owner = p % S == rank;                             // of the new position, its last
+  const int p = (int)p0, mine = (p + S - 1 - rank) / S;         // cached positions of this block (the new one does not come through the cache)
+  copy_rows(kbase, 1, 1, mine);
+  copy_rows(vbase, 3, 1, mine);
+  const bool owner = p % S == rank;                             // of the new position
   if (p != (int)hint) {
     c = cosv[(size_t)p * (D / 2) + pair];
     s = sinv[(size_t)p * (D / 2) + pair];
@@ -291,105 +284,111 @@ __global__ void __cluster_dims__(kAttSplit, 1, 1) __launch_bounds__(kAttThreads,
         *reinterpret_cast<__nv_bfloat162*>((who == 4 ? k_cache : v_cache) + ((size_t)p * hkv + kvh) * D + 2 * pair) = r;
     }
   }
-  __syncthreads();
-  // ---- scores
-  for (int base = 0; base < mine; base += kKeys * kAttWarps * 4) {
-    if (base > 0) load_keys(base, mine - owner);               // (the new row does not come through the cache)
-#pragma unroll
-    for (int k = 0; k < kKeys; ++k) {
-      const int i = base + (k * kAttWarps + warp) * 4 + sub;
-      if (base + (k * kAttWarps + warp) * 4 >= mine) break;      // warp-uniform
-      float kf[16];
-      unpack8(kr[k][0], *reinterpret_cast<float(*)[8]>(kf));
-      unpack8(kr[k][1], *reinterpret_cast<float(*)[8]>(kf + 8));
-      if (owner && i == mine - 1) {
-#pragma unroll
-        for (int d = 0; d < 16; ++d) kf[d] = sk[e * 16 + d];
-      }
-#pragma unroll
-      for (int h = 0; h < H; ++h) {
-        float dot = 0.f;
-#pragma unroll
-        for (int d = 0; d < 16; d += 4) {
-          const float4 q = *reinterpret_cast<const float4*>(&sq[h][e * 16 + d]);
-          dot += kf[d] * q.x + kf[d + 1] * q.y + kf[d + 2] * q.z + kf[d + 3] * q.w;
-        }
-#pragma unroll
-        for (int o = 4; o; o >>= 1) dot += __shfl_xor_sync(0xFFFFFFFFu, dot, o);
-        if (e == h && i < mine) sc[h][i] = dot;
-      }
-    }
-  }
-  __syncthreads();
-  if (warp < H) {                                               // softmax of this block's positions, one warp per head
-    float mx = -3.0e38f, sum = 0.f;
-    for (int i = lane; i < mine; i += 32) mx = fmaxf(mx, sc[warp][i]);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-    for (int i = lane; i < mine; i += 32) {
-      const float w = __expf(sc[warp][i] - mx);
-      sc[warp][i] = w;
-      sum += w;
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    if (lane == 0) {
-      s_m[warp] = mx;
-      s_l[warp] = sum;
-    }
-  }
-  __syncthreads();
-  // ---- values: a lane holds four dimensions of a row, for all heads
-  float acc[H][4];
-#pragma unroll
-  for (int h = 0; h < H; ++h) acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.f;
-  for (int base = 0; base < mine; base += kAttWarps * kAhead) {
-    if (base > 0) load_values(base, mine - owner);
-#pragma unroll
-    for (int j = 0; j < kAhead; ++j) {
-      const int i = base + warp + kAttWarps * j;
-      if (i >= mine) break;
-      float4 v = make_float4(__uint_as_float(vr[j].x << 16), __uint_as_float(vr[j].x & 0xFFFF0000u), __uint_as_float(vr[j].y << 16),
-                             __uint_as_float(vr[j].y & 0xFFFF0000u));
-      if (owner && i == mine - 1) v = *reinterpret_cast<const float4*>(sv + 4 * lane);
-#pragma unroll
-      for (int h = 0; h < H; ++h) {
-        const float w = sc[h][i];
-        acc[h][0] += w * v.x; acc[h][1] += w * v.y; acc[h][2] += w * v.z; acc[h][3] += w * v.w;
-      }
-    }
-  }
-#pragma unroll
-  for (int h = 0; h < H; ++h) *reinterpret_cast<float4*>(&part[warp][h][4 * lane]) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+  // ---- scores: warps 2h and 2h + 1 take head h, a thread one position of a buffer
+  const int h = warp >> 1, half = warp & 1, chunks = (mine + kAttRows - 1) / kAttRows;
+  float mx = -3.0e38f;
+  copy_wait<3>();
   __syncthreads();
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every block of the cluster has started
-  for (int x = tid; x < H * D; x += kAttThreads) {
-    const int h = x >> 7, d = x & 127;
-    float o = 0.f;
+  if (owner && half == 0) {                                     // of the new position: four dimensions per lane
+    const float4 k4 = *reinterpret_cast<const float4*>(sk + 4 * lane), q4 = *reinterpret_cast<const float4*>(&sq[h][4 * lane]);
+    float d = k4.x * q4.x + k4.y * q4.y + k4.z * q4.z + k4.w * q4.w;
 #pragma unroll
-    for (int w = 0; w < kAttWarps; ++w) o += part[w][h][d];
-    cluster_write(&in_out[h][rank][d], h % S, o);
+    for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xFFFFFFFFu, d, o);
+    if (lane == 0) cluster_write(&all[p], h, d);
+    mx = d;
   }
-  if (tid < H) {
-    cluster_write(&in_m[tid][rank], tid % S, s_m[tid]);
-    cluster_write(&in_l[tid][rank], tid % S, s_l[tid]);
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    if (chunk > 0) {                                            // (groups after this chunk's: values 1 and keys 2, then keys chunk + 1)
+      if (chunk == 1) copy_wait<2>();
+      else copy_wait<1>();
+      __syncthreads();
+    }
+    const int row = half * 32 + lane, i = chunk * kAttRows + row;
+    if (i < mine) {
+      const uint4* kr = reinterpret_cast<const uint4*>(rows + (chunk & 1) * kAttBuffer + row * kAttPitch);
+      float d = 0.f;
+#pragma unroll
+      for (int x = 0; x < 16; ++x) {
+        const uint4 raw4 = kr[x];
+        const float4 q0 = *reinterpret_cast<const float4*>(&sq[h][8 * x]), q1 = *reinterpret_cast<const float4*>(&sq[h][8 * x + 4]);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw4.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw4.y));
+        const float2 e = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw4.z)), f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw4.w));
+        d += a.x * q0.x + a.y * q0.y + b.x * q0.z + b.y * q0.w + e.x * q1.x + e.y * q1.y + f.x * q1.z + f.y * q1.w;
+      }
+      sc[h][i] = d;
+      cluster_write(&all[i * S + rank], h, d);
+      mx = fmaxf(mx, d);
+    }
+    if (chunks > 1) {
+      __syncthreads();                                          // the buffer is free
+      copy_rows(kbase, chunk & 1, chunk + 2, mine);
+    }
   }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+  if (lane < S) cluster_write(&in_m[h][rank * 2 + half], lane, mx);
+  copy_wait<0>();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  for (int x = tid; x < H / S * D; x += kAttThreads) {
-    const int h = (x >> 7) * S + rank, d = x & 127;
-    if (h >= nh) break;
-    float mx = in_m[h][0];
+  mx = in_m[h][0];
 #pragma unroll
-    for (int r = 1; r < S; ++r) mx = fmaxf(mx, in_m[h][r]);
-    float sum = 0.f, acc_o = 0.f;
-#pragma unroll
-    for (int r = 0; r < S; ++r) {
-      const float w = __expf(in_m[h][r] - mx);                  // (a block without positions: m = -3e38, weight zero)
-      sum += w * in_l[h][r];
-      acc_o += w * in_out[h][r][d];
+  for (int r = 1; r < 2 * S; ++r) mx = fmaxf(mx, in_m[h][r]);
+  // ---- values: a warp sums half of the dimensions for its head, position after position; a lane holds two dimensions
+  float a0 = 0.f, a1 = 0.f;
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    if (chunk > 1) {
+      copy_wait<1>();
+      __syncthreads();
     }
-    out[(size_t)(head0 + h) * D + d] = __float2bfloat16_rn(acc_o / sum);
+    const unsigned char* vr = rows + (2 + (chunk & 1)) * kAttBuffer + half * 128 + lane * 4;
+    for (int base = chunk * kAttRows; base < min(mine, (chunk + 1) * kAttRows); base += 32, vr += 32 * kAttPitch) {
+      const float e = base + lane < mine ? __expf(sc[h][base + lane] - mx) : 0.f;
+      const int n = min(32, mine - base);
+      if (n == 32) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float w = __shfl_sync(0xFFFFFFFFu, e, j);
+          const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(vr + j * kAttPitch));
+          a0 += w * v.x; a1 += w * v.y;
+        }
+      } else {
+#pragma unroll 4
+        for (int j = 0; j < n; ++j) {
+          const float w = __shfl_sync(0xFFFFFFFFu, e, j);
+          const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(vr + j * kAttPitch));
+          a0 += w * v.x; a1 += w * v.y;
+        }
+      }
+    }
+    if (chunks > 2) {
+      __syncthreads();
+      copy_rows(vbase, 2 + (chunk & 1), chunk + 2, mine);
+    }
+  }
+  cluster_write(&part[rank][half * 64 + 2 * lane], h, a0);
+  cluster_write(&part[rank][half * 64 + 2 * lane + 1], h, a1);
+  // ---- the head this block finishes: sum of its weights, then the streams and the new row
+  float mo = in_m[rank][0];
+#pragma unroll
+  for (int r = 1; r < 2 * S; ++r) mo = fmaxf(mo, in_m[rank][r]);
+  if (tid < D) {
+    float sum = 0.f;
+    for (int t = tid; t <= p; t += D) sum += __expf(all[t] - mo);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if (lane == 0) red[warp] = sum;
+  }
+  copy_wait<0>();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (tid < D && rank < nh) {
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) sum += red[w];
+    const float last = __expf(all[p] - mo);
+    const float acc = part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid] + last * sv[tid];
+    out[(size_t)(head0 + rank) * D + tid] = __float2bfloat16_rn(acc / sum);
   }
 }
 
@@ -408,10 +407,11 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const __nv_bfloat16* __rest
 }
 
 template <typename Kern, typename... Args>
-int launch_pdl(Kern kern, dim3 grid, dim3 block, cudaStream_t st, Args... args) {
+int launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -429,7 +429,7 @@ int htr_dec_add_rmsnorm(void* resid, const void* delta, const void* weight, void
   if (rows <= 0) return HTR_OK;
   if (!resid || !weight || !out) return HTR_ERR_NULL;
   if (h <= 0 || h % 2 || h > 8192) return HTR_ERR_BAD_SHAPE;
-  const int e = launch_pdl(add_rmsnorm_kernel, dim3(rows), dim3(256), static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(resid),
+  const int e = launch_pdl(add_rmsnorm_kernel, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(resid),
                            static_cast<const __nv_bfloat16*>(delta), static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(out), h, eps);
   return e ? HTR_ERR_CUDA : HTR_OK;
 }
@@ -439,7 +439,7 @@ int htr_dec_rope_cache(const void* qkv, const int64_t* pos, const float* cosv, c
   if (rows <= 0) return HTR_OK;
   if (!qkv || !pos || !cosv || !sinv || !q_out || !k_cache || !v_cache) return HTR_ERR_NULL;
   if (head_dim <= 0 || head_dim % 2 || head_dim > 2048 || q_heads <= 0 || kv_heads <= 0 || capacity <= 0) return HTR_ERR_BAD_SHAPE;
-  const int e = launch_pdl(rope_cache_kernel, dim3(q_heads + 2 * kv_heads, rows), dim3(head_dim / 2), static_cast<cudaStream_t>(stream),
+  const int e = launch_pdl(rope_cache_kernel, dim3(q_heads + 2 * kv_heads, rows), dim3(head_dim / 2), 0, static_cast<cudaStream_t>(stream),
                            static_cast<const __nv_bfloat16*>(qkv), reinterpret_cast<const long long*>(pos), cosv, sinv,
                            static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), q_heads,
                            kv_heads, head_dim, capacity, status);
@@ -451,7 +451,7 @@ int htr_dec_attention(const void* q, const void* k_cache, const void* v_cache, c
   if (rows <= 0) return HTR_OK;
   if (!q || !k_cache || !v_cache || !pos || !out) return HTR_ERR_NULL;
   if (head_dim != 128 || q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads || capacity <= 0) return HTR_ERR_BAD_SHAPE;
-  const int e = launch_pdl(attention_kernel, dim3(q_heads, rows), dim3(128), static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(q),
+  const int e = launch_pdl(attention_kernel, dim3(q_heads, rows), dim3(128), 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(q),
                            static_cast<const __nv_bfloat16*>(k_cache), static_cast<const __nv_bfloat16*>(v_cache),
                            reinterpret_cast<const long long*>(pos), static_cast<__nv_bfloat16*>(out), q_heads, kv_heads, capacity, status);
   return e ? HTR_ERR_CUDA : HTR_OK;
@@ -461,7 +461,15 @@ int htr_dec_rope_attention(const void* qkv, const int64_t* pos, const float* cos
                            int q_heads, int kv_heads, int head_dim, int capacity, int* status, htr_stream_t stream) {
   if (!qkv || !pos || !cosv || !sinv || !k_cache || !v_cache || !out) return HTR_ERR_NULL;
   if (head_dim != 128 || q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads || capacity <= 0) return HTR_ERR_BAD_SHAPE;
-  const int e = launch_pdl(rope_attention_kernel, dim3(kAttSplit * kv_heads, (q_heads / kv_heads + kAttHeads - 1) / kAttHeads), dim3(kAttThreads), static_cast<cudaStream_t>(stream),
+  static bool allowed[64] = {false};                      // shared memory beyond 48 KB: opted in once per device
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return HTR_ERR_CUDA;
+  if (dev < 0 || dev >= 64 || !allowed[dev]) {
+    if (cudaFuncSetAttribute(rope_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttSmem) != cudaSuccess) return HTR_ERR_CUDA;
+    if (dev >= 0 && dev < 64) allowed[dev] = true;
+  }
+  const int e = launch_pdl(rope_attention_kernel, dim3(kAttSplit * kv_heads, (q_heads / kv_heads + kAttHeads - 1) / kAttHeads), dim3(kAttThreads),
+                           kAttSmem, static_cast<cudaStream_t>(stream),
                            static_cast<const __nv_bfloat16*>(qkv), reinterpret_cast<const long long*>(pos), cosv, sinv,
                            static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), static_cast<__nv_bfloat16*>(out), q_heads,
                            kv_heads, capacity, status);
@@ -473,7 +481,7 @@ int htr_dec_swiglu(const void* gate_up, void* out, int rows, int intermediate, h
   if (!gate_up || !out) return HTR_ERR_NULL;
   if (intermediate <= 0 || intermediate % 2) return HTR_ERR_BAD_SHAPE;
   const int total = rows * intermediate;
-  const int e = launch_pdl(swiglu_kernel, dim3((total / 2 + 255) / 256), dim3(256), static_cast<cudaStream_t>(stream),
+  const int e = launch_pdl(swiglu_kernel, dim3((total / 2 + 255) / 256), dim3(256), 0, static_cast<cudaStream_t>(stream),
                            static_cast<const __nv_bfloat16*>(gate_up), static_cast<__nv_bfloat16*>(out), intermediate, total);
   return e ? HTR_ERR_CUDA : HTR_OK;
 }

@@ -2,7 +2,7 @@
 //
 //   y = sv * Ho( diag(scale * CB) * V * Hi(su * x) ),  V[i,j] = bytesum(h_ij) - 510      (the linear of packed_gemv.cuh)
 //
-// What bounds a dependent launch (a token of the decoder: four of them per layer): the decode at an SM's issue rate, and what no
+// What bounds a dependent launch: the decode at an SM's issue rate, and what no
 // weight is decoded in -- the release behind the predecessor, the staging of the activations, the hand-over of partial sums, the
 // tail.  packed_gemv.cuh with three small thread blocks per SM hides those parts of overlapping launches from one another, but in a
 // chain they add up, its blocks get 7 or 8 units each where 6.9 would do, and a scheduler serves its oldest warps first, so that
@@ -161,16 +161,11 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     for (int k = 0; k < kG1Warps; ++k) tot += s_ss[k];
     const float inv = rsqrtf(tot / (float)n + p.eps);
 #pragma unroll
-    for (int i = 0; i < kHeld; ++i) {                        // (the roundings of the unfused operators)
-      const float4 v = held[i], w = make_float4(__uint_as_float(gain[i].x << 16), __uint_as_float(gain[i].x & 0xFFFF0000u),
-                                                __uint_as_float(gain[i].y << 16), __uint_as_float(gain[i].y & 0xFFFF0000u));
-      held[i] = make_float4(bf16_round(bf16_round(v.x * inv) * w.x), bf16_round(bf16_round(v.y * inv) * w.y),
-                            bf16_round(bf16_round(v.z * inv) * w.z), bf16_round(bf16_round(v.w * inv) * w.w));
-    }
-  } else {
+    for (int i = 0; i < kHeld; ++i) held[i] = norm_x(held[i], gain[i], inv);
+  } else {                                                   // (other prologues and the residual form do not come here)
 #pragma unroll
     for (int i = 0; i < kHeld; ++i)
-      if (warp + kG1Warps * i < count) held[i] = fused_x(p, p.x, 0, block_at(i) * 128 + 4 * lane, 1.f);
+      if (warp + kG1Warps * i < count) held[i] = load_x(p.x, 0, block_at(i) * 128 + 4 * lane, p.n_in, p.dtype);
   }
 #pragma unroll
   for (int i = 0; i < kHeld; ++i)
@@ -223,11 +218,8 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     const int row0 = rb * 128 + 4 * lane;
     const uint2 sc_raw = __ldg(reinterpret_cast<const uint2*>(p.scales + row0));
     const unsigned sv_bits = sign_nibble(p.sv, rb * 32 + lane);
-    float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), old = bias4;
-    if (r < 32 && row0 < p.m_out) {
-      if (p.bias) bias4 = load_quad(p.bias, row0, p.dtype);
-      if (p.residual) old = load_quad(p.y, row0, p.dtype);
-    }
+    float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < 32 && row0 < p.m_out && p.bias) bias4 = load_quad(p.bias, row0, p.dtype);
     named_sync_at(1 + buf, kG1Threads);
     float sum = 0.f;
 #pragma unroll
@@ -268,7 +260,6 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
       wht128(v, lane);
       float4 o = make_float4(flip(v[0] * kInvSqrt128, sv_bits & 1u) + bias4.x, flip(v[1] * kInvSqrt128, (sv_bits >> 1) & 1u) + bias4.y,
                              flip(v[2] * kInvSqrt128, (sv_bits >> 2) & 1u) + bias4.z, flip(v[3] * kInvSqrt128, sv_bits >> 3) + bias4.w);
-      if (p.residual) o = make_float4(old.x + bf16_round(o.x), old.y + bf16_round(o.y), old.z + bf16_round(o.z), old.w + bf16_round(o.w));
       if (row0 < p.m_out) store_quad(p.y, row0, p.dtype, o);
     }
     // (ytil is written again only behind the next barrier with the decode warps, which warp 0 reaches after this)

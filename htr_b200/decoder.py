@@ -9,9 +9,9 @@ projections (q|k|v, gate|up) are single packed linears, as the format prescribes
 Every packed linear goes through `htr_b200.ops.linear`.  The glue between them (residual add + RMSNorm, rotary embedding
 + KV-cache write, single-query grouped attention, SwiGLU) runs as four small fused kernels of the library
 (`htr_dec_*`, launched with programmatic stream serialisation so the following packed GEMV prefetches its weights while
-they run); `fused=False` evaluates the same glue with plain torch ops, which is how the kernels are checked.  A single token
-(and two of small layers) folds the norms, the SwiGLU and the residual adds into the packed GEMVs themselves
-(`ops.linear_fused`) and the rotary embedding and cache write into the attention kernel: five launches
+they run); `fused=False` evaluates the same glue with plain torch ops, which is how the kernels are checked.  Steps of at
+most 8 rows (decoding) fold the norms, the SwiGLU and the residual adds into the packed GEMVs themselves
+(`ops.linear_fused`) and, for a single token, the rotary embedding and cache write into the attention kernel: five launches
 per layer.  A decode step reads its position from a device tensor, so one CUDA graph captured once serves every step.
 """
 import dataclasses
@@ -191,12 +191,6 @@ class PackedDecoder:
         out = torch.stack((t1 * cos - t2 * sin, t1 * sin + t2 * cos), dim=-1)
         return out.flatten(-2).to(t.dtype)
 
-    def _folds(self, T):
-        """Whether a step of T rows runs with the glue folded into the GEMVs: one row; two rows of small layers, where launches count.
-        From there on the linears are faster on the tensor-core GEMM between separate glue kernels (8 layers of the 9B class,
-        2 / 3 / 8 rows: 810 / 946 / 1750 -> 774 / 788 / 815 us)."""
-        return T == 1 or (T == 2 and 2 * self.cfg.intermediate * self.cfg.hidden < 1 << 25)
-
     def _cache_rows(self):
         """Addresses of the first layer's cache rows and the bytes between layers."""
         return self.k_cache.data_ptr(), self.v_cache.data_ptr(), self.k_cache.stride(0) * self.k_cache.element_size()
@@ -205,7 +199,7 @@ class PackedDecoder:
         """The same step with the library's glue kernels (bf16 only)."""
         c, L_ = self.cfg, _lib.lib
         T = ids.shape[0]
-        if self.fold and self._folds(T):
+        if T <= ops.GEMV_MAX_M and self.fold:
             return self.forward_folded(ids, pos)
         dev = self.device
         st = torch.cuda.current_stream(dev).cuda_stream
@@ -239,7 +233,7 @@ class PackedDecoder:
         return ops.linear(h, *self.head)
 
     def forward_folded(self, ids, pos):
-        """Decode-sized step (at most 8 rows; see `_folds`) with the norms, the SwiGLU and the residual adds folded into the packed GEMVs
+        """Decode-sized step (at most 8 rows) with the norms, the SwiGLU and the residual adds folded into the packed GEMVs
         (`ops.linear_fused`): six launches per layer instead of nine, five for a single token."""
         c, L_ = self.cfg, _lib.lib
         T = ids.shape[0]
