@@ -36,6 +36,11 @@ struct Entry {
   decltype(&htr_linear_fused) linear_fused;
   decltype(&htr_linear_gemm_padded) linear_gemm_padded;
   decltype(&htr_linear_route_rows) route_rows;
+  decltype(&htr_linear_routed) linear_routed;
+  decltype(&htr_linear_routed_gemm) linear_routed_gemm;
+  decltype(&htr_route_plan_bytes) route_plan_bytes;
+  decltype(&htr_route_plan) route_plan;
+  decltype(&htr_moe_weighted_sum) moe_weighted_sum;
 } g_lib = {};
 
 // ---- workspaces: buffers that ops.py owns (one per device, stream and kind); this table only remembers where they are
@@ -230,6 +235,115 @@ PyObject* py_linear_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(y));
 }
 
+// ---- the launches of a mixture-of-experts step (two linears and a sum: in Python and ctypes 54 us of host work, more than the GPU
+// needs for a few tokens of small experts)
+
+bool vector_of(const at::Tensor* t, const at::Device& dev, at::ScalarType type) { return t && t->dim() == 1 && plain(*t, dev, type); }
+
+// four address tables of one length
+bool tables_of(PyObject* const* a, const at::Device& dev, const at::Tensor* (&t)[4]) {
+  for (int i = 0; i < 4; ++i) {
+    t[i] = tensor(a[i]);
+    if (!vector_of(t[i], dev, at::kLong) || t[i]->numel() != t[0]->numel() || t[i]->numel() > (1 << 24)) return false;
+  }
+  return true;
+}
+
+// linear_routed(x, route, four tables, mt, nt, K, x_div, prologue, out or None)
+PyObject* py_linear_routed(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 12) return none();
+  const at::Tensor *x = tensor(a[0]), *route = tensor(a[1]), *t[4];
+  if (!x || !x->is_cuda() || x->dim() != 2 || !x->is_contiguous()) return none();
+  const at::Device where = x->device();
+  if (!vector_of(route, where, at::kLong) || !tables_of(a + 2, where, t)) return none();
+  const int dt = dtype_code(x->scalar_type());
+  const long mt = PyLong_AsLong(a[6]), nt = PyLong_AsLong(a[7]), K = PyLong_AsLong(a[8]), x_div = PyLong_AsLong(a[9]), prologue = PyLong_AsLong(a[10]);
+  if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
+  const int64_t count = route->numel();
+  if (dt < 0 || count < 1 || count > (1 << 24) || mt < 1 || mt > (1 << 24) || nt < 1 || nt > (1 << 24) || x_div < 1 || x_div > (1 << 24)) return none();
+  const int dev = x->get_device();
+  OnDevice on(dev);
+  void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const at::Tensor* ws = find_workspace(kGemv, dev, st);
+  if (!ws) return none();
+  at::Tensor y;
+  if (a[11] == Py_None) {
+    y = at::detail::empty_cuda({count, (int64_t)mt * 16}, x->scalar_type(), where, std::nullopt);
+  } else {
+    const at::Tensor* o = tensor(a[11]);
+    if (!o || !plain(*o, where, x->scalar_type()) || o->dim() != 2 || o->size(0) != count || o->size(1) != mt * 16) return none();
+    y = *o;
+  }
+  if (g_lib.linear_routed(x->const_data_ptr(), dt, (int)x_div, x->size(1), route->const_data_ptr<int64_t>(), (int)count, (int)t[0]->numel(),
+                          static_cast<const void* const*>(t[0]->const_data_ptr()), static_cast<const void* const*>(t[1]->const_data_ptr()),
+                          static_cast<const uint8_t* const*>(t[2]->const_data_ptr()), static_cast<const uint8_t* const*>(t[3]->const_data_ptr()), (int)mt,
+                          (int)nt, (int)K, y.data_ptr(), (int)prologue, ws->data_ptr(), ws->numel(), st) != HTR_OK)
+    return none();
+  if (a[11] != Py_None) return Py_NewRef(a[11]);
+  return THPVariable_Wrap(std::move(y));
+}
+
+// linear_routed_gemm(x, plan, count, four tables, mt, nt, K, x_div, prologue)
+PyObject* py_linear_routed_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 12) return none();
+  const at::Tensor *x = tensor(a[0]), *plan = tensor(a[1]), *t[4];
+  if (!x || !x->is_cuda() || x->dim() != 2 || !x->is_contiguous()) return none();
+  const at::Device where = x->device();
+  if (!vector_of(plan, where, at::kByte) || !tables_of(a + 3, where, t)) return none();
+  const int dt = dtype_code(x->scalar_type());
+  const long count = PyLong_AsLong(a[2]), mt = PyLong_AsLong(a[7]), nt = PyLong_AsLong(a[8]), K = PyLong_AsLong(a[9]), x_div = PyLong_AsLong(a[10]),
+             prologue = PyLong_AsLong(a[11]);
+  if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
+  if (dt < 0 || count < 1 || count > (1 << 24) || mt < 1 || mt > (1 << 24) || nt < 1 || nt > (1 << 24) || x_div < 1 || x_div > (1 << 24)) return none();
+  if ((size_t)plan->numel() < g_lib.route_plan_bytes((int)count, (int)t[0]->numel())) return none();
+  const int dev = x->get_device();
+  OnDevice on(dev);
+  void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const at::Tensor* ws = find_workspace(kGemm, dev, st);
+  if (!ws) return none();
+  at::Tensor y = at::detail::empty_cuda({(int64_t)count, (int64_t)mt * 16}, x->scalar_type(), where, std::nullopt);
+  if (g_lib.linear_routed_gemm(x->const_data_ptr(), dt, (int)x_div, x->size(1), plan->const_data_ptr(), (int)count, (int)t[0]->numel(),
+                               static_cast<const void* const*>(t[0]->const_data_ptr()), static_cast<const void* const*>(t[1]->const_data_ptr()),
+                               static_cast<const uint8_t* const*>(t[2]->const_data_ptr()), static_cast<const uint8_t* const*>(t[3]->const_data_ptr()), (int)mt,
+                               (int)nt, (int)K, y.data_ptr(), (int)prologue, ws->data_ptr(), ws->numel(), st) != HTR_OK)
+    return none();
+  return THPVariable_Wrap(std::move(y));
+}
+
+// route_plan(route, four tables)
+PyObject* py_route_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 5) return none();
+  const at::Tensor *route = tensor(a[0]), *t[4];
+  if (!route || !route->is_cuda() || !vector_of(route, route->device(), at::kLong) || !tables_of(a + 1, route->device(), t)) return none();
+  const int64_t count = route->numel(), rows = t[0]->numel();
+  const size_t need = count < 1 || count > (1 << 24) ? 0 : g_lib.route_plan_bytes((int)count, (int)rows);
+  if (need == 0) return none();
+  const int dev = route->get_device();
+  OnDevice on(dev);
+  at::Tensor plan = at::detail::empty_cuda({(int64_t)need}, at::kByte, route->device(), std::nullopt);
+  if (g_lib.route_plan(route->const_data_ptr<int64_t>(), (int)count, (int)rows, static_cast<const void* const*>(t[0]->const_data_ptr()), plan.data_ptr(),
+                       need, c10::cuda::getCurrentCUDAStream(dev).stream()) != HTR_OK)
+    return none();
+  return THPVariable_Wrap(std::move(plan));
+}
+
+// moe_weighted_sum(dn [T * k, h], gates [T, k] float32)
+PyObject* py_moe_weighted_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 2) return none();
+  const at::Tensor *dn = tensor(a[0]), *gates = tensor(a[1]);
+  if (!dn || !gates || !dn->is_cuda() || dn->dim() != 2 || !dn->is_contiguous() || !plain(*gates, dn->device(), at::kFloat) || gates->dim() != 2) return none();
+  const int dt = dtype_code(dn->scalar_type());
+  const int64_t T = gates->size(0), k = gates->size(1), h = dn->size(1);
+  if (dt < 0 || T < 1 || T > (1 << 24) || k > (1 << 24) || h > (1 << 24) || dn->size(0) != T * k) return none();
+  const int dev = dn->get_device();
+  OnDevice on(dev);
+  at::Tensor y = at::detail::empty_cuda({T, h}, dn->scalar_type(), dn->device(), std::nullopt);
+  if (g_lib.moe_weighted_sum(dn->const_data_ptr(), dt, gates->const_data_ptr<float>(), (int)T, (int)k, (int)h, y.data_ptr(),
+                             c10::cuda::getCurrentCUDAStream(dev).stream()) != HTR_OK)
+    return none();
+  return THPVariable_Wrap(std::move(y));
+}
+
 // set_workspace(kind, device index, stream, buffer): the buffer that calls on this device and stream use from now on
 PyObject* py_set_workspace(PyObject*, PyObject* args) {
   int kind, device;
@@ -262,7 +376,13 @@ PyObject* py_bind(PyObject*, PyObject* table) {
   g_lib.linear_fused = reinterpret_cast<decltype(g_lib.linear_fused)>(at_name("htr_linear_fused"));
   g_lib.linear_gemm_padded = reinterpret_cast<decltype(g_lib.linear_gemm_padded)>(at_name("htr_linear_gemm_padded"));
   g_lib.route_rows = reinterpret_cast<decltype(g_lib.route_rows)>(at_name("htr_linear_route_rows"));
-  if (!g_lib.linear_gemm_padded || !g_lib.route_rows || !g_lib.linear_ex || !g_lib.linear_gemm || !g_lib.linear_padded || !g_lib.linear_fused) {
+  g_lib.linear_routed = reinterpret_cast<decltype(g_lib.linear_routed)>(at_name("htr_linear_routed"));
+  g_lib.linear_routed_gemm = reinterpret_cast<decltype(g_lib.linear_routed_gemm)>(at_name("htr_linear_routed_gemm"));
+  g_lib.route_plan_bytes = reinterpret_cast<decltype(g_lib.route_plan_bytes)>(at_name("htr_route_plan_bytes"));
+  g_lib.route_plan = reinterpret_cast<decltype(g_lib.route_plan)>(at_name("htr_route_plan"));
+  g_lib.moe_weighted_sum = reinterpret_cast<decltype(g_lib.moe_weighted_sum)>(at_name("htr_moe_weighted_sum"));
+  if (!g_lib.linear_routed || !g_lib.linear_routed_gemm || !g_lib.route_plan_bytes || !g_lib.route_plan || !g_lib.moe_weighted_sum ||
+      !g_lib.linear_gemm_padded || !g_lib.route_rows || !g_lib.linear_ex || !g_lib.linear_gemm || !g_lib.linear_padded || !g_lib.linear_fused) {
     PyErr_SetString(PyExc_ImportError, "bind: an entry point of libhtr_b200 is missing");
     return nullptr;
   }
@@ -286,6 +406,10 @@ PyMethodDef g_methods[] = {
     fast<py_linear>("linear"),
     fast<py_linear_padded>("linear_padded"),
     fast<py_linear_fused>("linear_fused"),
+    fast<py_linear_routed>("linear_routed"),
+    fast<py_linear_routed_gemm>("linear_routed_gemm"),
+    fast<py_route_plan>("route_plan"),
+    fast<py_moe_weighted_sum>("moe_weighted_sum"),
     {"set_workspace", py_set_workspace, METH_VARARGS, nullptr},
     {"bind", py_bind, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},

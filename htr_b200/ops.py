@@ -327,6 +327,10 @@ def linear_routed(x, route, tables, mt, nt, K, x_div=1, prologue=PROLOGUE_NONE, 
     x are [gate | up] of 2n bf16 values.  Nothing touches the host: the routing result stays on the device.
     peer_ptrs (a list of device addresses: the [count, m] result matrix of every rank of an NVLink box as mapped into this process,
     this rank's `out` among them) turns the launch into htr_linear_routed_peers: each row this rank computes is stored into all of them."""
+    if peer_ptrs is None and share <= 1:
+        y = _host.linear_routed(x, route, *tables, mt, nt, K, x_div, prologue, out)
+        if y is not None:
+            return y
     count = route.numel()
     dev = x.device
     if route.dtype != torch.int64 or not route.is_cuda or not x.is_contiguous() or x.dim() != 2:
@@ -359,6 +363,9 @@ def linear_routed(x, route, tables, mt, nt, K, x_div=1, prologue=PROLOGUE_NONE, 
 def route_plan(route, tables):
     """The pairs of a mixture-of-experts step sorted by expert (htr_route_plan), for `linear_routed_gemm`; None where the sizes are
     beyond the grouped GEMM."""
+    plan = _host.route_plan(route, *tables)
+    if plan is not None:
+        return plan
     count, rows, dev = route.numel(), int(tables[0].numel()), route.device
     need = _lib.lib.htr_route_plan_bytes(count, rows)
     if need == 0:
@@ -373,6 +380,10 @@ def route_plan(route, tables):
 def linear_routed_gemm(x, plan, count, tables, mt, nt, K, x_div=1, prologue=PROLOGUE_NONE, out=None):
     """`linear_routed` for steps in which pairs share experts: `plan` (from `route_plan`) in place of the route, each expert's weights
     decoded once per 16 of its pairs on the tensor cores.  Returns None where the sizes are beyond the grouped GEMM."""
+    if out is None:
+        y = _host.linear_routed_gemm(x, plan, count, *tables, mt, nt, K, x_div, prologue)
+        if y is not None:
+            return y
     dev, rows = x.device, int(tables[0].numel())
     need = _lib.lib.htr_linear_routed_gemm_workspace_bytes(count, rows, mt * 16, nt * 16, K)
     if need == 0:

@@ -30,8 +30,9 @@ PEER_ORDER = "kernel"
 
 
 # On one GPU the grouped GEMM decodes an expert's weights once for the pairs that share it, the routed GEMV once per pair.  Both
-# decode 4.2 to 4.5e12 weights a second (float32 activations stay on the GEMV, whose sums carry 24 bits), the GEMM's three extra launches and its reductions cost about 20 us: it wins from this many
-# weights saved on (64 experts of 4096 x 1536, top 8: from 4 tokens; 16 experts of 2048 x 1024, top 4: from 8 tokens).
+# decode 4.2 to 4.5e12 weights a second, the GEMM's three extra launches and its reductions cost about 20 us: it wins from this many
+# weights saved on (64 experts of 4096 x 1536, top 8: from 4 tokens; 16 experts of 2048 x 1024, top 4: from 8 tokens).  Float32
+# activations stay on the GEMV, whose sums carry 24 bits.
 GROUPED_GEMM_MIN_SAVED = 90_000_000
 
 
@@ -378,19 +379,20 @@ class ExpertParallelMoE:
                 if dn is not None:
                     return dn
         skip = self.world > 1 and not exchange                          # rows of skipped pairs must read as zero
-        alloc = torch.zeros if skip else torch.empty
+
+        def rows(width):                                                # None: the launch allocates them
+            return torch.zeros(T * k, width, dtype=x.dtype, device=dev) if skip else None
+
         # (with `exchange`, the gate_up rows of pairs owned elsewhere are never read: the down launch skips the same pairs)
         share = self.world if (x.is_cuda and self.plan_for_share) else 1  # one pair in `world` has its expert here
-        gu = ops.linear_routed(x, route, tabs["gate_up"], mt_gu, nt_gu, K, x_div=k, out=alloc(T * k, mt_gu * 16, dtype=x.dtype, device=dev),
-                               share=share)
+        gu = ops.linear_routed(x, route, tabs["gate_up"], mt_gu, nt_gu, K, x_div=k, out=rows(mt_gu * 16), share=share)
         if x.dtype == torch.bfloat16:
             act, prologue = gu, ops.PROLOGUE_SWIGLU
         else:
             inter = mt_gu * 8
             act, prologue = (torch.nn.functional.silu(gu[:, :inter]) * gu[:, inter:]).contiguous(), ops.PROLOGUE_NONE
         if not exchange:
-            return ops.linear_routed(act, route, tabs["down"], mt_dn, nt_dn, K, prologue=prologue, out=alloc(T * k, mt_dn * 16, dtype=x.dtype, device=dev),
-                                     share=share)
+            return ops.linear_routed(act, route, tabs["down"], mt_dn, nt_dn, K, prologue=prologue, out=rows(mt_dn * 16), share=share)
         ex = self._row_exchange(T * k, mt_dn * 16, x.dtype, dev)
         half = ex["flip"]
         ex["flip"] ^= 1
@@ -407,6 +409,10 @@ class ExpertParallelMoE:
         """y[t] = sum_j w[t, j] * dn[t * k + j] (htr_moe_weighted_sum: float32 sums in slot order, one rounding)."""
         from . import _lib
 
+        if topk_w.shape == (T, k):
+            out = _lib.host.moe_weighted_sum(dn, topk_w)                # the usual case; None: whatever it does not take
+            if out is not None:
+                return out
         dev = dn.device
         gates = topk_w.to(device=dev, dtype=torch.float32).contiguous()
         out = torch.empty(T, dn.shape[1], dtype=dn.dtype, device=dev)

@@ -35,3 +35,23 @@ def test_front_equals_general_path(M, dtype, monkeypatch):
         monkeypatch.setattr(ops._host, name, lambda *a: None)
     assert torch.equal(ops.linear(x, *w, bias), got[0])
     assert torch.equal(ops.linear_padded(x[:, :200].contiguous(), *w, bias[:136].contiguous(), m_out=136), padded)
+
+
+@pytest.mark.parametrize("T,hidden,inter", ((1, 256, 128), (16, 2048, 1024)))    # the routed GEMV; pairs that share experts on the grouped GEMM
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float32))
+def test_moe_fronts_equal_general_path(T, hidden, inter, dtype, monkeypatch):
+    from htr_b200 import ops, sharded, wire
+
+    dev, E, k = torch.device("cuda:0"), 8, 4
+    experts = [dict(gate_up=wire.random_packed(2 * inter, hidden, 3, seed=e, device=dev), down=wire.random_packed(hidden, inter, 3, seed=50 + e, device=dev))
+               for e in range(E)]
+    layer = sharded.ExpertParallelMoE(experts, device=dev)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, hidden, generator=g).to(dtype).to(dev)
+    score, ids = torch.randn(T, E, generator=g).to(dev).topk(k, dim=-1)
+    gates = score.softmax(-1)
+    layer(x, ids, gates)                                                 # the workspaces exist from here on
+    got = layer(x, ids, gates)
+    for name in ("linear_routed", "linear_routed_gemm", "route_plan", "moe_weighted_sum"):
+        monkeypatch.setattr(ops._host, name, lambda *a: None)
+    assert torch.equal(layer(x, ids, gates), got)
