@@ -41,6 +41,9 @@ struct Entry {
   decltype(&htr_route_plan_bytes) route_plan_bytes;
   decltype(&htr_route_plan) route_plan;
   decltype(&htr_moe_weighted_sum) moe_weighted_sum;
+  decltype(&htr_dec_rope_cache) rope_cache;
+  decltype(&htr_dec_attention) attention;
+  decltype(&htr_dec_rope_attention) rope_attention;
 } g_lib = {};
 
 // ---- workspaces: buffers that ops.py owns (one per device, stream and kind); this table only remembers where they are
@@ -344,6 +347,103 @@ PyObject* py_moe_weighted_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(y));
 }
 
+// ---- a decode-sized step of the decoder (the loop of PackedDecoder.forward_folded): five or six launches a layer, 85 us
+// of host work in Python, more than the GPU needs for layers of small models; 24 here (two layers of hidden 1024, a token: 210 -> 95 us).
+// Unlike the fronts above it may return None after part of the step is enqueued: the caller then starts again from the embeddings
+// (cache rows are written again with the same values).
+
+bool wire_of(PyObject* o, const at::Device& dev, Weight* w) {   // the tuple of four wire tensors
+  PyObject* item[4];
+  if (!o || !PyTuple_CheckExact(o) || PyTuple_GET_SIZE(o) != 4) return false;
+  for (int i = 0; i < 4; ++i) item[i] = PyTuple_GET_ITEM(o, i);
+  return weight(item, dev, w);
+}
+
+// decoder_folded(x, layers, head, ln_f, k_cache, v_cache, pos, cos, sin, status, q_heads, kv_heads, eps): logits; x is overwritten
+PyObject* py_decoder_folded(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 13) return none();
+  static PyObject *const kQkv = PyUnicode_InternFromString("qkv"), *const kO = PyUnicode_InternFromString("o"),
+                  *const kUp = PyUnicode_InternFromString("gate_up"), *const kDown = PyUnicode_InternFromString("down"),
+                  *const kLn1 = PyUnicode_InternFromString("ln1"), *const kLn2 = PyUnicode_InternFromString("ln2");
+  const at::Tensor *x = tensor(a[0]), *kc = tensor(a[4]), *vc = tensor(a[5]), *pos = tensor(a[6]), *cosv = tensor(a[7]), *sinv = tensor(a[8]), *status = tensor(a[9]);
+  if (!x || !kc || !vc || !pos || !cosv || !sinv || !status || !PyList_CheckExact(a[1]) || !x->is_cuda() || x->dim() != 2) return none();
+  const at::Device where = x->device();
+  const long hq = PyLong_AsLong(a[10]), hkv = PyLong_AsLong(a[11]);
+  const double eps = PyFloat_AsDouble(a[12]);
+  if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
+  constexpr int64_t D = 128;
+  const int64_t T = x->size(0), hidden = x->size(1);
+  const Py_ssize_t count = PyList_GET_SIZE(a[1]);
+  if (!plain(*x, where, at::kBFloat16) || T < 1 || T > HTR_GEMV_MAX_ROWS || hq < 1 || hkv < 1 || hq > 4096 || hkv > hq) return none();
+  if (!plain(*kc, where, at::kBFloat16) || !plain(*vc, where, at::kBFloat16) || kc->dim() != 4 || kc->sizes() != vc->sizes() || kc->size(0) < count ||
+      kc->size(2) != hkv || kc->size(3) != D)
+    return none();
+  const int64_t cap = kc->size(1), layer_bytes = cap * hkv * D * 2;
+  if (!vector_of(pos, where, at::kLong) || pos->numel() != T || !plain(*cosv, where, at::kFloat) || !plain(*sinv, where, at::kFloat) ||
+      cosv->numel() < cap * D / 2 || sinv->numel() < cap * D / 2 || !plain(*status, where, at::kInt) || status->numel() < 1)
+    return none();
+
+  struct Layer { Weight qkv, o, up, down; const void *ln1, *ln2; };
+  std::vector<Layer> layers;
+  layers.reserve((size_t)count);
+  const auto norm_of = [&](PyObject* o, const void** out) {
+    const at::Tensor* g = o ? tensor(o) : nullptr;
+    if (!g || !plain(*g, where, at::kBFloat16) || g->numel() != hidden) return false;
+    *out = g->const_data_ptr();
+    return true;
+  };
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    PyObject* d = PyList_GET_ITEM(a[1], i);
+    Layer l;
+    if (!PyDict_CheckExact(d) || !wire_of(PyDict_GetItem(d, kQkv), where, &l.qkv) || !wire_of(PyDict_GetItem(d, kO), where, &l.o) ||
+        !wire_of(PyDict_GetItem(d, kUp), where, &l.up) || !wire_of(PyDict_GetItem(d, kDown), where, &l.down) || !norm_of(PyDict_GetItem(d, kLn1), &l.ln1) ||
+        !norm_of(PyDict_GetItem(d, kLn2), &l.ln2))
+      return none();
+    if (l.qkv.nt * 16 != hidden || l.qkv.mt * 16 != (hq + 2 * hkv) * D || l.o.nt * 16 != hq * D || l.o.mt * 16 != hidden || l.up.nt * 16 != hidden ||
+        l.up.mt != 2 * l.down.nt || l.down.mt * 16 != hidden)
+      return none();
+    if (!layers.empty() && l.up.mt != layers[0].up.mt) return none();
+    layers.push_back(l);
+  }
+  Weight head;
+  const void* ln_f;
+  if (!wire_of(a[2], where, &head) || head.nt * 16 != hidden || !norm_of(a[3], &ln_f)) return none();
+
+  const int dev = x->get_device(), rows = (int)T;
+  OnDevice on(dev);
+  void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const at::Tensor* ws = find_workspace(kGemv, dev, st);
+  if (!ws) return none();
+  const auto empty = [&](int64_t columns) { return at::detail::empty_cuda({T, columns}, at::kBFloat16, where, std::nullopt); };
+  const at::Tensor qkv = empty((hq + 2 * hkv) * D), att = empty(hq * D), q = T > 1 ? empty(hq * D) : at::Tensor();
+  const at::Tensor gu = empty(count ? (int64_t)layers[0].up.mt * 16 : 0);
+  at::Tensor y = empty((int64_t)head.mt * 16);
+  const auto fused = [&](const void* in, const Weight& w, void* out, int prologue, const void* norm, int residual) {
+    return g_lib.linear_fused(in, rows, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, out, ws->data_ptr(), ws->numel(), st, prologue, norm, (float)eps,
+                              residual) == HTR_OK;
+  };
+  const int64_t* at_pos = pos->const_data_ptr<int64_t>();
+  const float *cp = cosv->const_data_ptr<float>(), *sp = sinv->const_data_ptr<float>();
+  int* sw = status->data_ptr<int>();
+  void* xp = x->data_ptr();
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    const Layer& l = layers[i];
+    void *kl = static_cast<char*>(kc->data_ptr()) + i * layer_bytes, *vl = static_cast<char*>(vc->data_ptr()) + i * layer_bytes;
+    if (!fused(xp, l.qkv, qkv.data_ptr(), HTR_PROLOGUE_RMSNORM, l.ln1, 0)) return none();
+    if (T == 1) {                                         // one token: rotary embedding, cache write and attention in one launch
+      if (g_lib.rope_attention(qkv.data_ptr(), at_pos, cp, sp, kl, vl, att.data_ptr(), (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+    } else {
+      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+    }
+    if (!fused(att.data_ptr(), l.o, xp, HTR_PROLOGUE_NONE, nullptr, 1) || !fused(xp, l.up, gu.data_ptr(), HTR_PROLOGUE_RMSNORM, l.ln2, 0) ||
+        !fused(gu.data_ptr(), l.down, xp, HTR_PROLOGUE_SWIGLU, nullptr, 1))
+      return none();
+  }
+  if (!fused(xp, head, y.data_ptr(), HTR_PROLOGUE_RMSNORM, ln_f, 0)) return none();
+  return THPVariable_Wrap(std::move(y));
+}
+
 // set_workspace(kind, device index, stream, buffer): the buffer that calls on this device and stream use from now on
 PyObject* py_set_workspace(PyObject*, PyObject* args) {
   int kind, device;
@@ -381,7 +481,10 @@ PyObject* py_bind(PyObject*, PyObject* table) {
   g_lib.route_plan_bytes = reinterpret_cast<decltype(g_lib.route_plan_bytes)>(at_name("htr_route_plan_bytes"));
   g_lib.route_plan = reinterpret_cast<decltype(g_lib.route_plan)>(at_name("htr_route_plan"));
   g_lib.moe_weighted_sum = reinterpret_cast<decltype(g_lib.moe_weighted_sum)>(at_name("htr_moe_weighted_sum"));
-  if (!g_lib.linear_routed || !g_lib.linear_routed_gemm || !g_lib.route_plan_bytes || !g_lib.route_plan || !g_lib.moe_weighted_sum ||
+  g_lib.rope_cache = reinterpret_cast<decltype(g_lib.rope_cache)>(at_name("htr_dec_rope_cache"));
+  g_lib.attention = reinterpret_cast<decltype(g_lib.attention)>(at_name("htr_dec_attention"));
+  g_lib.rope_attention = reinterpret_cast<decltype(g_lib.rope_attention)>(at_name("htr_dec_rope_attention"));
+  if (!g_lib.rope_cache || !g_lib.attention || !g_lib.rope_attention || !g_lib.linear_routed || !g_lib.linear_routed_gemm || !g_lib.route_plan_bytes || !g_lib.route_plan || !g_lib.moe_weighted_sum ||
       !g_lib.linear_gemm_padded || !g_lib.route_rows || !g_lib.linear_ex || !g_lib.linear_gemm || !g_lib.linear_padded || !g_lib.linear_fused) {
     PyErr_SetString(PyExc_ImportError, "bind: an entry point of libhtr_b200 is missing");
     return nullptr;
@@ -410,6 +513,7 @@ PyMethodDef g_methods[] = {
     fast<py_linear_routed_gemm>("linear_routed_gemm"),
     fast<py_route_plan>("route_plan"),
     fast<py_moe_weighted_sum>("moe_weighted_sum"),
+    fast<py_decoder_folded>("decoder_folded"),
     {"set_workspace", py_set_workspace, METH_VARARGS, nullptr},
     {"bind", py_bind, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},

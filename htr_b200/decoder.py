@@ -240,6 +240,12 @@ class PackedDecoder:
         dev = self.device
         st = torch.cuda.current_stream(dev).cuda_stream
         x = self.embed.index_select(0, ids)                     # residual stream, updated in place by the o and down projections
+        # the loop below as one native call; None: whatever it does not take (the first call on a stream, odd layouts, errors)
+        y = _lib.host.decoder_folded(x, self.layers, self.head, self.ln_f, self.k_cache, self.v_cache, pos, self.cos, self.sin, self.status,
+                                     c.q_heads, c.kv_heads, c.eps)
+        if y is not None:
+            return y
+        x = self.embed.index_select(0, ids)                     # (it may have been changed)
         q = torch.empty(T, c.q_heads, c.head_dim, dtype=self.dtype, device=dev)
         att = torch.empty_like(q)
         kp, vp, layer_bytes = self._cache_rows()

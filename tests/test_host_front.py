@@ -55,3 +55,25 @@ def test_moe_fronts_equal_general_path(T, hidden, inter, dtype, monkeypatch):
     for name in ("linear_routed", "linear_routed_gemm", "route_plan", "moe_weighted_sum"):
         monkeypatch.setattr(ops._host, name, lambda *a: None)
     assert torch.equal(layer(x, ids, gates), got)
+
+
+@pytest.mark.parametrize("T", (1, 2, 8))
+def test_decoder_front_equals_general_path(T, monkeypatch):
+    from htr_b200 import ops
+    from htr_b200.decoder import DecoderConfig, PackedDecoder
+
+    dev = torch.device("cuda:0")
+    dec = PackedDecoder(DecoderConfig(layers=3, hidden=256, q_heads=4, kv_heads=2, intermediate=384, vocab=512, max_len=64), dev, seed=T)
+    ids, pos = torch.arange(T, device=dev), torch.arange(5, 5 + T, device=dev)
+    dec.forward(ids, pos)                                                # the workspace exists from here on
+    took = []
+    front = ops._host.decoder_folded
+    monkeypatch.setattr(ops._host, "decoder_folded", lambda *a: took.append(front(*a)) or took[-1])
+    got, k, v = dec.forward(ids, pos), dec.k_cache.clone(), dec.v_cache.clone()
+    assert took[0] is not None
+    monkeypatch.setattr(ops._host, "decoder_folded", lambda *a: None)
+    assert torch.equal(dec.forward(ids, pos), got) and torch.equal(dec.k_cache, k) and torch.equal(dec.v_cache, v)
+    monkeypatch.setattr(ops._host, "decoder_folded", front)
+    dec.layers[1]["o"] = dec.layers[1]["qkv"]                            # another shape: refused as the general path refuses it
+    with pytest.raises(Exception):
+        dec.forward(ids, pos)
