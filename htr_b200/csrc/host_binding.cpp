@@ -44,6 +44,8 @@ struct Entry {
   decltype(&htr_dec_rope_cache) rope_cache;
   decltype(&htr_dec_attention) attention;
   decltype(&htr_dec_rope_attention) rope_attention;
+  decltype(&htr_dec_add_rmsnorm) add_rmsnorm;
+  decltype(&htr_dec_swiglu) swiglu;
 } g_lib = {};
 
 // ---- workspaces: buffers that ops.py owns (one per device, stream and kind); this table only remembers where they are
@@ -347,7 +349,7 @@ PyObject* py_moe_weighted_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(y));
 }
 
-// ---- a decode-sized step of the decoder (the loop of PackedDecoder.forward_folded): five or six launches a layer, 85 us
+// ---- a step of the decoder (the loops of PackedDecoder.forward_folded and forward_fused): a decode-sized one is five or six launches a layer, 85 us
 // of host work in Python, more than the GPU needs for layers of small models; 24 here (two layers of hidden 1024, a token: 210 -> 95 us).
 // Unlike the fronts above it may return None after part of the step is enqueued: the caller then starts again from the embeddings
 // (cache rows are written again with the same values).
@@ -359,9 +361,10 @@ bool wire_of(PyObject* o, const at::Device& dev, Weight* w) {   // the tuple of 
   return weight(item, dev, w);
 }
 
-// decoder_folded(x, layers, head, ln_f, k_cache, v_cache, pos, cos, sin, status, q_heads, kv_heads, eps): logits; x is overwritten
-PyObject* py_decoder_folded(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 13) return none();
+// decoder_step(x, layers, head, ln_f, k_cache, v_cache, pos, cos, sin, status, q_heads, kv_heads, eps, gemm_rows): logits; x is overwritten.
+// gemm_rows 0: the glue folded into the GEMVs (up to 8 rows); else separate glue kernels between tensor-core GEMMs, up to that many rows
+PyObject* py_decoder_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 14) return none();
   static PyObject *const kQkv = PyUnicode_InternFromString("qkv"), *const kO = PyUnicode_InternFromString("o"),
                   *const kUp = PyUnicode_InternFromString("gate_up"), *const kDown = PyUnicode_InternFromString("down"),
                   *const kLn1 = PyUnicode_InternFromString("ln1"), *const kLn2 = PyUnicode_InternFromString("ln2");
@@ -370,11 +373,13 @@ PyObject* py_decoder_folded(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Device where = x->device();
   const long hq = PyLong_AsLong(a[10]), hkv = PyLong_AsLong(a[11]);
   const double eps = PyFloat_AsDouble(a[12]);
+  const long gemm_rows = PyLong_AsLong(a[13]);
   if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
+  const bool folded = gemm_rows == 0;
   constexpr int64_t D = 128;
   const int64_t T = x->size(0), hidden = x->size(1);
   const Py_ssize_t count = PyList_GET_SIZE(a[1]);
-  if (!plain(*x, where, at::kBFloat16) || T < 1 || T > HTR_GEMV_MAX_ROWS || hq < 1 || hkv < 1 || hq > 4096 || hkv > hq) return none();
+  if (!plain(*x, where, at::kBFloat16) || T < 1 || T > (folded ? HTR_GEMV_MAX_ROWS : gemm_rows) || hq < 1 || hkv < 1 || hq > 4096 || hkv > hq) return none();
   if (!plain(*kc, where, at::kBFloat16) || !plain(*vc, where, at::kBFloat16) || kc->dim() != 4 || kc->sizes() != vc->sizes() || kc->size(0) < count ||
       kc->size(2) != hkv || kc->size(3) != D)
     return none();
@@ -412,10 +417,10 @@ PyObject* py_decoder_folded(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int dev = x->get_device(), rows = (int)T;
   OnDevice on(dev);
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
-  const at::Tensor* ws = find_workspace(kGemv, dev, st);
+  const at::Tensor* ws = find_workspace(folded ? kGemv : kGemm, dev, st);
   if (!ws) return none();
   const auto empty = [&](int64_t columns) { return at::detail::empty_cuda({T, columns}, at::kBFloat16, where, std::nullopt); };
-  const at::Tensor qkv = empty((hq + 2 * hkv) * D), att = empty(hq * D), q = T > 1 ? empty(hq * D) : at::Tensor();
+  const at::Tensor qkv = empty((hq + 2 * hkv) * D), att = empty(hq * D), q = T > 1 || !folded ? empty(hq * D) : at::Tensor();
   const at::Tensor gu = empty(count ? (int64_t)layers[0].up.mt * 16 : 0);
   at::Tensor y = empty((int64_t)head.mt * 16);
   const auto fused = [&](const void* in, const Weight& w, void* out, int prologue, const void* norm, int residual) {
@@ -426,6 +431,32 @@ PyObject* py_decoder_folded(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const float *cp = cosv->const_data_ptr<float>(), *sp = sinv->const_data_ptr<float>();
   int* sw = status->data_ptr<int>();
   void* xp = x->data_ptr();
+  if (!folded) {
+    const int inter = count ? layers[0].down.nt * 16 : 0;
+    const at::Tensor h = empty(hidden), delta = empty(hidden), act = empty(inter);
+    const auto gemm = [&](const at::Tensor& in, const Weight& w, const at::Tensor& out) {
+      for (int r = 0; r < rows; r += HTR_GEMM_MAX_ROWS)
+        if (g_lib.linear_gemm(static_cast<const char*>(in.const_data_ptr()) + (int64_t)r * w.nt * 32, HTR_DTYPE_BF16, std::min(rows - r, (int)HTR_GEMM_MAX_ROWS), w.qw,
+                              w.mt, w.nt, w.K, w.sc, w.su, w.sv, nullptr, static_cast<char*>(out.data_ptr()) + (int64_t)r * w.mt * 32, ws->data_ptr(),
+                              ws->numel(), st) != HTR_OK)
+          return false;
+      return true;
+    };
+    const auto norm = [&](const void* add, const void* gain) {
+      return g_lib.add_rmsnorm(xp, add, gain, h.data_ptr(), rows, (int)hidden, (float)eps, st) == HTR_OK;
+    };
+    for (Py_ssize_t i = 0; i < count; ++i) {
+      const Layer& l = layers[i];
+      void *kl = static_cast<char*>(kc->data_ptr()) + i * layer_bytes, *vl = static_cast<char*>(vc->data_ptr()) + i * layer_bytes;
+      if (!norm(i ? delta.data_ptr() : nullptr, l.ln1) || !gemm(h, l.qkv, qkv)) return none();
+      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (!gemm(att, l.o, delta) || !norm(delta.data_ptr(), l.ln2) || !gemm(h, l.up, gu)) return none();
+      if (g_lib.swiglu(gu.data_ptr(), act.data_ptr(), rows, inter, st) != HTR_OK || !gemm(act, l.down, delta)) return none();
+    }
+    if (!norm(count ? delta.data_ptr() : nullptr, ln_f) || !gemm(h, head, y)) return none();
+    return THPVariable_Wrap(std::move(y));
+  }
   for (Py_ssize_t i = 0; i < count; ++i) {
     const Layer& l = layers[i];
     void *kl = static_cast<char*>(kc->data_ptr()) + i * layer_bytes, *vl = static_cast<char*>(vc->data_ptr()) + i * layer_bytes;
@@ -484,7 +515,9 @@ PyObject* py_bind(PyObject*, PyObject* table) {
   g_lib.rope_cache = reinterpret_cast<decltype(g_lib.rope_cache)>(at_name("htr_dec_rope_cache"));
   g_lib.attention = reinterpret_cast<decltype(g_lib.attention)>(at_name("htr_dec_attention"));
   g_lib.rope_attention = reinterpret_cast<decltype(g_lib.rope_attention)>(at_name("htr_dec_rope_attention"));
-  if (!g_lib.rope_cache || !g_lib.attention || !g_lib.rope_attention || !g_lib.linear_routed || !g_lib.linear_routed_gemm || !g_lib.route_plan_bytes || !g_lib.route_plan || !g_lib.moe_weighted_sum ||
+  g_lib.add_rmsnorm = reinterpret_cast<decltype(g_lib.add_rmsnorm)>(at_name("htr_dec_add_rmsnorm"));
+  g_lib.swiglu = reinterpret_cast<decltype(g_lib.swiglu)>(at_name("htr_dec_swiglu"));
+  if (!g_lib.add_rmsnorm || !g_lib.swiglu || !g_lib.rope_cache || !g_lib.attention || !g_lib.rope_attention || !g_lib.linear_routed || !g_lib.linear_routed_gemm || !g_lib.route_plan_bytes || !g_lib.route_plan || !g_lib.moe_weighted_sum ||
       !g_lib.linear_gemm_padded || !g_lib.route_rows || !g_lib.linear_ex || !g_lib.linear_gemm || !g_lib.linear_padded || !g_lib.linear_fused) {
     PyErr_SetString(PyExc_ImportError, "bind: an entry point of libhtr_b200 is missing");
     return nullptr;
@@ -513,7 +546,7 @@ PyMethodDef g_methods[] = {
     fast<py_linear_routed_gemm>("linear_routed_gemm"),
     fast<py_route_plan>("route_plan"),
     fast<py_moe_weighted_sum>("moe_weighted_sum"),
-    fast<py_decoder_folded>("decoder_folded"),
+    fast<py_decoder_step>("decoder_step"),
     {"set_workspace", py_set_workspace, METH_VARARGS, nullptr},
     {"bind", py_bind, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},

@@ -204,6 +204,12 @@ class PackedDecoder:
         dev = self.device
         st = torch.cuda.current_stream(dev).cuda_stream
         x = self.embed.index_select(0, ids)                     # residual stream, updated in place
+        if T > ops.GEMV_MAX_M and ops.USE_GEMM:                 # the loop below as one native call, as in forward_folded
+            y = _lib.host.decoder_step(x, self.layers, self.head, self.ln_f, self.k_cache, self.v_cache, pos, self.cos, self.sin, self.status,
+                                       c.q_heads, c.kv_heads, c.eps, ops.GEMM_ROUTE_MAX)
+            if y is not None:
+                return y
+            x = self.embed.index_select(0, ids)                 # (it may have been changed)
         h = torch.empty_like(x)
         q = torch.empty(T, c.q_heads, c.head_dim, dtype=self.dtype, device=dev)
         att = torch.empty_like(q)
@@ -241,8 +247,8 @@ class PackedDecoder:
         st = torch.cuda.current_stream(dev).cuda_stream
         x = self.embed.index_select(0, ids)                     # residual stream, updated in place by the o and down projections
         # the loop below as one native call; None: whatever it does not take (the first call on a stream, odd layouts, errors)
-        y = _lib.host.decoder_folded(x, self.layers, self.head, self.ln_f, self.k_cache, self.v_cache, pos, self.cos, self.sin, self.status,
-                                     c.q_heads, c.kv_heads, c.eps)
+        y = _lib.host.decoder_step(x, self.layers, self.head, self.ln_f, self.k_cache, self.v_cache, pos, self.cos, self.sin, self.status,
+                                   c.q_heads, c.kv_heads, c.eps, 0)
         if y is not None:
             return y
         x = self.embed.index_select(0, ids)                     # (it may have been changed)

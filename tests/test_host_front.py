@@ -57,7 +57,7 @@ def test_moe_fronts_equal_general_path(T, hidden, inter, dtype, monkeypatch):
     assert torch.equal(layer(x, ids, gates), got)
 
 
-@pytest.mark.parametrize("T", (1, 2, 8))
+@pytest.mark.parametrize("T", (1, 2, 8, 9, 33))
 def test_decoder_front_equals_general_path(T, monkeypatch):
     from htr_b200 import ops
     from htr_b200.decoder import DecoderConfig, PackedDecoder
@@ -67,13 +67,13 @@ def test_decoder_front_equals_general_path(T, monkeypatch):
     ids, pos = torch.arange(T, device=dev), torch.arange(5, 5 + T, device=dev)
     dec.forward(ids, pos)                                                # the workspace exists from here on
     took = []
-    front = ops._host.decoder_folded
-    monkeypatch.setattr(ops._host, "decoder_folded", lambda *a: took.append(front(*a)) or took[-1])
+    front = ops._host.decoder_step
+    monkeypatch.setattr(ops._host, "decoder_step", lambda *a: took.append(front(*a)) or took[-1])
     got, k, v = dec.forward(ids, pos), dec.k_cache.clone(), dec.v_cache.clone()
     assert took[0] is not None
-    monkeypatch.setattr(ops._host, "decoder_folded", lambda *a: None)
+    monkeypatch.setattr(ops._host, "decoder_step", lambda *a: None)
     assert torch.equal(dec.forward(ids, pos), got) and torch.equal(dec.k_cache, k) and torch.equal(dec.v_cache, v)
-    monkeypatch.setattr(ops._host, "decoder_folded", front)
+    monkeypatch.setattr(ops._host, "decoder_step", front)
     dec.layers[1]["o"] = dec.layers[1]["qkv"]                            # another shape: refused as the general path refuses it
     with pytest.raises(Exception):
         dec.forward(ids, pos)
