@@ -318,7 +318,7 @@ def batch_sweep_record(torch, dev, weights_by_k, reps):
     resident copies of the main workload (more than L2 per width), stream-ordered launches through ops.linear, one CUDA graph."""
     from htr_b200 import ops
 
-    out = {"shape_m_x_n": [4096, 12288], "launch_form": "stream-ordered", "kernels": {"1": "packed_gemv_kernel<K,1>", "4": "packed_gemv_mma_kernel<K,8>",
+    out = {"shape_m_x_n": [4096, 12288], "launch_form": "stream-ordered", "kernels": {"1": "packed_gemv1_kernel<K>", "4": "packed_gemm_tc_kernel<K>",
                                                                                       "8": "packed_gemm_tc_kernel<K>", "16": "packed_gemm_tc_kernel<K>", "64": "packed_gemm_tc_kernel<K>"}}
     for K, ws in weights_by_k.items():
         n = ws[0][0].shape[1] * 16

@@ -262,7 +262,9 @@ struct GemvStages {
 template <int K, int MT>
 constexpr int gemv_smem_bytes() { return MT * kStageCols * 4 + GemvStages<K>::value * kGemvWarps * 8 * (32 * K); }
 
-template <int K, int MT>
+// DEP: the one-row form of a launch that depends on the one before it (not for independent inputs and grouped launches, which gain
+// nothing from its early loads and lose 1.4 % by their registers)
+template <int K, int MT, bool DEP>
 __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1)) packed_gemv_kernel(const GemvParams p) {
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   float* smem = reinterpret_cast<float*>(dyn_smem);                               // [MT][kStageCols], later reductions
@@ -349,8 +351,8 @@ __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1))
   unsigned sign_first = 0u;
   uint2 gain_first = make_uint2(0u, 0u);
   const int hb_first = (cgi >> 1) + warp;
-  const bool early = MT == 1 && p.group == 0 && hb_first < (min(CG, cgi + u_end - u_begin) + 1) >> 1;
-  if constexpr (MT == 1) {
+  const bool early = DEP && hb_first < (min(CG, cgi + u_end - u_begin) + 1) >> 1;
+  if constexpr (DEP) {
     if (early) {
       asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(sign_first) : "l"(p.su + hb_first * 16 + (lane >> 1)));   // (nothing waits for it here)
       if (p.prologue == 1) gain_first = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(p.norm_w) + hb_first * 128 + 4 * lane));
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1))
       for (int sgi = 1; sgi < kDepth; ++sgi) issue(sgi * kStageBytes);
       ring_primed = true;
     }
-    if constexpr (MT == 1) {
+    if constexpr (DEP) {
       if (early) x_first = load_quad(x_ptr, hb_first * 128 + 4 * lane, p.dtype);
     }
     __shared__ float s_ss[kGemvWarps];
@@ -419,7 +421,7 @@ __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1))
     const int nblk = hb1 - hb0, items = MT * nblk;
     float4 xv_first = make_float4(0.f, 0.f, 0.f, 0.f);
     const int first_r = MT == 1 ? 0 : warp / nblk;                  // (one activation row: no divisions in the staging)
-    const bool staged_early = MT == 1 && early && u == u_begin;
+    const bool staged_early = DEP && early && u == u_begin;
     if (staged_early && p.prologue == 1) xv_first = norm_x(x_first, gain_first, s_row_inv[0]);
     else if (warp < items && first_r < p.rows)                      // the first item's loads go out before the copy burst
       xv_first = fused_x(p, x_ptr, first_r, (hb0 + warp - first_r * nblk) * 128 + 4 * lane, p.prologue == 1 ? s_row_inv[first_r] : 1.f);
@@ -503,13 +505,13 @@ __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1))
     uint2 sc_raw = make_uint2(0u, 0u);
     float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), old_first = bias4;
     unsigned sv_bits = 0;
-    const bool old_read = MT == 1 && predecessor_done;
+    const bool old_read = DEP && predecessor_done;
     if (warp < p.rows) {
       sc_raw = __ldg(reinterpret_cast<const uint2*>(scales_ptr + row0));
       sv_bits = sign_nibble(sv_ptr, (rb - rb_base) * 32 + lane);
       if (p.bias && row0 < p.m_out) bias4 = load_quad(p.bias, row0, p.dtype);
     }
-    if constexpr (MT == 1) {                           // (the residual row too: only its finisher writes it, and the wait above is behind)
+    if constexpr (DEP) {                               // (the residual row too: only its finisher writes it, and the wait above is behind)
       if (p.residual && warp == 0 && predecessor_done) old_first = load_quad(y_ptr, row0, p.dtype);
     }
     if (!predecessor_done) {                           // deferred wait of the independent-input form
