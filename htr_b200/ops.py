@@ -6,7 +6,8 @@ for one B200 (148 SMs, HBM3e) rather than copied from the 40-CU part the referen
 
   M == 0            empty result                                             (htr/ops.py:73-74)
   1 <= M <= 4       one launch of the streaming GEMV (activation transform, decode + dot, split reduce,
-                    output transform fused)                                  (replaces htr/ops.py:75-76,95-101)
+                    output transform fused)                                  (replaces htr/ops.py:75-76,95-101);
+                    2 to 4 16-bit rows of linears of at least 2^22 weights take the GEMM below (htr_linear_route_rows)
   4 < M <= 512      the tensor-core packed GEMM (tcgen05 + TMEM), up to 256 rows per launch (128 for float32
                     activations); decoded tiles go straight into the MMA operand    (replaces htr/ops.py:77-93).
                     The GEMV handles up to 8 rows and HTR_GEMV_ROUTE_MAX=8 keeps them there; measured, the GEMM wins from 5.
@@ -50,7 +51,6 @@ def _padded_gemv_rows(dtype):
     if dtype == torch.float32 or not USE_GEMM:
         return 1 << 30
     return GEMV_ROUTE_MAX if GEMV_ROUTE_MAX < GEMV_MAX_M else 2 * GEMV_MAX_M
-
 
 
 class _ThreadState(threading.local):
