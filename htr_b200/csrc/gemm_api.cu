@@ -14,6 +14,18 @@ namespace htr {
 // range of the whole row itself (every CTA of a row reads the row once, 16 bytes per load and all of them in flight; that is
 // cheaper than a second launch or a grid-wide exchange).  xsum[row][slice] holds the slice's sum, added up in slice order by the
 // GEMM's epilogue.  Rows beyond `rows` are written as zeros so that the padded batch is harmless; columns from n_in on read as zeros.
+//
+// Range scale of a row: the power of two 2^k with max|x| * sqrt(128) in (2^13, 2^14] * 2^k, in both directions, so that neither a large
+// row leaves the fp16 range nor a small one sinks into its subnormals (fp16 numbers are 2^-24 apart below 2^-14: unscaled, a row of
+// rms 1e-5 kept 9 bits).  |H128 x| / sqrt(128) <= sqrt(128) * max|x|.  k stays in [-120, 118], so that the scale, its reciprocal and
+// their products with 1/sqrt(128) are normal float32 numbers; two planes carry 4e-8 (2-norm) down to rows of rms 1e-36, 3e-7 at 3e-38.
+// The epilogue multiplies by 2^k last, so that the steps before it see ordinary magnitudes.
+__device__ __forceinline__ float range_scale(float mx) {
+  const uint32_t bits = __float_as_uint(mx * (11.32f / 16384.f));
+  const uint32_t e = (bits >> 23) + ((bits & 0x7FFFFFu) != 0u);   // rounded up; inf and NaN end at the upper limit, zero at the lower
+  return __uint_as_float(min(max(e, 127u - 120u), 127u + 118u) << 23);
+}
+
 template <int DT>
 __global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x, int rows, int np, int n, int n_in, int planes, int per,
                                                       const uint8_t* __restrict__ su, __half* __restrict__ xb, float* __restrict__ xsum,
@@ -77,8 +89,7 @@ __global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x
   if constexpr (DT == HTR_DTYPE_F32) mx = __uint_as_float(top);
   else if constexpr (DT == HTR_DTYPE_BF16) mx = __uint_as_float(top << 16);
   else mx = __half2float(__ushort_as_half((unsigned short)top));
-  const float bound = mx * 11.32f;                           // |H128 x| / sqrt(128) <= sqrt(128) * amax
-  const float scale = bound > 16384.f ? exp2f(ceilf(log2f(bound / 16384.f))) : 1.f;
+  const float scale = range_scale(mx);
   if (tid == 0 && slice == 0) tok[r] = scale;
   const float inv = kInvSqrt128 / scale;
   float sum = 0.f;
@@ -228,8 +239,7 @@ __global__ void __launch_bounds__(kGroupRhtWarps * 32) rht_group_kernel(const vo
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < kGroupRhtWarps; ++k) mx = fmaxf(mx, red[k]);
-  const float bound = mx * 11.32f;                           // |H128 x| / sqrt(128) <= sqrt(128) * amax
-  const float scale = bound > 16384.f ? exp2f(ceilf(log2f(bound / 16384.f))) : 1.f;
+  const float scale = range_scale(mx);
   if (tid == 0) tok[slot] = scale;
   const float inv = kInvSqrt128 / scale;
   const int c = (lane & 15) >> 2, j = lane & 3;

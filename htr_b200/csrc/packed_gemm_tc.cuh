@@ -10,7 +10,8 @@
 // conversion instruction); the constant 1534 = 1024 + 510 is removed in the epilogue with the row sums of the activations, as the
 // reference does (htr_kernels.cu:312-313).  B holds the transformed activations as one fp16 plane `hi`, or two, hi and
 // lo = fp16(xt - hi), concatenated along N, so that the products carry ~22 bits of the activations; the two accumulator halves are
-// added after the MMA.  A per-row power-of-two scale keeps |xt| inside the fp16 range (htr_kernels.cu:205-206).
+// added after the MMA.  A per-row power-of-two scale puts |xt| just inside the fp16 range (htr_kernels.cu:205-206; here small rows are
+// scaled up as well).
 //
 // What bounds it: producing A.  A weight costs about four issue slots (window, hash multiply-add, byte sum, half a pack) whatever
 // the batch, so the goal is that the decode warps do nothing else.  Two properties of the layout serve that:
@@ -325,12 +326,12 @@ __device__ __forceinline__ float gemm_xsum_share(const GemmParams& p, int j, int
 __device__ __forceinline__ void gemm_finish_row(const GemmParams& p, const GemmTail& t, int j, int lane, float4 r4, float xs, float tok) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) xs += __shfl_xor_sync(kFullWarp, xs, o);
-  const float off = 1534.0f * xs, rs = p.cb * tok;
-  float v[4] = {(r4.x - off) * (t.s[0] * rs), (r4.y - off) * (t.s[1] * rs), (r4.z - off) * (t.s[2] * rs), (r4.w - off) * (t.s[3] * rs)};
+  const float off = 1534.0f * xs, out = kInvSqrt128 * tok;  // (the range scale last: a row scale times a small tok could underflow)
+  float v[4] = {(r4.x - off) * (t.s[0] * p.cb), (r4.y - off) * (t.s[1] * p.cb), (r4.z - off) * (t.s[2] * p.cb), (r4.w - off) * (t.s[3] * p.cb)};
   wht128(v, lane);
   gemm_store_rows(p, t.pairs ? __ldcg(t.pairs + j) : j, t.row0,
-                  make_float4(flip(v[0] * kInvSqrt128, t.sv_bits & 1u) + t.bias.x, flip(v[1] * kInvSqrt128, (t.sv_bits >> 1) & 1u) + t.bias.y,
-                              flip(v[2] * kInvSqrt128, (t.sv_bits >> 2) & 1u) + t.bias.z, flip(v[3] * kInvSqrt128, t.sv_bits >> 3) + t.bias.w));
+                  make_float4(flip(v[0] * out, t.sv_bits & 1u) + t.bias.x, flip(v[1] * out, (t.sv_bits >> 1) & 1u) + t.bias.y,
+                              flip(v[2] * out, (t.sv_bits >> 2) & 1u) + t.bias.z, flip(v[3] * out, t.sv_bits >> 3) + t.bias.w));
 }
 
 // rows j0, j0 + step, ... of row block rb from the partial sums of thread blocks first .. first + contributors - 1, added in that

@@ -39,3 +39,46 @@ def test_padded_gemm(coracle, dtype, tol, n_in, m_out, n_pad, m_pad, M):
     ref = coracle.linear(torch.nn.functional.pad(x, (0, n_pad - n_in)).float().numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy())[:, :m_out] + bias.float().numpy()
     y = ops.linear_padded(x.to(dev), *[t.to(dev) for t in (qw, sc, su, sv)], bias=bias.to(dev), m_out=m_out)
     assert tuple(y.shape) == (M, m_out) and rel(y.float().cpu().numpy(), ref) <= tol
+
+
+@pytest.mark.parametrize("dtype,M,tol", ((torch.bfloat16, 4, 4e-3), (torch.float16, 3, 4e-3), (torch.bfloat16, 14, 4e-3), (torch.float32, 14, 5e-5)))
+@pytest.mark.parametrize("padded", (False, True))
+def test_rows_of_any_magnitude(coracle, dtype, M, tol, padded):
+    """The activations reach the MMA as fp16 numbers under a scale per row: each row of a call, however small or large, keeps the accuracy of
+    rows near 1 (the tolerances of the tests above), next to rows of other magnitudes and a row of zeros.  float16 stays above its subnormals."""
+    from htr_b200 import ops, wire
+
+    dev = torch.device("cuda:0")
+    m, n = 2048, 2048
+    qw, sc, su, sv = wire.random_packed(m, n, 4, seed=M)
+    x = torch.randn(M, n, generator=torch.Generator().manual_seed(M))
+    x[:, ::97] *= 10.0
+    powers = (0, -3, -4) if dtype == torch.float16 else (0, -8, 30, -3, -5, -6, -12, -20, -30, -36, 8, 2, 33, 0)
+    for r in range(M):
+        x[r] = (x[r].double() * 10.0 ** powers[r]).float()
+    if M > 4:
+        x[M - 1] = 0
+    x = x.to(dtype)
+    d = [t.to(dev) for t in (qw, sc, su, sv)]
+    n_in, m_out = (n - 40, m - 8) if padded else (n, m)
+    x[:, n_in:] = 0
+    ref = coracle.linear(x.float().numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy())[:, :m_out]
+    if padded and dtype == torch.float32:
+        y = torch.empty(M, m_out, device=dev)                     # (ops keeps float32 rows of padded linears on the GEMV)
+        from htr_b200 import _lib
+
+        ws = torch.zeros(_lib.lib.htr_linear_gemm_workspace_bytes(M, m, n, 4), dtype=torch.uint8, device=dev)
+        xs = x[:, :n_in].contiguous().to(dev)
+        rc = _lib.lib.htr_linear_gemm_padded(xs.data_ptr(), _lib.F32, M, n_in, d[0].data_ptr(), m // 16, n // 16, 4, d[1].data_ptr(), d[2].data_ptr(),
+                                             d[3].data_ptr(), None, y.data_ptr(), m_out, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+    else:
+        y = ops.linear_padded(x[:, :n_in].contiguous().to(dev), *d, m_out=m_out) if padded else ops.linear(x.to(dev), *d)
+    y = y.float().cpu().numpy()
+    for r in range(M):
+        if not x[r].any():
+            assert not y[r].any()
+        else:
+            s = float(np.abs(ref[r]).max())                       # (norms of the smallest rows would underflow)
+            assert rel(y[r] / s, ref[r] / s) <= tol, (r, powers[r])
+    assert all(c == 0 for c in ops.gemm_error_codes())

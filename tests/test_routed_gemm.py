@@ -41,3 +41,32 @@ def test_grouped_gemm_equals_routed_gemv(K, m, n, E, T, k):
         assert float((got[~skipped].float() - want[~skipped].float()).norm() / want[~skipped].float().norm()) <= 1e-3
     assert all(c == 0 for c in ops.gemm_error_codes())
     assert ops.route_plan(torch.zeros(5000, dtype=torch.int64, device=dev), tables) is None
+
+
+@pytest.mark.parametrize("dtype,tol", ((torch.float32, 5e-5), (torch.bfloat16, 1e-3)))
+def test_pairs_of_any_magnitude(dtype, tol):
+    """Rows of every magnitude side by side in one tile, plain and behind SwiGLU (whose products are where small rows come from): each row as
+    near to the routed GEMV, which stages float32 values, as ordinary rows are above."""
+    from htr_b200 import ops, wire
+
+    dev, m, n, E = torch.device("cuda:0"), 256, 384, 2
+    experts = [wire.random_packed(m, n, 3, seed=7 + e, device=dev) for e in range(E)]
+    tables = [torch.tensor([experts[e][i].data_ptr() for e in range(E)], dtype=torch.int64, device=dev) for i in range(4)]
+    g = torch.Generator().manual_seed(3)
+    scales = torch.tensor([10.0 ** p for p in (0, -3, -4, -5, -6, -8, -12, -20, -30, 4, 20, 30, -1, 0)], dtype=torch.float64)
+    T = scales.numel()
+    route = (torch.arange(T) % E).to(dev)
+    plan = ops.route_plan(route, tables)
+    x = (torch.randn(T, n, generator=g).double() * scales[:, None]).to(dtype).to(dev)
+
+    def close(got, want):
+        s = want.double().abs().amax(dim=1, keepdim=True)
+        err = ((got.double() - want.double()) / s).norm(dim=1) / (want.double() / s).norm(dim=1)
+        assert float(err.max()) <= tol, err.tolist()
+
+    close(ops.linear_routed_gemm(x, plan, T, tables, m // 16, n // 16, 3), ops.linear_routed(x, route, tables, m // 16, n // 16, 3))
+    if dtype == torch.bfloat16:
+        gu = torch.cat([x * 0 + torch.randn(T, n, generator=g).to(dtype).to(dev), x], dim=1).contiguous()
+        close(ops.linear_routed_gemm(gu, plan, T, tables, m // 16, n // 16, 3, prologue=ops.PROLOGUE_SWIGLU),
+              ops.linear_routed(gu, route, tables, m // 16, n // 16, 3, prologue=ops.PROLOGUE_SWIGLU))
+    assert all(c == 0 for c in ops.gemm_error_codes())
