@@ -285,7 +285,7 @@ __device__ __forceinline__ bool finishers_all(bool mine) {
 
 // ---- finishing of a row block: one warp per activation row, lane holds rows 4 lane .. + 3 of the block
 struct GemmTail {
-  float s[4];                                               // row scales
+  float s[4];                                               // row scales times the codebook's
   unsigned sv_bits;
   float4 bias;
   int row0;                                                 // row of this problem's weight
@@ -311,7 +311,7 @@ struct GemmTail {
     row0 = rb * 128 + 4 * lane;
     const uint2 raw = __ldg(reinterpret_cast<const uint2*>(scales + row0));
     const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-    s[0] = s01.x; s[1] = s01.y; s[2] = s23.x; s[3] = s23.y;
+    s[0] = s01.x * p.cb; s[1] = s01.y * p.cb; s[2] = s23.x * p.cb; s[3] = s23.y * p.cb;
     sv_bits = sign_nibble(sv, rb * 32 + lane);
     bias = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p.bias && row0 < p.m_out) bias = load_quad(p.bias, row0, p.dtype);
@@ -327,7 +327,7 @@ __device__ __forceinline__ void gemm_finish_row(const GemmParams& p, const GemmT
 #pragma unroll
   for (int o = 16; o; o >>= 1) xs += __shfl_xor_sync(kFullWarp, xs, o);
   const float off = 1534.0f * xs, out = kInvSqrt128 * tok;  // (the range scale last: a row scale times a small tok could underflow)
-  float v[4] = {(r4.x - off) * (t.s[0] * p.cb), (r4.y - off) * (t.s[1] * p.cb), (r4.z - off) * (t.s[2] * p.cb), (r4.w - off) * (t.s[3] * p.cb)};
+  float v[4] = {(r4.x - off) * t.s[0], (r4.y - off) * t.s[1], (r4.z - off) * t.s[2], (r4.w - off) * t.s[3]};
   wht128(v, lane);
   gemm_store_rows(p, t.pairs ? __ldcg(t.pairs + j) : j, t.row0,
                   make_float4(flip(v[0] * out, t.sv_bits & 1u) + t.bias.x, flip(v[1] * out, (t.sv_bits >> 1) & 1u) + t.bias.y,

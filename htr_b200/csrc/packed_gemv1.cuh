@@ -16,6 +16,13 @@
 //  * a weight costs half an instruction less: its byte sum, as the bits of a float, is a subnormal number (n * 2^-149 exactly), and
 //    multiplied with activations staged times 2^80 it needs neither a magic constant nor its subtraction.  The constant 510 goes in
 //    per 16 columns, as -510 times their sum added to the accumulator first, so that the sums stay centred (no cancellation at the end).
+// Range.  The products are normal numbers while the largest activation that a thread block stages lies within 2^-36 .. 2^36.  A block of
+// any other drops its sums and runs once more (gemv1_wide) under a power of two made for them; partial sums leave in their own unit, so
+// that blocks with different powers add up, and the range of the results is that of packed_gemv.cuh.  The check (three votes of a staging
+// warp, read by the idle finishers) costs the smallest launches 0.1 us and the others nothing: 1024x1024 3.73 -> 3.84, 1024x4096 4.62 -> 4.72,
+// 12288x4096 13.02 -> 13.02, 4096x12288 12.67 -> 12.67, 151936x4096 106.0 -> 104.9.  Dearer forms, at 1024x4096 / 12288x4096: a vote at the
+// barrier before the decode 4.82 / 13.18, both passes as a loop 5.08 / 13.41, the second pass inlined 4.98 / 13.35, a vote on the sums
+// 4.84 / 13.23.
 // us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.4 -> 4.9, 4096x12288 K4 13.8 -> 12.7, 151936x4096 K4
 // 131 -> 102 (6.1e12 weights a second, 21 per cycle and SM).
 #pragma once
@@ -26,9 +33,18 @@ namespace htr {
 constexpr int kG1DecodeWarps = 16, kG1FinishWarps = 4, kG1Warps = kG1DecodeWarps + kG1FinishWarps, kG1Threads = kG1Warps * 32;
 constexpr int kG1Alu = 2;                                    // byte sums of four that go to the shift/logic pipe (1, 3, 4: 2 to 3 % slower)
 constexpr int kG1MaxCols = 16384;                            // staged activations of a row: 64 KB
-constexpr float kG1Up = 1.2089258196146292e24f;              // 2^80: staged activations
-constexpr float kG1Down = 1.6940658945086007e-21f;           // 2^-69 = 2^80 * 2^-149: unit of the accumulators
-constexpr float kG1Out = 5.902958103587057e20f;              // 2^69
+constexpr int kG1Up = 80;                                    // activations are staged times 2^80 ...
+constexpr float kG1Least = 1.4551915e-11f, kG1Most = 6.871948e10f;   // ... where the largest is in [2^-36, 2^36): transformed within 2^-40 .. 2^40
+__device__ __forceinline__ float power_of_two(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
+
+struct G1Shared {
+  float red[2][kG1DecodeWarps][64];                          // sums of a row block: [buffer][decode warp][its 64 rows]
+  float ytil[128];
+  float ss[kG1Warps];
+  unsigned range[kG1Warps];                                  // of what a warp has staged: 1 = a value of at least kG1Most, 2 = of kG1Least, 4 = not zero
+  unsigned top[kG1Warps];                                    // gemv1_wide: its largest, as bits of a float
+  int arrival;
+};
 
 template <int K>
 struct G1Ring {
@@ -69,15 +85,13 @@ __device__ __forceinline__ void unit_fma_subnormal(const uint32_t (&V)[K + 1], c
   }
 }
 
-template <int K>
-__global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvParams p) {
+// The work of a thread block; true (for all its threads) where the activations are out of the usual range and nothing was delivered.
+// WIDE: the second run, under a power of two made for them.
+template <int K, bool WIDE>
+__device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
   using Ring = G1Ring<K>;
   constexpr int kTileBytes = Ring::tile_bytes, kSlotBytes = Ring::slot_bytes, R = Ring::slots;
   extern __shared__ __align__(128) unsigned char dyn_smem[];
-  __shared__ __align__(16) float s_red[2][kG1DecodeWarps][64];   // sums of a row block: [buffer][decode warp][its 64 rows]
-  __shared__ __align__(16) float ytil[128];
-  __shared__ float s_ss[kG1Warps];
-  __shared__ int s_arrival;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nt = p.nt, n = nt * 16, HB = nt >> 3;
   const EvenRuns runs((p.mt >> 3) * HB, gridDim.x);
@@ -129,6 +143,8 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
+  int shift = kG1Up;
+  auto scaled = [&](float f) { return WIDE ? f * power_of_two(shift >> 1) * power_of_two(shift - (shift >> 1)) : f * power_of_two(kG1Up); };
   auto stage = [&](int hb, unsigned sg, float4 x4) {
     float v[4] = {flip(x4.x, sg & 1u), flip(x4.y, (sg >> 1) & 1u), flip(x4.z, (sg >> 2) & 1u), flip(x4.w, sg >> 3)};
     wht128(v, lane);
@@ -136,13 +152,13 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     float sum = 0.f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float f = v[k] * kInvSqrt128;
-      dst[staged_col<K>(4 * (lane & 3) + k)] = f * kG1Up;
+      const float f = scaled(v[k] * kInvSqrt128);
+      dst[staged_col<K>(4 * (lane & 3) + k)] = f;
       sum += f;
     }
     sum += __shfl_xor_sync(kFullWarp, sum, 1);
     sum += __shfl_xor_sync(kFullWarp, sum, 2);
-    if ((lane & 3) == 0) xoff[hb * 8 + (lane >> 2)] = -510.0f * sum * kG1Down;
+    if ((lane & 3) == 0) xoff[hb * 8 + (lane >> 2)] = sum * __uint_as_float(0x80000000u | 510u);   // -510 * 2^-149, the unit of the byte sums
   };
   float4 held[kHeld];                                        // every load of a warp is in flight before the first is used
   if (p.prologue == 1) {
@@ -154,11 +170,11 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     for (int i = 0; i < kHeld; ++i) ss += held[i].x * held[i].x + held[i].y * held[i].y + held[i].z * held[i].z + held[i].w * held[i].w;
 #pragma unroll
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(kFullWarp, ss, o);
-    if (lane == 0) s_ss[warp] = ss;
+    if (lane == 0) sh.ss[warp] = ss;
     __syncthreads();
     float tot = 0.f;
 #pragma unroll
-    for (int k = 0; k < kG1Warps; ++k) tot += s_ss[k];
+    for (int k = 0; k < kG1Warps; ++k) tot += sh.ss[k];
     const float inv = rsqrtf(tot / (float)n + p.eps);
 #pragma unroll
     for (int i = 0; i < kHeld; ++i) held[i] = norm_x(held[i], gain[i], inv);
@@ -167,10 +183,33 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     for (int i = 0; i < kHeld; ++i)
       if (warp + kG1Warps * i < count) held[i] = load_x(p.x, 0, block_at(i) * 128 + 4 * lane, p.n_in, p.dtype);
   }
+  float top = 0.f;
+  auto range = [&](float4 v) { top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); };
+  if constexpr (WIDE) {
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i)
+      if (warp + kG1Warps * i < count) range(held[i]);
+    const unsigned own = __reduce_max_sync(kFullWarp, __float_as_uint(top));
+    if (lane == 0) sh.top[warp] = own;
+    __syncthreads();
+    // the largest activation to [2^96, 2^97), transformed at most 11.4 times that; -32 to 223
+    shift = 96 + 127 - (int)(__reduce_max_sync(kFullWarp, sh.top[lane < kG1Warps ? lane : 0]) >> 23);
+  }
 #pragma unroll
   for (int i = 0; i < kHeld; ++i)
-    if (warp + kG1Warps * i < count) stage(block_at(i), (signs[i] >> (4 * (lane & 1))) & 15u, held[i]);
+    if (warp + kG1Warps * i < count) {
+      if constexpr (!WIDE) range(held[i]);
+      stage(block_at(i), (signs[i] >> (4 * (lane & 1))) & 15u, held[i]);
+    }
+  if constexpr (!WIDE) {
+    const bool beyond = __any_sync(kFullWarp, top >= kG1Most), usual = __any_sync(kFullWarp, top >= kG1Least), some = __any_sync(kFullWarp, top > 0.f);
+    if (lane == 0) sh.range[warp] = (beyond ? 1u : 0u) | (usual ? 2u : 0u) | (some ? 4u : 0u);
+  }
   __syncthreads();
+  auto again = [&]() {                                       // all warps read the same words and decide alike
+    const unsigned all = __reduce_or_sync(kFullWarp, sh.range[lane < kG1Warps ? lane : 0]);
+    return !WIDE && ((all & 1u) != 0u || (all & 6u) == 4u);
+  };
 
   if (warp < kG1DecodeWarps) {
     float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -199,17 +238,18 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
       // ---- this warp's part of row block rb: leave it for the finishers (two buffers)
       const int buf = seg & 1;
       if (seg >= 2) named_sync_at(3 + buf, kG1Threads);
-      *reinterpret_cast<float2*>(&s_red[buf][warp][g * 16 + 2 * q]) = make_float2(acc[0].x + acc[0].y, acc[1].x + acc[1].y);
+      *reinterpret_cast<float2*>(&sh.red[buf][warp][g * 16 + 2 * q]) = make_float2(acc[0].x + acc[0].y, acc[1].x + acc[1].y);
       acc[0] = acc[1] = make_float2(0.f, 0.f);
       named_arrive_at(1 + buf, kG1Threads);
       start = stop;
     }
     async_wait<0>();
-    return;
+    return again();
   }
 
   // ---- finishers: thread r owns row r of the row block
   const int r = tid - kG1DecodeWarps * 32, segs = (u_end - 1) / HB - u_begin / HB + 1;
+  const bool drop = again();
   for (int seg = 0, start = u_begin; seg < segs; ++seg) {
     const int rb = start / HB, buf = seg & 1;
     const int first = runs.owner(rb * HB), contributors = runs.owner((rb + 1) * HB - 1) - first + 1;
@@ -223,8 +263,10 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     named_sync_at(1 + buf, kG1Threads);
     float sum = 0.f;
 #pragma unroll
-    for (int w = 0; w < kG1DecodeWarps / 2; ++w) sum += s_red[buf][2 * w + (r >> 6)][r & 63];
+    for (int w = 0; w < kG1DecodeWarps / 2; ++w) sum += sh.red[buf][2 * w + (r >> 6)][r & 63];
     if (seg + 2 < segs) named_arrive_at(3 + buf, kG1Threads);
+    if (drop) continue;
+    sum = WIDE ? sum * power_of_two((149 - shift) >> 1) * power_of_two(149 - shift - ((149 - shift) >> 1)) : sum * power_of_two(149 - kG1Up);
     bool finish = true;
     if (contributors > 1) {
       // a thread block has two partials: its first row block's and that of a later one (only its last is read by others)
@@ -232,10 +274,10 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
       named_sync<5, kG1FinishWarps * 32>();
       if (r == 0) {
         __threadfence();                                     // the partials of the thread block (ordered by the barrier) before the arrival
-        s_arrival = atomicAdd(p.counters + rb, 1);           // (they are read with loads served by L2, after this atomic)
+        sh.arrival = atomicAdd(p.counters + rb, 1);           // (they are read with loads served by L2, after this atomic)
       }
       named_sync<5, kG1FinishWarps * 32>();
-      finish = s_arrival == contributors - 1;
+      finish = sh.arrival == contributors - 1;
       if (finish) {
         if (r == 0) p.counters[rb] = 0;
         const int head = runs.begin(first) < rb * HB ? 1 : 0;
@@ -251,11 +293,11 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
       }
     }
     if (!finish) continue;
-    ytil[r] = sum * kG1Out;
+    sh.ytil[r] = sum;
     named_sync<5, kG1FinishWarps * 32>();
     if (r < 32) {
       const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.y));
-      const float4 y4 = *reinterpret_cast<const float4*>(ytil + 4 * lane);
+      const float4 y4 = *reinterpret_cast<const float4*>(sh.ytil + 4 * lane);
       float v[4] = {y4.x * (s01.x * p.cb), y4.y * (s01.y * p.cb), y4.z * (s23.x * p.cb), y4.w * (s23.y * p.cb)};
       wht128(v, lane);
       float4 o = make_float4(flip(v[0] * kInvSqrt128, sv_bits & 1u) + bias4.x, flip(v[1] * kInvSqrt128, (sv_bits >> 1) & 1u) + bias4.y,
@@ -264,6 +306,19 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const GemvP
     }
     // (ytil is written again only behind the next barrier with the decode warps, which warp 0 reaches after this)
   }
+  return drop;
+}
+
+template <int K>
+__device__ __noinline__ void gemv1_wide(const GemvParams& p, G1Shared& sh) {
+  __syncthreads();                                           // the first run's words and sums have been read
+  gemv1_run<K, true>(p, sh);
+}
+
+template <int K>
+__global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __grid_constant__ GemvParams p) {
+  __shared__ __align__(16) G1Shared sh;
+  if (gemv1_run<K, false>(p, sh)) gemv1_wide<K>(p, sh);
 }
 
 // host side, defined once per K in packed_gemv_k*.cu

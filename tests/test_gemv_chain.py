@@ -35,3 +35,33 @@ def test_one_row(coracle, K, m, n):
         xb = torch.randn(1, n, generator=g).to(dt)
         yb = ops.linear(xb.to(dev), *d)
         assert rel(yb.float().cpu().numpy(), coracle.linear(xb.float().numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy())) <= 4e-3
+
+
+@pytest.mark.parametrize("dtype,tol", ((torch.float32, 5e-6), (torch.bfloat16, 4e-3)))
+@pytest.mark.parametrize("m,n", ((128, 16384), (1024, 2048), (2176, 5760)))
+def test_one_row_of_any_magnitude(coracle, m, n, dtype, tol):
+    """Byte sums are multiplied as subnormal numbers with activations under a power-of-two factor, one per thread block: it must follow the
+    range of float32 and bf16, also where thread blocks of one launch choose different ones (columns of different magnitude)."""
+    from htr_b200 import ops, wire
+
+    dev = torch.device("cuda:0")
+    qw, sc, su, sv = wire.random_packed(m, n, 4, seed=m + n)
+    d = [t.to(dev) for t in (qw, sc, su, sv)]
+    g = torch.Generator().manual_seed(n)
+    x = torch.randn(1, n, generator=g)
+    for left, right in ((-36, -36), (-30, -30), (-20, -20), (-13, -11), (11, 13), (16, 16), (25, 25), (33, 33), (30, -30), (-25, 0), (0, 14), (13, 30), (-20, -36)):
+        xs = x.double().clone()
+        xs[:, :n // 2] *= 10.0 ** left
+        xs[:, n // 2:] *= 10.0 ** right
+        xs = xs.float().to(dtype)
+        ref = coracle.linear(xs.float().numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy())
+        y = ops.linear(xs.to(dev), *d)
+        assert bool(torch.isfinite(y).all()) and torch.equal(ops.linear(xs.to(dev), *d), y)
+        s = float(np.abs(ref).max())                                  # (squares of the ends would leave float64's sums of float32)
+        assert rel(y.float().cpu().numpy() / s, ref / s) <= tol, (left, right)
+    zero = ops.linear(torch.zeros(1, n, dtype=dtype, device=dev), *d)
+    assert not bool(zero.any())
+    for bad in (float("inf"), float("nan")):
+        xs = x.clone()
+        xs[0, 17] = bad
+        assert not bool(torch.isfinite(ops.linear(xs.to(dtype).to(dev), *d)).any())
