@@ -128,6 +128,25 @@ struct OnDevice {
 
 PyObject* none() { Py_RETURN_NONE; }
 
+// an argument that is a C int; false for anything else (another type, a value beyond its range), with no Python error left behind
+bool int_of(PyObject* o, int* out) {
+  const long v = PyLong_AsLong(o);
+  if (v == -1 && PyErr_Occurred()) {
+    PyErr_Clear();
+    return false;
+  }
+  *out = (int)v;
+  return *out == v;
+}
+bool float_of(PyObject* o, double* out) {
+  *out = PyFloat_AsDouble(o);
+  if (*out == -1.0 && PyErr_Occurred()) {
+    PyErr_Clear();
+    return false;
+  }
+  return true;
+}
+
 // linear(x, qweight, scales, su, sv, bias, flags, gemv_rows, gemm_rows): up to gemv_rows activation rows as one GEMV, up to
 // gemm_rows on the tensor-core GEMM
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -138,7 +157,8 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!x || !x->is_cuda() || x->dim() < 1 || !x->is_contiguous() || !weight(a + 1, x->device(), &w)) return none();
   const int dt = dtype_code(x->scalar_type());
   const int64_t cols = (int64_t)w.nt * 16, rows64 = cols ? x->numel() / cols : 0;
-  const long flags = PyLong_AsLong(a[6]), gemv_rows = PyLong_AsLong(a[7]), gemm_rows = PyLong_AsLong(a[8]);
+  int flags, gemv_rows, gemm_rows;
+  if (!int_of(a[6], &flags) || !int_of(a[7], &gemv_rows) || !int_of(a[8], &gemm_rows)) return none();
   if (dt < 0 || x->size(-1) != cols || rows64 < 1 || !bias_of(a[5], *x, (int64_t)w.mt * 16, &bias)) return none();
   // (the rule of ops._gemv_rows)
   int64_t most = gemv_rows;
@@ -177,14 +197,16 @@ PyObject* py_linear_padded(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const void* bias;
   if (!x || !x->is_cuda() || x->dim() < 1 || !x->is_contiguous() || !weight(a + 1, x->device(), &w)) return none();
   const int dt = dtype_code(x->scalar_type());
-  const int64_t n_in = x->size(-1), m_out = PyLong_AsLong(a[6]);
+  const int64_t n_in = x->size(-1);
+  int m_out, gemv_rows;
+  if (!int_of(a[6], &m_out) || !int_of(a[7], &gemv_rows)) return none();
   if (dt < 0 || n_in < 1 || n_in > (int64_t)w.nt * 16 || m_out < 1 || m_out > (int64_t)w.mt * 16 || !bias_of(a[5], *x, m_out, &bias)) return none();
   const int64_t rows = x->numel() / n_in, esize = x->element_size();
   if (rows < 1) return none();
   const int dev = x->get_device();
   OnDevice on(dev);
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
-  const bool gemm = rows > PyLong_AsLong(a[7]);
+  const bool gemm = rows > gemv_rows;
   const at::Tensor* ws = find_workspace(gemm ? kGemm : kGemv, dev, st);
   if (!ws) return none();
   at::Tensor y = output(*x, m_out);
@@ -195,7 +217,7 @@ PyObject* py_linear_padded(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int64_t r = 0; r < rows; r += step) {
     const int here = (int)(rows - r < step ? rows - r : step);
     if (launch(xp + r * n_in * esize, dt, here, (int)n_in, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, bias, yp + r * m_out * esize,
-                            (int)m_out, ws->data_ptr(), ws->numel(), st) != HTR_OK)
+               m_out, ws->data_ptr(), ws->numel(), st) != HTR_OK)
       return none();
   }
   return THPVariable_Wrap(std::move(y));
@@ -207,10 +229,12 @@ PyObject* py_linear_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor* x = tensor(a[0]);
   Weight w;
   if (!x || !x->is_cuda() || x->dim() != 2 || x->scalar_type() != at::kBFloat16 || !x->is_contiguous() || !weight(a + 1, x->device(), &w)) return none();
-  const long prologue = PyLong_AsLong(a[6]);
-  const double eps = PyFloat_AsDouble(a[8]);
-  if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
-  const bool residual = PyObject_IsTrue(a[9]) == 1;
+  int prologue;
+  double eps;
+  if (!int_of(a[6], &prologue) || !float_of(a[8], &eps)) return none();
+  const int truth = PyObject_IsTrue(a[9]);
+  if (truth < 0) { PyErr_Clear(); return none(); }
+  const bool residual = truth == 1;
   const int64_t rows = x->size(0), cols = (int64_t)w.nt * 16 * (prologue == HTR_PROLOGUE_SWIGLU ? 2 : 1), m = (int64_t)w.mt * 16;
   if (rows < 1 || rows > HTR_GEMV_MAX_ROWS || x->size(1) != cols) return none();
   const void* norm = nullptr;
@@ -234,7 +258,7 @@ PyObject* py_linear_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
     y = *o;
   }
   if (g_lib.linear_fused(x->const_data_ptr(), (int)rows, w.qw, w.mt, w.nt, w.K, w.sc, w.su, w.sv, y.data_ptr(), ws->data_ptr(), ws->numel(), st,
-                         (int)prologue, norm, (float)eps, residual ? 1 : 0) != HTR_OK)
+                         prologue, norm, (float)eps, residual ? 1 : 0) != HTR_OK)
     return none();
   if (a[5] != Py_None) return Py_NewRef(a[5]);
   return THPVariable_Wrap(std::move(y));
@@ -262,8 +286,8 @@ PyObject* py_linear_routed(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Device where = x->device();
   if (!vector_of(route, where, at::kLong) || !tables_of(a + 2, where, t)) return none();
   const int dt = dtype_code(x->scalar_type());
-  const long mt = PyLong_AsLong(a[6]), nt = PyLong_AsLong(a[7]), K = PyLong_AsLong(a[8]), x_div = PyLong_AsLong(a[9]), prologue = PyLong_AsLong(a[10]);
-  if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
+  int mt, nt, K, x_div, prologue;
+  if (!int_of(a[6], &mt) || !int_of(a[7], &nt) || !int_of(a[8], &K) || !int_of(a[9], &x_div) || !int_of(a[10], &prologue)) return none();
   const int64_t count = route->numel();
   if (dt < 0 || count < 1 || count > (1 << 24) || mt < 1 || mt > (1 << 24) || nt < 1 || nt > (1 << 24) || x_div < 1 || x_div > (1 << 24)) return none();
   const int dev = x->get_device();
@@ -279,10 +303,10 @@ PyObject* py_linear_routed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!o || !plain(*o, where, x->scalar_type()) || o->dim() != 2 || o->size(0) != count || o->size(1) != mt * 16) return none();
     y = *o;
   }
-  if (g_lib.linear_routed(x->const_data_ptr(), dt, (int)x_div, x->size(1), route->const_data_ptr<int64_t>(), (int)count, (int)t[0]->numel(),
+  if (g_lib.linear_routed(x->const_data_ptr(), dt, x_div, x->size(1), route->const_data_ptr<int64_t>(), (int)count, (int)t[0]->numel(),
                           static_cast<const void* const*>(t[0]->const_data_ptr()), static_cast<const void* const*>(t[1]->const_data_ptr()),
-                          static_cast<const uint8_t* const*>(t[2]->const_data_ptr()), static_cast<const uint8_t* const*>(t[3]->const_data_ptr()), (int)mt,
-                          (int)nt, (int)K, y.data_ptr(), (int)prologue, ws->data_ptr(), ws->numel(), st) != HTR_OK)
+                          static_cast<const uint8_t* const*>(t[2]->const_data_ptr()), static_cast<const uint8_t* const*>(t[3]->const_data_ptr()), mt,
+                          nt, K, y.data_ptr(), prologue, ws->data_ptr(), ws->numel(), st) != HTR_OK)
     return none();
   if (a[11] != Py_None) return Py_NewRef(a[11]);
   return THPVariable_Wrap(std::move(y));
@@ -296,21 +320,21 @@ PyObject* py_linear_routed_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Device where = x->device();
   if (!vector_of(plan, where, at::kByte) || !tables_of(a + 3, where, t)) return none();
   const int dt = dtype_code(x->scalar_type());
-  const long count = PyLong_AsLong(a[2]), mt = PyLong_AsLong(a[7]), nt = PyLong_AsLong(a[8]), K = PyLong_AsLong(a[9]), x_div = PyLong_AsLong(a[10]),
-             prologue = PyLong_AsLong(a[11]);
-  if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
+  int count, mt, nt, K, x_div, prologue;
+  if (!int_of(a[2], &count) || !int_of(a[7], &mt) || !int_of(a[8], &nt) || !int_of(a[9], &K) || !int_of(a[10], &x_div) || !int_of(a[11], &prologue))
+    return none();
   if (dt < 0 || count < 1 || count > (1 << 24) || mt < 1 || mt > (1 << 24) || nt < 1 || nt > (1 << 24) || x_div < 1 || x_div > (1 << 24)) return none();
-  if ((size_t)plan->numel() < g_lib.route_plan_bytes((int)count, (int)t[0]->numel())) return none();
+  if ((size_t)plan->numel() < g_lib.route_plan_bytes(count, (int)t[0]->numel())) return none();
   const int dev = x->get_device();
   OnDevice on(dev);
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
   const at::Tensor* ws = find_workspace(kGemm, dev, st);
   if (!ws) return none();
   at::Tensor y = at::detail::empty_cuda({(int64_t)count, (int64_t)mt * 16}, x->scalar_type(), where, std::nullopt);
-  if (g_lib.linear_routed_gemm(x->const_data_ptr(), dt, (int)x_div, x->size(1), plan->const_data_ptr(), (int)count, (int)t[0]->numel(),
+  if (g_lib.linear_routed_gemm(x->const_data_ptr(), dt, x_div, x->size(1), plan->const_data_ptr(), count, (int)t[0]->numel(),
                                static_cast<const void* const*>(t[0]->const_data_ptr()), static_cast<const void* const*>(t[1]->const_data_ptr()),
-                               static_cast<const uint8_t* const*>(t[2]->const_data_ptr()), static_cast<const uint8_t* const*>(t[3]->const_data_ptr()), (int)mt,
-                               (int)nt, (int)K, y.data_ptr(), (int)prologue, ws->data_ptr(), ws->numel(), st) != HTR_OK)
+                               static_cast<const uint8_t* const*>(t[2]->const_data_ptr()), static_cast<const uint8_t* const*>(t[3]->const_data_ptr()), mt,
+                               nt, K, y.data_ptr(), prologue, ws->data_ptr(), ws->numel(), st) != HTR_OK)
     return none();
   return THPVariable_Wrap(std::move(y));
 }
@@ -371,10 +395,9 @@ PyObject* py_decoder_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor *x = tensor(a[0]), *kc = tensor(a[4]), *vc = tensor(a[5]), *pos = tensor(a[6]), *cosv = tensor(a[7]), *sinv = tensor(a[8]), *status = tensor(a[9]);
   if (!x || !kc || !vc || !pos || !cosv || !sinv || !status || !PyList_CheckExact(a[1]) || !x->is_cuda() || x->dim() != 2) return none();
   const at::Device where = x->device();
-  const long hq = PyLong_AsLong(a[10]), hkv = PyLong_AsLong(a[11]);
-  const double eps = PyFloat_AsDouble(a[12]);
-  const long gemm_rows = PyLong_AsLong(a[13]);
-  if (PyErr_Occurred()) { PyErr_Clear(); return none(); }
+  int hq, hkv, gemm_rows;
+  double eps;
+  if (!int_of(a[10], &hq) || !int_of(a[11], &hkv) || !float_of(a[12], &eps) || !int_of(a[13], &gemm_rows)) return none();
   const bool folded = gemm_rows == 0;
   constexpr int64_t D = 128;
   const int64_t T = x->size(0), hidden = x->size(1);
@@ -449,8 +472,8 @@ PyObject* py_decoder_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
       const Layer& l = layers[i];
       void *kl = static_cast<char*>(kc->data_ptr()) + i * layer_bytes, *vl = static_cast<char*>(vc->data_ptr()) + i * layer_bytes;
       if (!norm(i ? delta.data_ptr() : nullptr, l.ln1) || !gemm(h, l.qkv, qkv)) return none();
-      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
-      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
       if (!gemm(att, l.o, delta) || !norm(delta.data_ptr(), l.ln2) || !gemm(h, l.up, gu)) return none();
       if (g_lib.swiglu(gu.data_ptr(), act.data_ptr(), rows, inter, st) != HTR_OK || !gemm(act, l.down, delta)) return none();
     }
@@ -462,10 +485,10 @@ PyObject* py_decoder_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     void *kl = static_cast<char*>(kc->data_ptr()) + i * layer_bytes, *vl = static_cast<char*>(vc->data_ptr()) + i * layer_bytes;
     if (!fused(xp, l.qkv, qkv.data_ptr(), HTR_PROLOGUE_RMSNORM, l.ln1, 0)) return none();
     if (T == 1) {                                         // one token: rotary embedding, cache write and attention in one launch
-      if (g_lib.rope_attention(qkv.data_ptr(), at_pos, cp, sp, kl, vl, att.data_ptr(), (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.rope_attention(qkv.data_ptr(), at_pos, cp, sp, kl, vl, att.data_ptr(), hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
     } else {
-      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
-      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, (int)hq, (int)hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
     }
     if (!fused(att.data_ptr(), l.o, xp, HTR_PROLOGUE_NONE, nullptr, 1) || !fused(xp, l.up, gu.data_ptr(), HTR_PROLOGUE_RMSNORM, l.ln2, 0) ||
         !fused(gu.data_ptr(), l.down, xp, HTR_PROLOGUE_SWIGLU, nullptr, 1))

@@ -141,6 +141,8 @@ def linear_padded(x, qweight, scales, su, sv, bias=None, m_out=None):
     if bias is not None and (bias.dtype != x2.dtype or bias.numel() != m_out):
         raise _lib.HTRError("htr::linear: bias must have the activation dtype and m_out elements")
     M, K = x2.shape[0], W // 8
+    if M and not 1 <= m_out <= mt * 16:
+        raise _lib.HTRError(f"htr::linear_padded: m_out = {m_out}, the weight has {mt * 16} rows")
     y = torch.empty((M, m_out), dtype=x2.dtype, device=x2.device)
     if M:
         qweight, scales, su, sv = qweight.contiguous(), scales.contiguous(), su.contiguous(), sv.contiguous()

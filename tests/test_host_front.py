@@ -77,3 +77,24 @@ def test_decoder_front_equals_general_path(T, monkeypatch):
     dec.layers[1]["o"] = dec.layers[1]["qkv"]                            # another shape: refused as the general path refuses it
     with pytest.raises(Exception):
         dec.forward(ids, pos)
+
+
+def test_integers_beyond_their_range_are_refused(monkeypatch):
+    """Sizes that do not fit a C integer: the error or the result of the general path, never a Python error left set by the front."""
+    from htr_b200 import _lib, ops, wire
+
+    dev = torch.device("cuda:0")
+    w = wire.random_packed(384, 256, 4, seed=1, device=dev)
+    x = torch.randn(3, 256, device=dev).bfloat16()
+    want = ops.linear(x, *w)
+    for m_out in (2 ** 31, 2 ** 40, 2 ** 63, 2 ** 70, -(2 ** 70), 0, 385):
+        with pytest.raises(_lib.HTRError):
+            ops.linear_padded(x, *w, m_out=m_out)
+    with pytest.raises(_lib.HTRError):
+        ops.linear_fused(x, *w, prologue=3)
+    monkeypatch.setattr(ops, "GEMM_ROUTE_MAX", 2 ** 70)
+    assert torch.equal(ops.linear(x, *w), want)
+    for bad in (2 ** 31, 2 ** 70, -(2 ** 70), "1", None):                # the front itself: None, no exception
+        assert ops._host.linear(x, *w, None, 0, 4, bad) is None
+        assert ops._host.linear_padded(x, *w, None, bad, 4) is None and ops._host.linear_padded(x, *w, None, 384, bad) is None
+        assert ops._host.linear_fused(x, *w, None, bad, None, 1e-6, False) is None
