@@ -30,6 +30,8 @@
 namespace {
 
 struct Entry {
+  decltype(&htr_linear_workspace_bytes) linear_workspace_bytes;
+  decltype(&htr_linear_gemm_workspace_bytes) linear_gemm_workspace_bytes;
   decltype(&htr_linear_ex) linear_ex;
   decltype(&htr_linear_gemm) linear_gemm;
   decltype(&htr_linear_padded) linear_padded;
@@ -375,8 +377,8 @@ PyObject* py_moe_weighted_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // ---- a step of the decoder (the loops of PackedDecoder.forward_folded and forward_fused): a decode-sized one is five or six launches a layer, 85 us
 // of host work in Python, more than the GPU needs for layers of small models; 24 here (two layers of hidden 1024, a token: 210 -> 95 us).
-// Unlike the fronts above it may return None after part of the step is enqueued: the caller then starts again from the embeddings
-// (cache rows are written again with the same values).
+// Whatever could refuse a launch of the step (shapes, alignment, workspace) is looked at before the first one, so that None means that
+// nothing is enqueued and x is as it was; a launch that fails all the same (a CUDA error) raises.
 
 bool wire_of(PyObject* o, const at::Device& dev, Weight* w) {   // the tuple of four wire tensors
   PyObject* item[4];
@@ -442,6 +444,24 @@ PyObject* py_decoder_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
   const at::Tensor* ws = find_workspace(folded ? kGemv : kGemm, dev, st);
   if (!ws) return none();
+  const auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  Weight fits[5] = {};                                    // per role, the shape looked at last: layers are mostly alike
+  const auto serves = [&](const Weight& w, int role) {
+    if (!a16(w.qw) || !a16(w.sc)) return false;
+    if (w.mt == fits[role].mt && w.nt == fits[role].nt && w.K == fits[role].K) return true;
+    if (w.mt % 8 || w.nt % 8 || w.mt / 8 >= 16383 || (int64_t)(w.mt / 8) * (w.nt / 4) > 0x3FFFFFFF) return false;   // (limits of the launches)
+    for (int r = 0; r < rows; r += folded ? rows : (int)HTR_GEMM_MAX_ROWS) {
+      const size_t need = folded ? g_lib.linear_workspace_bytes(rows, w.mt * 16, w.nt * 16, w.K)
+                                 : g_lib.linear_gemm_workspace_bytes(std::min(rows - r, (int)HTR_GEMM_MAX_ROWS), w.mt * 16, w.nt * 16, w.K);
+      if (need == 0 || need > (size_t)ws->numel()) return false;
+    }
+    fits[role] = w;
+    return true;
+  };
+  for (const Layer& l : layers)
+    if (!serves(l.qkv, 0) || !serves(l.o, 1) || !serves(l.up, 2) || !serves(l.down, 3) || !a16(l.ln1) || !a16(l.ln2)) return none();
+  if (!serves(head, 4) || !a16(ln_f) || !a16(x->const_data_ptr()) || hq % hkv || cap < 1 || (!folded && (hidden > 8192 || T > (1 << 16)))) return none();
+  const auto failed = []() -> PyObject* { TORCH_CHECK(false, "decoder_step: a launch failed; part of the step is enqueued"); };
   const auto empty = [&](int64_t columns) { return at::detail::empty_cuda({T, columns}, at::kBFloat16, where, std::nullopt); };
   const at::Tensor qkv = empty((hq + 2 * hkv) * D), att = empty(hq * D), q = T > 1 || !folded ? empty(hq * D) : at::Tensor();
   const at::Tensor gu = empty(count ? (int64_t)layers[0].up.mt * 16 : 0);
@@ -471,30 +491,30 @@ PyObject* py_decoder_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (Py_ssize_t i = 0; i < count; ++i) {
       const Layer& l = layers[i];
       void *kl = static_cast<char*>(kc->data_ptr()) + i * layer_bytes, *vl = static_cast<char*>(vc->data_ptr()) + i * layer_bytes;
-      if (!norm(i ? delta.data_ptr() : nullptr, l.ln1) || !gemm(h, l.qkv, qkv)) return none();
-      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
-      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
-      if (!gemm(att, l.o, delta) || !norm(delta.data_ptr(), l.ln2) || !gemm(h, l.up, gu)) return none();
-      if (g_lib.swiglu(gu.data_ptr(), act.data_ptr(), rows, inter, st) != HTR_OK || !gemm(act, l.down, delta)) return none();
+      if (!norm(i ? delta.data_ptr() : nullptr, l.ln1) || !gemm(h, l.qkv, qkv)) return failed();
+      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return failed();
+      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return failed();
+      if (!gemm(att, l.o, delta) || !norm(delta.data_ptr(), l.ln2) || !gemm(h, l.up, gu)) return failed();
+      if (g_lib.swiglu(gu.data_ptr(), act.data_ptr(), rows, inter, st) != HTR_OK || !gemm(act, l.down, delta)) return failed();
     }
-    if (!norm(count ? delta.data_ptr() : nullptr, ln_f) || !gemm(h, head, y)) return none();
+    if (!norm(count ? delta.data_ptr() : nullptr, ln_f) || !gemm(h, head, y)) return failed();
     return THPVariable_Wrap(std::move(y));
   }
   for (Py_ssize_t i = 0; i < count; ++i) {
     const Layer& l = layers[i];
     void *kl = static_cast<char*>(kc->data_ptr()) + i * layer_bytes, *vl = static_cast<char*>(vc->data_ptr()) + i * layer_bytes;
-    if (!fused(xp, l.qkv, qkv.data_ptr(), HTR_PROLOGUE_RMSNORM, l.ln1, 0)) return none();
+    if (!fused(xp, l.qkv, qkv.data_ptr(), HTR_PROLOGUE_RMSNORM, l.ln1, 0)) return failed();
     if (T == 1) {                                         // one token: rotary embedding, cache write and attention in one launch
-      if (g_lib.rope_attention(qkv.data_ptr(), at_pos, cp, sp, kl, vl, att.data_ptr(), hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.rope_attention(qkv.data_ptr(), at_pos, cp, sp, kl, vl, att.data_ptr(), hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return failed();
     } else {
-      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
-      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return none();
+      if (g_lib.rope_cache(qkv.data_ptr(), at_pos, cp, sp, q.data_ptr(), kl, vl, rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return failed();
+      if (g_lib.attention(q.data_ptr(), kl, vl, at_pos, att.data_ptr(), rows, hq, hkv, (int)D, (int)cap, sw, st) != HTR_OK) return failed();
     }
     if (!fused(att.data_ptr(), l.o, xp, HTR_PROLOGUE_NONE, nullptr, 1) || !fused(xp, l.up, gu.data_ptr(), HTR_PROLOGUE_RMSNORM, l.ln2, 0) ||
         !fused(gu.data_ptr(), l.down, xp, HTR_PROLOGUE_SWIGLU, nullptr, 1))
-      return none();
+      return failed();
   }
-  if (!fused(xp, head, y.data_ptr(), HTR_PROLOGUE_RMSNORM, ln_f, 0)) return none();
+  if (!fused(xp, head, y.data_ptr(), HTR_PROLOGUE_RMSNORM, ln_f, 0)) return failed();
   return THPVariable_Wrap(std::move(y));
 }
 
@@ -524,6 +544,8 @@ PyObject* py_bind(PyObject*, PyObject* table) {
     PyObject* v = PyDict_Check(table) ? PyDict_GetItemString(table, name) : nullptr;
     return v ? PyLong_AsVoidPtr(v) : nullptr;
   };
+  g_lib.linear_workspace_bytes = reinterpret_cast<decltype(g_lib.linear_workspace_bytes)>(at_name("htr_linear_workspace_bytes"));
+  g_lib.linear_gemm_workspace_bytes = reinterpret_cast<decltype(g_lib.linear_gemm_workspace_bytes)>(at_name("htr_linear_gemm_workspace_bytes"));
   g_lib.linear_ex = reinterpret_cast<decltype(g_lib.linear_ex)>(at_name("htr_linear_ex"));
   g_lib.linear_gemm = reinterpret_cast<decltype(g_lib.linear_gemm)>(at_name("htr_linear_gemm"));
   g_lib.linear_padded = reinterpret_cast<decltype(g_lib.linear_padded)>(at_name("htr_linear_padded"));
@@ -540,7 +562,7 @@ PyObject* py_bind(PyObject*, PyObject* table) {
   g_lib.rope_attention = reinterpret_cast<decltype(g_lib.rope_attention)>(at_name("htr_dec_rope_attention"));
   g_lib.add_rmsnorm = reinterpret_cast<decltype(g_lib.add_rmsnorm)>(at_name("htr_dec_add_rmsnorm"));
   g_lib.swiglu = reinterpret_cast<decltype(g_lib.swiglu)>(at_name("htr_dec_swiglu"));
-  if (!g_lib.add_rmsnorm || !g_lib.swiglu || !g_lib.rope_cache || !g_lib.attention || !g_lib.rope_attention || !g_lib.linear_routed || !g_lib.linear_routed_gemm || !g_lib.route_plan_bytes || !g_lib.route_plan || !g_lib.moe_weighted_sum ||
+  if (!g_lib.linear_workspace_bytes || !g_lib.linear_gemm_workspace_bytes || !g_lib.add_rmsnorm || !g_lib.swiglu || !g_lib.rope_cache || !g_lib.attention || !g_lib.rope_attention || !g_lib.linear_routed || !g_lib.linear_routed_gemm || !g_lib.route_plan_bytes || !g_lib.route_plan || !g_lib.moe_weighted_sum ||
       !g_lib.linear_gemm_padded || !g_lib.route_rows || !g_lib.linear_ex || !g_lib.linear_gemm || !g_lib.linear_padded || !g_lib.linear_fused) {
     PyErr_SetString(PyExc_ImportError, "bind: an entry point of libhtr_b200 is missing");
     return nullptr;

@@ -209,7 +209,6 @@ class PackedDecoder:
                                        c.q_heads, c.kv_heads, c.eps, ops.GEMM_ROUTE_MAX)
             if y is not None:
                 return y
-            x = self.embed.index_select(0, ids)                 # (it may have been changed)
         h = torch.empty_like(x)
         q = torch.empty(T, c.q_heads, c.head_dim, dtype=self.dtype, device=dev)
         att = torch.empty_like(q)
@@ -251,7 +250,6 @@ class PackedDecoder:
                                    c.q_heads, c.kv_heads, c.eps, 0)
         if y is not None:
             return y
-        x = self.embed.index_select(0, ids)                     # (it may have been changed)
         q = torch.empty(T, c.q_heads, c.head_dim, dtype=self.dtype, device=dev)
         att = torch.empty_like(q)
         kp, vp, layer_bytes = self._cache_rows()

@@ -98,3 +98,48 @@ def test_integers_beyond_their_range_are_refused(monkeypatch):
         assert ops._host.linear(x, *w, None, 0, 4, bad) is None
         assert ops._host.linear_padded(x, *w, None, bad, 4) is None and ops._host.linear_padded(x, *w, None, 384, bad) is None
         assert ops._host.linear_fused(x, *w, None, bad, None, 1e-6, False) is None
+
+
+@pytest.mark.parametrize("T", (1, 3, 9, 300))
+def test_a_refused_decoder_step_leaves_nothing_behind(T):
+    """None from the native loop means that nothing was enqueued, also where only a late linear is the reason: the residual stream and the
+    caches are as they were.  Reasons: a weight that is not 16-byte aligned, a workspace that is too small for one of the linears."""
+    from htr_b200 import _lib, ops
+    from htr_b200.decoder import DecoderConfig, PackedDecoder
+
+    dev = torch.device("cuda:0")
+    dec = PackedDecoder(DecoderConfig(layers=2, hidden=256, q_heads=4, kv_heads=2, intermediate=384, vocab=65536, max_len=512), dev, seed=T)
+    ids, pos = torch.arange(T, device=dev), torch.arange(5, 5 + T, device=dev)
+    want = dec.forward(ids, pos)                                         # the workspaces exist from here on
+    c, gemm_rows = dec.cfg, 0 if T <= ops.GEMV_MAX_M else ops.GEMM_ROUTE_MAX
+    dec.k_cache.zero_(), dec.v_cache.zero_()
+
+    def step():
+        x = dec.embed.index_select(0, ids)
+        y = ops._host.decoder_step(x, dec.layers, dec.head, dec.ln_f, dec.k_cache, dec.v_cache, pos, dec.cos, dec.sin, dec.status, c.q_heads, c.kv_heads,
+                                   c.eps, gemm_rows)
+        if y is None:
+            assert torch.equal(x, dec.embed.index_select(0, ids)) and not bool(dec.k_cache.any()) and not bool(dec.v_cache.any())
+        return y
+
+    qw = dec.layers[1]["down"][0]
+    shifted = torch.zeros(qw.numel() + 1, dtype=qw.dtype, device=dev)[1:].view_as(qw)
+    shifted.copy_(qw)
+    good = dec.layers[1]["down"]
+    dec.layers[1]["down"] = (shifted, *good[1:])
+    assert step() is None
+    with pytest.raises(_lib.HTRError):
+        dec.forward(ids, pos)
+    dec.layers[1]["down"] = good
+    dec.k_cache.zero_(), dec.v_cache.zero_()
+    kind, stream = (0 if gemm_rows == 0 else 1), torch.cuda.current_stream().cuda_stream
+    rows = min(T, ops.GEMM_MAX_M)
+    size = _lib.lib.htr_linear_workspace_bytes if kind == 0 else _lib.lib.htr_linear_gemm_workspace_bytes
+    need = max(size(rows, t[0].shape[0] * 16, t[0].shape[1] * 16, t[0].shape[2] // 8) for t in (*(dec.layers[0][k] for k in ("qkv", "o", "gate_up", "down")), dec.head))
+    small = torch.zeros(need - 1, dtype=torch.uint8, device=dev)         # too little for one of them
+    ops._host.set_workspace(kind, dev.index, stream, small)
+    try:
+        assert step() is None
+    finally:
+        ops._host.set_workspace(kind, dev.index, stream, (ops._WORKSPACES if kind == 0 else ops._GEMM_WS)[(dev.index, stream)])
+    assert torch.equal(step(), want)
