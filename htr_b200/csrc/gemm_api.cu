@@ -396,18 +396,23 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   if (g.stages < 2) return HTR_ERR_TOO_LARGE;
   // Three forms, by their cost in units of one decoded 128 x 128 block (0.43 us, or as long as the MMAs of a wide batch take):
   //  * up to sixteen thread blocks share a row block as a cluster and reduce on chip;
-  //  * a thread block takes a whole row block, in as many waves as there are row blocks per SM: all its warps finish it from shared
+  //  * a thread block takes a whole row block, in as many waves as there are row blocks per SM: its decode warps finish it from shared
   //    memory, about four blocks' time and a thirtieth of one per activation row;
   //  * every thread block of the GPU takes an even run (flat) and a row block's partial sums meet in global memory at one last arriver:
-  //    nine blocks' time for the hand-over (measured 2 to 3 us) and the partials, which that one reads at 100 bytes a nanosecond.  Row
-  //    blocks inside a run are finished by four warps beside the decode, half a block's time per activation row: many rows wait for them.
-  // Measured, flat / whole row blocks: 28672x1024, 64 rows 31.5 / 22.2 us; 151936x4096, 32 rows 147 / 182; 12288x4096, 200 rows 41.4 / 39.0;
-  // clusters over flat: 2048x2048, 8 / 200 rows 11.5 / 33.2 -> 7.6 / 16.9.
+  //    nine blocks' time for the hand-over (measured 2 to 3 us) and the partials, which that one reads row by row.  Row blocks inside a
+  //    run are finished by four warps beside the decode, half a block's time per activation row: many rows wait for them.
+  // us, flat / whole row blocks: 28672x1024, 64 rows 31.6 / 18.8; 151936x4096, 32 rows 146 / 171; 12288x4096, 64 rows 23.7 / 25.0, 160 rows
+  // 34.3 / 32.3, 200 rows 39.8 / 33.8, 256 rows 48.8 / 44.7; flat / clusters: 2048x2048, 8 / 200 rows 11.8 / 6.7, 35.1 / 14.6.
+  // (Beyond 128 rows a partial is read at less than half the rate: 12288x4096, 128 rows 29.7 / 29.9, 160 rows 34.3 / 32.3.)
+  // The tensor cores cut each sum off towards zero, so the error of a result grows with the blocks that one accumulator takes: 2048x4096,
+  // float32, 2 / 8 / 32 blocks 3.5e-6 / 1.1e-5 / 4.1e-5 (2-norm, normal activations), five times that where the activations have a mean.
+  // A change of these terms that gives float32 rows longer sums loses precision; beyond 128 rows there is one plane, whose own rounding
+  // (2e-4) hides it.
   const double unit = ncols > 192 ? 1.2 : 1.0;
   const long long slots = sms, units = (long long)g.rbs * g.hb;
   const long long flat_grid = slots < units ? slots : units, flat_run = (units + flat_grid - 1) / flat_grid;
   const double beside = (double)(flat_run / g.hb) * M * 0.5;
-  double best = (flat_run * unit > beside ? flat_run * unit : beside) + 9 + (double)((g.hb / flat_run + 1) * g.np) / 84;
+  double best = (flat_run * unit > beside ? flat_run * unit : beside) + 9 + (double)((g.hb / flat_run + 1) * g.np) / (g.np > 128 ? 32 : 84);
   g.split = 0;
   for (int s = (int)(slots / g.rbs < 16 ? slots / g.rbs : 16); s >= 2; --s) {
     const double cost = (double)((g.hb + s - 1) / s) * unit;

@@ -31,9 +31,14 @@
 // of each block (one bulk copy, completion counted on an mbarrier); one lane of warp 17 issues the eight MMAs of a block.  Stage s of
 // the ring is {64 tensor-memory columns of A, one B tile} with full[s] and freed[s] (tcgen05.commit); with up to seven
 // stages the decode runs ahead while the activation transform before the launch still works and while an accumulator is read.
-// Warps 18-21 finish row blocks: they move the accumulator to a partial sum in memory and, where it is the last, add the partials,
-// apply scales, output transform and signs, and store.  (Done by the decode warps, that chain of dependent loads cost 12 000 cycles
-// per row block, a fifth of the LM head at 8 rows.)  The last row block of a thread block is finished by all its warps.
+// Warps 18-21 finish the row blocks of a flat run: they move the accumulator to a partial sum in memory and, where it is the last, add the
+// partials, apply scales, output transform and signs, and store.  (Done by the decode warps, that chain of dependent loads cost 12 000
+// cycles per row block, a fifth of the LM head at 8 rows.)  The last row block of a run is finished by all warps.
+// A thread block with one row block, or a part of one (clusters, whole row blocks), has no use for them: its decode warps fetch what
+// their rows need (scales, signs, activation sums, lane i those of the i-th row) behind their last block, beside the last MMAs, move the
+// accumulator, four warps per quadrant, and finish.  With the finishers in their place a row waited for its own loads and 200 rows left
+// tensor memory one column group at a time.  us, before -> after: 32768x256, 8 / 200 rows 11.9 -> 10.0, 34.6 -> 24.8; 4096x4096, 8 / 256 rows
+// 9.9 -> 9.0, 25.9 -> 22.8; 2048x2048, 8 rows 7.5 -> 6.7; 4096x12288, 128 rows 27.5 -> 25.0.
 //
 // Decomposition.  Work = (row block) x (128-column blocks).  Where the row blocks are few, `split` thread blocks share one as a
 // cluster and reduce through distributed shared memory; else every thread block takes an even contiguous run that may cross row
@@ -323,9 +328,13 @@ __device__ __forceinline__ float gemm_xsum_share(const GemmParams& p, int j, int
   for (int y = lane; y < p.xsum_slices; y += 32) xs += __ldcg(p.xsum + (size_t)j * p.xsum_slices + y);
   return xs;
 }
-__device__ __forceinline__ void gemm_finish_row(const GemmParams& p, const GemmTail& t, int j, int lane, float4 r4, float xs, float tok) {
+__device__ __forceinline__ float gemm_xsum_total(float xs) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) xs += __shfl_xor_sync(kFullWarp, xs, o);
+  return xs;
+}
+// xs: the whole row sum of the activations
+__device__ __forceinline__ void gemm_finish_row(const GemmParams& p, const GemmTail& t, int j, int lane, float4 r4, float xs, float tok) {
   const float off = 1534.0f * xs, out = kInvSqrt128 * tok;  // (the range scale last: a row scale times a small tok could underflow)
   float v[4] = {(r4.x - off) * t.s[0], (r4.y - off) * t.s[1], (r4.z - off) * t.s[2], (r4.w - off) * t.s[3]};
   wht128(v, lane);
@@ -362,8 +371,8 @@ __device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, in
         rb4.x += vb[q].x; rb4.y += vb[q].y; rb4.z += vb[q].z; rb4.w += vb[q].w;
       }
     }
-    gemm_finish_row(p, tail, j, lane, ra, xa, ta);
-    if (jb != j) gemm_finish_row(p, tail, jb, lane, rb4, xb, tb);
+    gemm_finish_row(p, tail, j, lane, ra, gemm_xsum_total(xa), ta);
+    if (jb != j) gemm_finish_row(p, tail, jb, lane, rb4, gemm_xsum_total(xb), tb);
   }
 }
 
@@ -433,6 +442,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
   }
 
+  // cluster form: what a decode warp needs to finish its rows j0, j0 + split * DW, ... (at most sixteen) of the one row block
+  GemmTail tail;
+  float xs_of = 0.f, tok_of = 0.f;                          // lane i: activation sum and scale of the i-th of these rows
+  const int row_step = p.split * DW, row_first = part_id + p.split * warp;
   if (warp < DW) {
     // ================= decode warps
     const int quad = warp & 3, half = (warp >> 2) & 1, strip = 2 * quad + half, group = warp >> 3;
@@ -527,8 +540,40 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       stage += around ? 2 - NS : 2;
       parity ^= around ? 1u : 0u;
     }
-    if (!ok) s_fail = 1;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (!GROUP && p.split > 0) {
+      // these loads, and the wait for the transform that they need, lie beside the last MMAs; then the accumulator goes to the ring as
+      // the thread block's partial [np][128], hi + lo added: four warps of a quadrant take alternate groups of 8 columns
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      tail.load<false>(p, blockIdx.x / p.split, lane);
+      const int j = row_first + lane * row_step;
+      if (j < p.rows) {
+        float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+        for (int y = 0; y < p.xsum_slices; y += 4)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) part[q] += y + q < p.xsum_slices ? __ldcg(p.xsum + (size_t)j * p.xsum_slices + y + q) : 0.f;
+        xs_of = (part[0] + part[2]) + (part[1] + part[3]);
+        tok_of = __ldcg(p.tok + j);
+      }
+      ok = ok && __all_sync(kFullWarp, mbar_wait(smem_u32(&s_done), 0u, &s_fail));
+      if (ok) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int li = lane & 15, row = 32 * quad + (lane & 16) + (li < 8 ? 2 * li : 2 * li - 15);   // weight row of this tensor-memory lane
+        const uint32_t acc_addr = s_tmem + ((uint32_t)(32 * quad) << 16);
+        float* mine = reinterpret_cast<float*>(ring);
+        for (int j0 = 8 * (warp >> 2); j0 < np; j0 += 2 * DW) {
+          uint32_t hi[8], lo[8];
+          tmem_load8(acc_addr + j0, hi);
+          if (p.planes == 2) tmem_load8(acc_addr + np + j0, lo);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 8; ++i) mine[(j0 + i) * 128 + row] = p.planes == 2 ? __uint_as_float(hi[i]) + __uint_as_float(lo[i]) : __uint_as_float(hi[i]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      }
+    }
+    if (!ok) s_fail = 1;
   } else {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -602,8 +647,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
           mbar_wait(smem_u32(&s_done), (uint32_t)seg & 1u, nullptr);   // ... this one lets the MMAs in flight retire first
         }
       }
-    } else {
-      // ================= finishers
+    } else if (GROUP || p.split == 0) {
+      // ================= finishers (cluster form: the decode warps do that)
       const int fw = warp - (DW + 2), quad = warp & 3;
       const uint32_t acc_addr = s_tmem + ((uint32_t)(32 * quad) << 16);
       const int li = lane & 15, row = 32 * quad + (lane & 16) + (li < 8 ? 2 * li : 2 * li - 15);   // weight row of this tensor-memory lane
@@ -623,7 +668,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         }
         // accumulator -> partial [np][128], hi + lo added here.  A thread block has two partials: its first row block's, which other
         // thread blocks may read, and one for all later ones (of which only the last is read by others)
-        float* mine = !GROUP && p.split > 0 ? reinterpret_cast<float*>(ring) : p.part + (size_t)(2 * blockIdx.x + (seg > 0 ? 1 : 0)) * ((size_t)np * 128);
+        float* mine = p.part + (size_t)(2 * blockIdx.x + (seg > 0 ? 1 : 0)) * ((size_t)np * 128);
         for (int j0 = 0; j0 < np; j0 += 8) {
           uint32_t hi[8], lo[8];
           tmem_load8(acc_addr + j0, hi);
@@ -632,14 +677,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float v = p.planes == 2 ? __uint_as_float(hi[j]) + __uint_as_float(lo[j]) : __uint_as_float(hi[j]);
-            if (!GROUP && p.split > 0) mine[(j0 + j) * 128 + row] = v;
-            else __stcg(mine + (j0 + j) * 128 + row, v);
+            __stcg(mine + (j0 + j) * 128 + row, v);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&s_drained));    // the MMAs of the next row block may start
-        if ((!GROUP && p.split > 0) || stop >= u_end) break;             // the last row block: all warps finish it, below
+        if (stop >= u_end) break;                            // the last row block: all warps finish it, below
         // only the run's first row block can have other contributors here, thread blocks before this one
         const int first = runs.owner(rb * HB), contributors = blockIdx.x - first + 1;
         bool finish = true;
@@ -675,21 +719,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       for (int e = tid; e < np * 128; e += kGemmThreads) result[e] = __uint_as_float(0x7FC00000u);
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // (done before by the roles that needed it)
-    GemmTail tail;
-    tail.load<false>(p, blockIdx.x / p.split, lane);
-    const uint32_t result_addr = smem_u32(result);
-    for (int j = part_id + p.split * warp; j < p.rows; j += p.split * kGemmWarps) {
-      const float xs = gemm_xsum_share(p, j, lane), tok = __ldcg(p.tok + j);
-      float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int r = 0; r < p.split; ++r) {
-        uint32_t remote;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(result_addr + (uint32_t)(j * 128 + 4 * lane) * 4u), "r"(r));
-        float4 v;
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
-        r4.x += v.x; r4.y += v.y; r4.z += v.z; r4.w += v.w;
+    if (warp < DW) {
+      const uint32_t result_addr = smem_u32(result) + (uint32_t)lane * 16u;
+      for (int i = 0; row_first + i * row_step < p.rows; ++i) {
+        const int j = row_first + i * row_step;
+        float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < p.split; ++r) {
+          uint32_t remote;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(result_addr + (uint32_t)j * 512u), "r"(r));
+          float4 v;
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+          r4.x += v.x; r4.y += v.y; r4.z += v.z; r4.w += v.w;
+        }
+        gemm_finish_row(p, tail, j, lane, r4, __shfl_sync(kFullWarp, xs_of, i), __shfl_sync(kFullWarp, tok_of, i));
       }
-      gemm_finish_row(p, tail, j, lane, r4, xs, tok);
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // nobody leaves while its shared memory may still be read
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

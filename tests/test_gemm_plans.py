@@ -82,3 +82,26 @@ def test_rows_of_any_magnitude(coracle, dtype, M, tol, padded):
             s = float(np.abs(ref[r]).max())                       # (norms of the smallest rows would underflow)
             assert rel(y[r] / s, ref[r] / s) <= tol, (r, powers[r])
     assert all(c == 0 for c in ops.gemm_error_codes())
+
+
+@pytest.mark.parametrize("K,m,n,rows", ((3, 19072, 128, (9, 16, 17, 255, 256)), (4, 2048, 2048, (9, 15, 64, 65, 256)), (5, 640, 2176, (1, 33, 241, 256)),
+                                        (8, 128, 1024, (5, 128, 129)), (2, 32768, 256, (8, 200))))
+def test_rows_of_one_row_block(coracle, K, m, n, rows):
+    """Thread blocks with one row block or a part of one: the decode warps finish rows 16 at a time (per member of a cluster), each with the
+    sums and scales that its lane brought.  Row counts at the edges; every row has its own magnitude, so that a mixed-up scale shows."""
+    from htr_b200 import ops, wire
+
+    dev = torch.device("cuda:0")
+    qw, sc, su, sv = wire.random_packed(m, n, K, seed=m + n)
+    d = [t.to(dev) for t in (qw, sc, su, sv)]
+    g = torch.Generator().manual_seed(K)
+    x = (torch.randn(256, n, generator=g) + torch.randn(256, 1, generator=g)) * 2.0 ** torch.randint(-12, 12, (256, 1), generator=g)
+    x, bias = x.bfloat16(), torch.randn(m, generator=g).bfloat16()
+    few = slice(0, 640) if m > 4096 else slice(0, m)                     # (rows of the weight that the oracle computes)
+    ref = coracle.linear(x.float().numpy(), qw[:few.stop // 16].numpy(), sc[few].numpy(), su.numpy(), sv[:few.stop // 8].numpy())
+    for M in rows:
+        y = ops.linear(x[:M].to(dev), *d, bias.to(dev)) if M > 1 else ops.linear_padded(x[:M].to(dev), *d, bias=bias.to(dev), m_out=m)
+        want = ref[:M] + bias[few].float().numpy()
+        err = np.linalg.norm(y[:, few].float().cpu().numpy() - want, axis=1) / np.linalg.norm(want, axis=1)
+        assert err.max() <= 4e-3, (M, int(err.argmax()), float(err.max()))
+    assert all(c == 0 for c in ops.gemm_error_codes())
