@@ -174,8 +174,9 @@ static int gemv_kind(int M, int dtype = HTR_DTYPE_BF16, int n = 0, int prologue 
 }
 
 // From two 16-bit rows on, linears of at least this many weights run on the tensor-core GEMM (htr_linear_route_rows).  Measured at
-// K4, two / four bf16 rows, GEMV -> GEMM: 1024x4096 10.3 / 14.4 -> 7.8 us, 4096x12288 18.4 / 22.8 -> 17.1, 151936x4096 169 / 219 -> 126;
-// at 2 million weights and below the second launch costs what the decode saves (1024x1024, four fp16 rows: 5.9 against 7.0).
+// K4, two / four bf16 rows, GEMV -> GEMM: 1024x4096 10.3 / 14.4 -> 7.1 / 7.2 us, 4096x12288 18.9 / 23.2 -> 17.0 / 17.4, 151936x4096 170 / 222 ->
+// 128 / 130; at 2 million weights four fp16 rows lose (2048x1024: 5.9 against 6.2).  (Two to four bf16 rows would gain there too since the
+// finishing of small batches moved to the decode warps: 1024x2048, 4 rows 11.6 against 6.5; the line is older than that.)
 constexpr long long kRouteSmall = 1 << 22;
 
 static int make_plan(int M, int m, int n, int K, Plan* out, int kind = 0) {
@@ -254,8 +255,9 @@ static int make_plan(int M, int m, int n, int K, Plan* out, int kind = 0) {
 // where most blocks of a run end a row block (32768x256: 5.2 against 5.6).
 constexpr long long kChainSmall = 1 << 18;
 // The linears inside a decoder's layers (a residual or an activation folded in, a norm before fewer rows than a vocabulary has) stay on
-// packed_gemv.cuh.  The chain form would save 5 % of a token there, but it adds in another order: each rounding to bf16 between the
-// layers that falls the other way is carried on, and over 36 layers the logits move by 4.7 % (2-norm).  After the last one nothing follows.
+// packed_gemv.cuh, so that a decoder's results stay what they were.  The chain form would save 5 % of a token there, but it adds in another
+// order, and bf16 layers carry each rounding that falls the other way on: over 36 layers the logits move by 4.7 % (2-norm).  That is no
+// loss of precision: against float64 both orders are equally far off (1.45 % each over 24 layers of hidden 1024, 1.7 % from one another).
 constexpr int kChainLastRows = 1 << 15;
 static bool chain_serves(int m, int n) { return n <= kG1MaxCols && (long long)m * n >= kChainSmall && (n >= 512 || m < 16384); }
 static size_t chain_partial_bytes(int grid) { return (size_t)grid * 2 * 128 * sizeof(float); }

@@ -23,8 +23,8 @@
 // 12288x4096 13.02 -> 13.02, 4096x12288 12.67 -> 12.67, 151936x4096 106.0 -> 104.9.  Dearer forms, at 1024x4096 / 12288x4096: a vote at the
 // barrier before the decode 4.82 / 13.18, both passes as a loop 5.08 / 13.41, the second pass inlined 4.98 / 13.35, a vote on the sums
 // 4.84 / 13.23.
-// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.4 -> 4.9, 4096x12288 K4 13.8 -> 12.7, 151936x4096 K4
-// 131 -> 102 (6.1e12 weights a second, 21 per cycle and SM).
+// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.4 -> 4.7, 4096x12288 K4 13.8 -> 12.7, 151936x4096 K4
+// 131 -> 105 (5.9e12 weights a second, 20 per cycle and SM).
 #pragma once
 #include "packed_gemv.cuh"
 

@@ -35,7 +35,7 @@ GEMM_MAX_M = _lib.GEMM_MAX_ROWS
 # above this many rows the weight is decoded once to bf16 and a library GEMM runs (the packed GEMM decodes once per 256-row launch)
 GEMM_ROUTE_MAX = int(os.environ.get("HTR_GEMM_ROUTE_MAX", "512"))
 # batches above this many rows leave the GEMV for the tensor-core GEMM (the GEMV itself handles up to 8 rows, but from 5 rows
-# on the GEMM is faster: 25 us against 41-44 us at 4096x12288, 190 us against 384-408 us on the 151936x4096 head)
+# on the GEMM is faster: 18 us against 41-44 us at 4096x12288, 129 us against 384-408 us on the 151936x4096 head)
 GEMV_ROUTE_MAX = min(GEMV_MAX_M, int(os.environ.get("HTR_GEMV_ROUTE_MAX", "4")))
 
 

@@ -223,8 +223,8 @@ int htr_linear_fused(const void* x, int M, const void* qweight, int mt, int nt, 
                      const void* norm_weight, float eps, int residual);
 
 /* Tensor-core form of the packed linear for prefill-sized batches, 1 <= M <= HTR_GEMM_MAX_ROWS rows per call:
- * decoded tiles go straight into the shared-memory operand of tcgen05.mma, accumulators live in TMEM; two launches
- * (activation transform to fp16 hi/lo planes, then the GEMM with the same split reduction and epilogue as the GEMV).
+ * decoded tiles go straight into the tensor-memory operand of tcgen05.mma, accumulators live there too; two launches
+ * (activation transform to fp16 hi/lo planes under a power of two per row, so that rows of any magnitude keep their bits, then the GEMM).
  * The workspace starts with the same zero-initialised counter region as htr_linear's, followed by one status word at
  * htr_linear_gemm_error_offset(): non-zero after a call means a bounded device-side wait expired; the rows of the
  * affected 128-row blocks are then written as NaN.  Stands in for the prefill branch of _linear_impl, dequant_w + F.linear (htr/ops.py:89-93). */

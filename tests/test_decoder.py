@@ -132,3 +132,51 @@ def test_single_token_rope_attention_equals_the_two_kernels():
         assert torch.equal(k1, k2) and torch.equal(v1, v2)                 # the same cache rows
         assert float((got.float() - want.float()).abs().max()) <= 2e-2 * float(want.float().abs().max())
     assert int(status.item()) == 0                                          # every position was inside the caches
+
+
+@pytest.mark.parametrize("layers", (2, 8))
+def test_folded_and_separate_steps_are_equally_near_to_float64(layers):
+    """Folded steps (norms, SwiGLU and residual adds inside the CUDA-core GEMVs) and steps of separate kernels (tensor-core GEMM for rows, one-row
+    chain GEMV for tokens) add in different orders, and dozens of bf16 roundings carry that on.  Neither is nearer to the network in float64:
+    both lie at the level of the bf16 roundings, 2^-9 a step, which add up as the square root of their number."""
+    from htr_b200 import wire
+    from htr_b200.decoder import DecoderConfig, PackedDecoder
+
+    dev = torch.device("cuda:0")
+    cfg = DecoderConfig(layers=layers, hidden=512, q_heads=4, kv_heads=2, head_dim=128, intermediate=1024, vocab=1024, K=4, K_head=4, max_len=32)
+    weights = PackedDecoder.random_weights(cfg, dev, 11)
+    ids = torch.randint(0, cfg.vocab, (8,), generator=torch.Generator().manual_seed(2)).to(dev)
+    pos = torch.arange(8, device=dev)
+    model = PackedDecoder(cfg, dev, weights=weights)
+
+    def norm(x, w):
+        return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + cfg.eps) * w.double()
+
+    def rope(t):
+        cos, sin = model.cos[pos].double()[:, None, :], model.sin[pos].double()[:, None, :]
+        return torch.stack((t[..., ::2] * cos - t[..., 1::2] * sin, t[..., ::2] * sin + t[..., 1::2] * cos), dim=-1).flatten(-2)
+
+    def dense(w):
+        return wire.dequant(*w, dtype=torch.float32).double()        # (rounds at 1e-7, the steps below at 4e-3)
+
+    x, inter, rep = model.embed[ids].double(), cfg.intermediate, cfg.q_heads // cfg.kv_heads
+    for L in model.layers:
+        q, k, v = (norm(x, L["ln1"]) @ dense(L["qkv"]).T).split((cfg.q_heads * 128, cfg.kv_heads * 128, cfg.kv_heads * 128), dim=-1)
+        q, k = rope(q.view(8, -1, 128)), rope(k.view(8, -1, 128)).repeat_interleave(rep, 1)
+        s = torch.einsum("thd,shd->hts", q, k) / 128 ** 0.5
+        s = s.masked_fill(pos[None, None, :] > pos[None, :, None], float("-inf")).softmax(-1)
+        x = x + torch.einsum("hts,shd->thd", s, v.view(8, -1, 128).repeat_interleave(rep, 1)).reshape(8, -1) @ dense(L["o"]).T
+        gu = norm(x, L["ln2"]) @ dense(L["gate_up"]).T
+        x = x + (torch.nn.functional.silu(gu[:, :inter]) * gu[:, inter:]) @ dense(L["down"]).T
+    exact = norm(x, model.ln_f) @ dense(model.head).T
+    errors = {}
+    for fold in (True, False):
+        for tokens in (False, True):
+            model = PackedDecoder(cfg, dev, weights=weights)
+            model.fold = fold
+            y = torch.cat([model.forward(ids[i:i + 1], pos[i:i + 1]) for i in range(8)]) if tokens else model.forward(ids, pos)
+            errors[fold, tokens] = float((y.double() - exact).norm() / exact.norm())
+    steps = 12 * layers + 2                                           # bf16 roundings on the way of a value, each at most 2^-9 (2-norm: about half)
+    assert max(errors.values()) <= 2.0 ** -9 * steps ** 0.5, errors
+    for tokens in (False, True):
+        assert 0.8 <= errors[True, tokens] / errors[False, tokens] <= 1.25, errors
