@@ -16,15 +16,14 @@
 //  * a weight costs half an instruction less: its byte sum, as the bits of a float, is a subnormal number (n * 2^-149 exactly), and
 //    multiplied with activations staged times 2^80 it needs neither a magic constant nor its subtraction.  The constant 510 goes in
 //    per 16 columns, as -510 times their sum added to the accumulator first, so that the sums stay centred (no cancellation at the end).
-// Range.  The products are normal numbers while the largest activation that a thread block stages lies within 2^-36 .. 2^36.  A block of
-// any other drops its sums and runs once more (gemv1_wide) under a power of two made for them; partial sums leave in their own unit, so
-// that blocks with different powers add up, and the range of the results is that of packed_gemv.cuh.  The check (three votes of a staging
-// warp, read by the idle finishers) costs the smallest launches 0.1 us and the others nothing: 1024x1024 3.73 -> 3.84, 1024x4096 4.62 -> 4.72,
-// 12288x4096 13.02 -> 13.02, 4096x12288 12.67 -> 12.67, 151936x4096 106.0 -> 104.9.  Dearer forms, at 1024x4096 / 12288x4096: a vote at the
-// barrier before the decode 4.82 / 13.18, both passes as a loop 5.08 / 13.41, the second pass inlined 4.98 / 13.35, a vote on the sums
-// 4.84 / 13.23.
-// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.4 -> 4.7, 4096x12288 K4 13.8 -> 12.7, 151936x4096 K4
-// 131 -> 105 (5.9e12 weights a second, 20 per cycle and SM).
+// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.4 -> 4.7, 4096x12288 K4 13.8 -> 12.6, 151936x4096 K4
+// 131 -> 106 (5.9e12 weights a second, 20 per cycle and SM).
+// Range.  A transformed activation beyond 2^46 overflows under the factor 2^80, and where all of a row lie below 2^-56 the products sink into the
+// subnormals.  Both show in the sums of a row block: then all 128 are infinite, or all below 2^-33.  The barrier before the epilogue votes
+// on that (the only cost to other rows: half a per cent), and such a row block is summed again by the finishers alone, slowly and
+// without the factor (gemv1_any_range), so that the range of the results is that of packed_gemv.cuh.  Looking at the activations instead costs
+// launches of the usual range 1 to 4 %: a vote at the barrier before the decode, votes of the staging warps and a second run of the
+// thread block under another factor, a scan of the staged row by the finishers.
 #pragma once
 #include "packed_gemv.cuh"
 
@@ -33,18 +32,12 @@ namespace htr {
 constexpr int kG1DecodeWarps = 16, kG1FinishWarps = 4, kG1Warps = kG1DecodeWarps + kG1FinishWarps, kG1Threads = kG1Warps * 32;
 constexpr int kG1Alu = 2;                                    // byte sums of four that go to the shift/logic pipe (1, 3, 4: 2 to 3 % slower)
 constexpr int kG1MaxCols = 16384;                            // staged activations of a row: 64 KB
-constexpr int kG1Up = 80;                                    // activations are staged times 2^80 ...
-constexpr float kG1Least = 1.4551915e-11f, kG1Most = 6.871948e10f;   // ... where the largest is in [2^-36, 2^36): transformed within 2^-40 .. 2^40
-__device__ __forceinline__ float power_of_two(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
-
-struct G1Shared {
-  float red[2][kG1DecodeWarps][64];                          // sums of a row block: [buffer][decode warp][its 64 rows]
-  float ytil[128];
-  float ss[kG1Warps];
-  unsigned range[kG1Warps];                                  // of what a warp has staged: 1 = a value of at least kG1Most, 2 = of kG1Least, 4 = not zero
-  unsigned top[kG1Warps];                                    // gemv1_wide: its largest, as bits of a float
-  int arrival;
-};
+constexpr float kG1Up = 1.2089258196146292e24f;              // 2^80: staged activations
+constexpr float kG1Down = 1.6940658945086007e-21f;           // 2^-69 = 2^80 * 2^-149: unit of the accumulators
+constexpr float kG1Out = 5.902958103587057e20f;              // 2^69
+// A sum of at least this shows that its activations kept their bits: one of them, transformed, is then at least 2^-33 / (16384 columns * 510
+// * 1.1) = 2^-56, and products near that are rounded at 2^-80, 2^-24 of the largest.
+constexpr float kG1Least = 1.1641532e-10f;                   // 2^-33
 
 template <int K>
 struct G1Ring {
@@ -85,13 +78,81 @@ __device__ __forceinline__ void unit_fma_subnormal(const uint32_t (&V)[K + 1], c
   }
 }
 
-// The work of a thread block; true (for all its threads) where the activations are out of the usual range and nothing was delivered.
-// WIDE: the second run, under a power of two made for them.
-template <int K, bool WIDE>
-__device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
+// barrier of the finishers; true where any of them brings true
+__device__ __forceinline__ bool finishers_any(bool mine) {
+  int any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %1, 0;\n\tbar.red.or.pred p, 5, %2, q;\n\tselp.s32 %0, 1, 0, p;\n\t}"
+               : "=r"(any)
+               : "r"((int)mine), "n"(kG1FinishWarps * 32)
+               : "memory");
+  return any != 0;
+}
+
+// The sum of row r of row block rb over all its columns, by the finishers alone and without the factor 2^80: for activations whose sums
+// left the range of the fast form (see Range above).  Four 128-column blocks at a time; f holds their transformed activations.
+template <int K>
+static __device__ __noinline__ float gemv1_any_range(const GemvParams& p, float (*f)[128], int rb, int r) {
+  const int nt = p.nt, n = nt * 16, HB = nt >> 3, lane = r & 31, fw = r >> 5, q = (r & 15) >> 1;
+  float ss = 0.f;
+  bool some = false;                                         // (a row of zeros ends here: its sums are zeros as they are)
+  for (int col = 4 * r; col < n; col += 4 * kG1FinishWarps * 32) {
+    const float4 v = load_x(p.x, 0, col, p.n_in, p.dtype);
+    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    some = some || v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f;
+  }
+  if (!finishers_any(some)) return 0.f;
+  float inv = 0.f;
+  if (p.prologue == 1) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(kFullWarp, ss, o);
+    if (lane == 0) f[0][fw] = ss;
+    named_sync<5, kG1FinishWarps * 32>();
+    inv = rsqrtf((f[0][0] + f[0][1] + f[0][2] + f[0][3]) / (float)n + p.eps);
+    named_sync<5, kG1FinishWarps * 32>();
+  }
+  const uint32_t* strip = p.qw + (size_t)(rb * 8 + (r >> 4)) * nt * (8 * K);
+  float sum = 0.f;
+#pragma unroll 1
+  for (int first = 0; first < HB; first += kG1FinishWarps) {
+    const int hb = first + fw, col = hb * 128 + 4 * lane;
+    if (hb < HB) {
+      float4 x4 = load_x(p.x, 0, col, p.n_in, p.dtype);
+      if (p.prologue == 1) x4 = norm_x(x4, __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(p.norm_w) + col)), inv);
+      const unsigned sg = sign_nibble(p.su, hb * 32 + lane);
+      float v[4] = {flip(x4.x, sg & 1u), flip(x4.y, (sg >> 1) & 1u), flip(x4.z, (sg >> 2) & 1u), flip(x4.w, sg >> 3)};
+      wht128(v, lane);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) f[fw][4 * lane + k] = v[k] * kInvSqrt128;
+    }
+    named_sync<5, kG1FinishWarps * 32>();
+#pragma unroll 1
+    for (int tile = 0; tile < 8 * min(kG1FinishWarps, HB - first); ++tile) {
+      uint32_t V[K + 1], s[32];
+      read_unit_words<K>(strip + (size_t)(first * 8 + tile) * (8 * K), q, V);
+      unit_states<K>(V, s);
+      float part = 0.f;
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        const uint32_t h = (r & 1 ? s[16 + c] : s[c]) * kGenMul + kGenAdd;
+        part += (float)((int)bytesum_add(h, 0u) - 510) * f[tile >> 3][(tile & 7) * 16 + c];
+      }
+      sum += part;
+    }
+    named_sync<5, kG1FinishWarps * 32>();
+  }
+  return sum;
+}
+
+template <int K>
+__global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __grid_constant__ GemvParams p) {
   using Ring = G1Ring<K>;
   constexpr int kTileBytes = Ring::tile_bytes, kSlotBytes = Ring::slot_bytes, R = Ring::slots;
   extern __shared__ __align__(128) unsigned char dyn_smem[];
+  __shared__ __align__(16) float s_red[2][kG1DecodeWarps][64];   // sums of a row block: [buffer][decode warp][its 64 rows]
+  __shared__ __align__(16) float ytil[128];
+  __shared__ float s_ss[kG1Warps];
+  __shared__ int s_arrival;
+  __shared__ __align__(16) float s_any[kG1FinishWarps][128];   // gemv1_any_range
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nt = p.nt, n = nt * 16, HB = nt >> 3;
   const EvenRuns runs((p.mt >> 3) * HB, gridDim.x);
@@ -143,8 +204,6 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  int shift = kG1Up;
-  auto scaled = [&](float f) { return WIDE ? f * power_of_two(shift >> 1) * power_of_two(shift - (shift >> 1)) : f * power_of_two(kG1Up); };
   auto stage = [&](int hb, unsigned sg, float4 x4) {
     float v[4] = {flip(x4.x, sg & 1u), flip(x4.y, (sg >> 1) & 1u), flip(x4.z, (sg >> 2) & 1u), flip(x4.w, sg >> 3)};
     wht128(v, lane);
@@ -152,13 +211,13 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
     float sum = 0.f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float f = scaled(v[k] * kInvSqrt128);
-      dst[staged_col<K>(4 * (lane & 3) + k)] = f;
+      const float f = v[k] * kInvSqrt128;
+      dst[staged_col<K>(4 * (lane & 3) + k)] = f * kG1Up;
       sum += f;
     }
     sum += __shfl_xor_sync(kFullWarp, sum, 1);
     sum += __shfl_xor_sync(kFullWarp, sum, 2);
-    if ((lane & 3) == 0) xoff[hb * 8 + (lane >> 2)] = sum * __uint_as_float(0x80000000u | 510u);   // -510 * 2^-149, the unit of the byte sums
+    if ((lane & 3) == 0) xoff[hb * 8 + (lane >> 2)] = -510.0f * sum * kG1Down;
   };
   float4 held[kHeld];                                        // every load of a warp is in flight before the first is used
   if (p.prologue == 1) {
@@ -170,11 +229,11 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
     for (int i = 0; i < kHeld; ++i) ss += held[i].x * held[i].x + held[i].y * held[i].y + held[i].z * held[i].z + held[i].w * held[i].w;
 #pragma unroll
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(kFullWarp, ss, o);
-    if (lane == 0) sh.ss[warp] = ss;
+    if (lane == 0) s_ss[warp] = ss;
     __syncthreads();
     float tot = 0.f;
 #pragma unroll
-    for (int k = 0; k < kG1Warps; ++k) tot += sh.ss[k];
+    for (int k = 0; k < kG1Warps; ++k) tot += s_ss[k];
     const float inv = rsqrtf(tot / (float)n + p.eps);
 #pragma unroll
     for (int i = 0; i < kHeld; ++i) held[i] = norm_x(held[i], gain[i], inv);
@@ -183,33 +242,10 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
     for (int i = 0; i < kHeld; ++i)
       if (warp + kG1Warps * i < count) held[i] = load_x(p.x, 0, block_at(i) * 128 + 4 * lane, p.n_in, p.dtype);
   }
-  float top = 0.f;
-  auto range = [&](float4 v) { top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); };
-  if constexpr (WIDE) {
-#pragma unroll
-    for (int i = 0; i < kHeld; ++i)
-      if (warp + kG1Warps * i < count) range(held[i]);
-    const unsigned own = __reduce_max_sync(kFullWarp, __float_as_uint(top));
-    if (lane == 0) sh.top[warp] = own;
-    __syncthreads();
-    // the largest activation to [2^96, 2^97), transformed at most 11.4 times that; -32 to 223
-    shift = 96 + 127 - (int)(__reduce_max_sync(kFullWarp, sh.top[lane < kG1Warps ? lane : 0]) >> 23);
-  }
 #pragma unroll
   for (int i = 0; i < kHeld; ++i)
-    if (warp + kG1Warps * i < count) {
-      if constexpr (!WIDE) range(held[i]);
-      stage(block_at(i), (signs[i] >> (4 * (lane & 1))) & 15u, held[i]);
-    }
-  if constexpr (!WIDE) {
-    const bool beyond = __any_sync(kFullWarp, top >= kG1Most), usual = __any_sync(kFullWarp, top >= kG1Least), some = __any_sync(kFullWarp, top > 0.f);
-    if (lane == 0) sh.range[warp] = (beyond ? 1u : 0u) | (usual ? 2u : 0u) | (some ? 4u : 0u);
-  }
+    if (warp + kG1Warps * i < count) stage(block_at(i), (signs[i] >> (4 * (lane & 1))) & 15u, held[i]);
   __syncthreads();
-  auto again = [&]() {                                       // all warps read the same words and decide alike
-    const unsigned all = __reduce_or_sync(kFullWarp, sh.range[lane < kG1Warps ? lane : 0]);
-    return !WIDE && ((all & 1u) != 0u || (all & 6u) == 4u);
-  };
 
   if (warp < kG1DecodeWarps) {
     float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -238,18 +274,17 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
       // ---- this warp's part of row block rb: leave it for the finishers (two buffers)
       const int buf = seg & 1;
       if (seg >= 2) named_sync_at(3 + buf, kG1Threads);
-      *reinterpret_cast<float2*>(&sh.red[buf][warp][g * 16 + 2 * q]) = make_float2(acc[0].x + acc[0].y, acc[1].x + acc[1].y);
+      *reinterpret_cast<float2*>(&s_red[buf][warp][g * 16 + 2 * q]) = make_float2(acc[0].x + acc[0].y, acc[1].x + acc[1].y);
       acc[0] = acc[1] = make_float2(0.f, 0.f);
       named_arrive_at(1 + buf, kG1Threads);
       start = stop;
     }
     async_wait<0>();
-    return again();
+    return;
   }
 
   // ---- finishers: thread r owns row r of the row block
   const int r = tid - kG1DecodeWarps * 32, segs = (u_end - 1) / HB - u_begin / HB + 1;
-  const bool drop = again();
   for (int seg = 0, start = u_begin; seg < segs; ++seg) {
     const int rb = start / HB, buf = seg & 1;
     const int first = runs.owner(rb * HB), contributors = runs.owner((rb + 1) * HB - 1) - first + 1;
@@ -263,10 +298,8 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
     named_sync_at(1 + buf, kG1Threads);
     float sum = 0.f;
 #pragma unroll
-    for (int w = 0; w < kG1DecodeWarps / 2; ++w) sum += sh.red[buf][2 * w + (r >> 6)][r & 63];
+    for (int w = 0; w < kG1DecodeWarps / 2; ++w) sum += s_red[buf][2 * w + (r >> 6)][r & 63];
     if (seg + 2 < segs) named_arrive_at(3 + buf, kG1Threads);
-    if (drop) continue;
-    sum = WIDE ? sum * power_of_two((149 - shift) >> 1) * power_of_two(149 - shift - ((149 - shift) >> 1)) : sum * power_of_two(149 - kG1Up);
     bool finish = true;
     if (contributors > 1) {
       // a thread block has two partials: its first row block's and that of a later one (only its last is read by others)
@@ -274,10 +307,10 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
       named_sync<5, kG1FinishWarps * 32>();
       if (r == 0) {
         __threadfence();                                     // the partials of the thread block (ordered by the barrier) before the arrival
-        sh.arrival = atomicAdd(p.counters + rb, 1);           // (they are read with loads served by L2, after this atomic)
+        s_arrival = atomicAdd(p.counters + rb, 1);           // (they are read with loads served by L2, after this atomic)
       }
       named_sync<5, kG1FinishWarps * 32>();
-      finish = sh.arrival == contributors - 1;
+      finish = s_arrival == contributors - 1;
       if (finish) {
         if (r == 0) p.counters[rb] = 0;
         const int head = runs.begin(first) < rb * HB ? 1 : 0;
@@ -293,11 +326,16 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
       }
     }
     if (!finish) continue;
-    sh.ytil[r] = sum;
-    named_sync<5, kG1FinishWarps * 32>();
+    sum *= kG1Out;
+    ytil[r] = sum;
+    if (!finishers_any(fabsf(sum) >= kG1Least && fabsf(sum) <= 3.402823466e38f)) {
+      sum = gemv1_any_range<K>(p, s_any, rb, r);
+      ytil[r] = sum;
+      named_sync<5, kG1FinishWarps * 32>();
+    }
     if (r < 32) {
       const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&sc_raw.y));
-      const float4 y4 = *reinterpret_cast<const float4*>(sh.ytil + 4 * lane);
+      const float4 y4 = *reinterpret_cast<const float4*>(ytil + 4 * lane);
       float v[4] = {y4.x * (s01.x * p.cb), y4.y * (s01.y * p.cb), y4.z * (s23.x * p.cb), y4.w * (s23.y * p.cb)};
       wht128(v, lane);
       float4 o = make_float4(flip(v[0] * kInvSqrt128, sv_bits & 1u) + bias4.x, flip(v[1] * kInvSqrt128, (sv_bits >> 1) & 1u) + bias4.y,
@@ -306,19 +344,6 @@ __device__ __forceinline__ bool gemv1_run(const GemvParams& p, G1Shared& sh) {
     }
     // (ytil is written again only behind the next barrier with the decode warps, which warp 0 reaches after this)
   }
-  return drop;
-}
-
-template <int K>
-__device__ __noinline__ void gemv1_wide(const GemvParams& p, G1Shared& sh) {
-  __syncthreads();                                           // the first run's words and sums have been read
-  gemv1_run<K, true>(p, sh);
-}
-
-template <int K>
-__global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __grid_constant__ GemvParams p) {
-  __shared__ __align__(16) G1Shared sh;
-  if (gemv1_run<K, false>(p, sh)) gemv1_wide<K>(p, sh);
 }
 
 // host side, defined once per K in packed_gemv_k*.cu
