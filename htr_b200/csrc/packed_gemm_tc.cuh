@@ -397,10 +397,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   }
   const int U = (GROUP ? tiles * p.rb_per_tile : p.mt >> 3) * HB;
   const EvenRuns runs(U, gridDim.x);
-  int u_begin, u_end, part_id = 0;
+  int u_begin, u_end;
   if (!GROUP && p.split > 0) {
-    const int rb = blockIdx.x / p.split;
-    part_id = blockIdx.x - rb * p.split;
+    const int rb = blockIdx.x / p.split, part_id = blockIdx.x - rb * p.split;
     u_begin = rb * HB + part_id * HB / p.split;
     u_end = rb * HB + (part_id + 1) * HB / p.split;
   } else {
@@ -445,7 +444,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   // cluster form: what a decode warp needs to finish its rows j0, j0 + split * DW, ... (at most sixteen) of the one row block
   GemmTail tail;
   float xs_of = 0.f, tok_of = 0.f;                          // lane i: activation sum and scale of the i-th of these rows
-  const int row_step = p.split * DW, row_first = part_id + p.split * warp;
   if (warp < DW) {
     // ================= decode warps
     const int quad = warp & 3, half = (warp >> 2) & 1, strip = 2 * quad + half, group = warp >> 3;
@@ -546,7 +544,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       // the thread block's partial [np][128], hi + lo added: four warps of a quadrant take alternate groups of 8 columns
       asm volatile("griddepcontrol.wait;" ::: "memory");
       tail.load<false>(p, blockIdx.x / p.split, lane);
-      const int j = row_first + lane * row_step;
+      const int j = (int)(blockIdx.x % p.split) + p.split * (warp + lane * DW);
       if (j < p.rows) {
         float part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 2
@@ -721,8 +719,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (warp < DW) {
       const uint32_t result_addr = smem_u32(result) + (uint32_t)lane * 16u;
-      for (int i = 0; row_first + i * row_step < p.rows; ++i) {
-        const int j = row_first + i * row_step;
+      const int row_first = (int)(blockIdx.x % p.split) + p.split * warp;
+      for (int i = 0; row_first + i * (p.split * DW) < p.rows; ++i) {
+        const int j = row_first + i * (p.split * DW);
         float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int r = 0; r < p.split; ++r) {
           uint32_t remote;
