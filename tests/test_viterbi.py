@@ -127,3 +127,41 @@ def test_tiles_shared_by_a_cluster_equal_tiles_of_one_block(K, B):
     assert torch.equal(got, want[:B]) and torch.equal(c, cost[:B])
     opened, _ = encoder.viterbi(x.to(dev), w.to(dev), None, K, tailbite=False, return_cost=True)
     assert torch.equal(encoder.viterbi(x[:B].to(dev), w[:B].to(dev), None, K, tailbite=False), opened[:B])
+
+
+@pytest.mark.parametrize("K", (2, 3, 4, 5, 6, 8))
+@pytest.mark.parametrize("T", (1, 2, 3, 4, 5, 6, 7, 8, 12, 13, 19, 255))
+def test_lengths_around_the_kept_rows(coracle, T, K):
+    """The traceback goes from kept row to kept row (every 1 to 6 steps): lengths that end at, before and behind one, with and without
+    the circle (which needs T*K >= 16 to close), negative weights among them."""
+    from htr_b200 import encoder
+
+    dev = torch.device("cuda:0")
+    x, w = tiles(3, T, 11 * T + K)
+    w[1, T // 2] *= -1.0
+    x[2] = torch.round(x[2])
+    w[2] = 1.0
+    for tailbite in (False, True) if T * K >= 16 else (False,):
+        want, want_cost = coracle.viterbi(x.numpy(), w.numpy(), K, tailbite=tailbite)
+        got, cost = encoder.viterbi(x.to(dev), w.to(dev), None, K, tailbite=tailbite, return_cost=True)
+        assert np.array_equal(got.cpu().numpy(), want)
+        assert np.array_equal(cost.cpu().numpy().view(np.uint32), want_cost.view(np.uint32))
+
+
+@pytest.mark.parametrize("K", (2, 3, 4, 5, 6, 8))
+@pytest.mark.parametrize("T", (256, 10))
+def test_two_tiles_of_a_block_equal_one(K, T):
+    """More tiles than SMs are searched in pairs, a lone one twice, the last few of a long call in a launch of their own: the same bits as
+    in calls of few tiles."""
+    from htr_b200 import encoder
+
+    dev = torch.device("cuda:0")
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    x, w = tiles(2 * sms + 9, T, 30 + K)
+    x, w = x.to(dev), w.to(dev)
+    for tailbite in (True, False):
+        few = [encoder.viterbi(x[b:b + 20], w[b:b + 20], None, K, tailbite=tailbite, return_cost=True) for b in range(0, x.shape[0], 20)]
+        want, cost = torch.cat([s for s, _ in few]), torch.cat([c for _, c in few])
+        for B in (sms + 1, 2 * sms, 2 * sms + 9):
+            got, c = encoder.viterbi(x[:B], w[:B], None, K, tailbite=tailbite, return_cost=True)
+            assert torch.equal(got, want[:B]) and torch.equal(c, cost[:B])
