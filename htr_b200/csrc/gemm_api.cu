@@ -10,10 +10,21 @@ namespace htr {
 // Output layout = the B operand tiles of the GEMM, one contiguous block per 128 columns of x:
 //   xb[64-column unit][column group g][k-group kc][column r][8 k]   column = g*8 + r: activation row (hi plane), np + row (lo plane)
 // with the k order of the A operand inside a unit (packed_gemm_tc.cuh): position 16 j + 4 c + e holds column 16 c + 4 j + e.
-// grid (np, slices): a CTA transforms one slice of one activation row (one 128-column block per warp and turn), after finding the
-// range of the whole row itself (every CTA of a row reads the row once, 16 bytes per load and all of them in flight; that is
-// cheaper than a second launch or a grid-wide exchange).  xsum[row][slice] holds the slice's sum, added up in slice order by the
-// GEMM's epilogue.  Rows beyond `rows` are written as zeros so that the padded batch is harmless; columns from n_in on read as zeros.
+// grid (rows, slices): a thread block transforms one slice of one activation row, after finding the range of the whole row itself (16
+// bytes per load; cheaper than an exchange between slices).  A warp takes four 128-column blocks at a time, eight lanes each, a lane the
+// 16 columns of one tile, so that four of the seven butterfly stages stay in a lane and a value crosses lanes three times (one block per
+// warp, four values a lane: five times, and shuffles pass 32 lanes a cycle and SM).  xsum[row][slice] holds the slice's sum, added up in
+// slice order by the GEMM's epilogue.  Columns from n_in on read as zeros; B columns of the padded batch that have no row stay as they
+// are: they reach only accumulator columns that nobody reads.
+//
+// What bounds it: latency -- of the wait for the kernel before it, of the row, of instructions that nobody has fetched yet (a kernel this
+// short runs every line once) -- and the stores, 16 bytes apart by the B layout, a line of L1 each.  So
+//  * the thread blocks, which are resident long before they may read x, go through the whole code once on zeros before the wait (`passes`
+//    = 2, nothing is loaded or stored), which brings it into the SM's instruction caches;
+//  * there are as many of them as fit on the few SMs that the GEMM before leaves free: clusters of the next GEMM waited for those that did not.
+// us for transform + GEMM in a chain (graph), 4096x12288 K3 4 rows / K5 16 rows / 12288x4096 K2 64 rows / 151936x4096 K4 8 rows / 4096x4000 K3
+// 11 rows: one block per warp in 12 / 12 / 4 / 4 / 4 slices of 256 threads 18.1 / 21.9 / 23.6 / 128.7 / 9.25; four per warp, 24 warps, one slice
+// 18.3 / 18.3 / 23.1 / 127.7 / 9.18, two 17.3 / 20.6 / 23.1 / 127.0 / 10.6, four 17.1 / 20.5 / 25.9 / 127.2 / 11.0.
 //
 // Range scale of a row: the power of two 2^k with max|x| * sqrt(128) in (2^13, 2^14] * 2^k, in both directions, so that neither a large
 // row leaves the fp16 range nor a small one sinks into its subnormals (fp16 numbers are 2^-24 apart below 2^-14: unscaled, a row of
@@ -26,102 +37,118 @@ __device__ __forceinline__ float range_scale(float mx) {
   return __uint_as_float(min(max(e, 127u - 120u), 127u + 118u) << 23);
 }
 
+constexpr int kRhtWarps = 24, kRhtMaxSlices = 4;
+
 template <int DT>
-__global__ void __launch_bounds__(256) rht_f16_kernel(const void* __restrict__ x, int rows, int np, int n, int n_in, int planes, int per,
-                                                      const uint8_t* __restrict__ su, __half* __restrict__ xb, float* __restrict__ xsum,
-                                                      float* __restrict__ tok) {
-  __shared__ float red[8];
+__global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ x, int np, int n, int n_in, int planes,
+                                                                 const uint8_t* __restrict__ su, __half* __restrict__ xb, float* __restrict__ xsum,
+                                                                 float* __restrict__ tok, int passes) {
+  __shared__ unsigned red_top[kRhtWarps];
+  __shared__ float red_sum[kRhtWarps];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the GEMM may start fetching packed words now
-  const int r = blockIdx.x, slice = blockIdx.y, slices = gridDim.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int blocks = n >> 7;
-  const int hb0 = slice * 8 * per + warp;                    // this warp's 128-column blocks: hb0, hb0 + 8, ... (`per` of them)
+  const int r = blockIdx.x, slice = blockIdx.y, slices = gridDim.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int blocks = n >> 7, groups = (blocks + 4 * slices - 1) / (4 * slices);   // of four blocks, in this slice
+  const int u = (lane >> 2) & 1, c = lane & 3;               // this lane's tile inside a block of a group
   const int ncols = np * planes;
-  const size_t unit_halves = (size_t)ncols * 64;
-  const size_t col_hi = (size_t)(r >> 3) * 512 + (r & 7) * 8, col_lo = (size_t)((np + r) >> 3) * 512 + ((np + r) & 7) * 8;
-  // four consecutive columns 4 lane .. + 3 of a block: tile c = (lane % 16) / 4, step j = lane % 4 of unit lane / 16
-  const int c = (lane & 15) >> 2, j = lane & 3;
-  const size_t in_unit = (size_t)(2 * j + (c >> 1)) * 64 + 4 * (c & 1);
-  auto tile_offset = [&](int hb) { return (size_t)(2 * hb + (lane >> 4)) * unit_halves + in_unit; };
-  const unsigned sg_first = hb0 < blocks ? sign_nibble(su, hb0 * 32 + lane) : 0u;   // the signs do not depend on earlier kernels
-  asm volatile("griddepcontrol.wait;" ::: "memory");         // x may come from the preceding kernel, the last GEMM may still read xb
-  if (r >= rows) {
-    for (int i = 0; i < per; ++i) {
-      const int hb = hb0 + 8 * i;
-      if (hb < blocks) {
-        *reinterpret_cast<uint2*>(xb + tile_offset(hb) + col_hi) = make_uint2(0u, 0u);
-        if (planes == 2) *reinterpret_cast<uint2*>(xb + tile_offset(hb) + col_lo) = make_uint2(0u, 0u);
+  // column 16 c + 4 j + e of unit u goes to position 16 j + 4 c + e
+  __half* const out = xb + (size_t)u * ncols * 64 + (size_t)(r >> 3) * 512 + (r & 7) * 8 + (c >> 1) * 64 + 4 * (c & 1);
+  const size_t to_lo = (size_t)(np >> 3) * 512;
+#pragma unroll 1
+  for (int pass = 0; pass < passes; ++pass) {
+    const bool real = pass + 1 == passes;
+    if (real) asm volatile("griddepcontrol.wait;" ::: "memory");     // x may come from the preceding kernel, the last GEMM may still read xb
+    // range of the whole row: magnitudes of floats compare like their bit patterns, so 16-bit pairs take the packed integer maximum
+    uint32_t top = 0u;
+    constexpr int kPer16 = DT == HTR_DTYPE_F32 ? 4 : 8;      // elements in 16 bytes
+    const uint4* row16 = reinterpret_cast<const uint4*>(static_cast<const char*>(x) + (size_t)r * n_in * (16 / kPer16));
+    const int scan = real ? n_in / kPer16 : 0;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < scan; e += blockDim.x) {
+      const uint4 v = __ldg(row16 + e);
+      if constexpr (DT == HTR_DTYPE_F32) {
+        constexpr uint32_t m = 0x7FFFFFFFu;
+        top = max(max(top, v.x & m), max(v.y & m, max(v.z & m, v.w & m)));
+      } else {
+        constexpr uint32_t m = 0x7FFF7FFFu;
+        top = __vmaxu2(__vmaxu2(top, v.x & m), __vmaxu2(v.y & m, __vmaxu2(v.z & m, v.w & m)));
       }
     }
-    if (tid == 0) {
-      xsum[(size_t)r * slices + slice] = 0.f;
-      if (slice == 0) tok[r] = 1.f;
-    }
-    return;
-  }
-  // this lane's values of its first block: the load is in flight beside those of the scan
-  auto values = [&](int hb) {
-    const int col = hb * 128 + 4 * lane;
-    return hb < blocks && col < n_in ? load_quad(x, (size_t)r * n_in + col, DT) : make_float4(0.f, 0.f, 0.f, 0.f);
-  };
-  const float4 first = values(hb0);
-  // range of the whole row: magnitudes of floats compare like their bit patterns, so 16-bit pairs take the packed integer maximum
-  uint32_t top = 0u;
-  constexpr int kPer16 = DT == HTR_DTYPE_F32 ? 4 : 8;        // elements in 16 bytes
-  const uint4* row16 = reinterpret_cast<const uint4*>(static_cast<const char*>(x) + (size_t)r * n_in * (16 / kPer16));
-#pragma unroll 8
-  for (int e = tid; e < n_in / kPer16; e += 256) {
-    const uint4 v = __ldg(row16 + e);
-    if constexpr (DT == HTR_DTYPE_F32) {
-      constexpr uint32_t m = 0x7FFFFFFFu;
-      top = max(max(top, v.x & m), max(v.y & m, max(v.z & m, v.w & m)));
-    } else {
-      constexpr uint32_t m = 0x7FFF7FFFu;
-      top = __vmaxu2(__vmaxu2(top, v.x & m), __vmaxu2(v.y & m, __vmaxu2(v.z & m, v.w & m)));
-    }
-  }
-  if constexpr (DT != HTR_DTYPE_F32) top = max(top >> 16, top & 0xFFFFu);
-  top = __reduce_max_sync(kFullWarp, top);
-  if (lane == 0) red[warp] = __uint_as_float(top);
-  __syncthreads();
+    if constexpr (DT != HTR_DTYPE_F32) top = max(top >> 16, top & 0xFFFFu);
+    top = __reduce_max_sync(kFullWarp, top);
+    if (lane == 0) red_top[warp] = top;
+    __syncthreads();
+    top = __reduce_max_sync(kFullWarp, lane < warps ? red_top[lane] : 0u);
+    float mx;
+    if constexpr (DT == HTR_DTYPE_F32) mx = __uint_as_float(top);
+    else if constexpr (DT == HTR_DTYPE_BF16) mx = __uint_as_float(top << 16);
+    else mx = __half2float(__ushort_as_half((unsigned short)top));
+    const float scale = range_scale(mx), inv = kInvSqrt128 / scale;
+    float sum = 0.f;
+#pragma unroll 1
+    for (int g = warp; g < groups; g += warps) {
+      const int hb = 4 * (slice * groups + g) + (lane >> 3);
+      float2 v[8];
+      const int col = hb * 128 + 64 * u + 16 * c;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) top = max(top, __float_as_uint(red[k]));
-  float mx;
-  if constexpr (DT == HTR_DTYPE_F32) mx = __uint_as_float(top);
-  else if constexpr (DT == HTR_DTYPE_BF16) mx = __uint_as_float(top << 16);
-  else mx = __half2float(__ushort_as_half((unsigned short)top));
-  const float scale = range_scale(mx);
-  if (tid == 0 && slice == 0) tok[r] = scale;
-  const float inv = kInvSqrt128 / scale;
-  float sum = 0.f;
-#pragma unroll 2
-  for (int i = 0; i < per; ++i) {
-    const int hb = hb0 + 8 * i;
-    if (hb >= blocks) break;                                 // warp-uniform: the shuffles inside stay converged
-    const float4 mine = i == 0 ? first : values(hb);         // (second touch: L1)
-    const unsigned sg = i == 0 ? sg_first : sign_nibble(su, hb * 32 + lane);
-    float v[4] = {flip(mine.x, sg & 1u), flip(mine.y, (sg >> 1) & 1u), flip(mine.z, (sg >> 2) & 1u), flip(mine.w, sg >> 3)};
-    wht128(v, lane);
-    __half hi[4], lo[4];
+      for (int h = 0; h < 4; ++h) {
+        const float4 q = real && hb < blocks && col + 4 * h < n_in ? load_quad(x, (size_t)r * n_in + col + 4 * h, DT) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[2 * h] = make_float2(q.x, q.y);
+        v[2 * h + 1] = make_float2(q.z, q.w);
+      }
+      const int byte = hb < blocks ? hb * 16 + 8 * u + 2 * c : 0;
+      const uint32_t signs = (uint32_t)su[byte] | ((uint32_t)su[byte + 1] << 8);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float t = v[k] * inv;
-      hi[k] = __float2half_rn(t);
-      lo[k] = __float2half_rn(t - __half2float(hi[k]));
-      sum += planes == 2 ? __half2float(hi[k]) + __half2float(lo[k]) : __half2float(hi[k]);   // exactly what the MMA will see
+      for (int i = 0; i < 8; ++i) v[i] = make_float2(flip(v[i].x, (signs >> (2 * i)) & 1u), flip(v[i].y, (signs >> (2 * i + 1)) & 1u));
+      const float2 minus = make_float2(-1.f, -1.f);
+#pragma unroll
+      for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (!(i & bit)) {
+            const float2 a = v[i], b = v[i | bit];
+            v[i] = __fadd2_rn(a, b);
+            v[i | bit] = __ffma2_rn(b, minus, a);                    // a - b, as rounded
+          }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = make_float2(v[i].x + v[i].y, v[i].x - v[i].y);
+#pragma unroll
+      for (int bit = 1; bit < 8; bit <<= 1) {
+        const float sgn = (lane & bit) ? -1.0f : 1.0f;               // the upper partner of a butterfly keeps (other - own)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          v[i] = make_float2(fmaf(sgn, v[i].x, __shfl_xor_sync(kFullWarp, v[i].x, bit)), fmaf(sgn, v[i].y, __shfl_xor_sync(kFullWarp, v[i].y, bit)));
+      }
+      __half* const at = out + (size_t)hb * ncols * 128;
+      const bool store = real && hb < blocks;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        __half2 hi[2], lo[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float2 t = __fmul2_rn(v[2 * j + e], make_float2(inv, inv));
+          hi[e] = __float22half2_rn(t);
+          const float2 back = __half22float2(hi[e]);
+          lo[e] = __float22half2_rn(__ffma2_rn(back, minus, t));
+          const float2 rest = __half22float2(lo[e]);
+          sum += planes == 2 ? (back.x + rest.x) + (back.y + rest.y) : back.x + back.y;   // exactly what the MMA will see
+        }
+        if (store) *reinterpret_cast<uint2*>(at + 128 * j) = *reinterpret_cast<const uint2*>(hi);
+        if (store && planes == 2) *reinterpret_cast<uint2*>(at + 128 * j + to_lo) = *reinterpret_cast<const uint2*>(lo);
+      }
     }
-    const size_t at = tile_offset(hb);
-    *reinterpret_cast<uint2*>(xb + at + col_hi) = *reinterpret_cast<const uint2*>(hi);
-    if (planes == 2) *reinterpret_cast<uint2*>(xb + at + col_lo) = *reinterpret_cast<const uint2*>(lo);
-  }
 #pragma unroll
-  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullWarp, sum, o);
-  __syncthreads();
-  if (lane == 0) red[warp] = sum;
-  __syncthreads();
-  if (tid == 0) {
-    float s = 0.f;
-    for (int k = 0; k < 8; ++k) s += red[k];
-    xsum[(size_t)r * slices + slice] = s;
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullWarp, sum, o);
+    if (lane == 0) red_sum[warp] = sum;
+    __syncthreads();
+    if (warp == 0) {
+      sum = lane < warps ? red_sum[lane] : 0.f;
+#pragma unroll
+      for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullWarp, sum, o);
+      if (real && lane == 0) {
+        xsum[(size_t)r * slices + slice] = sum;
+        if (slice == 0) tok[r] = scale;
+      }
+    }
   }
 }
 
@@ -294,26 +321,30 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
   return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// 128-column blocks per warp of the transform: one for small batches (most CTAs), more when the rows alone fill the GPU
-int gemm_rht_per(int np, int n) {
-  const int max_per = (n / 128 + 7) / 8;
-  int per = np / 48;
-  if (per < 1) per = 1;
-  return per > max_per ? max_per : per;
-}
-int gemm_rht_slices(int np, int n) {
-  const int per = gemm_rht_per(np, n);
-  return (n / 128 + 8 * per - 1) / (8 * per);
-}
+// Slices of a row, warps of a thread block, rounds of the transform before a GEMM of `grid` thread blocks.  With 64 registers a thread, an
+// SM holds one thread block of 24 warps, two of 16, four of 8; `idle` SMs are free while the GEMM before (most often the same) runs, and a
+// GEMM in clusters loses where the transform needs others.  Long rows take 24 warps whatever the number, short ones have work for 8.
+// us (slices x warps): 4096x12288 K5 16 rows 1x24 / 2x24 18.3 / 20.5; 8 rows 2x24 / 4x24 16.7 / 18.4; 64 rows 1x8 / 2x24 26.1 / 21.8; 4096x4096 K4
+// 32 rows 1x16 / 1x24 9.6 / 11.2, 64 rows 1x8 / 1x16 11.7 / 12.6; 14720x12544 K2 28 float32 rows 1x24 / 2x24 54.2 / 50.7.  Beyond 48 rows the round
+// on zeros costs more than it saves, because other thread blocks wait for the place (4096x12288 128 rows 24.8 / 23.5).
+struct RhtShape {
+  int slices, warps, passes;
+  RhtShape(int rows, int n, int grid, int sms) {
+    const int groups = (n + 511) / 512, idle = sms - grid;
+    warps = groups >= 9 ? (rows > 128 ? 16 : 24) : groups <= 4 || (idle >= 16 && rows > 2 * idle && rows <= 4 * idle) ? 8 : 16;
+    slices = groups < 8 ? 1 : idle >= rows ? (idle / rows < kRhtMaxSlices ? idle / rows : kRhtMaxSlices) : rows <= 16 || (rows <= 64 && groups >= 16) ? 2 : 1;
+    passes = rows > 48 ? 1 : 2;
+  }
+};
 
-int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
-                cudaStream_t st) {
-  const int per = gemm_rht_per(np, n);
-  const dim3 grid(np, gemm_rht_slices(np, n));
+int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const RhtShape& shape, const uint8_t* su, __half* xb,
+                float* xsum, float* tok, cudaStream_t st) {
+  const dim3 grid(rows, shape.slices);
+  const int threads = 32 * shape.warps;
   switch (dtype) {
-    case HTR_DTYPE_BF16: return launch_chained(rht_f16_kernel<HTR_DTYPE_BF16>, grid, 256, 0, st, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
-    case HTR_DTYPE_F16: return launch_chained(rht_f16_kernel<HTR_DTYPE_F16>, grid, 256, 0, st, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
-    default: return launch_chained(rht_f16_kernel<HTR_DTYPE_F32>, grid, 256, 0, st, x, rows, np, n, n_in, planes, per, su, xb, xsum, tok);
+    case HTR_DTYPE_BF16: return launch_chained(rht_f16_kernel<HTR_DTYPE_BF16>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, shape.passes);
+    case HTR_DTYPE_F16: return launch_chained(rht_f16_kernel<HTR_DTYPE_F16>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, shape.passes);
+    default: return launch_chained(rht_f16_kernel<HTR_DTYPE_F32>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, shape.passes);
   }
 }
 
@@ -426,7 +457,7 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   g.grid = g.split > 0 ? g.rbs * g.split : (int)flat_grid;
   size_t off = kCounterRegion + kErrorRegion;
   g.off_xb = off; off += align256((size_t)ncols * n * 2);
-  g.off_xsum = off; off += align256((size_t)g.np * gemm_rht_slices(g.np, n) * 4);
+  g.off_xsum = off; off += align256((size_t)g.np * kRhtMaxSlices * 4);
   g.off_tok = off; off += align256((size_t)g.np * 4);
   g.off_part = off;
   if (g.split == 0) off += align256((size_t)g.grid * 2 * g.np * 128 * 4);
@@ -527,13 +558,14 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   p.split = g.split;
   p.stages = g.stages;
   p.m_out = m_out;
-  p.xsum_slices = gemm_rht_slices(g.np, n);
+  const RhtShape shape(M, n, g.grid, g.sms);
+  p.xsum_slices = shape.slices;
   p.cb = (float)codebook_scale();
   p.plan = nullptr;
   p.npeer = npeer;
   p.peer_offset = peer_offset;
   for (int i = 0; i < 8; ++i) p.peer_y[i] = i < npeer ? peer_y[i] : nullptr;
-  int e = run_rht_f16(x, dtype, M, g.np, n, n_in, planes, su, reinterpret_cast<__half*>(ws + g.off_xb), reinterpret_cast<float*>(ws + g.off_xsum),
+  int e = run_rht_f16(x, dtype, M, g.np, n, n_in, planes, shape, su, reinterpret_cast<__half*>(ws + g.off_xb), reinterpret_cast<float*>(ws + g.off_xsum),
                       reinterpret_cast<float*>(ws + g.off_tok), st);
   if (e) { t_gemm_cuda = e; return HTR_ERR_CUDA; }
   e = launch_gemm(K, p, g.grid, g.smem, st);

@@ -765,9 +765,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   if (warp == DW + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem), "r"((uint32_t)kGemmTmemCols) : "memory");
 }
 
-int gemm_rht_slices(int np, int n);
-int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const uint8_t* su, __half* xb, float* xsum, float* tok,
-                cudaStream_t st);
 template <int K>
 int launch_packed_gemm_tc(const GemmParams& p, int grid, int smem, cudaStream_t st);   // p.plan set: the grouped form
 // clusters of `split` thread blocks that the GPU holds at once (0: none), for the cluster form of the plan

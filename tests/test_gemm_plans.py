@@ -105,3 +105,26 @@ def test_rows_of_one_row_block(coracle, K, m, n, rows):
         err = np.linalg.norm(y[:, few].float().cpu().numpy() - want, axis=1) / np.linalg.norm(want, axis=1)
         assert err.max() <= 4e-3, (M, int(err.argmax()), float(err.max()))
     assert all(c == 0 for c in ops.gemm_error_codes())
+
+
+@pytest.mark.parametrize("n", (128, 384, 512, 640, 2176, 4096, 4224, 8320, 16512))
+@pytest.mark.parametrize("m", (128, 19072))
+def test_activation_transform_shapes(coracle, m, n):
+    """Slices, warps and rounds of the activation transform change with the rows, the blocks of a row (four per warp and turn) and the SMs that
+    the GEMM leaves free: every form of it, rows at the edges, in the three types; rows of their own magnitude, so that a scale of another row shows."""
+    from htr_b200 import ops, wire
+
+    if m > 4096 and n > 640:
+        pytest.skip("a launch that fills the GPU takes the same shapes at fewer columns")
+    dev = torch.device("cuda:0")
+    qw, sc, su, sv = wire.random_packed(m, n, 3, seed=m + n)
+    d = [t.to(dev) for t in (qw, sc, su, sv)]
+    g = torch.Generator().manual_seed(n)
+    x = torch.randn(256, n, generator=g) * 2.0 ** torch.randint(-8, 8, (256, 1), generator=g)
+    ref = {dt: coracle.linear(x.to(dt).float().numpy(), qw[:8].numpy(), sc[:128].numpy(), su.numpy(), sv[:16].numpy()) for dt in (torch.bfloat16, torch.float32)}
+    for dt, tol, rows in ((torch.bfloat16, 4e-3, (5, 8, 9, 16, 17, 48, 49, 64, 65, 129, 256)), (torch.float32, 2e-4, (5, 17, 49, 128))):
+        for M in rows:
+            y = ops.linear(x[:M].to(dt).to(dev), *d)[:, :128].float().cpu().numpy()
+            err = np.linalg.norm(y - ref[dt][:M], axis=1) / np.linalg.norm(ref[dt][:M], axis=1)
+            assert err.max() <= tol, (dt, M, int(err.argmax()), float(err.max()))
+    assert all(c == 0 for c in ops.gemm_error_codes())
