@@ -355,7 +355,7 @@ constexpr size_t kCounterRegion = 1 << 16;   // same fixed counter region as the
 constexpr size_t kErrorRegion = 256;
 
 struct GemmPlan {
-  int np, rbs, hb, split, grid, stages, smem, sms;
+  int np, rbs, hb, split, grid, stages, smem, sms, inbox;
   size_t off_xb, off_xsum, off_tok, off_part, total;
 };
 
@@ -455,6 +455,22 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   const long long waves = (g.rbs + slots - 1) / slots;
   if (waves * (g.hb * unit + M / 30.0) + (waves - 1) * 4 < best) g.split = 1;
   g.grid = g.split > 0 ? g.rbs * g.split : (int)flat_grid;
+  // A cluster's partials are sent to the thread blocks that finish their rows where an inbox of np x 512 bytes fits beside the rings, with
+  // fewer stages of B if need be (a run needs no more than it has blocks).  us, fetched from where they were made / sent: 4096x12288 K3 4
+  // rows 17.1 / 16.6, 4096x4096 K4 32 rows 9.5 / 8.8, 2048x2048 K4 64 rows 8.3 / 7.4, 640x1024 K4 64 rows 7.4 / 6.6; but 768x384 K2 137 rows
+  // 8.6 / 9.4: a number sent is an instruction of its own, and at many rows they outweigh the barriers.
+  g.inbox = 0;
+  if (g.split > 1 && g.np <= 64) {
+    const int inbox_bytes = g.split * ((g.np + g.split - 1) / g.split) * 512, run = (g.hb + g.split - 1) / g.split, least = run < 2 ? 2 : run < 4 ? run : 4;
+    int stages = g.stages;
+    while (stages > least && gemm_smem_bytes(g.np, planes, stages, words) + inbox_bytes > budget) --stages;
+    const int smem = gemm_smem_bytes(g.np, planes, stages, words);
+    if (smem + inbox_bytes <= budget) {
+      g.stages = stages;
+      g.inbox = smem - 128;                                  // (behind the words; the last 128 bytes are for the alignment of the first)
+      g.smem = smem + inbox_bytes;
+    }
+  }
   size_t off = kCounterRegion + kErrorRegion;
   g.off_xb = off; off += align256((size_t)ncols * n * 2);
   g.off_xsum = off; off += align256((size_t)g.np * kRhtMaxSlices * 4);
@@ -556,6 +572,9 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   p.dtype = dtype;
   p.hb = g.hb;
   p.split = g.split;
+  p.run_q = g.split > 0 ? g.hb / g.split : g.rbs * g.hb / g.grid;
+  p.run_rem = g.split > 0 ? g.hb % g.split : g.rbs * g.hb % g.grid;
+  p.inbox = g.inbox;
   p.stages = g.stages;
   p.m_out = m_out;
   const RhtShape shape(M, n, g.grid, g.sms);

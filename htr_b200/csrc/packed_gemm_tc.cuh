@@ -87,6 +87,9 @@ struct GemmParams {
   int dtype;
   int hb;                 // 128-column blocks per row block (n / 128)
   int split;              // > 0: thread blocks per row block (cluster form); 0: flat ranges
+  int run_q, run_rem;     // blocks of a thread block's run (cluster form: of its part of the row block): run_q, one more for the first run_rem
+  int inbox;              // > 0: offset in shared memory where a thread block of a cluster receives the partial sums of its rows; 0: the
+                          // partials stay where they are and are fetched from there (many activation rows)
   int stages;
   int xsum_slices;
   float cb;
@@ -199,6 +202,15 @@ __device__ __forceinline__ void tmem_store_strip(uint32_t taddr, const uint32_t 
                "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
                "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                : "memory");
+}
+
+// one float to the same place in the shared memory of thread block `rank` of the cluster, counted in bytes on its mbarrier
+__device__ __forceinline__ void send_partial(uint32_t at, uint32_t bar, int rank, float v) {
+  asm volatile(
+      "{\n\t.reg .b32 a, b;\n\tmapa.shared::cluster.u32 a, %0, %2;\n\tmapa.shared::cluster.u32 b, %1, %2;\n\t"
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [a], %3, [b];\n\t}" ::"r"(at),
+      "r"(bar), "r"(rank), "f"(v)
+      : "memory");
 }
 
 // 8 consecutive accumulator columns of this thread's tensor-memory lane (complete after tcgen05.wait::ld)
@@ -379,7 +391,7 @@ __device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, in
 template <int K, bool GROUP>
 __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const GemmParams p) {
   extern __shared__ __align__(128) unsigned char gsm[];
-  __shared__ __align__(8) unsigned long long s_full[kGemmMaxStages], s_freed[kGemmMaxStages], s_done, s_drained;
+  __shared__ __align__(8) unsigned long long s_full[kGemmMaxStages], s_freed[kGemmMaxStages], s_done, s_drained, s_inbox;
   __shared__ uint32_t s_tmem;
   __shared__ int s_arrival;
   __shared__ int s_owed[kGemmFinishWarps];                  // row blocks below it have been delivered by the finisher warp
@@ -396,15 +408,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     tiles = group_tiles(p.plan);
   }
   const int U = (GROUP ? tiles * p.rb_per_tile : p.mt >> 3) * HB;
-  const EvenRuns runs(U, gridDim.x);
-  int u_begin, u_end;
+  EvenRuns runs(p.run_q, p.run_rem, 0);
+  if constexpr (GROUP) runs = EvenRuns(U, gridDim.x);
+  // first row block and first block in it of the run (cluster form: its only row block; divisions cost a start of cold instructions)
+  int rb0, hb0, part_id = 0, u_begin, u_end;
   if (!GROUP && p.split > 0) {
-    const int rb = blockIdx.x / p.split, part_id = blockIdx.x - rb * p.split;
-    u_begin = rb * HB + part_id * HB / p.split;
-    u_end = rb * HB + (part_id + 1) * HB / p.split;
+    rb0 = blockIdx.x;
+    if (p.split > 1) {
+      asm("mov.u32 %0, %%clusterid.x;" : "=r"(rb0));
+      asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(part_id));
+    }
+    hb0 = runs.begin(part_id);
+    u_begin = rb0 * HB + hb0;
+    u_end = rb0 * HB + runs.begin(part_id + 1);
   } else {
     u_begin = runs.begin(blockIdx.x);
     u_end = runs.begin(blockIdx.x + 1);
+    rb0 = u_begin / HB;
+    hb0 = u_begin - rb0 * HB;
   }
   if (GROUP && u_begin == u_end) return;                    // fewer blocks than thread blocks (an empty plan among others)
   const int b_tile_bytes = ncols * 256;
@@ -412,18 +433,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   const uint32_t ring_addr = smem_u32(ring);
   const int a_col = gemm_acc_cols(ncols);
 
-  if (tid == 0) {
-    for (int s = 0; s < kGemmMaxStages; ++s) {
-      mbar_init(smem_u32(&s_full[s]), kGemmGroupWarps + 1);             // the warps of the group that decodes the block, and the B
+  if (warp == 0) {
+    if (lane < kGemmMaxStages) {
+      mbar_init(smem_u32(&s_full[lane]), kGemmGroupWarps + 1);          // the warps of the group that decodes the block, and the B
                                                                         // lane's arrive.expect_tx (with the bytes of the tile)
-      mbar_init(smem_u32(&s_freed[s]), 1);                              // tcgen05.commit
+      mbar_init(smem_u32(&s_freed[lane]), 1);                           // tcgen05.commit
     }
-    mbar_init(smem_u32(&s_done), 1);                                    // tcgen05.commit: the MMAs of a row block have retired
-    mbar_init(smem_u32(&s_drained), kGemmFinishWarps);                  // one arrival per finisher warp: its accumulator has been read
-    s_fail = 0;
-    for (int i = 0; i < kGemmFinishWarps; ++i) s_owed[i] = u_begin / HB;
+    if (lane == 0) {
+      mbar_init(smem_u32(&s_done), 1);                                  // tcgen05.commit: the MMAs of a row block have retired
+      mbar_init(smem_u32(&s_drained), kGemmFinishWarps);                // one arrival per finisher warp: its accumulator has been read
+      mbar_init(smem_u32(&s_inbox), 1);                                 // the partial sums of this thread block's rows, from the whole cluster
+      s_fail = 0;
+      for (int i = 0; i < kGemmFinishWarps; ++i) s_owed[i] = rb0;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
+    if (!GROUP && p.inbox > 0 && lane == 0) mbar_expect_tx(smem_u32(&s_inbox), (uint32_t)(p.split * ((p.rows - part_id + p.split - 1) / p.split) * 512));
   }
+  if (!GROUP && p.inbox > 0) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (waited for before the first partial is sent)
   if (warp == DW + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"((uint32_t)kGemmTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -436,7 +463,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   if (!GROUP && warp == kGemmWarps - 1 && lane < 6) {
     // the row scales and signs of the first and the last row block are needed at the very end, in a chain of dependent loads:
     // bring them to L2 now (256 bytes of scales and 16 of signs per row block)
-    const size_t rb = lane & 1 ? (u_end - 1) / HB : u_begin / HB;
+    const size_t rb = lane & 1 ? (u_end - 1) / HB : rb0;
     const char* at = lane < 4 ? reinterpret_cast<const char*>(p.scales + rb * 128) + (lane >> 1) * 128 : reinterpret_cast<const char*>(p.sv + rb * 16);
     asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
   }
@@ -472,8 +499,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       return reinterpret_cast<const char*>(base) + (size_t)(rb * 8 + strip) * nt * (32 * K) + lane * 16;
     };
     {
-      const int u = u_begin + group, hb = u % HB;
-      pf_rb = u / HB;
+      int hb = hb0 + group;
+      pf_rb = rb0;
+      while (hb >= HB) { hb -= HB; ++pf_rb; }
       pf = strip_row(pf_rb) + (size_t)hb * (256 * K);
       pf_in_rb = HB - hb;
     }
@@ -543,8 +571,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       // these loads, and the wait for the transform that they need, lie beside the last MMAs; then the accumulator goes to the ring as
       // the thread block's partial [np][128], hi + lo added: four warps of a quadrant take alternate groups of 8 columns
       asm volatile("griddepcontrol.wait;" ::: "memory");
-      tail.load<false>(p, blockIdx.x / p.split, lane);
-      const int j = (int)(blockIdx.x % p.split) + p.split * (warp + lane * DW);
+      tail.load<false>(p, rb0, lane);
+      const int j = part_id + p.split * (warp + lane * DW);
       if (j < p.rows) {
         float part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 2
@@ -555,10 +583,29 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         tok_of = __ldcg(p.tok + j);
       }
       ok = ok && __all_sync(kFullWarp, mbar_wait(smem_u32(&s_done), 0u, &s_fail));
-      if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int li = lane & 15, row = 32 * quad + (lane & 16) + (li < 8 ? 2 * li : 2 * li - 15);   // weight row of this tensor-memory lane
-        const uint32_t acc_addr = s_tmem + ((uint32_t)(32 * quad) << 16);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int li = lane & 15, row = 32 * quad + (lane & 16) + (li < 8 ? 2 * li : 2 * li - 15);   // weight row of this tensor-memory lane
+      const uint32_t acc_addr = s_tmem + ((uint32_t)(32 * quad) << 16);
+      if (p.inbox > 0) {
+        const uint32_t inbox = smem_u32(ring) + (uint32_t)p.inbox, own_rows = (np + p.split - 1) / p.split;
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every thread block's inbox is ready
+        for (int j0 = 8 * (warp >> 2); j0 < np; j0 += 2 * DW) {
+          uint32_t hi[8], lo[8];
+          if (ok) {
+            tmem_load8(acc_addr + j0, hi);
+            if (p.planes == 2) tmem_load8(acc_addr + np + j0, lo);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          }
+          int index = j0 / p.split, owner = j0 - index * p.split;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            float v = p.planes == 2 ? __uint_as_float(hi[i]) + __uint_as_float(lo[i]) : __uint_as_float(hi[i]);
+            if (!ok) v = __uint_as_float(0x7FC00000u);       // a bounded wait gave up: NaN, so that the row carries it whoever finishes it
+            if (j0 + i < p.rows) send_partial(inbox + ((part_id * own_rows + index) * 128 + row) * 4, smem_u32(&s_inbox), owner, v);
+            if (++owner == p.split) { owner = 0; ++index; }
+          }
+        }
+      } else if (ok) {
         float* mine = reinterpret_cast<float*>(ring);
         for (int j0 = 8 * (warp >> 2); j0 < np; j0 += 2 * DW) {
           uint32_t hi[8], lo[8];
@@ -568,8 +615,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
 #pragma unroll
           for (int i = 0; i < 8; ++i) mine[(j0 + i) * 128 + row] = p.planes == 2 ? __uint_as_float(hi[i]) + __uint_as_float(lo[i]) : __uint_as_float(hi[i]);
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
     if (!ok) s_fail = 1;
   } else {
@@ -580,10 +627,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       // ================= B lane: one bulk copy per 128-column block (the activation transform wrote the tiles contiguously)
       if (elect_one()) {
         asm volatile("griddepcontrol.wait;" ::: "memory");  // the transformed activations come from the preceding kernel
-        int s = 0, issued = 0, hb = u_begin % HB;
-        int rb_left = GROUP ? p.rb_per_tile - (u_begin / HB) % p.rb_per_tile : 0;   // row blocks of this tile still to come, this one included
+        int s = 0, issued = 0, hb = hb0;
+        int rb_left = GROUP ? p.rb_per_tile - rb0 % p.rb_per_tile : 0;   // row blocks of this tile still to come, this one included
         const char* xb = reinterpret_cast<const char*>(p.xb);
-        if constexpr (GROUP) xb += (size_t)(u_begin / HB / p.rb_per_tile) * HB * b_tile_bytes;
+        if constexpr (GROUP) xb += (size_t)(rb0 / p.rb_per_tile) * HB * b_tile_bytes;
         uint32_t use = 0u;
         for (int u = u_begin; u < u_end; ++u) {
           if (use > 0 && !mbar_wait(smem_u32(&s_freed[s]), (use - 1u) & 1u, &s_fail, kSleepNs)) { s_fail = 1; break; }
@@ -617,7 +664,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         uint32_t ph = 0u;
         bool ok = true;
         for (int u = u_begin; u < u_end && ok; ++seg) {
-          const int stop = min(u_end, (u / HB + 1) * HB);
+          const int stop = min(u_end, (rb0 + seg + 1) * HB);
           if (seg > 0 && !mbar_wait(smem_u32(&s_drained), (uint32_t)(seg - 1) & 1u, &s_fail)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           uint32_t fresh = 0u;                               // 0: the first MMA of a row block overwrites the accumulator
@@ -653,7 +700,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       bool ok = true, predecessor_done = false;
       int seg = 0;
       for (int u = u_begin; u < u_end; ++seg) {
-        const int rb = u / HB, stop = (rb + 1) * HB;
+        const int rb = rb0 + seg, stop = (rb + 1) * HB;
         ok = __all_sync(kFullWarp, mbar_wait(smem_u32(&s_done), (uint32_t)seg & 1u, &s_fail, kSleepNs));
         if (s_fail) ok = false;
         if (!ok) s_fail = 1;
@@ -704,6 +751,33 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       if (!ok) s_fail = 1;
     }
     __syncwarp();
+    if (!GROUP && p.inbox > 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // (its arrival; complete long ago)
+  }
+  if (!GROUP && p.inbox > 0) {
+    // ---- reduction inside the cluster: every thread block has sent its partials of row j to thread block j % split, which adds them in rank
+    // order and finishes the row.  (Partials fetched from where they were made wait for a barrier of the cluster before and one after, so
+    // that nobody leaves too early, 1.5 us together.)
+    if (warp < DW) {
+      const bool here = __all_sync(kFullWarp, mbar_wait(smem_u32(&s_inbox), 0u, nullptr));
+      const int own_rows = (np + p.split - 1) / p.split, row_first = part_id + p.split * warp;
+      const float4* in = reinterpret_cast<const float4*>(ring + p.inbox) + lane;
+      for (int i = 0; row_first + i * (p.split * DW) < p.rows; ++i) {
+        float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int r = 0; r < p.split; ++r) {
+          const float4 v = in[(r * own_rows + warp + i * DW) * 32];
+          r4.x += v.x; r4.y += v.y; r4.z += v.z; r4.w += v.w;
+        }
+        if (!here) r4.x = r4.y = r4.z = r4.w = __uint_as_float(0x7FC00000u);
+        gemm_finish_row(p, tail, row_first + i * (p.split * DW), lane, r4, __shfl_sync(kFullWarp, xs_of, i), __shfl_sync(kFullWarp, tok_of, i));
+      }
+      if (!here) s_fail = 1;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid == 0 && s_fail) atomicCAS(p.error, 0, 1);
+    if (warp == DW + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem), "r"((uint32_t)kGemmTmemCols) : "memory");
+    return;
   }
   __syncthreads();
   const bool bad = s_fail != 0;
@@ -715,11 +789,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     float* result = reinterpret_cast<float*>(ring);
     if (bad)                                                 // a bounded wait gave up: the rows come out as NaN, beside the error word
       for (int e = tid; e < np * 128; e += kGemmThreads) result[e] = __uint_as_float(0x7FC00000u);
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (p.split > 1) {
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else if (bad) {
+      __syncthreads();
+    }
     if (warp < DW) {
       const uint32_t result_addr = smem_u32(result) + (uint32_t)lane * 16u;
-      const int row_first = (int)(blockIdx.x % p.split) + p.split * warp;
+      const int row_first = part_id + p.split * warp;
       for (int i = 0; row_first + i * (p.split * DW) < p.rows; ++i) {
         const int j = row_first + i * (p.split * DW);
         float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -733,8 +811,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         gemm_finish_row(p, tail, j, lane, r4, __shfl_sync(kFullWarp, xs_of, i), __shfl_sync(kFullWarp, tok_of, i));
       }
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // nobody leaves while its shared memory may still be read
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (p.split > 1) {                                       // nobody leaves while its shared memory may still be read
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
   } else {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int rb = (u_end - 1) / HB;

@@ -122,7 +122,7 @@ def test_activation_transform_shapes(coracle, m, n):
     g = torch.Generator().manual_seed(n)
     x = torch.randn(256, n, generator=g) * 2.0 ** torch.randint(-8, 8, (256, 1), generator=g)
     ref = {dt: coracle.linear(x.to(dt).float().numpy(), qw[:8].numpy(), sc[:128].numpy(), su.numpy(), sv[:16].numpy()) for dt in (torch.bfloat16, torch.float32)}
-    for dt, tol, rows in ((torch.bfloat16, 4e-3, (5, 8, 9, 16, 17, 48, 49, 64, 65, 129, 256)), (torch.float32, 2e-4, (5, 17, 49, 128))):
+    for dt, tol, rows in ((torch.bfloat16, 4e-3, (5, 8, 9, 16, 17, 48, 49, 64, 65, 129, 256)), (torch.float32, 5e-5, (5, 17, 49, 128))):
         for M in rows:
             y = ops.linear(x[:M].to(dt).to(dev), *d)[:, :128].float().cpu().numpy()
             err = np.linalg.norm(y - ref[dt][:M], axis=1) / np.linalg.norm(ref[dt][:M], axis=1)
