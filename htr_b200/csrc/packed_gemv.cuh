@@ -103,7 +103,21 @@ struct GemvParams {
   int g_table_rows;  // rows of the four tables: a route entry outside [0, g_table_rows) skips its problem like a null weight pointer
   int g_xdiv;
   long long g_xrow_bytes, g_yrow_bytes;
+  // Quotients without divisions (filled in by the launchers).  Flat form: units / grid, units % grid, ceil(2^32 / grid), grid / units and
+  // 1 / cg; one-row kernel of a chain: blocks of a run (one more in the first run_rem) and ceil(2^32 / blocks per row block)
+  int run_q, run_rem;
+  unsigned grid_magic, hb_magic;
+  float per_unit, per_cg;
 };
+inline unsigned reciprocal(int divisor) { return divisor > 1 ? (unsigned)((0x100000000ull + divisor - 1) / divisor) : 0u; }
+// the fields of p that FlatRuns needs, for a launch of `grid` thread blocks in the flat form
+inline void set_flat_runs(GemvParams& p, int grid) {
+  p.run_q = p.units / grid;
+  p.run_rem = p.units % grid;
+  p.grid_magic = reciprocal(grid);
+  p.per_unit = (float)grid / (float)p.units;
+  p.per_cg = 1.0f / (float)p.cg;
+}
 
 // Called by every thread of the block that has just stored the output rows of a row block into the peers' buffers.
 __device__ __forceinline__ void signal_peers_when_last(const GemvParams& p, int* counters, int row_blocks) {
@@ -153,6 +167,29 @@ __device__ __forceinline__ float4 fused_x(const GemvParams& p, const void* x, in
 
 // owner CTA of unit x when CTA b starts at floor(b*U/G)
 __device__ __host__ inline int unit_owner(long long x, long long G, long long U) { return (int)(((x + 1) * G - 1) / U); }
+// The same without a division, which is dozens of cold instructions (64 bits: a subroutine) at the start of every thread block and
+// between its last sum and its partial.  Quotients come as the upper product with ceil(2^32 / divisor), exact while dividend times divisor
+// stays below 2^32 (here less than grid^3; 0 stands for the divisor 1), or from a float32 guess that is then corrected.
+__device__ __forceinline__ int quotient(int x, unsigned magic) { return magic ? (int)__umulhi((unsigned)x, magic) : x; }
+__device__ __forceinline__ int quotient(int x, int divisor, float reciprocal) {
+  int q = (int)((float)x * reciprocal);
+  while (q * divisor > x) --q;
+  while (x - q * divisor >= divisor) ++q;
+  return q;
+}
+struct FlatRuns {
+  int q, rem;             // U / G, U % G
+  unsigned grid_magic;
+  float per_unit;         // G / U
+  __device__ __forceinline__ explicit FlatRuns(const GemvParams& p) : q(p.run_q), rem(p.run_rem), grid_magic(p.grid_magic), per_unit(p.per_unit) {}
+  __device__ __forceinline__ int begin(int b) const { return b * q + quotient(b * rem, grid_magic); }
+  __device__ __forceinline__ int owner(int x) const {
+    int b = (int)(((float)x + 0.5f) * per_unit);
+    while (begin(b) > x) --b;
+    while (begin(b + 1) <= x) ++b;
+    return b;
+  }
+};
 
 
 __device__ __forceinline__ void async_copy16(uint32_t smem_addr, const void* gptr) {
@@ -273,17 +310,18 @@ __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1))
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int h = warp & 1, c = warp >> 1, g = lane >> 3, q = lane & 7;
-  const int U = p.units, G = gridDim.x, CG = p.cg, nt = p.nt, n = nt * 16, m = p.mt * 16;
+  const int CG = p.cg, nt = p.nt, n = nt * 16, m = p.mt * 16;
   // split form: grid (split, row blocks), the parts of a row block differ by at most one unit; flat form: even unit ranges
   int u_begin, u_end, slot_index;
+  const FlatRuns runs(p);
   if (p.split > 0) {
     const int part = blockIdx.x, base = blockIdx.y * CG;
     u_begin = base + part * p.cg_quot + min(part, p.cg_rem);
     u_end = u_begin + p.cg_quot + (part < p.cg_rem ? 1 : 0);
     slot_index = part;
   } else {
-    u_begin = (int)((long long)blockIdx.x * U / G);
-    u_end = (int)(((long long)blockIdx.x + 1) * U / G);
+    u_begin = runs.begin(blockIdx.x);
+    u_end = runs.begin(blockIdx.x + 1);
     slot_index = 0;                                     // found per row block below
   }
   constexpr int kTileWords = 8 * K, kTileBytes = 32 * K, kTileChunks = 2 * K;    // 16-byte chunks per tile
@@ -294,7 +332,7 @@ __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1))
   const uint32_t* my_ring = ring + (warp * 8 + g) * kTileWords;
   const uint32_t ring_dst = (uint32_t)__cvta_generic_to_shared(my_ring) + q * 16;
 
-  int rb = p.split > 0 ? (int)blockIdx.y : u_begin / CG;
+  int rb = p.split > 0 ? (int)blockIdx.y : quotient(u_begin, CG, p.per_cg);
   int cgi = u_begin - rb * CG;
 
   // tensors of this CTA's problem (grouped form: one row block per CTA, so they never change inside a launch)
@@ -495,8 +533,8 @@ __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1))
     if (p.split > 0) {
       contributors = p.split;
     } else {
-      const int first = unit_owner((long long)rb * CG, G, U);
-      contributors = unit_owner((long long)(rb + 1) * CG - 1, G, U) - first + 1;
+      const int first = runs.owner(rb * CG);
+      contributors = runs.owner((rb + 1) * CG - 1) - first + 1;
       slot_index = blockIdx.x - first;
     }
     float* ytil = smem + 4 * MT * 128;                  // [MT][128], disjoint from red (MT*kStageCols >= 5*MT*128)

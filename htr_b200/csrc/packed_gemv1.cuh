@@ -16,8 +16,13 @@
 //  * a weight costs half an instruction less: its byte sum, as the bits of a float, is a subnormal number (n * 2^-149 exactly), and
 //    multiplied with activations staged times 2^80 it needs neither a magic constant nor its subtraction.  The constant 510 goes in
 //    per 16 columns, as -510 times their sum added to the accumulator first, so that the sums stay centred (no cancellation at the end).
-// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.4 -> 4.7, 4096x12288 K4 13.8 -> 12.6, 151936x4096 K4
-// 131 -> 106 (5.9e12 weights a second, 20 per cycle and SM).
+// Every launch runs its code from cold instruction caches, so that what stands on the way to the first loads and behind the wait costs more
+// than its instructions: run boundaries need no division (host, or the reciprocal of the blocks per row block), and the staging is
+// compiled for one, two, five and seven blocks a warp instead of seven with most of them skipped (1024x4096 K4 4.65 -> 4.13, 4096x12288
+// K4 12.7 -> 12.4, 1024x2048 K3 4.15 -> 3.63 us).  A round on zeros before the wait, as in the activation transform of the GEMM,
+// was slower here (4.65 -> 6.5): a thread block starts when its SM is free, shortly before the wait ends.
+// us per launch in a chain, bf16, packed_gemv.cuh -> here: 1024x4096 K4 6.4 -> 4.1, 4096x12288 K4 13.8 -> 12.4, 151936x4096 K4
+// 131 -> 105 (5.9e12 weights a second, 20 per cycle and SM).
 // Range.  A transformed activation beyond 2^46 overflows under the factor 2^80, and where all of a row lie below 2^-56 the products sink into the
 // subnormals.  Both show in the sums of a row block: then all 128 are infinite, or all below 2^-33.  The barrier before the epilogue votes
 // on that (the only cost to other rows: half a per cent), and such a row block is summed again by the finishers alone, slowly and
@@ -143,7 +148,8 @@ static __device__ __noinline__ float gemv1_any_range(const GemvParams& p, float 
   return sum;
 }
 
-template <int K>
+// HELD: 128-column blocks of activations that a warp stages at most
+template <int K, int HELD>
 __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __grid_constant__ GemvParams p) {
   using Ring = G1Ring<K>;
   constexpr int kTileBytes = Ring::tile_bytes, kSlotBytes = Ring::slot_bytes, R = Ring::slots;
@@ -155,8 +161,11 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __gri
   __shared__ __align__(16) float s_any[kG1FinishWarps][128];   // gemv1_any_range
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nt = p.nt, n = nt * 16, HB = nt >> 3;
-  const EvenRuns runs((p.mt >> 3) * HB, gridDim.x);
+  // (no divisions on the way to the first loads: a few dozen cold instructions each)
+  const EvenRuns runs(p.run_q, p.run_rem, 0);
   const int u_begin = runs.begin(blockIdx.x), u_end = runs.begin(blockIdx.x + 1);
+  const auto row_block = [&](int u) { return p.hb_magic ? (int)__umulhi((unsigned)u, p.hb_magic) : u; };
+  const int rb0 = row_block(u_begin), hb0 = u_begin - rb0 * HB;
   float* xs = reinterpret_cast<float*>(dyn_smem + Ring::bytes);  // [n] staged activations, by column
   float* xoff = xs + n;                                          // [n / 16] offset of every tile
 
@@ -177,8 +186,9 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __gri
     async_commit();
   };
   if (warp < kG1DecodeWarps) {
-    const int u = u_begin + group, rb = u / HB, hb = u - rb * HB;
-    pf_left = max(u_end - u, 0);
+    const bool next = hb0 + group >= HB;                     // (HB = 1: the second group begins in the next row block)
+    const int rb = rb0 + (next ? 1 : 0), hb = next ? 0 : hb0 + group;
+    pf_left = max(u_end - u_begin - group, 0);
     pf_in_rb = HB - hb;
     pf = reinterpret_cast<const char*>(p.qw) + ((size_t)(rb * 8 + 4 * h + g) * nt + (size_t)hb * 8 + c) * kTileBytes + q * 16;
 #pragma unroll
@@ -187,8 +197,8 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __gri
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // ---- activations of every column this thread block meets: `count` blocks from its first one on, around the end of the row.
   // A warp takes every 20th; signs and norm weights do not depend on the preceding kernel and are fetched before the wait
-  constexpr int kHeld = (kG1MaxCols / 128 + kG1Warps - 1) / kG1Warps;
-  const int hb0 = u_begin % HB, count = min(u_end - u_begin, HB);
+  constexpr int kHeld = HELD;
+  const int count = min(u_end - u_begin, HB);
   auto block_at = [&](int i) { const int hb = hb0 + warp + kG1Warps * i; return hb >= HB ? hb - HB : hb; };
   unsigned signs[kHeld];
   uint2 gain[kHeld];
@@ -252,7 +262,7 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __gri
     uint32_t at = 0u, refill = (R - 1) * kSlotBytes;         // ring slots of this trip and of the one before it
     int seg = 0, u = u_begin + group;
     for (int start = u_begin; start < u_end; ++seg) {
-      const int rb = start / HB, stop = min(u_end, (rb + 1) * HB);
+      const int rb = rb0 + seg, stop = min(u_end, (rb + 1) * HB);
       const float* xt = xs + (u - rb * HB) * 128 + c * 16;
       const float* ot = xoff + (u - rb * HB) * 8 + c;
 #pragma unroll 1
@@ -284,11 +294,10 @@ __global__ void __launch_bounds__(kG1Threads, 1) packed_gemv1_kernel(const __gri
   }
 
   // ---- finishers: thread r owns row r of the row block
-  const int r = tid - kG1DecodeWarps * 32, segs = (u_end - 1) / HB - u_begin / HB + 1;
-  for (int seg = 0, start = u_begin; seg < segs; ++seg) {
-    const int rb = start / HB, buf = seg & 1;
+  const int r = tid - kG1DecodeWarps * 32, segs = row_block(u_end - 1) - rb0 + 1;
+  for (int seg = 0; seg < segs; ++seg) {
+    const int rb = rb0 + seg, buf = seg & 1;
     const int first = runs.owner(rb * HB), contributors = runs.owner((rb + 1) * HB - 1) - first + 1;
-    start = (rb + 1) * HB;
     // operands of the epilogue are fetched now so that their latency hides behind the hand-over
     const int row0 = rb * 128 + 4 * lane;
     const uint2 sc_raw = __ldg(reinterpret_cast<const uint2*>(p.scales + row0));

@@ -31,7 +31,9 @@ static int launch_one(const GemvParams& p, int grid, cudaStream_t stream) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = gemv_overlap_enabled() ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, packed_gemv_kernel<K, MT, DEP>, p);
+  GemvParams q = p;
+  if (p.split == 0) set_flat_runs(q, grid);
+  return (int)cudaLaunchKernelEx(&cfg, packed_gemv_kernel<K, MT, DEP>, q);
 }
 
 template <int K, int MT>
@@ -55,13 +57,13 @@ int launch_packed_gemv<HTR_INST_K>(const GemvParams& p, int mt_rows, int grid, c
   return (int)cudaErrorInvalidValue;
 }
 
-template <>
-int launch_packed_gemv1<HTR_INST_K>(const GemvParams& p, int grid, cudaStream_t stream) {
+template <int HELD>
+static int launch_gemv1(const GemvParams& p, int grid, cudaStream_t stream) {
   static bool allowed[64] = {false};                      // shared memory beyond 48 KB: opted in once per device
   int dev = 0;
   if (const cudaError_t e = cudaGetDevice(&dev)) return (int)e;
   if (dev < 0 || dev >= 64 || !allowed[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(packed_gemv1_kernel<HTR_INST_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemv1_smem_bytes<HTR_INST_K>(kG1MaxCols));
+    const cudaError_t e = cudaFuncSetAttribute(packed_gemv1_kernel<HTR_INST_K, HELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemv1_smem_bytes<HTR_INST_K>(kG1MaxCols));
     if (e != cudaSuccess) return (int)e;
     if (dev >= 0 && dev < 64) allowed[dev] = true;
   }
@@ -75,7 +77,22 @@ int launch_packed_gemv1<HTR_INST_K>(const GemvParams& p, int grid, cudaStream_t 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = gemv_overlap_enabled() ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, packed_gemv1_kernel<HTR_INST_K>, p);
+  GemvParams q = p;
+  const int hb = p.nt >> 3, units = (p.mt >> 3) * hb;
+  q.run_q = units / grid;
+  q.run_rem = units % grid;
+  q.hb_magic = reciprocal(hb);
+  return (int)cudaLaunchKernelEx(&cfg, packed_gemv1_kernel<HTR_INST_K, HELD>, q);
+}
+
+template <>
+int launch_packed_gemv1<HTR_INST_K>(const GemvParams& p, int grid, cudaStream_t stream) {
+  constexpr int kColsOfOne = kG1Warps * 128;
+  const int n = p.nt * 16;
+  if (n <= kColsOfOne) return launch_gemv1<1>(p, grid, stream);
+  if (n <= 2 * kColsOfOne) return launch_gemv1<2>(p, grid, stream);
+  if (n <= 5 * kColsOfOne) return launch_gemv1<5>(p, grid, stream);
+  return launch_gemv1<(kG1MaxCols + kColsOfOne - 1) / kColsOfOne>(p, grid, stream);
 }
 
 template <>

@@ -65,3 +65,26 @@ def test_one_row_of_any_magnitude(coracle, m, n, dtype, tol):
         xs = x.clone()
         xs[0, 17] = bad
         assert not bool(torch.isfinite(ops.linear(xs.to(dtype).to(dev), *d)).any())
+
+
+@pytest.mark.parametrize("n", (512, 2560, 2688, 5120, 5248, 12800, 12928))
+@pytest.mark.parametrize("m", (2048, 4864))
+def test_one_row_at_the_widths_where_the_staging_changes(coracle, m, n):
+    """A warp stages one, two, five or seven blocks of the row at most, and runs begin anywhere in a row block (their boundaries come from
+    a multiplication with the reciprocal)."""
+    from htr_b200 import ops, wire
+
+    dev = torch.device("cuda:0")
+    qw, sc, su, sv = wire.random_packed(m, n, 3, seed=m + n)
+    d = [t.to(dev) for t in (qw, sc, su, sv)]
+    x = torch.randn(1, n, generator=torch.Generator().manual_seed(n))
+    ref = coracle.linear(x.numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy())
+    assert rel(ops.linear(x.to(dev), *d).cpu().numpy(), ref) <= 5e-6
+
+
+def test_run_boundaries_by_reciprocal():
+    """The quotient by the blocks of a row block, as the launcher and the kernel form it, over everything that a workspace admits."""
+    for hb in list(range(2, 129)):
+        magic = (2 ** 32 + hb - 1) // hb
+        u = np.unique(np.concatenate([np.arange(0, 4 * hb), np.arange(1, 16385) * hb - 1, np.arange(1, 16385) * hb])).astype(np.uint64)
+        assert np.array_equal((u * np.uint64(magic)) >> np.uint64(32), u // np.uint64(hb))
