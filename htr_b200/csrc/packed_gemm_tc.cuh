@@ -391,7 +391,7 @@ __device__ __forceinline__ void gemm_finish_flat(const GemmParams& p, int rb, in
 template <int K, bool GROUP>
 __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const GemmParams p) {
   extern __shared__ __align__(128) unsigned char gsm[];
-  __shared__ __align__(8) unsigned long long s_full[kGemmMaxStages], s_freed[kGemmMaxStages], s_done, s_drained, s_inbox;
+  __shared__ __align__(8) unsigned long long s_full[kGemmMaxStages], s_freed[kGemmMaxStages], s_done, s_drained, s_inbox, s_nobody;
   __shared__ uint32_t s_tmem;
   __shared__ int s_arrival;
   __shared__ int s_owed[kGemmFinishWarps];                  // row blocks below it have been delivered by the finisher warp
@@ -442,6 +442,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     if (lane == 0) {
       mbar_init(smem_u32(&s_done), 1);                                  // tcgen05.commit: the MMAs of a row block have retired
       mbar_init(smem_u32(&s_drained), kGemmFinishWarps);                // one arrival per finisher warp: its accumulator has been read
+      if (GROUP) mbar_init(smem_u32(&s_nobody), DW);                    // before the first block of a warp
       mbar_init(smem_u32(&s_inbox), 1);                                 // the partial sums of this thread block's rows, from the whole cluster
       s_fail = 0;
       for (int i = 0; i < kGemmFinishWarps; ++i) s_owed[i] = rb0;
@@ -538,6 +539,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     uint32_t at = 0u, refill = (R - 1) * Ring::slot_bytes;  // ring slots of this block and of the one before it
     int stage = group;
     uint32_t parity = 1u;                                   // of freed[stage]: passes at once on the first round
+    // A stage is told of when its stores have landed: behind the second one, or (experts) half a block later, while the next block is decoded.
+    // The wait leaves issue slots empty, but the MMAs lose half a block at every boundary of row blocks: us, at once / later, 16 tokens
+    // on 64 experts 272 / 268, 4096x12288 K3 4 rows 16.6 / 16.2, but 12288x4096 K2 64 rows 22.9 / 23.2, 151936x4096 K4 8 rows 127.3 / 127.9
+    // (and choosing at run time costs 2 % by itself).
+    uint32_t stored = GROUP ? smem_u32(&s_nobody) : 0u;     // full[] of the stage stored last
+    auto deliver = [&](uint32_t to) {
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(to);
+    };
     bool ok = true;
 #pragma unroll 1
     for (int left = u_end - u_begin - group; left > 0; left -= 2) {
@@ -550,6 +562,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       uint32_t V[K], w[16];
       read_own_words<K>(blk, c, g, V);
       decode_unit<K>(V, lane, w);
+      if constexpr (GROUP) deliver(stored);
       // the MMAs that read this stage NS blocks ago must have retired
       const uint32_t bar = smem_u32(&s_freed[0]) + 8u * stage;
       if (!__all_sync(kFullWarp, mbar_try(bar, parity, 1000u)) && !__all_sync(kFullWarp, mbar_wait_slow(bar, parity, &s_fail, 0u))) { ok = false; break; }
@@ -558,14 +571,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       read_own_words<K>(blk + 128 * K, c, g, V);
       decode_unit<K>(V, lane, w);
       tmem_store_strip(a_addr + 64 * stage + 32, w);
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_full[0]) + 8u * stage);
+      if constexpr (GROUP) stored = smem_u32(&s_full[0]) + 8u * stage;
+      else deliver(smem_u32(&s_full[0]) + 8u * stage);
       const bool around = stage + 2 >= NS;
       stage += around ? 2 - NS : 2;
       parity ^= around ? 1u : 0u;
     }
+    if constexpr (GROUP) deliver(stored);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (!GROUP && p.split > 0) {
       // these loads, and the wait for the transform that they need, lie beside the last MMAs; then the accumulator goes to the ring as
