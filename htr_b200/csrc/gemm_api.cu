@@ -236,8 +236,10 @@ __global__ void __launch_bounds__(kGroupRhtWarps * 32) rht_group_kernel(const vo
                                                                         const int* __restrict__ plan, int cap, const uint8_t* const* su_table,
                                                                         __half* __restrict__ xb, float* __restrict__ xsum, float* __restrict__ tok) {
   __shared__ float red[kGroupRhtWarps];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // in this order: the GEMM behind this kernel starts when every thread block has come here, and then the plan, which an earlier kernel
+  // wrote, is complete, so that it can look up its experts and fetch their words while this kernel still works
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int pair = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blocks = n >> 7;
   const int slot = __ldcg(plan + group_plan_ints(cap) + pair);
   if (slot < 0) return;

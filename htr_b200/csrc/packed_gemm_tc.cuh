@@ -403,10 +403,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   const int np = p.np, ncols = p.planes * np;               // accumulator columns: hi plane, then lo plane if present
   const int nt = p.nt, HB = p.hb, NS = p.stages;
   int tiles = 1;
-  if constexpr (GROUP) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // the plan comes from an earlier kernel
-    tiles = group_tiles(p.plan);
-  }
+  if constexpr (GROUP) tiles = group_tiles(p.plan);         // (complete: the transform before this launch lets it start only then)
   const int U = (GROUP ? tiles * p.rb_per_tile : p.mt >> 3) * HB;
   EvenRuns runs(p.run_q, p.run_rem, 0);
   if constexpr (GROUP) runs = EvenRuns(U, gridDim.x);
