@@ -241,10 +241,8 @@ __global__ void __launch_bounds__(kGroupRhtWarps * 32) rht_group_kernel(const vo
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int pair = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blocks = n >> 7;
+  // the row does not depend on the plan: its loads go out beside the chain slot -> expert -> signs, whose end is needed behind the barrier only
   const int slot = __ldcg(plan + group_plan_ints(cap) + pair);
-  if (slot < 0) return;
-  const int t = slot / kGroupRows, r = slot % kGroupRows;
-  const uint8_t* su = su_table[group_expert(plan, cap, t)];
   const size_t row = (size_t)(pair / x_div) * x_stride;
   float v[kGroupRhtBlocks][4];
   float mx = 0.f;
@@ -261,6 +259,15 @@ __global__ void __launch_bounds__(kGroupRhtWarps * 32) rht_group_kernel(const vo
     }
     v[i][0] = q.x; v[i][1] = q.y; v[i][2] = q.z; v[i][3] = q.w;
     mx = fmaxf(mx, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
+  }
+  if (slot < 0) return;                                      // no expert here (the whole thread block)
+  const int t = slot / kGroupRows, r = slot % kGroupRows;
+  const uint8_t* su = su_table[group_expert(plan, cap, t)];
+  unsigned sg[kGroupRhtBlocks];
+#pragma unroll
+  for (int i = 0; i < kGroupRhtBlocks; ++i) {
+    const int hb = warp + kGroupRhtWarps * i;
+    sg[i] = hb < blocks ? sign_nibble(su, hb * 32 + lane) : 0u;
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFullWarp, mx, o));
@@ -280,9 +287,8 @@ __global__ void __launch_bounds__(kGroupRhtWarps * 32) rht_group_kernel(const vo
   for (int i = 0; i < kGroupRhtBlocks; ++i) {
     const int hb = warp + kGroupRhtWarps * i;
     if (hb >= blocks) break;                                 // warp-uniform
-    const unsigned sg = sign_nibble(su, hb * 32 + lane);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[i][k] = flip(v[i][k], (sg >> k) & 1u);
+    for (int k = 0; k < 4; ++k) v[i][k] = flip(v[i][k], (sg[i] >> k) & 1u);
     wht128(v[i], lane);
     __half hi[4], lo[4];
 #pragma unroll
