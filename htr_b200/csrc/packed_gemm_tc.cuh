@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   const uint32_t ring_addr = smem_u32(ring);
   const int a_col = gemm_acc_cols(ncols);
 
-  if (warp == 0) {
+  if (warp == kGemmWarps - 2) {                             // (not a warp whose first words are on the way)
     if (lane < kGemmMaxStages) {
       mbar_init(smem_u32(&s_full[lane]), kGemmGroupWarps + 1);          // the warps of the group that decodes the block, and the B
                                                                         // lane's arrive.expect_tx (with the bytes of the tile)
