@@ -13,8 +13,9 @@ namespace htr {
 // grid (rows, slices): a thread block transforms one slice of one activation row, after finding the range of the whole row itself (16
 // bytes per load; cheaper than an exchange between slices).  A warp takes four 128-column blocks at a time, eight lanes each, a lane the
 // 16 columns of one tile, so that four of the seven butterfly stages stay in a lane and a value crosses lanes three times (one block per
-// warp, four values a lane: five times, and shuffles pass 32 lanes a cycle and SM).  xsum[row][slice] holds the slice's sum, added up in
-// slice order by the GEMM's epilogue.  Columns from n_in on read as zeros; B columns of the padded batch that have no row stay as they
+// warp, four values a lane: five times, and shuffles pass 32 lanes a cycle and SM).  xsum[row][i] holds the sum of columns 1024 i and on.
+// Butterflies go from the lowest column bit to the highest, and sums are formed over four columns, the 32 fours of a block (halves, quarters,
+// ...) and the eight blocks one after another, whatever the grid: dozens of bf16 layers turn another order of these sums into percents.  Columns from n_in on read as zeros; B columns of the padded batch that have no row stay as they
 // are: they reach only accumulator columns that nobody reads.
 //
 // What bounds it: latency -- of the wait for the kernel before it, of the row, of instructions that nobody has fetched yet (a kernel this
@@ -37,17 +38,17 @@ __device__ __forceinline__ float range_scale(float mx) {
   return __uint_as_float(min(max(e, 127u - 120u), 127u + 118u) << 23);
 }
 
-constexpr int kRhtWarps = 24, kRhtMaxSlices = 4;
+constexpr int kRhtWarps = 24, kRhtMaxSlices = 4, kRhtBlocks = 512;   // (blocks of a slice: longer rows take more slices)
 
 template <int DT>
 __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ x, int np, int n, int n_in, int planes,
                                                                  const uint8_t* __restrict__ su, __half* __restrict__ xb, float* __restrict__ xsum,
                                                                  float* __restrict__ tok, int passes) {
   __shared__ unsigned red_top[kRhtWarps];
-  __shared__ float red_sum[kRhtWarps];
+  __shared__ float block_sum[kRhtBlocks];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the GEMM may start fetching packed words now
   const int r = blockIdx.x, slice = blockIdx.y, slices = gridDim.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int blocks = n >> 7, groups = (blocks + 4 * slices - 1) / (4 * slices);   // of four blocks, in this slice
+  const int blocks = n >> 7, groups = 2 * ((blocks + 8 * slices - 1) / (8 * slices));   // of four blocks, in this slice
   const int u = (lane >> 2) & 1, c = lane & 3;               // this lane's tile inside a block of a group
   const int ncols = np * planes;
   // column 16 c + 4 j + e of unit u goes to position 16 j + 4 c + e
@@ -83,7 +84,6 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
     else if constexpr (DT == HTR_DTYPE_BF16) mx = __uint_as_float(top << 16);
     else mx = __half2float(__ushort_as_half((unsigned short)top));
     const float scale = range_scale(mx), inv = kInvSqrt128 / scale;
-    float sum = 0.f;
 #pragma unroll 1
     for (int g = warp; g < groups; g += warps) {
       const int hb = 4 * (slice * groups + g) + (lane >> 3);
@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
       const uint32_t signs = (uint32_t)su[byte] | ((uint32_t)su[byte + 1] << 8);
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = make_float2(flip(v[i].x, (signs >> (2 * i)) & 1u), flip(v[i].y, (signs >> (2 * i + 1)) & 1u));
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = make_float2(v[i].x + v[i].y, v[i].x - v[i].y);
       const float2 minus = make_float2(-1.f, -1.f);
 #pragma unroll
       for (int bit = 1; bit < 8; bit <<= 1)
@@ -110,8 +112,6 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
             v[i | bit] = __ffma2_rn(b, minus, a);                    // a - b, as rounded
           }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = make_float2(v[i].x + v[i].y, v[i].x - v[i].y);
-#pragma unroll
       for (int bit = 1; bit < 8; bit <<= 1) {
         const float sgn = (lane & bit) ? -1.0f : 1.0f;               // the upper partner of a butterfly keeps (other - own)
 #pragma unroll
@@ -120,9 +120,11 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
       }
       __half* const at = out + (size_t)hb * ncols * 128;
       const bool store = real && hb < blocks;
+      float sum[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         __half2 hi[2], lo[2];
+        sum[j] = 0.f;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const float2 t = __fmul2_rn(v[2 * j + e], make_float2(inv, inv));
@@ -130,25 +132,33 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
           const float2 back = __half22float2(hi[e]);
           lo[e] = __float22half2_rn(__ffma2_rn(back, minus, t));
           const float2 rest = __half22float2(lo[e]);
-          sum += planes == 2 ? (back.x + rest.x) + (back.y + rest.y) : back.x + back.y;   // exactly what the MMA will see
+          sum[j] += planes == 2 ? back.x + rest.x : back.x;          // exactly what the MMA will see
+          sum[j] += planes == 2 ? back.y + rest.y : back.y;
         }
         if (store) *reinterpret_cast<uint2*>(at + 128 * j) = *reinterpret_cast<const uint2*>(hi);
         if (store && planes == 2) *reinterpret_cast<uint2*>(at + 128 * j + to_lo) = *reinterpret_cast<const uint2*>(lo);
       }
+      // the block's sum over its fours, index 4 w + j in lane w: bits 4 and 3 by an exchange of halves (a lane keeps what its own bit says),
+      // then bits 2, 1 and 0
+      const int w = lane & 7;
+      const bool upper = w & 4, second = w & 2;
+      float a = (upper ? sum[2] : sum[0]) + __shfl_xor_sync(kFullWarp, upper ? sum[0] : sum[2], 4);
+      const float b = (upper ? sum[3] : sum[1]) + __shfl_xor_sync(kFullWarp, upper ? sum[1] : sum[3], 4);
+      a = (second ? b : a) + __shfl_xor_sync(kFullWarp, second ? a : b, 2);
+      a += __shfl_xor_sync(kFullWarp, a, 1);
+      a += __shfl_xor_sync(kFullWarp, a, 4);
+      a += __shfl_xor_sync(kFullWarp, a, 2);
+      if (w == 0) block_sum[4 * g + (lane >> 3)] = a;
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullWarp, sum, o);
-    if (lane == 0) red_sum[warp] = sum;
     __syncthreads();
-    if (warp == 0) {
-      sum = lane < warps ? red_sum[lane] : 0.f;
+    for (int i = threadIdx.x; i < groups / 2; i += blockDim.x) {
+      float all = 0.f;
 #pragma unroll
-      for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullWarp, sum, o);
-      if (real && lane == 0) {
-        xsum[(size_t)r * slices + slice] = sum;
-        if (slice == 0) tok[r] = scale;
-      }
+      for (int k = 0; k < 8; ++k) all += block_sum[8 * i + k];
+      const int at = slice * (groups / 2) + i, count = (blocks + 7) >> 3;
+      if (real && at < count) xsum[(size_t)r * count + at] = all;
     }
+    if (real && slice == 0 && threadIdx.x == 0) tok[r] = scale;
   }
 }
 
@@ -329,6 +339,8 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
   return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+int gemm_xsums(int n) { return (n + 1023) / 1024; }            // sums that the transform leaves of a row
+
 // Slices of a row, warps of a thread block, rounds of the transform before a GEMM of `grid` thread blocks.  With 64 registers a thread, an
 // SM holds one thread block of 24 warps, two of 16, four of 8; `idle` SMs are free while the GEMM before (most often the same) runs, and a
 // GEMM in clusters loses where the transform needs others.  Long rows take 24 warps whatever the number, short ones have work for 8.
@@ -341,6 +353,7 @@ struct RhtShape {
     const int groups = (n + 511) / 512, idle = sms - grid;
     warps = groups >= 9 ? (rows > 128 ? 16 : 24) : groups <= 4 || (idle >= 16 && rows > 2 * idle && rows <= 4 * idle) ? 8 : 16;
     slices = groups < 8 ? 1 : idle >= rows ? (idle / rows < kRhtMaxSlices ? idle / rows : kRhtMaxSlices) : rows <= 16 || (rows <= 64 && groups >= 16) ? 2 : 1;
+    slices = max(slices, (n + 128 * kRhtBlocks - 1) / (128 * kRhtBlocks));
     passes = rows > 48 ? 1 : 2;
   }
 };
@@ -481,7 +494,7 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   }
   size_t off = kCounterRegion + kErrorRegion;
   g.off_xb = off; off += align256((size_t)ncols * n * 2);
-  g.off_xsum = off; off += align256((size_t)g.np * kRhtMaxSlices * 4);
+  g.off_xsum = off; off += align256((size_t)g.np * gemm_xsums(n) * 4);
   g.off_tok = off; off += align256((size_t)g.np * 4);
   g.off_part = off;
   if (g.split == 0) off += align256((size_t)g.grid * 2 * g.np * 128 * 4);
@@ -582,11 +595,12 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   p.split = g.split;
   p.run_q = g.split > 0 ? g.hb / g.split : g.rbs * g.hb / g.grid;
   p.run_rem = g.split > 0 ? g.hb % g.split : g.rbs * g.hb % g.grid;
+  p.part_magic = g.split > 0 ? (65536 + g.split - 1) / g.split : 0;
   p.inbox = g.inbox;
   p.stages = g.stages;
   p.m_out = m_out;
   const RhtShape shape(M, n, g.grid, g.sms);
-  p.xsum_slices = shape.slices;
+  p.xsum_slices = gemm_xsums(n);
   p.cb = (float)codebook_scale();
   p.plan = nullptr;
   p.npeer = npeer;

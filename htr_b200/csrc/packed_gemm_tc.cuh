@@ -38,11 +38,12 @@
 // their rows need (scales, signs, activation sums, lane i those of the i-th row) behind their last block, beside the last MMAs, move the
 // accumulator, four warps per quadrant, and finish.  With the finishers in their place a row waited for its own loads and 200 rows left
 // tensor memory one column group at a time.  us, before -> after: 32768x256, 8 / 200 rows 11.9 -> 10.0, 34.6 -> 24.8; 4096x4096, 8 / 256 rows
-// 9.9 -> 9.0, 25.9 -> 22.8; 2048x2048, 8 rows 7.5 -> 6.7; 4096x12288, 128 rows 27.5 -> 25.0.
+// 9.9 -> 9.0, 25.9 -> 22.8; 2048x2048, 8 rows 7.5 -> 6.7; 4096x12288, 128 rows 27.5 -> 25.0 (each before the inbox below).
 //
 // Decomposition.  Work = (row block) x (128-column blocks).  Where the row blocks are few, `split` thread blocks share one as a
-// cluster and reduce through distributed shared memory; else every thread block takes an even contiguous run that may cross row
-// blocks (flat), publishes a partial [np][128] per row block it touches, and the last arriver adds them in thread-block order.
+// cluster: each sends its partial sums of a row into the shared memory of the one that finishes that row (st.async, up to 64 rows), or,
+// where no inbox fits or the rows are many, fetches the others' between two cluster barriers.  4096x12288 K3, 4 rows: 17.1 -> 16.5 us for
+// the inbox.  Else every thread block takes an even contiguous run that may cross row blocks (flat), publishes a partial [np][128] per row block it touches, and the last arriver adds them in thread-block order.
 // Both are deterministic and nobody waits for another thread block except inside a cluster.  One thread block per SM, not two: the
 // partial sums of a row block are half as many, and no SM waits for the slower of two.
 //
@@ -87,7 +88,9 @@ struct GemmParams {
   int dtype;
   int hb;                 // 128-column blocks per row block (n / 128)
   int split;              // > 0: thread blocks per row block (cluster form); 0: flat ranges
-  int run_q, run_rem;     // blocks of a thread block's run (cluster form: of its part of the row block): run_q, one more for the first run_rem
+  int run_q, run_rem;     // blocks of a thread block's run: run_q, one more for the first run_rem (cluster form: hb / split and the remainder,
+                          // parts from block part * hb / split on)
+  int part_magic;         // 65536 / split, rounded up
   int inbox;              // > 0: offset in shared memory where a thread block of a cluster receives the partial sums of its rows; 0: the
                           // partials stay where they are and are fetched from there (many activation rows)
   int stages;
@@ -408,16 +411,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   EvenRuns runs(p.run_q, p.run_rem, 0);
   if constexpr (GROUP) runs = EvenRuns(U, gridDim.x);
   // first row block and first block in it of the run (cluster form: its only row block; divisions cost a start of cold instructions)
-  int rb0, hb0, part_id = 0, u_begin, u_end;
+  int rb0, hb0, part_id = 0, part = 0, u_begin, u_end;
   if (!GROUP && p.split > 0) {
     rb0 = blockIdx.x;
     if (p.split > 1) {
       asm("mov.u32 %0, %%clusterid.x;" : "=r"(rb0));
       asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(part_id));
     }
-    hb0 = runs.begin(part_id);
+    // part * HB / split, the quotient of the remainders by a reciprocal (exact: at most 16 * 15 by at most 16).  The last part is always one
+    // of the longer ones: it goes to the first thread block of the cluster, which starts first (2944x1664 K6, 37 rows: 8.3 -> 8.0 us)
+    part = p.split - 1 - part_id;
+    hb0 = part * p.run_q + ((part * p.run_rem * p.part_magic) >> 16);
     u_begin = rb0 * HB + hb0;
-    u_end = rb0 * HB + runs.begin(part_id + 1);
+    u_end = rb0 * HB + (part + 1) * p.run_q + (((part + 1) * p.run_rem * p.part_magic) >> 16);
   } else {
     u_begin = runs.begin(blockIdx.x);
     u_end = runs.begin(blockIdx.x + 1);
@@ -610,7 +616,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
           for (int i = 0; i < 8; ++i) {
             float v = p.planes == 2 ? __uint_as_float(hi[i]) + __uint_as_float(lo[i]) : __uint_as_float(hi[i]);
             if (!ok) v = __uint_as_float(0x7FC00000u);       // a bounded wait gave up: NaN, so that the row carries it whoever finishes it
-            if (j0 + i < p.rows) send_partial(inbox + ((part_id * own_rows + index) * 128 + row) * 4, smem_u32(&s_inbox), owner, v);
+            if (j0 + i < p.rows) send_partial(inbox + ((part * own_rows + index) * 128 + row) * 4, smem_u32(&s_inbox), owner, v);
             if (++owner == p.split) { owner = 0; ++index; }
           }
         }
@@ -763,11 +769,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     if (!GROUP && p.inbox > 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // (its arrival; complete long ago)
   }
   if (!GROUP && p.inbox > 0) {
-    // ---- reduction inside the cluster: every thread block has sent its partials of row j to thread block j % split, which adds them in rank
-    // order and finishes the row.  (Partials fetched from where they were made wait for a barrier of the cluster before and one after, so
+    // ---- reduction inside the cluster: every thread block has sent its partials of row j to thread block j % split, which adds them in the
+    // order of the parts and finishes the row.  (Partials fetched from where they were made wait for a barrier of the cluster before and one after, so
     // that nobody leaves too early, 1.5 us together.)
     if (warp < DW) {
-      const bool here = __all_sync(kFullWarp, mbar_wait(smem_u32(&s_inbox), 0u, nullptr));
+      // A peer whose own wait gave up still sends, but up to two of its limits later, and into shared memory that must not be gone by then.
+      bool here = mbar_wait(smem_u32(&s_inbox), 0u, nullptr);
+      for (int limit = 0; limit < 3 && !here; ++limit) here = mbar_wait(smem_u32(&s_inbox), 0u, nullptr);
+      here = __all_sync(kFullWarp, here);
       const int own_rows = (np + p.split - 1) / p.split, row_first = part_id + p.split * warp;
       const float4* in = reinterpret_cast<const float4*>(ring + p.inbox) + lane;
       for (int i = 0; row_first + i * (p.split * DW) < p.rows; ++i) {
@@ -794,7 +803,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
 
   if (!GROUP && p.split > 0) {
     // ---- split reduction inside the cluster: every thread block keeps its partial [np][128] where it is; thread block r of the
-    // cluster sums rows r, r + split, ... over all of them (in rank order) and finishes those rows itself
+    // cluster sums rows r, r + split, ... over all of them (in the order of the parts) and finishes those rows itself
     float* result = reinterpret_cast<float*>(ring);
     if (bad)                                                 // a bounded wait gave up: the rows come out as NaN, beside the error word
       for (int e = tid; e < np * 128; e += kGemmThreads) result[e] = __uint_as_float(0x7FC00000u);
@@ -812,7 +821,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int r = 0; r < p.split; ++r) {
           uint32_t remote;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(result_addr + (uint32_t)j * 512u), "r"(r));
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(result_addr + (uint32_t)j * 512u), "r"(p.split - 1 - r));
           float4 v;
           asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
           r4.x += v.x; r4.y += v.y; r4.z += v.z; r4.w += v.w;

@@ -128,3 +128,16 @@ def test_activation_transform_shapes(coracle, m, n):
             err = np.linalg.norm(y - ref[dt][:M], axis=1) / np.linalg.norm(ref[dt][:M], axis=1)
             assert err.max() <= tol, (dt, M, int(err.argmax()), float(err.max()))
     assert all(c == 0 for c in ops.gemm_error_codes())
+
+
+@pytest.mark.parametrize("n", (1664, 4096, 12288, 16512))
+@pytest.mark.parametrize("dtype,few,many", ((torch.bfloat16, 9, 16), (torch.bfloat16, 17, 32), (torch.bfloat16, 33, 48), (torch.float16, 49, 64), (torch.float32, 9, 16)))
+def test_rows_do_not_depend_on_the_shape_of_the_transform(n, dtype, few, many):
+    """The same plan of the GEMM (batches padded to the same size), but other slices of the activation transform: sums are formed in one order,
+    so that not a bit of a row changes."""
+    from htr_b200 import ops, wire
+
+    dev = torch.device("cuda:0")
+    w = [t.to(dev) for t in wire.random_packed(2048, n, 3, seed=n)]
+    x = torch.randn(many, n, generator=torch.Generator().manual_seed(n)).to(dtype).to(dev)
+    assert torch.equal(ops.linear(x, *w)[:few], ops.linear(x[:few], *w))
