@@ -60,10 +60,12 @@ __global__ void __launch_bounds__(256) rht_kernel(const void* __restrict__ x, in
 //            column bits and two tile bits as packed pairs (row 2q, row 2q+1), then the row bit;
 //   phase 2  thread = columns c, c + 64 of the 64 rows of one parity: the six row bits as packed pairs (c, c + 64), then the last
 //            column bit, signs, cast, store.
-// The exchange buffer swaps 16-byte groups by row pair so that both sides are free of bank conflicts.  16-bit results change
-// hands with the neighbour lane so that a store carries two adjacent columns.
-// Measured at 4096 x 12288 K4, bf16: 54 us, where one value per shuffle and shared-memory access with scalar stores took 108; issue
-// slots 52 % busy, a quarter of the stalls are instruction fetches of the unrolled body.
+// The exchange buffer swaps 16-byte groups by row pair so that both sides are free of bank conflicts.  A register of the 16-bit results holds
+// one column of two rows; the neighbour lane has the next column, and one shuffle and one byte permutation leave two adjacent columns of
+// one row in each, for one store (with a register of two columns of one row, two selections more per pair of values and half a shuffle less).
+// Measured, bf16: 4096 x 12288 K4 52.5 -> 48.1 us for that exchange, 28672 x 8192 K4 230 -> 208; one value per shuffle and shared-memory access
+// with scalar stores took 108.  A quarter of the stalls are instruction fetches of the unrolled body, so that instructions count twice.
+// Without gain: words of the next wave's blocks prefetched to L2, magic constants cancelled in the first butterfly (50 us).
 constexpr int kDqThreads = 128;
 constexpr int kDqSmem = 128 * 128 * 4;
 
@@ -87,10 +89,15 @@ __global__ void __launch_bounds__(kDqThreads, 3) dequant_w_kernel(const uint32_t
                                                                   const uint8_t* __restrict__ su, const uint8_t* __restrict__ sv, float cb,
                                                                   void* __restrict__ W, int nt) {
   extern __shared__ __align__(16) float blk[];               // [128][128], groups of four columns swapped by row pair
-  __shared__ __align__(16) uint32_t s_sign[128];             // sign mask of a row, rows of one parity together
+  __shared__ __align__(16) uint32_t s_sign[OUT == HTR_DTYPE_F32 ? 128 : 64];   // sign masks: of a row, or of two rows of one parity in halves
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cbk = blockIdx.x, rb = blockIdx.y, n = nt * 16;
-  s_sign[(tid & 1) * 64 + (tid >> 1)] = ((sv[rb * 16 + (tid >> 3)] >> (tid & 7)) & 1) ? 0x80008000u : 0u;
+  if constexpr (OUT == HTR_DTYPE_F32) {
+    s_sign[(tid & 1) * 64 + (tid >> 1)] = ((sv[rb * 16 + (tid >> 3)] >> (tid & 7)) & 1) << 31;
+  } else if (tid < 64) {                                     // rows 4 i + parity, 4 i + parity + 2
+    const unsigned b = sv[rb * 16 + ((tid & 31) >> 1)] >> (4 * (tid & 1) + (tid >> 5));
+    s_sign[tid] = ((b & 1) << 15) | ((b & 4) << 29);
+  }
   {
     const int q = lane & 7, half = (lane >> 3) & 1, strip = 2 * warp + (lane >> 4);
     const uint32_t* words = qw + ((size_t)(rb * 8 + strip) * nt + (size_t)(cbk * 8 + half * 4)) * (8 * K) + q * K;
@@ -158,43 +165,46 @@ __global__ void __launch_bounds__(kDqThreads, 3) dequant_w_kernel(const uint32_t
   dq_stage<64, 5>(v);
   const int gc = cbk * 128 + c;
   const uint32_t su0 = (su[gc >> 3] >> (gc & 7)) & 1u, su1 = (su[(gc + 64) >> 3] >> (gc & 7)) & 1u;
-  const uint32_t* masks = s_sign + parity * 64;
   const size_t row0 = (size_t)rb * 128 + parity;
+  if constexpr (OUT == HTR_DTYPE_F32) {
+    const uint32_t* masks = s_sign + parity * 64;
 #pragma unroll
-  for (int i = 0; i < 64; i += 4) {
-    const uint4 m4 = *reinterpret_cast<const uint4*>(masks + i);
-    const uint32_t m[4] = {m4.x, m4.y, m4.z, m4.w};
-    if constexpr (OUT == HTR_DTYPE_F32) {
+    for (int i = 0; i < 64; i += 4) {
+      const uint4 m4 = *reinterpret_cast<const uint4*>(masks + i);
+      const uint32_t m[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float2 a = v[i + k];
         float* dst = static_cast<float*>(W) + (row0 + 2 * (i + k)) * n + gc;
-        dst[0] = __uint_as_float(__float_as_uint(a.x + a.y) ^ ((m[k] & 0x80000000u) ^ (su0 << 31)));
-        dst[64] = __uint_as_float(__float_as_uint(a.x - a.y) ^ ((m[k] & 0x80000000u) ^ (su1 << 31)));
+        dst[0] = __uint_as_float(__float_as_uint(a.x + a.y) ^ (m[k] ^ (su0 << 31)));
+        dst[64] = __uint_as_float(__float_as_uint(a.x - a.y) ^ (m[k] ^ (su1 << 31)));
       }
-    } else {
-      const uint32_t flips = (su0 << 15) | (su1 << 31);
-      uint32_t w[4];                                         // columns c (low half) and c + 64 (high half)
+    }
+  } else {
+    // a register takes one column of two rows; the even lane stores the first row of its column and its neighbour's, the odd lane the second
+    const uint32_t* masks = s_sign + parity * 32;
+    const uint32_t flip0 = su0 * 0x80008000u, flip1 = su1 * 0x80008000u, pick = lane & 1 ? 0x3276u : 0x5410u;
+    uint16_t* dst = static_cast<uint16_t*>(W) + (row0 + 2 * (lane & 1)) * n + (gc & ~1);
+    const auto narrow = [](float lo, float hi) {
+      if constexpr (OUT == HTR_DTYPE_BF16) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&h);
+      } else {
+        const __half2 h = __floats2half2_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&h);
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < 64; i += 8) {
+      const uint4 m4 = *reinterpret_cast<const uint4*>(masks + i / 2);
+      const uint32_t m[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float2 a = v[i + k];
-        if constexpr (OUT == HTR_DTYPE_BF16) {
-          const __nv_bfloat162 h = __floats2bfloat162_rn(a.x + a.y, a.x - a.y);
-          w[k] = *reinterpret_cast<const uint32_t*>(&h) ^ m[k] ^ flips;
-        } else {
-          const __half2 h = __floats2half2_rn(a.x + a.y, a.x - a.y);
-          w[k] = *reinterpret_cast<const uint32_t*>(&h) ^ m[k] ^ flips;
-        }
-      }
-      const bool odd = lane & 1;
-#pragma unroll
-      for (int k = 0; k < 4; k += 2) {
-        // the even lane keeps row k and takes its neighbour's, the odd lane row k + 1
-        const uint32_t other = __shfl_xor_sync(kFullWarp, odd ? w[k] : w[k + 1], 1), mine = odd ? w[k + 1] : w[k];
-        const uint32_t left = odd ? other : mine, right = odd ? mine : other;
-        uint32_t* dst = reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(W) + (row0 + 2 * (i + k + (odd ? 1 : 0))) * n + (gc & ~1));
-        dst[0] = __byte_perm(left, right, 0x5410);
-        dst[32] = __byte_perm(left, right, 0x7632);
+        const float2 a = v[i + 2 * k], b = v[i + 2 * k + 1];
+        const uint32_t w0 = narrow(a.x + a.y, b.x + b.y) ^ m[k] ^ flip0, w1 = narrow(a.x - a.y, b.x - b.y) ^ m[k] ^ flip1;
+        uint32_t* at = reinterpret_cast<uint32_t*>(dst + (size_t)(2 * (i + 2 * k)) * n);
+        at[0] = __byte_perm(w0, __shfl_xor_sync(kFullWarp, w0, 1), pick);
+        at[32] = __byte_perm(w1, __shfl_xor_sync(kFullWarp, w1, 1), pick);
       }
     }
   }
