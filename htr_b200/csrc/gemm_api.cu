@@ -13,9 +13,9 @@ namespace htr {
 // grid (rows, slices): a thread block transforms one slice of one activation row, after finding the range of the whole row itself (16
 // bytes per load; cheaper than an exchange between slices).  A warp takes four 128-column blocks at a time, eight lanes each, a lane the
 // 16 columns of one tile, so that four of the seven butterfly stages stay in a lane and a value crosses lanes three times (one block per
-// warp, four values a lane: five times, and shuffles pass 32 lanes a cycle and SM).  xsum[row][i] holds the sum of columns 1024 i and on.
-// Butterflies go from the lowest column bit to the highest, and sums are formed over four columns, the 32 fours of a block (halves, quarters,
-// ...) and the eight blocks one after another, whatever the grid: dozens of bf16 layers turn another order of these sums into percents.  Columns from n_in on read as zeros; B columns of the padded batch that have no row stay as they
+// warp, four values a lane: five times, and shuffles pass 32 lanes a cycle and SM).  xsum[row][i] holds the sum of the i-th 8 `per`
+// blocks.  Butterflies go from the lowest column bit to the highest, and sums are formed over four columns of every eighth block, the 32 fours of
+// a block (halves, quarters, ...) and eight blocks one after another, whatever the grid: dozens of bf16 layers turn another order into percents.  Columns from n_in on read as zeros; B columns of the padded batch that have no row stay as they
 // are: they reach only accumulator columns that nobody reads.
 //
 // What bounds it: latency -- of the wait for the kernel before it, of the row, of instructions that nobody has fetched yet (a kernel this
@@ -43,12 +43,12 @@ constexpr int kRhtWarps = 24, kRhtMaxSlices = 4, kRhtBlocks = 512;   // (blocks 
 template <int DT>
 __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ x, int np, int n, int n_in, int planes,
                                                                  const uint8_t* __restrict__ su, __half* __restrict__ xb, float* __restrict__ xsum,
-                                                                 float* __restrict__ tok, int passes) {
+                                                                 float* __restrict__ tok, int per, int passes) {
   __shared__ unsigned red_top[kRhtWarps];
   __shared__ float block_sum[kRhtBlocks];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the GEMM may start fetching packed words now
   const int r = blockIdx.x, slice = blockIdx.y, slices = gridDim.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int blocks = n >> 7, groups = 2 * ((blocks + 8 * slices - 1) / (8 * slices));   // of four blocks, in this slice
+  const int blocks = n >> 7, sums = (blocks + 8 * per - 1) / (8 * per), own = (sums + slices - 1) / slices;   // sums of a row, of this slice
   const int u = (lane >> 2) & 1, c = lane & 3;               // this lane's tile inside a block of a group
   const int ncols = np * planes;
   // column 16 c + 4 j + e of unit u goes to position 16 j + 4 c + e
@@ -85,60 +85,62 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
     else mx = __half2float(__ushort_as_half((unsigned short)top));
     const float scale = range_scale(mx), inv = kInvSqrt128 / scale;
 #pragma unroll 1
-    for (int g = warp; g < groups; g += warps) {
-      const int hb = 4 * (slice * groups + g) + (lane >> 3);
-      float2 v[8];
-      const int col = hb * 128 + 64 * u + 16 * c;
+    for (int g = warp; g < 2 * own; g += warps) {            // half of the blocks of a sum: four of every eight
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int i8 = 0; i8 < per; ++i8) {
+        const int hb = 8 * (per * (slice * own + (g >> 1)) + i8) + 4 * (g & 1) + (lane >> 3);
+        float2 v[8];
+        const int col = hb * 128 + 64 * u + 16 * c;
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const float4 q = real && hb < blocks && col + 4 * h < n_in ? load_quad(x, (size_t)r * n_in + col + 4 * h, DT) : make_float4(0.f, 0.f, 0.f, 0.f);
-        v[2 * h] = make_float2(q.x, q.y);
-        v[2 * h + 1] = make_float2(q.z, q.w);
-      }
-      const int byte = hb < blocks ? hb * 16 + 8 * u + 2 * c : 0;
-      const uint32_t signs = (uint32_t)su[byte] | ((uint32_t)su[byte + 1] << 8);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = make_float2(flip(v[i].x, (signs >> (2 * i)) & 1u), flip(v[i].y, (signs >> (2 * i + 1)) & 1u));
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = make_float2(v[i].x + v[i].y, v[i].x - v[i].y);
-      const float2 minus = make_float2(-1.f, -1.f);
-#pragma unroll
-      for (int bit = 1; bit < 8; bit <<= 1)
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (!(i & bit)) {
-            const float2 a = v[i], b = v[i | bit];
-            v[i] = __fadd2_rn(a, b);
-            v[i | bit] = __ffma2_rn(b, minus, a);                    // a - b, as rounded
-          }
-#pragma unroll
-      for (int bit = 1; bit < 8; bit <<= 1) {
-        const float sgn = (lane & bit) ? -1.0f : 1.0f;               // the upper partner of a butterfly keeps (other - own)
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          v[i] = make_float2(fmaf(sgn, v[i].x, __shfl_xor_sync(kFullWarp, v[i].x, bit)), fmaf(sgn, v[i].y, __shfl_xor_sync(kFullWarp, v[i].y, bit)));
-      }
-      __half* const at = out + (size_t)hb * ncols * 128;
-      const bool store = real && hb < blocks;
-      float sum[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        __half2 hi[2], lo[2];
-        sum[j] = 0.f;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float2 t = __fmul2_rn(v[2 * j + e], make_float2(inv, inv));
-          hi[e] = __float22half2_rn(t);
-          const float2 back = __half22float2(hi[e]);
-          lo[e] = __float22half2_rn(__ffma2_rn(back, minus, t));
-          const float2 rest = __half22float2(lo[e]);
-          sum[j] += planes == 2 ? back.x + rest.x : back.x;          // exactly what the MMA will see
-          sum[j] += planes == 2 ? back.y + rest.y : back.y;
+        for (int h = 0; h < 4; ++h) {
+          const float4 q = real && hb < blocks && col + 4 * h < n_in ? load_quad(x, (size_t)r * n_in + col + 4 * h, DT) : make_float4(0.f, 0.f, 0.f, 0.f);
+          v[2 * h] = make_float2(q.x, q.y);
+          v[2 * h + 1] = make_float2(q.z, q.w);
         }
-        if (store) *reinterpret_cast<uint2*>(at + 128 * j) = *reinterpret_cast<const uint2*>(hi);
-        if (store && planes == 2) *reinterpret_cast<uint2*>(at + 128 * j + to_lo) = *reinterpret_cast<const uint2*>(lo);
+        const int byte = hb < blocks ? hb * 16 + 8 * u + 2 * c : 0;
+        const uint32_t signs = (uint32_t)su[byte] | ((uint32_t)su[byte + 1] << 8);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = make_float2(flip(v[i].x, (signs >> (2 * i)) & 1u), flip(v[i].y, (signs >> (2 * i + 1)) & 1u));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = make_float2(v[i].x + v[i].y, v[i].x - v[i].y);
+        const float2 minus = make_float2(-1.f, -1.f);
+#pragma unroll
+        for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (!(i & bit)) {
+              const float2 a = v[i], b = v[i | bit];
+              v[i] = __fadd2_rn(a, b);
+              v[i | bit] = __ffma2_rn(b, minus, a);                    // a - b, as rounded
+            }
+#pragma unroll
+        for (int bit = 1; bit < 8; bit <<= 1) {
+          const float sgn = (lane & bit) ? -1.0f : 1.0f;               // the upper partner of a butterfly keeps (other - own)
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            v[i] = make_float2(fmaf(sgn, v[i].x, __shfl_xor_sync(kFullWarp, v[i].x, bit)), fmaf(sgn, v[i].y, __shfl_xor_sync(kFullWarp, v[i].y, bit)));
+        }
+        __half* const at = out + (size_t)hb * ncols * 128;
+        const bool store = real && hb < blocks;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          __half2 hi[2], lo[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float2 t = __fmul2_rn(v[2 * j + e], make_float2(inv, inv));
+            hi[e] = __float22half2_rn(t);
+            const float2 back = __half22float2(hi[e]);
+            lo[e] = __float22half2_rn(__ffma2_rn(back, minus, t));
+            const float2 rest = __half22float2(lo[e]);
+            sum[j] += planes == 2 ? back.x + rest.x : back.x;          // exactly what the MMA will see
+            sum[j] += planes == 2 ? back.y + rest.y : back.y;
+          }
+          if (store) *reinterpret_cast<uint2*>(at + 128 * j) = *reinterpret_cast<const uint2*>(hi);
+          if (store && planes == 2) *reinterpret_cast<uint2*>(at + 128 * j + to_lo) = *reinterpret_cast<const uint2*>(lo);
+        }
       }
-      // the block's sum over its fours, index 4 w + j in lane w: bits 4 and 3 by an exchange of halves (a lane keeps what its own bit says),
+      // the sum over the fours of a block, index 4 w + j in lane w: bits 4 and 3 by an exchange of halves (a lane keeps what its own bit says),
       // then bits 2, 1 and 0
       const int w = lane & 7;
       const bool upper = w & 4, second = w & 2;
@@ -151,12 +153,12 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
       if (w == 0) block_sum[4 * g + (lane >> 3)] = a;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < groups / 2; i += blockDim.x) {
+    for (int i = threadIdx.x; i < own; i += blockDim.x) {
       float all = 0.f;
 #pragma unroll
       for (int k = 0; k < 8; ++k) all += block_sum[8 * i + k];
-      const int at = slice * (groups / 2) + i, count = (blocks + 7) >> 3;
-      if (real && at < count) xsum[(size_t)r * count + at] = all;
+      const int at = slice * own + i;
+      if (real && at < sums) xsum[(size_t)r * sums + at] = all;
     }
     if (real && slice == 0 && threadIdx.x == 0) tok[r] = scale;
   }
@@ -339,7 +341,9 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
   return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-int gemm_xsums(int n) { return (n + 1023) / 1024; }            // sums that the transform leaves of a row
+// blocks that a lane of the transform adds up one after another, and the sums that it leaves of a row
+int gemm_rht_per(int np, int n) { return min(max(np / 48, 1), (n + 1023) / 1024); }
+int gemm_xsums(int np, int n) { return (n / 128 + 8 * gemm_rht_per(np, n) - 1) / (8 * gemm_rht_per(np, n)); }
 
 // Slices of a row, warps of a thread block, rounds of the transform before a GEMM of `grid` thread blocks.  With 64 registers a thread, an
 // SM holds one thread block of 24 warps, two of 16, four of 8; `idle` SMs are free while the GEMM before (most often the same) runs, and a
@@ -363,9 +367,9 @@ int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int
   const dim3 grid(rows, shape.slices);
   const int threads = 32 * shape.warps;
   switch (dtype) {
-    case HTR_DTYPE_BF16: return launch_chained(rht_f16_kernel<HTR_DTYPE_BF16>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, shape.passes);
-    case HTR_DTYPE_F16: return launch_chained(rht_f16_kernel<HTR_DTYPE_F16>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, shape.passes);
-    default: return launch_chained(rht_f16_kernel<HTR_DTYPE_F32>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, shape.passes);
+    case HTR_DTYPE_BF16: return launch_chained(rht_f16_kernel<HTR_DTYPE_BF16>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, gemm_rht_per(np, n), shape.passes);
+    case HTR_DTYPE_F16: return launch_chained(rht_f16_kernel<HTR_DTYPE_F16>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, gemm_rht_per(np, n), shape.passes);
+    default: return launch_chained(rht_f16_kernel<HTR_DTYPE_F32>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, gemm_rht_per(np, n), shape.passes);
   }
 }
 
@@ -494,7 +498,7 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   }
   size_t off = kCounterRegion + kErrorRegion;
   g.off_xb = off; off += align256((size_t)ncols * n * 2);
-  g.off_xsum = off; off += align256((size_t)g.np * gemm_xsums(n) * 4);
+  g.off_xsum = off; off += align256((size_t)g.np * gemm_xsums(g.np, n) * 4);
   g.off_tok = off; off += align256((size_t)g.np * 4);
   g.off_part = off;
   if (g.split == 0) off += align256((size_t)g.grid * 2 * g.np * 128 * 4);
@@ -600,7 +604,7 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   p.stages = g.stages;
   p.m_out = m_out;
   const RhtShape shape(M, n, g.grid, g.sms);
-  p.xsum_slices = gemm_xsums(n);
+  p.xsum_slices = gemm_xsums(g.np, n);
   p.cb = (float)codebook_scale();
   p.plan = nullptr;
   p.npeer = npeer;
