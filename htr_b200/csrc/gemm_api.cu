@@ -351,13 +351,13 @@ int gemm_xsums(int np, int n) { return (n / 128 + 8 * gemm_rht_per(np, n) - 1) /
 // us (slices x warps): 4096x12288 K5 16 rows 1x24 / 2x24 18.3 / 20.5; 8 rows 2x24 / 4x24 16.7 / 18.4; 64 rows 1x8 / 2x24 26.1 / 21.8; 4096x4096 K4
 // 32 rows 1x16 / 1x24 9.6 / 11.2, 64 rows 1x8 / 1x16 11.7 / 12.6; 14720x12544 K2 28 float32 rows 1x24 / 2x24 54.2 / 50.7.  Beyond 48 rows the round
 // on zeros costs more than it saves, because other thread blocks wait for the place (4096x12288 128 rows 24.8 / 23.5).
-// Behind a GEMM that fills the GPU nothing is resident early: one round, and more thread blocks for few long rows (two rounds of two slices / one of
+// Behind a GEMM that fills the GPU (but for three SMs) nothing is resident early: one round, and more thread blocks for few long rows (two rounds of two slices / one of
 // two / one of four: 7168x15104 K8 13 float32 rows 37.2 / 36.5 / 35.2, 18560x13696 K3 5 rows 64.1 / 63.6 / 62.8, 32768x4096 K4 5 rows 37.1 / 36.7 / 37.0).
 struct RhtShape {
   int slices, warps, passes;
   RhtShape(int rows, int n, int grid, int sms) {
     const int groups = (n + 511) / 512, idle = sms - grid;
-    const bool full = idle == 0 && groups >= 8;
+    const bool full = idle < 4 && groups >= 8;
     warps = groups >= 9 ? (rows > 128 ? 16 : 24) : groups <= 4 || (idle >= 16 && rows > 2 * idle && rows <= 4 * idle) ? 8 : 16;
     slices = groups < 8 ? 1 : idle >= rows ? (idle / rows < kRhtMaxSlices ? idle / rows : kRhtMaxSlices) : rows <= 16 || (rows <= 64 && groups >= 16) ? (full && rows <= 16 && groups > 16 ? 4 : 2) : 1;
     slices = max(slices, (n + 128 * kRhtBlocks - 1) / (128 * kRhtBlocks));
