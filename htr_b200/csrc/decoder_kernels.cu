@@ -10,6 +10,7 @@
 #include <cstdint>
 
 #include "../../include/htr_b200.h"
+#include "htr_common.cuh"
 
 namespace {
 
@@ -214,7 +215,7 @@ __global__ void __cluster_dims__(kAttSplit, 1, 1) __launch_bounds__(kAttThreads,
   __shared__ float in_m[H][S * 2];                              // largest scores: two warps per head and block
   __shared__ float red[4];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this block runs: its shared memory may be written (waited for below)
+  htr::cluster_arrive_relaxed();                                  // this block runs: its shared memory may be written (waited for below)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = blockIdx.x % S, kvh = blockIdx.x / S, rep = hq / hkv, head0 = kvh * rep + blockIdx.y * H;
   const int nh = min(H, rep - (int)blockIdx.y * H);            // query heads of this cluster
@@ -260,7 +261,7 @@ __global__ void __cluster_dims__(kAttSplit, 1, 1) __launch_bounds__(kAttThreads,
     if (status && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) atomicOr(status, 4);
     for (int x = tid; x < nh * D && rank == 0; x += kAttThreads) out[(size_t)head0 * D + x] = __float2bfloat16_rn(0.f);
     copy_wait<0>();
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    htr::cluster_wait();
     return;
   }
   const int p = (int)p0, mine = (p + S - 1 - rank) / S;         // cached positions of this block (the new one does not come through the cache)
@@ -291,7 +292,7 @@ __global__ void __cluster_dims__(kAttSplit, 1, 1) __launch_bounds__(kAttThreads,
   float mx = -3.0e38f;
   copy_wait<3>();
   __syncthreads();
-  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every block of the cluster has started
+  htr::cluster_wait();                                           // every block of the cluster has started
   if (owner && half == 0) {                                     // of the new position: four dimensions per lane
     const float4 k4 = *reinterpret_cast<const float4*>(sk + 4 * lane), q4 = *reinterpret_cast<const float4*>(&sq[h][4 * lane]);
     float d = k4.x * q4.x + k4.y * q4.y + k4.z * q4.z + k4.w * q4.w;
@@ -331,8 +332,7 @@ __global__ void __cluster_dims__(kAttSplit, 1, 1) __launch_bounds__(kAttThreads,
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
   if (lane < S) cluster_write(&in_m[h][rank * 2 + half], lane, mx);
   copy_wait<0>();
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  htr::cluster_sync();
   mx = in_m[h][0];
 #pragma unroll
   for (int r = 1; r < 2 * S; ++r) mx = fmaxf(mx, in_m[h][r]);
@@ -382,8 +382,7 @@ __global__ void __cluster_dims__(kAttSplit, 1, 1) __launch_bounds__(kAttThreads,
     if (lane == 0) red[warp] = sum;
   }
   copy_wait<0>();
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  htr::cluster_sync();
   if (tid < D && rank < nh) {
     float sum = 0.f;
 #pragma unroll

@@ -70,6 +70,25 @@ __device__ __forceinline__ void wht128(float (&v)[4], int lane) {
   }
 }
 
+// Barriers of a cluster.  The .aligned forms (bar.sync, bar.arrive and bar.red are such forms too) want the whole warp at the instruction; a
+// branch on a lane or a thread before one does not promise that by itself, hence the __syncwarp in front of every such barrier.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  cluster_arrive();
+  cluster_wait();
+}
+
 // even contiguous runs of `units` over `grid` thread blocks: the first `rem` of them hold one more
 struct EvenRuns {
   int q, rem;

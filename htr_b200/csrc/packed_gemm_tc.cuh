@@ -296,6 +296,7 @@ __device__ __forceinline__ void decode_unit(const uint32_t (&own)[K], int lane, 
 // barrier of the finisher warps; true where every thread brought true
 __device__ __forceinline__ bool finishers_all(bool mine) {
   int all;
+  __syncwarp();
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %1, 0;\n\tbar.red.and.pred p, 1, %2, q;\n\tselp.s32 %0, 1, 0, p;\n\t}"
                : "=r"(all)
                : "r"((int)mine), "n"(kGemmFinishWarps * 32)
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     __syncwarp();
     if (!GROUP && p.inbox > 0 && lane == 0) mbar_expect_tx(smem_u32(&s_inbox), (uint32_t)(p.split * ((p.rows - part_id + p.split - 1) / p.split) * 512));
   }
-  if (!GROUP && p.inbox > 0) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (waited for before the first partial is sent)
+  if (!GROUP && p.inbox > 0) cluster_arrive();   // (waited for before the first partial is sent)
   if (warp == DW + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"((uint32_t)kGemmTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -603,7 +604,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       const uint32_t acc_addr = s_tmem + ((uint32_t)(32 * quad) << 16);
       if (p.inbox > 0) {
         const uint32_t inbox = smem_u32(ring) + (uint32_t)p.inbox, own_rows = (np + p.split - 1) / p.split;
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every thread block's inbox is ready
+        cluster_wait();   // every thread block's inbox is ready
         for (int j0 = 8 * (warp >> 2); j0 < np; j0 += 2 * DW) {
           uint32_t hi[8], lo[8];
           if (ok) {
@@ -766,7 +767,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       if (!ok) s_fail = 1;
     }
     __syncwarp();
-    if (!GROUP && p.inbox > 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // (its arrival; complete long ago)
+    if (!GROUP && p.inbox > 0) cluster_wait();   // (its arrival; complete long ago)
   }
   if (!GROUP && p.inbox > 0) {
     // ---- reduction inside the cluster: every thread block has sent its partials of row j to thread block j % split, which adds them in the
@@ -808,8 +809,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     if (bad)                                                 // a bounded wait gave up: the rows come out as NaN, beside the error word
       for (int e = tid; e < np * 128; e += kGemmThreads) result[e] = __uint_as_float(0x7FC00000u);
     if (p.split > 1) {
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      cluster_sync();
     } else if (bad) {
       __syncthreads();
     }
@@ -830,8 +830,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       }
     }
     if (p.split > 1) {                                       // nobody leaves while its shared memory may still be read
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      cluster_sync();
     }
   } else {
     asm volatile("griddepcontrol.wait;" ::: "memory");

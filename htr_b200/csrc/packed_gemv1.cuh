@@ -54,9 +54,18 @@ template <int K>
 constexpr int gemv1_smem_bytes(int n) { return G1Ring<K>::bytes + n * 4 + (n / 16) * 4; }
 
 template <int ID, int COUNT>
-__device__ __forceinline__ void named_sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory"); }
-__device__ __forceinline__ void named_sync_at(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
-__device__ __forceinline__ void named_arrive_at(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+__device__ __forceinline__ void named_sync() {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory");
+}
+__device__ __forceinline__ void named_sync_at(int id, int count) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void named_arrive_at(int id, int count) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
 
 // 32 weights (two tile rows x 16 columns) of a lane against the tile's staged activations
 template <int K, int ALU4>
@@ -86,6 +95,7 @@ __device__ __forceinline__ void unit_fma_subnormal(const uint32_t (&V)[K + 1], c
 // barrier of the finishers; true where any of them brings true
 __device__ __forceinline__ bool finishers_any(bool mine) {
   int any;
+  __syncwarp();
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %1, 0;\n\tbar.red.or.pred p, 5, %2, q;\n\tselp.s32 %0, 1, 0, p;\n\t}"
                : "=r"(any)
                : "r"((int)mine), "n"(kG1FinishWarps * 32)

@@ -135,12 +135,16 @@ __device__ __forceinline__ void tile_sync() {
   if constexpr (C == 1) {
     __syncthreads();
   } else {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 }
 // barrier of the threads that trace one tile back
-__device__ __forceinline__ void trace_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void trace_sync(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 
 // One step of this thread's states in N tiles at once: costs mc -> mn (of every block of the cluster).  mem: the tiles' shared memory,
 // one tile behind the other; the codebook values serve all of them.

@@ -1,0 +1,23 @@
+"""What the kernels' sources promise and no run on a healthy GPU would show (CPU)."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "htr_b200", "csrc")
+
+
+def source(path):
+    return re.sub(r"//[^\n]*", "", open(path).read()).replace("\\n\\t", " ")
+
+
+def test_whole_warps_at_aligned_barriers():
+    """bar.* and barrier.cluster.*.aligned are undefined where a warp's threads come one by one: each such instruction stands directly behind a
+    __syncwarp or another barrier."""
+    found = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        text = source(path)
+        for at in re.finditer(r"(?<![\w.])(bar\.(sync|arrive|red)|barrier\.cluster)", text):
+            before = text[:text.rindex("asm", 0, at.start())].rstrip()
+            assert re.search(r'(__syncwarp\(\);|"barrier\.cluster\.\w+\.\w+\.aligned;" ::: "memory"\);)$', before), (os.path.basename(path), before[-160:])
+            found += 1
+    assert found >= 10, found
