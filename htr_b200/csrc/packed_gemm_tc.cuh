@@ -155,19 +155,29 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// CLUSTER: what is waited for was written by other thread blocks of the cluster (the default acquires from this one's threads alone)
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity, unsigned hint_ns) {
   uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(bar), "r"(parity), "r"(hint_ns)
-      : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity), "r"(hint_ns)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity), "r"(hint_ns)
+        : "memory");
   return done != 0;
 }
 // (a role that waits most of the time sleeps between polls: the issue slots are the decode warps')
+template <bool CLUSTER = false>
 static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, const volatile int* fail, unsigned sleep_ns) {
   for (unsigned it = 0; it < kSpinLimit; ++it) {
-    if (mbar_try(bar, parity, 1000u)) return true;
+    if (mbar_try<CLUSTER>(bar, parity, 1000u)) return true;
     if ((it & 255u) == 255u && fail && *fail) return false;
     if (sleep_ns) __nanosleep(sleep_ns);
   }
@@ -175,8 +185,9 @@ static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity
 }
 // bounded wait for the phase with the given parity; false when the limit ran out or another role has already failed
 // (`fail` null: no early exit -- used on the failure path to let copies and MMAs in flight drain)
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* fail, unsigned sleep_ns = 0) {
-  return mbar_try(bar, parity, 1000u) || mbar_wait_slow(bar, parity, fail, sleep_ns);
+  return mbar_try<CLUSTER>(bar, parity, 1000u) || mbar_wait_slow<CLUSTER>(bar, parity, fail, sleep_ns);
 }
 
 // global -> shared bulk copy (16-byte aligned, size a multiple of 16), completion counted in bytes on an mbarrier
@@ -775,8 +786,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     // that nobody leaves too early, 1.5 us together.)
     if (warp < DW) {
       // A peer whose own wait gave up still sends, but up to two of its limits later, and into shared memory that must not be gone by then.
-      bool here = mbar_wait(smem_u32(&s_inbox), 0u, nullptr);
-      for (int limit = 0; limit < 3 && !here; ++limit) here = mbar_wait(smem_u32(&s_inbox), 0u, nullptr);
+      bool here = mbar_wait<true>(smem_u32(&s_inbox), 0u, nullptr);
+      for (int limit = 0; limit < 3 && !here; ++limit) here = mbar_wait<true>(smem_u32(&s_inbox), 0u, nullptr);
       here = __all_sync(kFullWarp, here);
       const int own_rows = (np + p.split - 1) / p.split, row_first = part_id + p.split * warp;
       const float4* in = reinterpret_cast<const float4*>(ring + p.inbox) + lane;

@@ -21,3 +21,11 @@ def test_whole_warps_at_aligned_barriers():
             assert re.search(r'(__syncwarp\(\);|"barrier\.cluster\.\w+\.\w+\.aligned;" ::: "memory"\);)$', before), (os.path.basename(path), before[-160:])
             found += 1
     assert found >= 10, found
+
+
+def test_partials_of_the_cluster_are_acquired_from_the_cluster():
+    """The inbox of the tensor-core GEMM is filled by other thread blocks: a wait that acquires from its own alone would not order their stores."""
+    text = source(os.path.join(CSRC, "packed_gemm_tc.cuh"))
+    waits = re.findall(r"mbar_wait(?:_slow)?(<\w+>)?\(smem_u32\(&s_inbox\)", text)
+    assert waits and all(w == "<true>" for w in waits)
+    assert "mbarrier.try_wait.parity.acquire.cluster.shared::cta" in text
