@@ -442,7 +442,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
     rb0 = u_begin / HB;
     hb0 = u_begin - rb0 * HB;
   }
-  if (GROUP && u_begin == u_end) return;                    // fewer blocks than thread blocks (an empty plan among others)
+  if (GROUP && u_begin == u_end) {                          // fewer blocks than thread blocks (an empty plan among others)
+    // not before the transform has: with an empty plan the grid would be over, and what comes behind it free to write, while that still reads
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   const int b_tile_bytes = ncols * 256;
   unsigned char* ring = gsm + (128 - (smem_u32(gsm) & 127)) % 128;
   const uint32_t ring_addr = smem_u32(ring);

@@ -29,3 +29,13 @@ def test_partials_of_the_cluster_are_acquired_from_the_cluster():
     waits = re.findall(r"mbar_wait(?:_slow)?(<\w+>)?\(smem_u32\(&s_inbox\)", text)
     assert waits and all(w == "<true>" for w in waits)
     assert "mbarrier.try_wait.parity.acquire.cluster.shared::cta" in text
+
+
+def test_no_thread_block_of_the_gemm_leaves_before_its_transform():
+    """A grid whose thread blocks all return without a wait is complete while the launch before it may still run, and later launches wait for
+    this grid alone.  The returns of the kernel before its roles begin stand behind a wait."""
+    text = source(os.path.join(CSRC, "packed_gemm_tc.cuh"))
+    start = text[text.index("packed_gemm_tc_kernel(const GemmParams p)"):]
+    start = start[:start.index("tcgen05.alloc")]
+    for at in re.finditer(r"\breturn\b", start):
+        assert re.search(r'"griddepcontrol\.wait;" ::: "memory"\);\s*$', start[:at.start()]), start[at.start() - 120:at.start()]

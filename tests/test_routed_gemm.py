@@ -70,3 +70,28 @@ def test_pairs_of_any_magnitude(dtype, tol):
         close(ops.linear_routed_gemm(gu, plan, T, tables, m // 16, n // 16, 3, prologue=ops.PROLOGUE_SWIGLU),
               ops.linear_routed(gu, route, tables, m // 16, n // 16, 3, prologue=ops.PROLOGUE_SWIGLU))
     assert all(c == 0 for c in ops.gemm_error_codes())
+
+
+@pytest.mark.parametrize("m,n", ((128, 128), (256, 4096)))
+def test_plans_without_a_pair_between_others(m, n):
+    """Steps of which every pair goes to an expert outside the tables (an empty plan: no thread block has work) between ordinary ones that use
+    the same scratch: the empty ones write nothing, the others give the bits that they give alone."""
+    from htr_b200 import ops, wire
+
+    dev, E, T = torch.device("cuda:0"), 4, 24
+    experts = [wire.random_packed(m, n, 3, seed=5 + e, device=dev) for e in range(E)]
+    tables = [torch.tensor([experts[e][i].data_ptr() for e in range(E)], dtype=torch.int64, device=dev) for i in range(4)]
+    g = torch.Generator().manual_seed(n)
+    x = torch.randn(T, n, generator=g).bfloat16().to(dev)
+    some, none = (torch.arange(T) % E).to(dev), torch.full((T,), E, dtype=torch.int64, device=dev)
+
+    def step(route, out):
+        return ops.linear_routed_gemm(x, ops.route_plan(route, tables), T, tables, m // 16, n // 16, 3, out=out)
+
+    want = step(some, torch.empty((T, m), dtype=torch.bfloat16, device=dev))
+    torch.cuda.synchronize()
+    outs = [(step(none, torch.full((T, m), 7.0, dtype=torch.bfloat16, device=dev)), step(some, torch.empty((T, m), dtype=torch.bfloat16, device=dev)))
+            for _ in range(20)]
+    for empty, full in outs:
+        assert bool((empty == 7.0).all()) and torch.equal(full, want)
+    assert all(c == 0 for c in ops.gemm_error_codes())
