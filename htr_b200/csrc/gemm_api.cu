@@ -379,6 +379,7 @@ int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int
 namespace {
 
 thread_local int t_gemm_cuda = 0;
+thread_local int t_gemm_withhold = 0;                      // (htr_gemm_withhold_tile)
 constexpr size_t kCounterRegion = 1 << 16;   // same fixed counter region as the GEMV workspace
 constexpr size_t kErrorRegion = 256;
 
@@ -605,6 +606,7 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   p.part_magic = g.split > 0 ? (65536 + g.split - 1) / g.split : 0;
   p.inbox = g.inbox;
   p.stages = g.stages;
+  p.withhold = t_gemm_withhold;
   p.m_out = m_out;
   const RhtShape shape(M, n, g.grid, g.sms);
   p.xsum_slices = gemm_xsums(g.np, n);
@@ -718,6 +720,7 @@ int htr_linear_routed_gemm(const void* x, int dtype, int x_div, int64_t x_row_st
   p.dtype = dtype;
   p.hb = n / 128;
   p.stages = g.stages;
+  p.withhold = t_gemm_withhold;
   p.xsum_slices = 1;
   p.cb = (float)codebook_scale();
   p.plan = pl;
@@ -734,5 +737,7 @@ int htr_linear_routed_gemm(const void* x, int dtype, int x_div, int64_t x_row_st
 int htr_linear_gemm_last_cuda_error(void) { return t_gemm_cuda; }
 
 size_t htr_linear_gemm_error_offset(void) { return kCounterRegion; }
+
+void htr_gemm_withhold_tile(int block) { t_gemm_withhold = block < 0 ? 0 : block + 1; }
 
 }  // extern "C"

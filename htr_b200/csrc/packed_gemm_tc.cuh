@@ -94,6 +94,7 @@ struct GemmParams {
   int inbox;              // > 0: offset in shared memory where a thread block of a cluster receives the partial sums of its rows; 0: the
                           // partials stay where they are and are fetched from there (many activation rows)
   int stages;
+  int withhold;           // test hook: the B tile of block withhold - 1 of the launch is never fetched (0: none)
   int xsum_slices;
   float cb;
   // Grouped form (GROUP instantiations: the experts of a mixture-of-experts step): the problems are the tiles of a device-side plan
@@ -614,6 +615,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         tok_of = __ldcg(p.tok + j);
       }
       ok = ok && __all_sync(kFullWarp, mbar_wait(smem_u32(&s_done), 0u, &s_fail));
+      ok = __all_sync(kFullWarp, ok && !s_fail);             // (an MMA lane that gave up says so before it commits what it had issued)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int li = lane & 15, row = 32 * quad + (lane & 16) + (li < 8 ? 2 * li : 2 * li - 15);   // weight row of this tensor-memory lane
       const uint32_t acc_addr = s_tmem + ((uint32_t)(32 * quad) << 16);
@@ -666,9 +668,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
         for (int u = u_begin; u < u_end; ++u) {
           if (use > 0 && !mbar_wait(smem_u32(&s_freed[s]), (use - 1u) & 1u, &s_fail, kSleepNs)) { s_fail = 1; break; }
           const uint32_t bar = smem_u32(&s_full[s]);
-          mbar_expect_tx(bar, (uint32_t)b_tile_bytes);
-          bulk_load(ring_addr + s * b_tile_bytes, xb + (size_t)hb * b_tile_bytes, (uint32_t)b_tile_bytes, bar);
-          ++issued;
+          if (u + 1 != p.withhold) {
+            mbar_expect_tx(bar, (uint32_t)b_tile_bytes);
+            bulk_load(ring_addr + s * b_tile_bytes, xb + (size_t)hb * b_tile_bytes, (uint32_t)b_tile_bytes, bar);
+            ++issued;
+          }
           if (++hb == HB) {
             hb = 0;
             if (GROUP && --rb_left == 0) {

@@ -232,6 +232,9 @@ int htr_linear_fused(const void* x, int M, const void* qweight, int mt, int nt, 
 #define HTR_GEMM_MAX_ROWS_F32 128 /* float32 activations travel as two fp16 planes: half as many rows per call */
 size_t htr_linear_gemm_workspace_bytes(int M, int m, int n, int K);
 size_t htr_linear_gemm_error_offset(void);
+/* Test hook: in the GEMM launches of this thread that follow, the activations of 128-column block `block` (row block * blocks per row
+ * block + block inside it) are never fetched, so that the bounded waits for them run out; block < 0: no longer. */
+void htr_gemm_withhold_tile(int block);
 int htr_linear_gemm_last_cuda_error(void);
 int htr_linear_gemm(const void* x, int dtype, int M, const void* qweight, int mt, int nt, int K, const void* scales,
                     const uint8_t* su, const uint8_t* sv, const void* bias /* may be NULL */, void* y, void* workspace,

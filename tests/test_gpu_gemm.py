@@ -69,3 +69,32 @@ def test_gemm_full_size_and_bit_stability(coracle):
     y1 = ops.linear(x[:1].to(dev), *d)
     assert rel(y1.float().cpu().numpy(), y[:1].float().cpu().numpy()) <= 4e-3
     assert all(c == 0 for c in ops.gemm_error_codes())
+
+
+@pytest.mark.parametrize("m,n,M,block", ((1024, 4096, 8, 3 * 32 + 17), (1024, 4096, 40, 5 * 32), (768, 384, 137, 2 * 3 + 1), (128, 128, 8, 0), (12288, 4096, 8, 40 * 32 + 5)))
+def test_rows_of_an_expired_wait_are_nan(m, n, M, block):
+    """One tile of activations is withheld, so that a bounded wait runs out (in clusters that send their partial sums, in clusters that fetch
+    them, in single thread blocks and in flat runs): every result of its row block is NaN, those of other thread blocks are as they are without,
+    the status word is set, and the next call is served again."""
+    from htr_b200 import _lib, ops, wire
+
+    dev = torch.device("cuda:0")
+    w = [t.to(dev) for t in wire.random_packed(m, n, 4, seed=m + M)]
+    x = torch.randn(M, n, generator=torch.Generator().manual_seed(M)).bfloat16().to(dev)
+    want = ops.linear(x, *w)
+    torch.cuda.synchronize()
+    _lib.lib.htr_gemm_withhold_tile(block)
+    try:
+        got = ops.linear(x, *w)
+    finally:
+        _lib.lib.htr_gemm_withhold_tile(-1)
+    lost = {rb for rb in range(m // 128) if bool(torch.isnan(got[:, 128 * rb:128 * rb + 128]).all())}
+    rb = block // (n // 128)
+    assert rb in lost and lost <= ({rb, rb + 1} if m == 12288 else {rb})   # (a flat run owes the next row block too)
+    kept = torch.tensor([r // 128 not in lost for r in range(m)], device=dev)
+    assert torch.equal(got[:, kept], want[:, kept])
+    codes = ops.gemm_error_codes()
+    for ws in ops._GEMM_WS.values():                              # (status word, and counters that an unfinished row block leaves)
+        ws.zero_()
+    assert any(c != 0 for c in codes)
+    assert torch.equal(ops.linear(x, *w), want)
