@@ -585,7 +585,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       if constexpr (GROUP) deliver(stored);
       // the MMAs that read this stage NS blocks ago must have retired
       const uint32_t bar = smem_u32(&s_freed[0]) + 8u * stage;
-      if (!__all_sync(kFullWarp, mbar_try(bar, parity, 1000u)) && !__all_sync(kFullWarp, mbar_wait_slow(bar, parity, &s_fail, 0u))) { ok = false; break; }
+      if (!__all_sync(kFullWarp, mbar_try(bar, parity, 1000u)) && !__all_sync(kFullWarp, mbar_wait_slow(bar, parity, &s_fail, 0u))) {
+        s_fail = 1;                                          // (before anything else that the MMA lane could take for progress)
+        ok = false;
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       tmem_store_strip(a_addr + 64 * stage, w);
       read_own_words<K>(blk + 128 * K, c, g, V);
@@ -597,7 +601,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       stage += around ? 2 - NS : 2;
       parity ^= around ? 1u : 0u;
     }
-    if constexpr (GROUP) deliver(stored);
+    if constexpr (GROUP)
+      if (ok) deliver(stored);                               // (a warp that gave up has told of all that it stored: a second arrival would count for the next round)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (!GROUP && p.split > 0) {
       // these loads, and the wait for the transform that they need, lie beside the last MMAs; then the accumulator goes to the ring as

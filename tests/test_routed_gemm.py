@@ -95,3 +95,35 @@ def test_plans_without_a_pair_between_others(m, n):
     for empty, full in outs:
         assert bool((empty == 7.0).all()) and torch.equal(full, want)
     assert all(c == 0 for c in ops.gemm_error_codes())
+
+
+def test_pairs_of_an_expired_wait_are_nan():
+    """One tile of activations is withheld: its row block of its experts' pairs comes out as NaN, and the row block behind it in the same thread
+    block's run (13 blocks, more than there are stages, so that the decode warps' own waits run out as well); all others keep their bits."""
+    from htr_b200 import _lib, ops, wire
+
+    dev, m, n, E, T = torch.device("cuda:0"), 256, 4096, 32, 64
+    experts = [wire.random_packed(m, n, 3, seed=60 + e, device=dev) for e in range(E)]
+    tables = [torch.tensor([experts[e][i].data_ptr() for e in range(E)], dtype=torch.int64, device=dev) for i in range(4)]
+    route = (torch.arange(T) % E).to(dev)                         # tile e holds the two pairs of expert e
+    x = torch.randn(T, n, generator=torch.Generator().manual_seed(1)).bfloat16().to(dev)
+    plan = ops.route_plan(route, tables)
+    want = ops.linear_routed_gemm(x, plan, T, tables, m // 16, n // 16, 3)
+    torch.cuda.synchronize()
+    for block in (0, 19 * 64 + 3, 19 * 64 + 40):
+        _lib.lib.htr_gemm_withhold_tile(block)
+        try:
+            got = ops.linear_routed_gemm(x, plan, T, tables, m // 16, n // 16, 3)
+        finally:
+            _lib.lib.htr_gemm_withhold_tile(-1)
+        codes = ops.gemm_error_codes()
+        assert any(c != 0 for c in codes)
+        for ws in ops._GEMM_WS.values():
+            ws.zero_()
+        unit = block // (n // 128)                                # row block, counted through the tiles
+        for at in range(E * 2):
+            rows, cols = route == at // 2, slice(128 * (at % 2), 128 * (at % 2) + 128)
+            lost = bool(torch.isnan(got[rows][:, cols]).all())
+            assert lost or torch.equal(got[rows][:, cols], want[rows][:, cols])
+            assert lost if at == unit else not lost or at == unit + 1
+    assert torch.equal(ops.linear_routed_gemm(x, plan, T, tables, m // 16, n // 16, 3), want)
