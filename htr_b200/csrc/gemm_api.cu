@@ -431,29 +431,40 @@ int launch_gemm(int K, const GemmParams& p, int grid, int smem, cudaStream_t st)
 // activation rows per launch after padding: accumulator columns come in multiples of 16
 int padded_rows(int M, int planes) { return planes == 2 ? (M + 7) / 8 * 8 : (M + 15) / 16 * 16; }
 
-int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
+int device_sms() {                                        // 0: a CUDA error
   int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return HTR_ERR_CUDA;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   static int seen_sms[64] = {0};                          // a device fact: asked once (every caller would store the same number)
   if (dev >= 0 && dev < 64) sms = seen_sms[dev];
   if (sms <= 0) {
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return HTR_ERR_CUDA;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 0;
     if (dev >= 0 && dev < 64) seen_sms[dev] = sms;
   }
+  return sms;
+}
+
+// Stages of a launch, as many as tensor memory and `budget` bytes of shared memory hold, and the shared memory of its two rings; 0: fewer than two
+int gemm_stages(int np, int planes, int K, int budget, int* smem) {
+  int stages = (kGemmTmemCols - gemm_acc_cols(np * planes)) / 64;
+  if (stages > kGemmMaxStages) stages = kGemmMaxStages;
+  while (stages > 1 && gemm_smem_bytes(np, planes, stages, gemm_word_bytes(K)) > budget) --stages;
+  *smem = gemm_smem_bytes(np, planes, stages, gemm_word_bytes(K));
+  return stages < 2 || *smem > budget ? 0 : stages;
+}
+
+int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   GemmPlan g;
-  g.sms = sms;
+  g.sms = device_sms();
+  if (g.sms <= 0) return HTR_ERR_CUDA;
   g.np = padded_rows(M, planes);
   g.rbs = m / 128;
   g.hb = n / 128;
   const int ncols = g.np * planes;
   if (ncols > kGemmMaxCols) return HTR_ERR_TOO_LARGE;
-  // one thread block per SM; as many stages as its tensor memory and shared memory hold
-  const int words = gemm_word_bytes(K), budget = 226 * 1024;
-  g.stages = (kGemmTmemCols - gemm_acc_cols(ncols)) / 64;
-  if (g.stages > kGemmMaxStages) g.stages = kGemmMaxStages;
-  while (g.stages > 1 && gemm_smem_bytes(g.np, planes, g.stages, words) > budget) --g.stages;
-  g.smem = gemm_smem_bytes(g.np, planes, g.stages, words);
-  if (g.stages < 2) return HTR_ERR_TOO_LARGE;
+  // one thread block per SM
+  const int words = gemm_word_bytes(K), budget = kGemmSmem;
+  g.stages = gemm_stages(g.np, planes, K, budget, &g.smem);
+  if (g.stages == 0) return HTR_ERR_TOO_LARGE;
   // Three forms, by their cost in units of one decoded 128 x 128 block (0.43 us, or as long as the MMAs of a wide batch take):
   //  * up to sixteen thread blocks share a row block as a cluster and reduce on chip;
   //  * a thread block takes a whole row block, in as many waves as there are row blocks per SM: its decode warps finish it from shared
@@ -469,7 +480,7 @@ int make_gemm_plan(int M, int m, int n, int K, int planes, GemmPlan* out) {
   // A change of these terms that gives float32 rows longer sums loses precision; beyond 128 rows there is one plane, whose own rounding
   // (2e-4) hides it.
   const double unit = ncols > 192 ? 1.2 : 1.0;
-  const long long slots = sms, units = (long long)g.rbs * g.hb;
+  const long long slots = g.sms, units = (long long)g.rbs * g.hb;
   const long long flat_grid = slots < units ? slots : units, flat_run = (units + flat_grid - 1) / flat_grid;
   const double beside = (double)(flat_run / g.hb) * M * 0.5;
   double best = (flat_run * unit > beside ? flat_run * unit : beside) + 9 + (double)((g.hb / flat_run + 1) * g.np) / (g.np > 128 ? 32 : 84);
@@ -639,12 +650,10 @@ static int group_layout(int count, int table_rows, int m, int n, int K, GroupLay
   g->cap = group_cap(count, table_rows);
   if (g->cap > kGroupMaxTiles || (long long)g->cap * (m / 128) > (int)(kCounterRegion / 4) || (long long)g->cap * (m / 128) * (n / 128) > 0x3FFFFFFF)
     return HTR_ERR_TOO_LARGE;
-  GemmPlan plan;                                             // stages, shared memory and thread blocks of a launch with these columns
-  const int rc = make_gemm_plan(kGroupRows, m, n, K, 2, &plan);
-  if (rc != HTR_OK) return rc;
-  g->stages = plan.stages;
-  g->smem = plan.smem;
-  g->grid = plan.sms;
+  g->stages = gemm_stages(kGroupRows, 2, K, kGemmGroupSmem, &g->smem);
+  if (g->stages == 0) return HTR_ERR_TOO_LARGE;
+  g->grid = device_sms();
+  if (g->grid <= 0) return HTR_ERR_CUDA;
   size_t off = kCounterRegion + kErrorRegion;
   g->off_xb = off; off += align256((size_t)g->cap * n * (2 * kGroupRows) * 2);
   g->off_xsum = off; off += align256((size_t)g->cap * kGroupRows * 4);

@@ -62,6 +62,7 @@ constexpr int kGemmFinishWarps = 4;
 constexpr int kGemmWarps = kGemmDecodeWarps + 2 + kGemmFinishWarps;
 constexpr int kGemmThreads = kGemmWarps * 32;
 constexpr int kGemmTmemCols = 512;                          // the accumulator first, then 64 columns of A per stage
+constexpr int kGemmSmem = 226 * 1024, kGemmGroupSmem = 220 * 1024;   // dynamic shared memory that a launch may ask for (grouped: beside 4 KB of tables)
 constexpr int kGemmMaxCols = 256;                           // accumulator columns (activation rows x planes) per launch
 constexpr int kLbo = 128;                                   // bytes between core matrices of B adjacent in K
 constexpr int kSboB = 1024;                                 // bytes between its 8-column groups (64 k x 8 columns x 2 bytes)
@@ -238,12 +239,12 @@ __device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&r)[8]) {
 
 // dynamic shared memory: the B ring (the cluster form reuses it for the [np][128] float partial of the thread block), then the
 // packed-word rings of the decode warps (`words` bytes)
-__host__ __device__ inline int gemm_stage_bytes(int ncols) { return ncols * 256; }
-__host__ __device__ inline int gemm_ring_bytes(int np, int planes, int stages) {
+__host__ __device__ constexpr int gemm_stage_bytes(int ncols) { return ncols * 256; }
+__host__ __device__ constexpr int gemm_ring_bytes(int np, int planes, int stages) {
   const int ring = stages * gemm_stage_bytes(np * planes), result = np * 128 * 4;
   return ring > result ? ring : result;
 }
-__host__ __device__ inline int gemm_smem_bytes(int np, int planes, int stages, int words) { return gemm_ring_bytes(np, planes, stages) + words + 128; }
+__host__ __device__ constexpr int gemm_smem_bytes(int np, int planes, int stages, int words) { return gemm_ring_bytes(np, planes, stages) + words + 128; }
 __host__ __device__ inline int gemm_acc_cols(int ncols) { return ncols < 32 ? 32 : ncols; }
 
 // ---- packed-word ring of a decode warp: one slot = the tiles of its strip in one 128-column block (two units of four tiles).

@@ -8,13 +8,16 @@
 namespace htr {
 namespace {
 
+// the grouped form's stages all fit at its 16 rows and two planes, whatever the width
+static_assert(gemm_smem_bytes(kGroupRows, 2, kGemmMaxStages, GemmRing<HTR_INST_K>::bytes) <= kGemmGroupSmem, "grouped GEMM: rings beyond the opt-in");
+
 // shared memory beyond 48 KB: opted in once per device (the 227 KB limit includes the static part)
 int allow_smem(int dev) {
   static bool allowed[64] = {false};
   if (dev >= 0 && dev < 64 && allowed[dev]) return 0;
-  const cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+  const cudaError_t e = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
   if (e != cudaSuccess) return (int)e;
-  const cudaError_t e2 = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  const cudaError_t e2 = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmGroupSmem);
   if (e2 != cudaSuccess) return (int)e2;
   const cudaError_t e3 = cudaFuncSetAttribute(packed_gemm_tc_kernel<HTR_INST_K, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // up to 16
   if (e3 != cudaSuccess) return (int)e3;
