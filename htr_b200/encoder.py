@@ -18,17 +18,6 @@ import torch
 
 from . import _lib, wire
 
-_WS = {}
-
-
-def _workspace(device, nbytes):
-    buf = _WS.get(device.index)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
-        _WS[device.index] = buf
-    return buf
-
-
 def codebook_f32(device):
     """cb[s] = float32(v(s) / rms) for all 65536 states, computed by the device function the search uses."""
     out = torch.empty(65536, dtype=torch.float32, device=device)
@@ -58,7 +47,8 @@ def viterbi(x, w, cb=None, K=4, tailbite=True, return_cost=False):
             need = _lib.lib.htr_viterbi_workspace_bytes(B, T, int(K))
             if need == 0:
                 raise _lib.HTRError(f"htr_viterbi: unsupported sizes B={B} T={T} K={K}")
-            ws = _workspace(x.device, need)
+            # of this call and stream alone, and the allocator's again afterwards: the kept rows of path costs are up to 0.6 GB (K = 3)
+            ws = torch.empty(need, dtype=torch.uint8, device=x.device)
             rc = _lib.lib.htr_viterbi(x32.data_ptr(), w32.data_ptr(), B, T, int(K), int(bool(tailbite)), states.data_ptr(), total.data_ptr(),
                                       ws.data_ptr(), ws.numel(), torch.cuda.current_stream(x.device).cuda_stream)
             _lib.check(rc, "htr_viterbi")

@@ -291,8 +291,9 @@ int htr_dec_rope_attention(const void* qkv, const int64_t* pos, const float* cos
  * htr/vit_v2.py:28-73 (built there for sm_86 / sm_120 only), the callable behind the reference's encode.VITERBI hook
  * (htr/encode.py:7,48): minimises sum_t w[t] * (x[t] - cb[s_t])^2, cb[s] = float32(v(s) / rms), over state sequences
  * s_t = ((s_{t-1} << K) & 0xFFFF) | bits; with tailbite != 0 the sequence closes into a circle.  states[B][T] receives the
- * 16-bit states (as int32), total[B] (may be NULL) the cost of the winning final state.  The workspace holds rows of path costs:
- * htr_viterbi_workspace_bytes(B, T, K) bytes (0 = unsupported arguments).
+ * 16-bit states (as int32), total[B] (may be NULL) the cost of the winning final state.  The workspace holds rows of path costs, 1 to 11 KB per
+ * step of every tile that is worked on at once (up to two per SM): htr_viterbi_workspace_bytes(B, T, K) bytes, which grow with B up to 407, 611,
+ * 412, 308, 154 and 77 MB at K = 2, 3, 4, 5, 6 and 8 (T = 256, 148 SMs); calls that run at the same time need one each (0 = unsupported arguments).
  * htr_codebook_f32 writes cb[0..65535] as the search computes it (test hook). */
 size_t htr_viterbi_workspace_bytes(int B, int T, int K);
 int htr_viterbi(const float* x, const float* w, int B, int T, int K, int tailbite, int32_t* states, float* total, void* workspace,

@@ -165,3 +165,26 @@ def test_two_tiles_of_a_block_equal_one(K, T):
         for B in (sms + 1, 2 * sms, 2 * sms + 9):
             got, c = encoder.viterbi(x[:B], w[:B], None, K, tailbite=tailbite, return_cost=True)
             assert torch.equal(got, want[:B]) and torch.equal(c, cost[:B])
+
+
+def test_workspace_of_a_call_is_its_own():
+    """The kept rows are gone when a call is over, and calls of two streams at the same time do not share them."""
+    from htr_b200 import encoder
+
+    dev = torch.device("cuda:0")
+    x, w = (t.to(dev) for t in tiles(96, 256, 5))
+    want = [encoder.viterbi(x[i::2], w[i::2], None, 3) for i in range(2)]
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated(dev)
+    got = encoder.viterbi(x, w, None, 3)
+    assert torch.cuda.memory_allocated(dev) - before <= got.numel() * got.element_size() + 4096
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    parts = [(x[i::2].contiguous(), w[i::2].contiguous()) for i in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        out = []
+        for s, p in zip(streams, parts):
+            with torch.cuda.stream(s):
+                out.append(encoder.viterbi(*p, None, 3))
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(out, want))
