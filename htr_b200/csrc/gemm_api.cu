@@ -1,5 +1,6 @@
 // C entry points of the tensor-core packed GEMM (batches of up to 256 activation rows per call).
 #include <cmath>
+#include <type_traits>
 
 #include "packed_gemm_tc.cuh"
 
@@ -10,22 +11,23 @@ namespace htr {
 // Output layout = the B operand tiles of the GEMM, one contiguous block per 128 columns of x:
 //   xb[64-column unit][column group g][k-group kc][column r][8 k]   column = g*8 + r: activation row (hi plane), np + row (lo plane)
 // with the k order of the A operand inside a unit (packed_gemm_tc.cuh): position 16 j + 4 c + e holds column 16 c + 4 j + e.
-// grid (rows, slices): a thread block transforms one slice of one activation row, after finding the range of the whole row itself (16
-// bytes per load; cheaper than an exchange between slices).  A warp takes four 128-column blocks at a time, eight lanes each, a lane the
-// 16 columns of one tile, so that four of the seven butterfly stages stay in a lane and a value crosses lanes three times (one block per
-// warp, four values a lane: five times, and shuffles pass 32 lanes a cycle and SM).  xsum[row][i] holds the sum of the i-th 8 `per`
-// blocks.  Butterflies go from the lowest column bit to the highest, and sums are formed over four columns of every eighth block, the 32 fours of
-// a block (halves, quarters, ...) and eight blocks one after another, whatever the grid: dozens of bf16 layers turn another order into percents.  Columns from n_in on read as zeros; B columns of the padded batch that have no row stay as they
-// are: they reach only accumulator columns that nobody reads.
+// A thread block transforms one slice of one activation row, after finding the range of the whole row itself (16 bytes per load; cheaper
+// than an exchange between slices).  xsum[row][i] holds the sum of the i-th 8 `per` blocks.  Butterflies go from the lowest column bit to
+// the highest, and sums are formed over four columns of every eighth block, the 32 fours of a block (halves, quarters, ...) and eight
+// blocks one after another, whatever the form and the grid: dozens of bf16 layers turn another order into percents.  Columns from n_in
+// on read as zeros; B columns of the padded batch that have no row stay as they are: they reach only accumulator columns that nobody reads.
 //
 // What bounds it: latency -- of the wait for the kernel before it, of the row, of instructions that nobody has fetched yet (a kernel this
-// short runs every line once) -- and the stores, 16 bytes apart by the B layout, a line of L1 each.  So
-//  * the thread blocks, which are resident long before they may read x, go through the whole code once on zeros before the wait (`passes`
-//    = 2, nothing is loaded or stored), which brings it into the SM's instruction caches;
-//  * there are as many of them as fit on the few SMs that the GEMM before leaves free: clusters of the next GEMM waited for those that did not.
-// us for transform + GEMM in a chain (graph), 4096x12288 K3 4 rows / K5 16 rows / 12288x4096 K2 64 rows / 151936x4096 K4 8 rows / 4096x4000 K3
-// 11 rows: one block per warp in 12 / 12 / 4 / 4 / 4 slices of 256 threads 18.1 / 21.9 / 23.6 / 128.7 / 9.25; four per warp, 24 warps, one slice
-// 18.3 / 18.3 / 23.1 / 127.7 / 9.18, two 17.3 / 20.6 / 23.1 / 127.0 / 10.6, four 17.1 / 20.5 / 25.9 / 127.2 / 11.0.
+// short runs every line once) -- and the stores, 16 bytes apart by the B layout, a line of L1 each.  Two forms:
+//  * one block per warp and turn, a thread block per sum: four columns a lane, so that a value crosses lanes five times, and every block of
+//    a short row has a warp of its own;
+//  * four blocks per warp, eight lanes each, a lane the 16 columns of one tile: a value crosses lanes three times, and one thread block takes
+//    a whole row or half of one.  Few thread blocks matter before a GEMM in clusters: those that do not fit on the SMs that the GEMM before
+//    leaves free keep its successor's clusters waiting.
+// us for transform + GEMM in a chain (graph) and behind an elementwise kernel, one block per warp / four: 1024x640 K4 16 rows 5.3, 7.2 / 5.7,
+// 7.3; 2048x2048 K4 96 rows 9.7, 11.5 / 10.3, 12.1; 4096x4096 K4 37 rows 11.8, 12.1 / 9.6, 12.8; 4096x12288 K5 16 rows 20.9, 21.4 / 17.9, 19.8.
+// (All warps through the code once on zeros before the wait, to fetch its instructions: 0 to 0.3 us less in a chain, where the wait is long, and
+// 0.7 to 1.7 more behind a kernel that lets its successors go at its end only; 4096x12288 K5 16 rows 17.7, 21.5.)
 //
 // Range scale of a row: the power of two 2^k with max|x| * sqrt(128) in (2^13, 2^14] * 2^k, in both directions, so that neither a large
 // row leaves the fp16 range nor a small one sinks into its subnormals (fp16 numbers are 2^-24 apart below 2^-14: unscaled, a row of
@@ -38,12 +40,12 @@ __device__ __forceinline__ float range_scale(float mx) {
   return __uint_as_float(min(max(e, 127u - 120u), 127u + 118u) << 23);
 }
 
-constexpr int kRhtWarps = 24, kRhtMaxSlices = 4, kRhtBlocks = 512;   // (blocks of a slice: longer rows take more slices)
+constexpr int kRhtWarps = 24, kRhtBlocks = 512;              // (blocks of a slice: longer rows take more slices)
 
 template <int DT>
 __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ x, int np, int n, int n_in, int planes,
                                                                  const uint8_t* __restrict__ su, __half* __restrict__ xb, float* __restrict__ xsum,
-                                                                 float* __restrict__ tok, int per, int passes) {
+                                                                 float* __restrict__ tok, int per) {
   __shared__ unsigned red_top[kRhtWarps];
   __shared__ float block_sum[kRhtBlocks];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the GEMM may start fetching packed words now
@@ -52,115 +54,200 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
   const int u = (lane >> 2) & 1, c = lane & 3;               // this lane's tile inside a block of a group
   const int ncols = np * planes;
   // column 16 c + 4 j + e of unit u goes to position 16 j + 4 c + e
-  __half* const out = xb + (size_t)u * ncols * 64 + (size_t)(r >> 3) * 512 + (r & 7) * 8 + (c >> 1) * 64 + 4 * (c & 1);
-  const size_t to_lo = (size_t)(np >> 3) * 512;
-#pragma unroll 1
-  for (int pass = 0; pass < passes; ++pass) {
-    const bool real = pass + 1 == passes;
-    if (real) asm volatile("griddepcontrol.wait;" ::: "memory");     // x may come from the preceding kernel, the last GEMM may still read xb
-    // range of the whole row: magnitudes of floats compare like their bit patterns, so 16-bit pairs take the packed integer maximum
-    uint32_t top = 0u;
-    constexpr int kPer16 = DT == HTR_DTYPE_F32 ? 4 : 8;      // elements in 16 bytes
-    const uint4* row16 = reinterpret_cast<const uint4*>(static_cast<const char*>(x) + (size_t)r * n_in * (16 / kPer16));
-    const int scan = real ? n_in / kPer16 : 0;
+  __half* out = xb + (size_t)u * ncols * 64 + (size_t)(r >> 3) * 512 + (r & 7) * 8 + (c >> 1) * 64 + 4 * (c & 1);
+  size_t to_lo = (size_t)(np >> 3) * 512;
+  constexpr int kPer16 = DT == HTR_DTYPE_F32 ? 4 : 8;        // elements in 16 bytes
+  const char* row = static_cast<const char*>(x) + (size_t)r * n_in * (16 / kPer16);
+  int todo = 2 * own, first = 8 * per * slice * own, col0 = 64 * u + 16 * c;
+  // x may come from the preceding kernel, the last GEMM may still read xb.  Operands of the wait are computed before it, while there is time
+  // (left to the compiler, behind it, in cold code: 4096x4096 K4, 256 rows 20.9 -> 21.3 us)
+  asm volatile("griddepcontrol.wait;" : "+l"(out), "+l"(to_lo), "+l"(row), "+r"(todo), "+r"(first), "+r"(col0) : : "memory");
+  // range of the whole row: magnitudes of floats compare like their bit patterns, so 16-bit pairs take the packed integer maximum
+  uint32_t top = 0u;
+  const uint4* row16 = reinterpret_cast<const uint4*>(row);
 #pragma unroll 4
-    for (int e = threadIdx.x; e < scan; e += blockDim.x) {
-      const uint4 v = __ldg(row16 + e);
-      if constexpr (DT == HTR_DTYPE_F32) {
-        constexpr uint32_t m = 0x7FFFFFFFu;
-        top = max(max(top, v.x & m), max(v.y & m, max(v.z & m, v.w & m)));
-      } else {
-        constexpr uint32_t m = 0x7FFF7FFFu;
-        top = __vmaxu2(__vmaxu2(top, v.x & m), __vmaxu2(v.y & m, __vmaxu2(v.z & m, v.w & m)));
-      }
+  for (int e = threadIdx.x; e < n_in / kPer16; e += blockDim.x) {
+    const uint4 v = __ldg(row16 + e);
+    if constexpr (DT == HTR_DTYPE_F32) {
+      constexpr uint32_t m = 0x7FFFFFFFu;
+      top = max(max(top, v.x & m), max(v.y & m, max(v.z & m, v.w & m)));
+    } else {
+      constexpr uint32_t m = 0x7FFF7FFFu;
+      top = __vmaxu2(__vmaxu2(top, v.x & m), __vmaxu2(v.y & m, __vmaxu2(v.z & m, v.w & m)));
     }
-    if constexpr (DT != HTR_DTYPE_F32) top = max(top >> 16, top & 0xFFFFu);
-    top = __reduce_max_sync(kFullWarp, top);
-    if (lane == 0) red_top[warp] = top;
-    __syncthreads();
-    top = __reduce_max_sync(kFullWarp, lane < warps ? red_top[lane] : 0u);
-    float mx;
-    if constexpr (DT == HTR_DTYPE_F32) mx = __uint_as_float(top);
-    else if constexpr (DT == HTR_DTYPE_BF16) mx = __uint_as_float(top << 16);
-    else mx = __half2float(__ushort_as_half((unsigned short)top));
-    const float scale = range_scale(mx), inv = kInvSqrt128 / scale;
+  }
+  if constexpr (DT != HTR_DTYPE_F32) top = max(top >> 16, top & 0xFFFFu);
+  top = __reduce_max_sync(kFullWarp, top);
+  if (lane == 0) red_top[warp] = top;
+  __syncthreads();
+  top = __reduce_max_sync(kFullWarp, lane < warps ? red_top[lane] : 0u);
+  float mx;
+  if constexpr (DT == HTR_DTYPE_F32) mx = __uint_as_float(top);
+  else if constexpr (DT == HTR_DTYPE_BF16) mx = __uint_as_float(top << 16);
+  else mx = __half2float(__ushort_as_half((unsigned short)top));
+  const float scale = range_scale(mx), inv = kInvSqrt128 / scale;
 #pragma unroll 1
-    for (int g = warp; g < 2 * own; g += warps) {            // half of the blocks of a sum: four of every eight
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int g = warp; g < todo; g += warps) {                 // half of the blocks of a sum: four of every eight
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-      for (int i8 = 0; i8 < per; ++i8) {
-        const int hb = 8 * (per * (slice * own + (g >> 1)) + i8) + 4 * (g & 1) + (lane >> 3);
-        float2 v[8];
-        const int col = hb * 128 + 64 * u + 16 * c;
+    for (int i8 = 0; i8 < per; ++i8) {
+      const int hb = first + 8 * (per * (g >> 1) + i8) + 4 * (g & 1) + (lane >> 3);
+      float2 v[8];
+      const int col = hb * 128 + col0;
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const float4 q = real && hb < blocks && col + 4 * h < n_in ? load_quad(x, (size_t)r * n_in + col + 4 * h, DT) : make_float4(0.f, 0.f, 0.f, 0.f);
-          v[2 * h] = make_float2(q.x, q.y);
-          v[2 * h + 1] = make_float2(q.z, q.w);
-        }
-        const int byte = hb < blocks ? hb * 16 + 8 * u + 2 * c : 0;
-        const uint32_t signs = (uint32_t)su[byte] | ((uint32_t)su[byte + 1] << 8);
+      for (int h = 0; h < 4; ++h) {
+        const float4 q = hb < blocks && col + 4 * h < n_in ? load_quad(row, col + 4 * h, DT) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[2 * h] = make_float2(q.x, q.y);
+        v[2 * h + 1] = make_float2(q.z, q.w);
+      }
+      const int byte = hb < blocks ? col >> 3 : 0;
+      const uint32_t signs = (uint32_t)su[byte] | ((uint32_t)su[byte + 1] << 8);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = make_float2(flip(v[i].x, (signs >> (2 * i)) & 1u), flip(v[i].y, (signs >> (2 * i + 1)) & 1u));
+      for (int i = 0; i < 8; ++i) v[i] = make_float2(flip(v[i].x, (signs >> (2 * i)) & 1u), flip(v[i].y, (signs >> (2 * i + 1)) & 1u));
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = make_float2(v[i].x + v[i].y, v[i].x - v[i].y);
-        const float2 minus = make_float2(-1.f, -1.f);
+      for (int i = 0; i < 8; ++i) v[i] = make_float2(v[i].x + v[i].y, v[i].x - v[i].y);
+      const float2 minus = make_float2(-1.f, -1.f);
 #pragma unroll
-        for (int bit = 1; bit < 8; bit <<= 1)
+      for (int bit = 1; bit < 8; bit <<= 1)
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (!(i & bit)) {
-              const float2 a = v[i], b = v[i | bit];
-              v[i] = __fadd2_rn(a, b);
-              v[i | bit] = __ffma2_rn(b, minus, a);                    // a - b, as rounded
-            }
-#pragma unroll
-        for (int bit = 1; bit < 8; bit <<= 1) {
-          const float sgn = (lane & bit) ? -1.0f : 1.0f;               // the upper partner of a butterfly keeps (other - own)
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            v[i] = make_float2(fmaf(sgn, v[i].x, __shfl_xor_sync(kFullWarp, v[i].x, bit)), fmaf(sgn, v[i].y, __shfl_xor_sync(kFullWarp, v[i].y, bit)));
-        }
-        __half* const at = out + (size_t)hb * ncols * 128;
-        const bool store = real && hb < blocks;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          __half2 hi[2], lo[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float2 t = __fmul2_rn(v[2 * j + e], make_float2(inv, inv));
-            hi[e] = __float22half2_rn(t);
-            const float2 back = __half22float2(hi[e]);
-            lo[e] = __float22half2_rn(__ffma2_rn(back, minus, t));
-            const float2 rest = __half22float2(lo[e]);
-            sum[j] += planes == 2 ? back.x + rest.x : back.x;          // exactly what the MMA will see
-            sum[j] += planes == 2 ? back.y + rest.y : back.y;
+        for (int i = 0; i < 8; ++i)
+          if (!(i & bit)) {
+            const float2 a = v[i], b = v[i | bit];
+            v[i] = __fadd2_rn(a, b);
+            v[i | bit] = __ffma2_rn(b, minus, a);                    // a - b, as rounded
           }
-          if (store) *reinterpret_cast<uint2*>(at + 128 * j) = *reinterpret_cast<const uint2*>(hi);
-          if (store && planes == 2) *reinterpret_cast<uint2*>(at + 128 * j + to_lo) = *reinterpret_cast<const uint2*>(lo);
-        }
-      }
-      // the sum over the fours of a block, index 4 w + j in lane w: bits 4 and 3 by an exchange of halves (a lane keeps what its own bit says),
-      // then bits 2, 1 and 0
-      const int w = lane & 7;
-      const bool upper = w & 4, second = w & 2;
-      float a = (upper ? sum[2] : sum[0]) + __shfl_xor_sync(kFullWarp, upper ? sum[0] : sum[2], 4);
-      const float b = (upper ? sum[3] : sum[1]) + __shfl_xor_sync(kFullWarp, upper ? sum[1] : sum[3], 4);
-      a = (second ? b : a) + __shfl_xor_sync(kFullWarp, second ? a : b, 2);
-      a += __shfl_xor_sync(kFullWarp, a, 1);
-      a += __shfl_xor_sync(kFullWarp, a, 4);
-      a += __shfl_xor_sync(kFullWarp, a, 2);
-      if (w == 0) block_sum[4 * g + (lane >> 3)] = a;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < own; i += blockDim.x) {
-      float all = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) all += block_sum[8 * i + k];
-      const int at = slice * own + i;
-      if (real && at < sums) xsum[(size_t)r * sums + at] = all;
+      for (int bit = 1; bit < 8; bit <<= 1) {
+        const float sgn = (lane & bit) ? -1.0f : 1.0f;               // the upper partner of a butterfly keeps (other - own)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          v[i] = make_float2(fmaf(sgn, v[i].x, __shfl_xor_sync(kFullWarp, v[i].x, bit)), fmaf(sgn, v[i].y, __shfl_xor_sync(kFullWarp, v[i].y, bit)));
+      }
+      __half* const at = out + (size_t)hb * ncols * 128;
+      const bool store = hb < blocks;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        __half2 hi[2], lo[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float2 t = __fmul2_rn(v[2 * j + e], make_float2(inv, inv));
+          hi[e] = __float22half2_rn(t);
+          const float2 back = __half22float2(hi[e]);
+          lo[e] = __float22half2_rn(__ffma2_rn(back, minus, t));
+          const float2 rest = __half22float2(lo[e]);
+          sum[j] += planes == 2 ? back.x + rest.x : back.x;          // exactly what the MMA will see
+          sum[j] += planes == 2 ? back.y + rest.y : back.y;
+        }
+        if (store) *reinterpret_cast<uint2*>(at + 128 * j) = *reinterpret_cast<const uint2*>(hi);
+        if (store && planes == 2) *reinterpret_cast<uint2*>(at + 128 * j + to_lo) = *reinterpret_cast<const uint2*>(lo);
+      }
     }
-    if (real && slice == 0 && threadIdx.x == 0) tok[r] = scale;
+    // the sum over the fours of a block, index 4 w + j in lane w: bits 4 and 3 by an exchange of halves (a lane keeps what its own bit says),
+    // then bits 2, 1 and 0
+    const int w = lane & 7;
+    const bool upper = w & 4, second = w & 2;
+    float a = (upper ? sum[2] : sum[0]) + __shfl_xor_sync(kFullWarp, upper ? sum[0] : sum[2], 4);
+    const float b = (upper ? sum[3] : sum[1]) + __shfl_xor_sync(kFullWarp, upper ? sum[1] : sum[3], 4);
+    a = (second ? b : a) + __shfl_xor_sync(kFullWarp, second ? a : b, 2);
+    a += __shfl_xor_sync(kFullWarp, a, 1);
+    a += __shfl_xor_sync(kFullWarp, a, 4);
+    a += __shfl_xor_sync(kFullWarp, a, 2);
+    if (w == 0) block_sum[4 * g + (lane >> 3)] = a;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < own; i += blockDim.x) {
+    float all = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) all += block_sum[8 * i + k];
+    const int at = slice * own + i;
+    if (at < sums) xsum[(size_t)r * sums + at] = all;
+  }
+  if (slice == 0 && threadIdx.x == 0) tok[r] = scale;
+}
+
+// One block per warp and turn: grid (rows, sums of a row), 8 warps
+template <int DT>
+__global__ void __launch_bounds__(256) rht_f16_short_kernel(const void* __restrict__ x, int np, int n, int n_in, int planes,
+                                                            const uint8_t* __restrict__ su, __half* __restrict__ xb, float* __restrict__ xsum,
+                                                            float* __restrict__ tok, int per) {
+  __shared__ float red[8];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the GEMM may start fetching packed words now
+  const int r = blockIdx.x, slice = blockIdx.y, slices = gridDim.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int blocks = n >> 7;
+  const int hb0 = slice * 8 * per + warp;                    // this warp's 128-column blocks: hb0, hb0 + 8, ... (`per` of them)
+  const int ncols = np * planes;
+  const size_t unit_halves = (size_t)ncols * 64;
+  const size_t col_hi = (size_t)(r >> 3) * 512 + (r & 7) * 8, col_lo = (size_t)((np + r) >> 3) * 512 + ((np + r) & 7) * 8;
+  // four consecutive columns 4 lane .. + 3 of a block: tile c = (lane % 16) / 4, step j = lane % 4 of unit lane / 16
+  const int c = (lane & 15) >> 2, j = lane & 3;
+  const size_t in_unit = (size_t)(2 * j + (c >> 1)) * 64 + 4 * (c & 1);
+  auto tile_offset = [&](int hb) { return (size_t)(2 * hb + (lane >> 4)) * unit_halves + in_unit; };
+  const unsigned sg_first = hb0 < blocks ? sign_nibble(su, hb0 * 32 + lane) : 0u;   // the signs do not depend on earlier kernels
+  asm volatile("griddepcontrol.wait;" ::: "memory");         // x may come from the preceding kernel, the last GEMM may still read xb
+  // this lane's values of its first block: the load is in flight beside those of the scan
+  auto values = [&](int hb) {
+    const int col = hb * 128 + 4 * lane;
+    return hb < blocks && col < n_in ? load_quad(x, (size_t)r * n_in + col, DT) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  const float4 first = values(hb0);
+  // range of the whole row: magnitudes of floats compare like their bit patterns, so 16-bit pairs take the packed integer maximum
+  uint32_t top = 0u;
+  constexpr int kPer16 = DT == HTR_DTYPE_F32 ? 4 : 8;        // elements in 16 bytes
+  const uint4* row16 = reinterpret_cast<const uint4*>(static_cast<const char*>(x) + (size_t)r * n_in * (16 / kPer16));
+#pragma unroll 8
+  for (int e = tid; e < n_in / kPer16; e += 256) {
+    const uint4 v = __ldg(row16 + e);
+    if constexpr (DT == HTR_DTYPE_F32) {
+      constexpr uint32_t m = 0x7FFFFFFFu;
+      top = max(max(top, v.x & m), max(v.y & m, max(v.z & m, v.w & m)));
+    } else {
+      constexpr uint32_t m = 0x7FFF7FFFu;
+      top = __vmaxu2(__vmaxu2(top, v.x & m), __vmaxu2(v.y & m, __vmaxu2(v.z & m, v.w & m)));
+    }
+  }
+  if constexpr (DT != HTR_DTYPE_F32) top = max(top >> 16, top & 0xFFFFu);
+  top = __reduce_max_sync(kFullWarp, top);
+  if (lane == 0) red[warp] = __uint_as_float(top);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) top = max(top, __float_as_uint(red[k]));
+  float mx;
+  if constexpr (DT == HTR_DTYPE_F32) mx = __uint_as_float(top);
+  else if constexpr (DT == HTR_DTYPE_BF16) mx = __uint_as_float(top << 16);
+  else mx = __half2float(__ushort_as_half((unsigned short)top));
+  const float scale = range_scale(mx);
+  if (tid == 0 && slice == 0) tok[r] = scale;
+  const float inv = kInvSqrt128 / scale;
+  float sum = 0.f;
+#pragma unroll 2
+  for (int i = 0; i < per; ++i) {
+    const int hb = hb0 + 8 * i;
+    if (hb >= blocks) break;                                 // warp-uniform: the shuffles inside stay converged
+    const float4 mine = i == 0 ? first : values(hb);         // (second touch: L1)
+    const unsigned sg = i == 0 ? sg_first : sign_nibble(su, hb * 32 + lane);
+    float v[4] = {flip(mine.x, sg & 1u), flip(mine.y, (sg >> 1) & 1u), flip(mine.z, (sg >> 2) & 1u), flip(mine.w, sg >> 3)};
+    wht128(v, lane);
+    __half hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float t = v[k] * inv;
+      hi[k] = __float2half_rn(t);
+      lo[k] = __float2half_rn(t - __half2float(hi[k]));
+      sum += planes == 2 ? __half2float(hi[k]) + __half2float(lo[k]) : __half2float(hi[k]);   // exactly what the MMA will see
+    }
+    const size_t at = tile_offset(hb);
+    *reinterpret_cast<uint2*>(xb + at + col_hi) = *reinterpret_cast<const uint2*>(hi);
+    if (planes == 2) *reinterpret_cast<uint2*>(xb + at + col_lo) = *reinterpret_cast<const uint2*>(lo);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullWarp, sum, o);
+  __syncthreads();
+  if (lane == 0) red[warp] = sum;
+  __syncthreads();
+  if (tid == 0) {
+    float s = 0.f;
+    for (int k = 0; k < 8; ++k) s += red[k];
+    xsum[(size_t)r * slices + slice] = s;
   }
 }
 
@@ -345,34 +432,51 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
 int gemm_rht_per(int np, int n) { return min(max(np / 48, 1), (n + 1023) / 1024); }
 int gemm_xsums(int np, int n) { return (n / 128 + 8 * gemm_rht_per(np, n) - 1) / (8 * gemm_rht_per(np, n)); }
 
-// Slices of a row, warps of a thread block, rounds of the transform before a GEMM of `grid` thread blocks.  With 64 registers a thread, an
-// SM holds one thread block of 24 warps, two of 16, four of 8; `idle` SMs are free while the GEMM before (most often the same) runs, and a
-// GEMM in clusters loses where the transform needs others.  Long rows take 24 warps whatever the number, short ones have work for 8.
-// us (slices x warps): 4096x12288 K5 16 rows 1x24 / 2x24 18.3 / 20.5; 8 rows 2x24 / 4x24 16.7 / 18.4; 64 rows 1x8 / 2x24 26.1 / 21.8; 4096x4096 K4
-// 32 rows 1x16 / 1x24 9.6 / 11.2, 64 rows 1x8 / 1x16 11.7 / 12.6; 14720x12544 K2 28 float32 rows 1x24 / 2x24 54.2 / 50.7.  Beyond 48 rows the round
-// on zeros costs more than it saves, because other thread blocks wait for the place (4096x12288 128 rows 24.8 / 23.5).
-// Behind a GEMM that fills the GPU (but for three SMs) nothing is resident early: one round, and more thread blocks for few long rows (two rounds of two slices / one of
-// two / one of four: 7168x15104 K8 13 float32 rows 37.2 / 36.5 / 35.2, 18560x13696 K3 5 rows 64.1 / 63.6 / 62.8, 32768x4096 K4 5 rows 37.1 / 36.7 / 37.0).
+// Form, slices of a row and warps of the transform's thread blocks before a GEMM of `grid` thread blocks.  Below 2560 columns one block per
+// warp is better (figures above), but for more than 128 rows of 2048 columns and more (2048x2048 K4, 200 rows: 14.8 / 14.0 us in a chain; at 2560
+// columns, 48 rows, 10.1 / 9.5).  The rest is about the SMs that a GEMM in clusters leaves free, `idle`, taken from the GEMM that comes: in a
+// chain of layers the one before is most often like it, and behind another kernel the transform finds the GPU empty and the numbers matter
+// little.  An SM holds one thread block of 24 warps, two of 16 or four of 8 at 64 registers a thread.
+//  * A slice has work for two warps per 1024 columns: 8 warps up to 4096 columns (more rows than 64 take 16: 4096x4096 K4, 96 rows 14.8 / 13.9),
+//    16 up to 8192, 24 beyond (4096x12288 K5, 16 rows, 16 / 24: 18.2 / 18.0).  More than 128 rows fill the SMs with 16 (200 rows 36.7 / 34.2).
+//  * Two slices where all fit (4096x12288 K5, 8 rows, 1 / 2: 18.6 / 17.2), and where one would not fit either (37 rows 22.3 / 21.5; 4096x8192 K3,
+//    48 rows 17.6 / 16.6); between the two one slice, all of them at once (4096x8192 K3, 24 rows 14.4 / 15.7).
+//  * Where the GEMM before leaves no SM free, the transform comes when all of them are: more and larger thread blocks for few rows (12288x4096 K2,
+//    11 rows, one slice of 8 / two of 24: 19.9 / 18.5; 7168x15104 K8, 13 float32 rows, two / four of 24: 36.5 / 35.2).
 struct RhtShape {
-  int slices, warps, passes;
-  RhtShape(int rows, int n, int grid, int sms) {
+  bool quad;                                                 // four blocks per warp
+  int slices, warps;
+  RhtShape(int rows, int np, int n, int grid, int sms) {
     const int groups = (n + 511) / 512, idle = sms - grid;
-    const bool full = idle < 4 && groups >= 8;
-    warps = groups >= 9 ? (rows > 128 ? 16 : 24) : groups <= 4 || (idle >= 16 && rows > 2 * idle && rows <= 4 * idle) ? 8 : 16;
-    slices = groups < 8 ? 1 : idle >= rows ? (idle / rows < kRhtMaxSlices ? idle / rows : kRhtMaxSlices) : rows <= 16 || (rows <= 64 && groups >= 16) ? (full && rows <= 16 && groups > 16 ? 4 : 2) : 1;
-    slices = max(slices, (n + 128 * kRhtBlocks - 1) / (128 * kRhtBlocks));
-    passes = rows > 48 || full ? 1 : 2;
+    const bool full = idle < 4, all_fit = !full && 2 * rows <= idle;
+    quad = n >= 2560 || (n >= 2048 && rows > 128);
+    slices = gemm_xsums(np, n);
+    warps = 8;
+    if (!quad) return;
+    if (all_fit) warps = groups <= 16 ? 8 : groups <= 32 ? 16 : 24;      // (of half a row)
+    else if (rows > 128) warps = 16;
+    else if (full || groups > 16) warps = 24;
+    else warps = groups <= 8 && rows <= 64 ? 8 : 16;
+    if (full) slices = rows <= 16 && groups > 16 ? 4 : rows <= 64 ? 2 : 1;
+    else if (warps == 24) slices = all_fit || (rows > idle && rows <= 64) ? 2 : 1;
+    else slices = all_fit || (groups > 8 && rows > 2 * idle && rows <= 128) ? 2 : 1;
+    const int least = (n + 128 * kRhtBlocks - 1) / (128 * kRhtBlocks);
+    if (slices < least) slices = least;
   }
 };
 
 int run_rht_f16(const void* x, int dtype, int rows, int np, int n, int n_in, int planes, const RhtShape& shape, const uint8_t* su, __half* xb,
                 float* xsum, float* tok, cudaStream_t st) {
   const dim3 grid(rows, shape.slices);
-  const int threads = 32 * shape.warps;
+  const int threads = 32 * shape.warps, per = gemm_rht_per(np, n);
+  const auto launch = [&](auto type) {
+    constexpr int DT = decltype(type)::value;
+    return launch_chained(shape.quad ? rht_f16_kernel<DT> : rht_f16_short_kernel<DT>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, per);
+  };
   switch (dtype) {
-    case HTR_DTYPE_BF16: return launch_chained(rht_f16_kernel<HTR_DTYPE_BF16>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, gemm_rht_per(np, n), shape.passes);
-    case HTR_DTYPE_F16: return launch_chained(rht_f16_kernel<HTR_DTYPE_F16>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, gemm_rht_per(np, n), shape.passes);
-    default: return launch_chained(rht_f16_kernel<HTR_DTYPE_F32>, grid, threads, 0, st, x, np, n, n_in, planes, su, xb, xsum, tok, gemm_rht_per(np, n), shape.passes);
+    case HTR_DTYPE_BF16: return launch(std::integral_constant<int, HTR_DTYPE_BF16>{});
+    case HTR_DTYPE_F16: return launch(std::integral_constant<int, HTR_DTYPE_F16>{});
+    default: return launch(std::integral_constant<int, HTR_DTYPE_F32>{});
   }
 }
 
@@ -619,7 +723,7 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   p.stages = g.stages;
   p.withhold = t_gemm_withhold;
   p.m_out = m_out;
-  const RhtShape shape(M, n, g.grid, g.sms);
+  const RhtShape shape(M, g.np, n, g.grid, g.sms);
   p.xsum_slices = gemm_xsums(g.np, n);
   p.cb = (float)codebook_scale();
   p.plan = nullptr;
@@ -632,6 +736,21 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   e = launch_gemm(K, p, g.grid, g.smem, st);
   if (e) t_gemm_cuda = e;
   return e ? HTR_ERR_CUDA : HTR_OK;
+}
+
+int htr_linear_gemm_shape(int dtype, int M, int m, int n, int K, int* shape) {
+  if (!width_ok(K)) return HTR_ERR_BAD_K;
+  if (dtype < HTR_DTYPE_BF16 || dtype > HTR_DTYPE_F32) return HTR_ERR_BAD_DTYPE;
+  const int planes = gemm_planes(dtype, M, false);
+  if (M < 1 || M > (planes == 2 ? HTR_GEMM_MAX_ROWS_F32 : HTR_GEMM_MAX_ROWS) || m <= 0 || n <= 0 || m % 128 || n % 128) return HTR_ERR_BAD_SHAPE;
+  if (!shape) return HTR_ERR_NULL;
+  GemmPlan g;
+  const int rc = make_gemm_plan(M, m, n, K, planes, &g);
+  if (rc != HTR_OK) return rc;
+  const RhtShape r(M, g.np, n, g.grid, g.sms);
+  const int all[5] = {g.split, g.grid, r.quad ? 1 : 0, r.slices, r.warps};
+  for (int i = 0; i < 5; ++i) shape[i] = all[i];
+  return HTR_OK;
 }
 
 // ---- grouped form: the experts of a mixture-of-experts step

@@ -236,6 +236,9 @@ size_t htr_linear_gemm_error_offset(void);
  * block + block inside it) are never fetched, so that the bounded waits for them run out; block < 0: no longer. */
 void htr_gemm_withhold_tile(int block);
 int htr_linear_gemm_last_cuda_error(void);
+/* What htr_linear_gemm launches for these sizes on the current device (for tests and benches): shape[5] = thread blocks per row block (0: even
+ * runs), thread blocks, and of the activation transform 1 where a warp takes four blocks at a time, slices of a row, warps of a thread block. */
+int htr_linear_gemm_shape(int dtype, int M, int m, int n, int K, int* shape);
 int htr_linear_gemm(const void* x, int dtype, int M, const void* qweight, int mt, int nt, int K, const void* scales,
                     const uint8_t* su, const uint8_t* sv, const void* bias /* may be NULL */, void* y, void* workspace,
                     size_t workspace_bytes, htr_stream_t stream);
