@@ -340,8 +340,8 @@ __global__ void __launch_bounds__(kGroupRhtWarps * 32) rht_group_kernel(const vo
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int pair = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blocks = n >> 7;
-  // the row does not depend on the plan: its loads go out beside the chain slot -> expert -> signs, whose end is needed behind the barrier only
   const int slot = __ldcg(plan + group_plan_ints(cap) + pair);
+  if (slot < 0) return;                                      // no expert here (the whole thread block): nobody may have written the row
   const size_t row = (size_t)(pair / x_div) * x_stride;
   float v[kGroupRhtBlocks][4];
   float mx = 0.f;
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(kGroupRhtWarps * 32) rht_group_kernel(const vo
     v[i][0] = q.x; v[i][1] = q.y; v[i][2] = q.z; v[i][3] = q.w;
     mx = fmaxf(mx, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
   }
-  if (slot < 0) return;                                      // no expert here (the whole thread block)
+  // the signs come from the end of a chain, slot -> expert -> signs, beside the row's loads: they are needed behind the barrier only
   const int t = slot / kGroupRows, r = slot % kGroupRows;
   const uint8_t* su = su_table[group_expert(plan, cap, t)];
   unsigned sg[kGroupRhtBlocks];

@@ -39,3 +39,10 @@ def test_no_thread_block_of_the_gemm_leaves_before_its_transform():
     start = start[:start.index("tcgen05.alloc")]
     for at in re.finditer(r"\breturn\b", start):
         assert re.search(r'"griddepcontrol\.wait;" ::: "memory"\);\s*$', start[:at.start()]), start[at.start() - 120:at.start()]
+
+
+def test_pairs_without_an_expert_are_left_before_their_row_is_read():
+    """The row of such a pair may never have been written (a gate_up launch skips it too), and reading it costs as much as a pair with work."""
+    text = source(os.path.join(CSRC, "gemm_api.cu"))
+    kernel = text[text.index("rht_group_kernel(const void*"):]
+    assert 0 < kernel.index("if (slot < 0) return;") < kernel.index("load_quad(x")
