@@ -718,7 +718,7 @@ static int gemm_launch(const void* x, int dtype, int M, int n_in, const void* qw
   p.split = g.split;
   p.run_q = g.split > 0 ? g.hb / g.split : g.rbs * g.hb / g.grid;
   p.run_rem = g.split > 0 ? g.hb % g.split : g.rbs * g.hb % g.grid;
-  p.part_magic = g.split > 0 ? (65536 + g.split - 1) / g.split : 0;
+  p.part_magic = g.split > 0 ? part_reciprocal(g.split) : 0;
   p.inbox = g.inbox;
   p.stages = g.stages;
   p.withhold = t_gemm_withhold;

@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "../../include/htr_b200.h"
+#include "run_arith.cuh"
 
 namespace htr {
 
@@ -88,14 +89,5 @@ __device__ __forceinline__ void cluster_sync() {
   cluster_arrive();
   cluster_wait();
 }
-
-// even contiguous runs of `units` over `grid` thread blocks: the first `rem` of them hold one more
-struct EvenRuns {
-  int q, rem;
-  __device__ __forceinline__ EvenRuns(int quotient, int remainder, int) : q(quotient), rem(remainder) {}   // divided elsewhere
-  __device__ __forceinline__ EvenRuns(int units, int grid) : q(units / grid), rem(units - (units / grid) * grid) {}
-  __device__ __forceinline__ int begin(int b) const { return b * q + min(b, rem); }
-  __device__ __forceinline__ int owner(int u) const { return u < rem * (q + 1) ? u / (q + 1) : rem + (u - rem * (q + 1)) / q; }
-};
 
 }  // namespace htr

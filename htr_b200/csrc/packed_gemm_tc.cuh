@@ -23,8 +23,9 @@
 //    Tensor-memory lane l < 8 of a strip holds weight row 2l, lane 8 + l row 2l + 1, and MMA step j takes columns 4j..4j+3 of each
 //    of the four tiles; the activation transform writes B in that k order.
 // The packed words take a ring per warp (16-byte cp.async, all slots but one in flight): plain loads into registers one block ahead
-// keep 16 KB per SM in flight and measured 12 weights per cycle and SM, the ring 22 (at any depth from 3 slots on), which is the
-// decode alone: 4.8 instructions per weight at 82 % of the issue slots.
+// keep 16 KB per SM in flight and measured 12 weights per cycle and SM, the ring 17 over the launch of an LM head (151936x4096 K4, 8 rows: 622
+// million weights in 127 us; the same at any depth from 3 slots on), at 80 % of the issue slots: 5.6 instructions a weight over the launch, of
+// which the decode unit is about four.
 //
 // Roles (22 warps, one thread block per SM).  Warps 0-15 decode, as two groups of eight that take alternate 128-column blocks;
 // inside a group warp w owns tensor-memory quadrant w % 4 and strip 2 (w % 4) + (w / 4) % 2.  One lane of warp 16 brings the B tile
@@ -42,10 +43,11 @@
 //
 // Decomposition.  Work = (row block) x (128-column blocks).  Where the row blocks are few, `split` thread blocks share one as a
 // cluster: each sends its partial sums of a row into the shared memory of the one that finishes that row (st.async, up to 64 rows), or,
-// where no inbox fits or the rows are many, fetches the others' between two cluster barriers.  4096x12288 K3, 4 rows: 17.1 -> 16.5 us for
-// the inbox.  Else every thread block takes an even contiguous run that may cross row blocks (flat), publishes a partial [np][128] per row block it touches, and the last arriver adds them in thread-block order.
-// Both are deterministic and nobody waits for another thread block except inside a cluster.  One thread block per SM, not two: the
-// partial sums of a row block are half as many, and no SM waits for the slower of two.
+// where no inbox fits or the rows are many, fetches the others' between two cluster barriers.  4096x12288 K3, 4 rows: 17.1 -> 16.5 us
+// for the inbox.  Else every thread block takes an even contiguous run that may cross row blocks (flat), publishes a partial [np][128]
+// per row block it touches, and the last arriver adds them in thread-block order.  Both are deterministic and nobody waits for another
+// thread block except inside a cluster.  One thread block per SM, not two: the partial sums of a row block are half as many, and no SM
+// waits for the slower of two.
 //
 // Every wait on an mbarrier is bounded: when it expires the thread block records an error code, stops issuing work, waits (bounded)
 // for its copies and MMAs in flight, writes NaN into the rows it owed, frees its tensor memory and returns; the host sees the code
@@ -91,7 +93,7 @@ struct GemmParams {
   int split;              // > 0: thread blocks per row block (cluster form); 0: flat ranges
   int run_q, run_rem;     // blocks of a thread block's run: run_q, one more for the first run_rem (cluster form: hb / split and the remainder,
                           // parts from block part * hb / split on)
-  int part_magic;         // 65536 / split, rounded up
+  int part_magic;         // part_reciprocal(split)
   int inbox;              // > 0: offset in shared memory where a thread block of a cluster receives the partial sums of its rows; 0: the
                           // partials stay where they are and are fetched from there (many activation rows)
   int stages;
@@ -432,12 +434,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       asm("mov.u32 %0, %%clusterid.x;" : "=r"(rb0));
       asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(part_id));
     }
-    // part * HB / split, the quotient of the remainders by a reciprocal (exact: at most 16 * 15 by at most 16).  The last part is always one
-    // of the longer ones: it goes to the first thread block of the cluster, which starts first (2944x1664 K6, 37 rows: 8.3 -> 8.0 us)
+    // The last part is always one of the longer ones: it goes to the first thread block of the cluster, which starts first (2944x1664 K6, 37
+    // rows: 8.3 -> 8.0 us)
     part = p.split - 1 - part_id;
-    hb0 = part * p.run_q + ((part * p.run_rem * p.part_magic) >> 16);
+    hb0 = part_begin(part, p.run_q, p.run_rem, p.part_magic);
     u_begin = rb0 * HB + hb0;
-    u_end = rb0 * HB + (part + 1) * p.run_q + (((part + 1) * p.run_rem * p.part_magic) >> 16);
+    u_end = rb0 * HB + part_begin(part + 1, p.run_q, p.run_rem, p.part_magic);
   } else {
     u_begin = runs.begin(blockIdx.x);
     u_end = runs.begin(blockIdx.x + 1);
@@ -603,7 +605,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
       parity ^= around ? 1u : 0u;
     }
     if constexpr (GROUP)
-      if (ok) deliver(stored);                               // (a warp that gave up has told of all that it stored: a second arrival would count for the next round)
+      if (ok) deliver(stored);                               // (a warp that gave up has told of all it stored: another arrival counts for the next round)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (!GROUP && p.split > 0) {
       // these loads, and the wait for the transform that they need, lie beside the last MMAs; then the accumulator goes to the ring as
@@ -796,8 +798,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) packed_gemm_tc_kernel(const G
   }
   if (!GROUP && p.inbox > 0) {
     // ---- reduction inside the cluster: every thread block has sent its partials of row j to thread block j % split, which adds them in the
-    // order of the parts and finishes the row.  (Partials fetched from where they were made wait for a barrier of the cluster before and one after, so
-    // that nobody leaves too early, 1.5 us together.)
+    // order of the parts and finishes the row.  (Partials fetched from where they were made wait for a barrier of the cluster before and one
+    // after, so that nobody leaves too early, 1.5 us together.)
     if (warp < DW) {
       // A peer whose own wait gave up still sends, but up to two of its limits later, and into shared memory that must not be gone by then.
       bool here = mbar_wait<true>(smem_u32(&s_inbox), 0u, nullptr);

@@ -109,7 +109,6 @@ struct GemvParams {
   unsigned grid_magic, hb_magic;
   float per_unit, per_cg;
 };
-inline unsigned reciprocal(int divisor) { return divisor > 1 ? (unsigned)((0x100000000ull + divisor - 1) / divisor) : 0u; }
 // the fields of p that FlatRuns needs, for a launch of `grid` thread blocks in the flat form
 inline void set_flat_runs(GemvParams& p, int grid) {
   p.run_q = p.units / grid;
@@ -164,33 +163,6 @@ __device__ __forceinline__ float4 fused_x(const GemvParams& p, const void* x, in
   }
   return load_x(x, r, col, p.n_in, p.dtype);
 }
-
-// owner CTA of unit x when CTA b starts at floor(b*U/G)
-__device__ __host__ inline int unit_owner(long long x, long long G, long long U) { return (int)(((x + 1) * G - 1) / U); }
-// The same without a division, which is dozens of cold instructions (64 bits: a subroutine) at the start of every thread block and
-// between its last sum and its partial.  Quotients come as the upper product with ceil(2^32 / divisor), exact while dividend times divisor
-// stays below 2^32 (here less than grid^3; 0 stands for the divisor 1), or from a float32 guess that is then corrected.
-__device__ __forceinline__ int quotient(int x, unsigned magic) { return magic ? (int)__umulhi((unsigned)x, magic) : x; }
-__device__ __forceinline__ int quotient(int x, int divisor, float reciprocal) {
-  int q = (int)((float)x * reciprocal);
-  while (q * divisor > x) --q;
-  while (x - q * divisor >= divisor) ++q;
-  return q;
-}
-struct FlatRuns {
-  int q, rem;             // U / G, U % G
-  unsigned grid_magic;
-  float per_unit;         // G / U
-  __device__ __forceinline__ explicit FlatRuns(const GemvParams& p) : q(p.run_q), rem(p.run_rem), grid_magic(p.grid_magic), per_unit(p.per_unit) {}
-  __device__ __forceinline__ int begin(int b) const { return b * q + quotient(b * rem, grid_magic); }
-  __device__ __forceinline__ int owner(int x) const {
-    int b = (int)(((float)x + 0.5f) * per_unit);
-    while (begin(b) > x) --b;
-    while (begin(b + 1) <= x) ++b;
-    return b;
-  }
-};
-
 
 __device__ __forceinline__ void async_copy16(uint32_t smem_addr, const void* gptr) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gptr) : "memory");
@@ -313,7 +285,7 @@ __global__ void __launch_bounds__(kGemvThreads, (MT == 1 ? 3 : MT == 2 ? 2 : 1))
   const int CG = p.cg, nt = p.nt, n = nt * 16, m = p.mt * 16;
   // split form: grid (split, row blocks), the parts of a row block differ by at most one unit; flat form: even unit ranges
   int u_begin, u_end, slot_index;
-  const FlatRuns runs(p);
+  const FlatRuns runs(p.run_q, p.run_rem, p.grid_magic, p.per_unit);
   if (p.split > 0) {
     const int part = blockIdx.x, base = blockIdx.y * CG;
     u_begin = base + part * p.cg_quot + min(part, p.cg_rem);

@@ -80,11 +80,3 @@ def test_one_row_at_the_widths_where_the_staging_changes(coracle, m, n):
     x = torch.randn(1, n, generator=torch.Generator().manual_seed(n))
     ref = coracle.linear(x.numpy(), qw.numpy(), sc.numpy(), su.numpy(), sv.numpy())
     assert rel(ops.linear(x.to(dev), *d).cpu().numpy(), ref) <= 5e-6
-
-
-def test_run_boundaries_by_reciprocal():
-    """The quotient by the blocks of a row block, as the launcher and the kernel form it, over everything that a workspace admits."""
-    for hb in list(range(2, 129)):
-        magic = (2 ** 32 + hb - 1) // hb
-        u = np.unique(np.concatenate([np.arange(0, 4 * hb), np.arange(1, 16385) * hb - 1, np.arange(1, 16385) * hb])).astype(np.uint64)
-        assert np.array_equal((u * np.uint64(magic)) >> np.uint64(32), u // np.uint64(hb))

@@ -89,6 +89,15 @@ def test_kernel_decode_arithmetic_on_the_host(tmp_path):
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout
 
 
+def test_runs_and_quotients_without_divisions(tmp_path):
+    """csrc/run_arith.cuh, from which the launchers and the kernels take their runs, compiled for the host and compared with exact division: one,
+    remainder 0, units just at the grid, and units beyond 2^24, where a float guess is not exact."""
+    exe = tmp_path / "host_runs_check"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-o", str(exe), os.path.join(ROOT, "tests", "host_runs_check.cpp")], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout
+
+
 def test_wire_helpers_agree_with_the_oracle(lib):
     from htr_b200 import wire
     from oracle import oracle as O
