@@ -14,11 +14,12 @@
 // What bounds it: per candidate the reference's operations x - c, d * d, w * (d * d), prev + ... occupy the FMA pipes for four
 // cycles of a warp (packed or not), so everything else has to go:
 //  * No step looks for the argument of a minimum (a comparison and two selects per candidate, half as much again as the four
-//    operations).  Every kLevels-th row of minima is kept in global memory instead (5 to 11 KB a step), and the way back computes the
+//    operations).  Every kLevels-th row of minima is kept in global memory instead (1 to 11 KB a step, K = 8 to 2), and the way back computes the
 //    few costs it meets again: from a state, the 2^(K kLevels) ancestors at the next kept row (vit_trace).  The first minimum of
 //    three operands at a time is one instruction for two candidates.
-//  * A thread owns the same states in every step, hence the same codebook values: three quarters of them stay in registers, the rest
-//    in shared memory (one 16-byte read per four; K = 2 has no room there and recomputes them from the state hash).
+//  * A thread owns the same states in every step, hence the same codebook values.  One block per tile or two tiles per block: three
+//    quarters of them stay in registers, the rest in shared memory (one 16-byte read per four); K = 2, whose cost arrays leave no room
+//    there, keeps half in registers and computes the others from the state hash.  Clusters: all in registers.
 //  * More tiles than thread blocks: a block takes two tiles step by step together, so that a value from shared memory serves both and a
 //    block barrier has twice the work on either side.  (Two tiles in turn, each with a barrier that is waited for only after the other
 //    tile's step, were slower: 0.75 against 0.67 ms a tile and two passes.)
@@ -57,7 +58,8 @@ struct VitParams {
   float one;         // 1, unknown to the compiler
 };
 
-// C: thread blocks of the cluster that share one tile (1, 2 or 4): each owns SJ / C consecutive j; N: tiles that a thread block works on in turn
+// C: thread blocks of the cluster that share one tile (1, 2 or 4): each owns SJ / C consecutive j; N: tiles that a thread block
+// works on step by step together
 template <int K, int C, int N>
 struct VitCfg {
   static constexpr int kNB = 1 << K, kSj = 1 << (16 - K);
@@ -70,6 +72,7 @@ struct VitCfg {
   static constexpr int kPer = kStates / kTT;                              // j of a thread
   static constexpr int kJb = K == 2 ? 4 : kPer < 8 ? kPer : 8;            // consecutive j of a group: they share their predecessor minima
   static constexpr int kGroups = kPer / kJb;                              // groups of a thread
+  static_assert(kJb % 4 == 0, "costs are handled four at a time");
   static constexpr int kPairs = kJb / 2;                                  // candidates are handled two at a time
   static constexpr int kBlocks = kStates / kJb;                           // (group, top) blocks of kJb states, in that order
   static constexpr int kRegBlocks = C > 1 ? kBlocks : kThreads == 512 ? kBlocks / 2 : kBlocks * 3 / 4;   // ... whose codebook values stay in registers
@@ -106,26 +109,18 @@ __device__ __forceinline__ float state_cost(uint32_t s, float prev, float xt, fl
 template <int C, int JB>
 __device__ __forceinline__ void spread_costs(float* at, const float (&v)[JB]) {
   if constexpr (C == 1) {
-    if constexpr (JB % 4 == 0) {
 #pragma unroll
-      for (int q = 0; q < JB / 4; ++q) *reinterpret_cast<float4*>(at + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-    } else {
-      *reinterpret_cast<float2*>(at) = make_float2(v[0], v[1]);
-    }
+    for (int q = 0; q < JB / 4; ++q) *reinterpret_cast<float4*>(at + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
   } else {
     const uint32_t mine = (uint32_t)__cvta_generic_to_shared(at);
 #pragma unroll
     for (int r = 0; r < C; ++r) {
       uint32_t to;
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine), "r"(r));
-      if constexpr (JB % 4 == 0) {
 #pragma unroll
-        for (int q = 0; q < JB / 4; ++q)
-          asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + 16 * q), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
-                       : "memory");
-      } else {
-        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(v[0]), "f"(v[1]) : "memory");
-      }
+      for (int q = 0; q < JB / 4; ++q)
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + 16 * q), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                     : "memory");
     }
   }
 }
@@ -178,7 +173,7 @@ __device__ __forceinline__ void vit_step(float* __restrict__ mem, int cur, int t
       const int blk = g * TT + tt;
       if (blk < Cfg::kRegBlocks) {
         nc[0] = negc[blk * PAIRS + 2 * q];
-        nc[1] = negc[blk * PAIRS + (2 * q + 1 < PAIRS ? 2 * q + 1 : 2 * q)];
+        nc[1] = negc[blk * PAIRS + 2 * q + 1];
       } else if constexpr (Cfg::kTable) {
         const float4 f = table[((blk - Cfg::kRegBlocks) * (PAIRS / 2) + q) * Cfg::kThreads];
         nc[0] = make_float2(f.x, f.y);
@@ -204,7 +199,7 @@ __device__ __forceinline__ void vit_step(float* __restrict__ mem, int cur, int t
 #pragma unroll
     for (int tt = 0; tt < TT; tt += 2)
 #pragma unroll
-      for (int q = 0; q < (PAIRS + 1) / 2; ++q) {
+      for (int q = 0; q < PAIRS / 2; ++q) {
         float2 na[2], nb[2];
         values(tt, q, na);
         values(tt + 1, q, nb);
@@ -213,7 +208,6 @@ __device__ __forceinline__ void vit_step(float* __restrict__ mem, int cur, int t
           const float pa = prev_col[h * Cfg::kTileFloats + (tt << SH)], pb = prev_col[h * Cfg::kTileFloats + ((tt + 1) << SH)];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            if (2 * q + e >= PAIRS) break;
             const float2 va = cost(h, na[e], pa), vb = cost(h, nb[e], pb);
             best[h][4 * q + 2 * e] = min3(best[h][4 * q + 2 * e], va.x, vb.x);
             best[h][4 * q + 2 * e + 1] = min3(best[h][4 * q + 2 * e + 1], va.y, vb.y);
@@ -360,7 +354,7 @@ __global__ void __launch_bounds__(VitCfg<K, C, N>::kThreads, 1) viterbi_kernel(c
   const int T = p.T, kept = (T - 1) / Cfg::kLevels;
   const int at_once = gridDim.x / C * N, cluster = blockIdx.x / C, rank = blockIdx.x % C, j_first = rank * (SJ / C);
 
-  // the negated codebook values of this thread's states, in block order (group, top): in registers, or half of them in shared memory
+  // the negated codebook values of this thread's states, in block order (group, top): in registers, the last ones in shared memory where there is a table
   float2 negc[Cfg::kRegBlocks * PAIRS];
 #pragma unroll
   for (int blk = 0; blk < (Cfg::kTable ? Cfg::kBlocks : Cfg::kRegBlocks); ++blk) {
