@@ -439,10 +439,12 @@ int gemm_xsums(int np, int n) { return (n / 128 + 8 * gemm_rht_per(np, n) - 1) /
 // little.  An SM holds one thread block of 24 warps, two of 16 or four of 8 at 64 registers a thread.
 //  * A slice has work for two warps per 1024 columns: 8 warps up to 4096 columns (more rows than 64 take 16: 4096x4096 K4, 96 rows 14.8 / 13.9),
 //    16 up to 8192, 24 beyond (4096x12288 K5, 16 rows, 16 / 24: 18.2 / 18.0).  More than 128 rows fill the SMs with 16 (200 rows 36.7 / 34.2).
-//  * Two slices where all fit (4096x12288 K5, 8 rows, 1 / 2: 18.6 / 17.2), and where one would not fit either (37 rows 22.3 / 21.5; 4096x8192 K3,
-//    48 rows 17.6 / 16.6); between the two one slice, all of them at once (4096x8192 K3, 24 rows 14.4 / 15.7).
+//  * Two slices where all fit (4096x12288 K5, 8 rows, 1 / 2: 18.6 / 17.2), four for long rows if they do (1024x16256 K4, 2 rows, 2 / 4: 11.2 / 10.4),
+//    and two where one would not fit either (4096x12288 37 rows 22.3 / 21.5; 4096x8192 K3, 48 rows 17.6 / 16.6); between the two one slice, all
+//    of them at once (4096x8192 K3, 24 rows 14.4 / 15.7).
 //  * Where the GEMM before leaves no SM free, the transform comes when all of them are: more and larger thread blocks for few rows (12288x4096 K2,
-//    11 rows, one slice of 8 / two of 24: 19.9 / 18.5; 7168x15104 K8, 13 float32 rows, two / four of 24: 36.5 / 35.2).
+//    11 rows, one slice of 8 / two of 24: 19.9 / 18.5; 2 rows two of 24 / four of 8: 19.8 / 18.1; 7168x15104 K8, 13 float32 rows, two / four of
+//    24: 36.5 / 35.2).
 struct RhtShape {
   bool quad;                                                 // four blocks per warp
   int slices, warps;
@@ -453,11 +455,14 @@ struct RhtShape {
     slices = gemm_xsums(np, n);
     warps = 8;
     if (!quad) return;
-    if (all_fit) warps = groups <= 16 ? 8 : groups <= 32 ? 16 : 24;      // (of half a row)
+    const bool four = full ? rows <= (groups > 16 ? 16 : 4) : groups > 16 && 4 * rows < idle;
+    if (all_fit) warps = groups <= 16 || four ? 8 : groups <= 32 ? 16 : 24;   // (of half a row or a quarter)
+    else if (full && four && groups <= 16) warps = 8;
     else if (rows > 128) warps = 16;
     else if (full || groups > 16) warps = 24;
     else warps = groups <= 8 && rows <= 64 ? 8 : 16;
-    if (full) slices = rows <= 16 && groups > 16 ? 4 : rows <= 64 ? 2 : 1;
+    if (four) slices = 4;
+    else if (full) slices = rows <= 64 ? 2 : 1;
     else if (warps == 24) slices = all_fit || (rows > idle && rows <= 64) ? 2 : 1;
     else slices = all_fit || (groups > 8 && rows > 2 * idle && rows <= 128) ? 2 : 1;
     const int least = (n + 128 * kRhtBlocks - 1) / (128 * kRhtBlocks);

@@ -120,17 +120,17 @@ def transform(dtype, M, m, n, K):
 
 TRANSFORM_SIZES = ((128, 128), (128, 384), (128, 2176), (256, 2048), (4096, 4096), (128, 8320), (4096, 6144), (4096, 12288), (128, 16512), (128, 65664),
                    (19072, 4224), (19072, 12288))
-TRANSFORM_ROWS = (5, 8, 9, 16, 17, 24, 37, 48, 49, 64, 65, 100, 128, 129, 200, 256)
+TRANSFORM_ROWS = (3, 5, 8, 9, 16, 17, 24, 37, 48, 49, 64, 65, 100, 128, 129, 200, 256)
 
 
 def test_every_form_of_the_transform_is_among_the_tested():
-    """Form and warps, and one slice or two where four blocks go to a warp, over all sizes that the rule looks at."""
+    """Form, warps, and slices where four blocks go to a warp, over the sizes that the rule looks at."""
     def form(shape):
-        return (shape[2], shape[4], min(shape[3], 2) if shape[2] else 0)
+        return (shape[2], shape[4], shape[3] if shape[2] else 0)
 
     tested = {form(transform(torch.bfloat16, M, m, n, 3)) for m, n in TRANSFORM_SIZES for M in TRANSFORM_ROWS}
     every = {form(transform(torch.bfloat16, M, m, n, 3)) for m in (128, 1024, 2048, 4096, 8192, 12288, 19072) for n in
-             (*range(128, 4480, 128), 5120, 6144, 8192, 8320, 10240, 12288, 16384, 66048) for M in range(5, 257)}
+             (*range(128, 4480, 128), 5120, 6144, 8192, 8320, 10240, 12288, 16384, 16512, 65664) for M in range(2, 257)}
     assert tested == every and len(every) >= 6, (tested, every)
 
 
