@@ -442,9 +442,9 @@ int gemm_xsums(int np, int n) { return (n / 128 + 8 * gemm_rht_per(np, n) - 1) /
 //  * Two slices where all fit (4096x12288 K5, 8 rows, 1 / 2: 18.6 / 17.2), four for long rows if they do (1024x16256 K4, 2 rows, 2 / 4: 11.2 / 10.4),
 //    and two where one would not fit either (4096x12288 37 rows 22.3 / 21.5; 4096x8192 K3, 48 rows 17.6 / 16.6); between the two one slice, all
 //    of them at once (4096x8192 K3, 24 rows 14.4 / 15.7).
-//  * Where the GEMM before leaves no SM free, the transform comes when all of them are: more and larger thread blocks for few rows (12288x4096 K2,
-//    11 rows, one slice of 8 / two of 24: 19.9 / 18.5; 2 rows two of 24 / four of 8: 19.8 / 18.1; 7168x15104 K8, 13 float32 rows, two / four of
-//    24: 36.5 / 35.2).
+//  * Where the GEMM before leaves no SM free, the transform comes when all of them are: larger thread blocks (12288x4096 K2, 11 rows, 8 / 24 warps:
+//    19.9 / 18.5), and more for few rows (2 rows, one slice of 8 / four: 18.4 / 18.1; 7168x15104 K8, 13 float32 rows, two / four of 24: 36.5 /
+//    35.2) and long ones (18560x13696 K3, 16 rows, one / two: 64.3 / 62.4).
 struct RhtShape {
   bool quad;                                                 // four blocks per warp
   int slices, warps;
@@ -462,7 +462,7 @@ struct RhtShape {
     else if (full || groups > 16) warps = 24;
     else warps = groups <= 8 && rows <= 64 ? 8 : 16;
     if (four) slices = 4;
-    else if (full) slices = rows <= 64 ? 2 : 1;
+    else if (full) slices = groups > 16 && rows <= 64 ? 2 : 1;
     else if (warps == 24) slices = all_fit || (rows > idle && rows <= 64) ? 2 : 1;
     else slices = all_fit || (groups > 8 && rows > 2 * idle && rows <= 128) ? 2 : 1;
     const int least = (n + 128 * kRhtBlocks - 1) / (128 * kRhtBlocks);

@@ -41,7 +41,8 @@ struct FlatRuns {
   int q, rem;
   unsigned grid_magic;
   float per_unit;
-  HTR_HD FlatRuns(int quotient, int remainder, unsigned magic, float blocks_per_unit) : q(quotient), rem(remainder), grid_magic(magic), per_unit(blocks_per_unit) {}
+  HTR_HD FlatRuns(int quotient, int remainder, unsigned magic, float blocks_per_unit)
+      : q(quotient), rem(remainder), grid_magic(magic), per_unit(blocks_per_unit) {}
   HTR_HD int begin(int b) const { return b * q + quotient(b * rem, grid_magic); }
   HTR_HD int owner(int x) const {
     int b = (int)(((float)x + 0.5f) * per_unit);

@@ -253,7 +253,8 @@ def gemm_into_peers(x2, qweight, scales, su, sv, bias, peer_ptrs, elem_offset):
 
 
 def gemm_error_codes():
-    """Status words of the GEMM workspaces (synchronises; for tests): non-zero means a bounded device-side wait expired."""
+    """Status words of the GEMM workspaces (synchronises; for tests): non-zero means a bounded device-side wait expired, and that the workspace
+    is to be zeroed before its next use."""
     off = _lib.lib.htr_linear_gemm_error_offset()
     return [int(ws[off:off + 4].view(torch.int32).item()) for ws in _GEMM_WS.values()]
 
