@@ -25,9 +25,9 @@ namespace htr {
 //    a whole row or half of one.  Few thread blocks matter before a GEMM in clusters: those that do not fit on the SMs that the GEMM before
 //    leaves free keep its successor's clusters waiting.
 // us for transform + GEMM in a chain (graph) and behind an elementwise kernel, one block per warp / four: 1024x640 K4 16 rows 5.3, 7.2 / 5.7,
-// 7.3; 2048x2048 K4 96 rows 9.7, 11.5 / 10.3, 12.1; 4096x4096 K4 37 rows 11.8, 12.1 / 9.6, 12.8; 4096x12288 K5 16 rows 20.9, 21.4 / 17.9, 19.8.
-// (All warps through the code once on zeros before the wait, to fetch its instructions: 0 to 0.3 us less in a chain, where the wait is long, and
-// 0.7 to 1.7 more behind a kernel that lets its successors go at its end only; 4096x12288 K5 16 rows 17.7, 21.5.)
+// 7.3; 2048x2048 K4 96 rows 9.7, 11.5 / 10.3, 12.1; 4096x4096 K4 37 rows 11.8, 12.1 / 9.6, 12.8; 4096x12288 K5 16 rows 20.9, 21.4 / 17.7, 19.8.
+// (All warps through the code once on zeros before the wait, to fetch its instructions: nothing in a chain, where the wait is long, and 0.7 to
+// 1.7 us more behind a kernel that lets its successors go at its end only; 4096x12288 K5 16 rows 17.7, 21.4.)
 //
 // Range scale of a row: the power of two 2^k with max|x| * sqrt(128) in (2^13, 2^14] * 2^k, in both directions, so that neither a large
 // row leaves the fp16 range nor a small one sinks into its subnormals (fp16 numbers are 2^-24 apart below 2^-14: unscaled, a row of
@@ -54,18 +54,16 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
   const int u = (lane >> 2) & 1, c = lane & 3;               // this lane's tile inside a block of a group
   const int ncols = np * planes;
   // column 16 c + 4 j + e of unit u goes to position 16 j + 4 c + e
-  __half* out = xb + (size_t)u * ncols * 64 + (size_t)(r >> 3) * 512 + (r & 7) * 8 + (c >> 1) * 64 + 4 * (c & 1);
-  size_t to_lo = (size_t)(np >> 3) * 512;
+  __half* const out = xb + (size_t)u * ncols * 64 + (size_t)(r >> 3) * 512 + (r & 7) * 8 + (c >> 1) * 64 + 4 * (c & 1);
+  const size_t to_lo = (size_t)(np >> 3) * 512;
   constexpr int kPer16 = DT == HTR_DTYPE_F32 ? 4 : 8;        // elements in 16 bytes
-  const char* row = static_cast<const char*>(x) + (size_t)r * n_in * (16 / kPer16);
-  int todo = 2 * own, first = 8 * per * slice * own, col0 = 64 * u + 16 * c;
-  // x may come from the preceding kernel, the last GEMM may still read xb.  Operands of the wait are computed before it, while there is time
-  // (left to the compiler, behind it, in cold code: 4096x4096 K4, 256 rows 20.9 -> 21.3 us)
-  asm volatile("griddepcontrol.wait;" : "+l"(out), "+l"(to_lo), "+l"(row), "+r"(todo), "+r"(first), "+r"(col0) : : "memory");
+  const char* const row = static_cast<const char*>(x) + (size_t)r * n_in * (16 / kPer16);
+  const int first = 8 * per * slice * own, col0 = 64 * u + 16 * c;
+  asm volatile("griddepcontrol.wait;" ::: "memory");         // x may come from the preceding kernel, the last GEMM may still read xb
   // range of the whole row: magnitudes of floats compare like their bit patterns, so 16-bit pairs take the packed integer maximum
   uint32_t top = 0u;
   const uint4* row16 = reinterpret_cast<const uint4*>(row);
-#pragma unroll 4
+#pragma unroll 1                                             // (few turns, and every line is fetched cold: by four, 4096x12288 K5, 16 rows 17.7 -> 18.0 us)
   for (int e = threadIdx.x; e < n_in / kPer16; e += blockDim.x) {
     const uint4 v = __ldg(row16 + e);
     if constexpr (DT == HTR_DTYPE_F32) {
@@ -87,7 +85,7 @@ __global__ void __launch_bounds__(1024) rht_f16_kernel(const void* __restrict__ 
   else mx = __half2float(__ushort_as_half((unsigned short)top));
   const float scale = range_scale(mx), inv = kInvSqrt128 / scale;
 #pragma unroll 1
-  for (int g = warp; g < todo; g += warps) {                 // half of the blocks of a sum: four of every eight
+  for (int g = warp; g < 2 * own; g += warps) {              // half of the blocks of a sum: four of every eight
     float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
     for (int i8 = 0; i8 < per; ++i8) {
@@ -437,8 +435,9 @@ int gemm_xsums(int np, int n) { return (n / 128 + 8 * gemm_rht_per(np, n) - 1) /
 // columns, 48 rows, 10.1 / 9.5).  The rest is about the SMs that a GEMM in clusters leaves free, `idle`, taken from the GEMM that comes: in a
 // chain of layers the one before is most often like it, and behind another kernel the transform finds the GPU empty and the numbers matter
 // little.  An SM holds one thread block of 24 warps, two of 16 or four of 8 at 64 registers a thread.
-//  * A slice has work for two warps per 1024 columns: 8 warps up to 4096 columns (more rows than 64 take 16: 4096x4096 K4, 96 rows 14.8 / 13.9),
-//    16 up to 8192, 24 beyond (4096x12288 K5, 16 rows, 16 / 24: 18.2 / 18.0).  More than 128 rows fill the SMs with 16 (200 rows 36.7 / 34.2).
+//  * Two turns of the scan, whatever the slices: 8 warps up to 4096 columns (more rows than 64 take 16: 4096x4096 K4, 96 rows 14.8 / 13.9), 16 up
+//    to 8192, 24 beyond (512x13568 K3, 2 rows, 8 / 24: 8.4 / 7.8).  More than 128 rows fill the SMs with 16 (4096x12288 K5, 200 rows, 24 / 16:
+//    36.7 / 34.2).
 //  * Two slices where all fit (4096x12288 K5, 8 rows, 1 / 2: 18.6 / 17.2), four for long rows if they do (1024x16256 K4, 2 rows, 2 / 4: 11.2 / 10.4),
 //    and two where one would not fit either (4096x12288 37 rows 22.3 / 21.5; 4096x8192 K3, 48 rows 17.6 / 16.6); between the two one slice, all
 //    of them at once (4096x8192 K3, 24 rows 14.4 / 15.7).
@@ -456,8 +455,7 @@ struct RhtShape {
     warps = 8;
     if (!quad) return;
     const bool four = full ? rows <= (groups > 16 ? 16 : 4) : groups > 16 && 4 * rows < idle;
-    if (all_fit) warps = groups <= 16 || four ? 8 : groups <= 32 ? 16 : 24;   // (of half a row or a quarter)
-    else if (full && four && groups <= 16) warps = 8;
+    if (full && four && groups <= 16) warps = 8;
     else if (rows > 128) warps = 16;
     else if (full || groups > 16) warps = 24;
     else warps = groups <= 8 && rows <= 64 ? 8 : 16;
